@@ -11,6 +11,7 @@
 #include <atomic>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/pakman_gb300.h"
@@ -561,33 +562,92 @@ pk_status pk_count(pk_job* j, const char* fasta, uint64_t n, const pk_params* p)
   return count_host(j, fasta, n, p);
 }
 
+// Row check of a loaded table on the host, for a budget with no room to check it on the
+// device beside the job's current table.
+static pk_status check_rows_host(const uint64_t* kw, const uint32_t* counts, uint64_t n, int k,
+                                 unsigned long long* chk) {
+  const bool wide = k > 32;
+  unsigned __int128 y = 0;
+  for (uint64_t i = 0; i < n; i++) {
+    const unsigned __int128 x = wide ? ((unsigned __int128)kw[2 * i + 1] << 64) | kw[2 * i]
+                                     : (unsigned __int128)kw[i];
+    const bool big = k < 64 && (x >> (2 * k)) != 0;
+    if (big || (i && !(y < x)) || counts[i] == 0) {
+      chk[0] = 4 * i + (big ? 0 : (i && !(y < x)) ? 1 : 2);
+      return PK_OK;
+    }
+    chk[1] += counts[i];
+    y = x;
+  }
+  return PK_OK;
+}
+
+static pk_status load_rule(unsigned long long bad) {
+  if (bad == ~0ull) return PK_OK;
+  const std::string row = std::to_string(bad >> 2);
+  switch (bad & 3) {
+    case 0: return fail(PK_ERR_INVALID, "row " + row + " is not a k-mer");
+    case 1: return fail(PK_ERR_INVALID, "rows must be ascending and unique (row " + row + ")");
+    default: return fail(PK_ERR_INVALID, "row " + row + " has count 0");
+  }
+}
+
 // An existing (k-mer, count) table in place of counting: host rows ascending and
 // unique, k-mers below 4^k.  The rows are laid out as the counting stages leave them
-// (every bucket's rows contiguous), so cutoff and macro-nodes run unchanged.
+// (every bucket's rows contiguous), so cutoff and macro-nodes run unchanged.  The rows go
+// to new buffers and are checked there, so a refused table leaves the job's current one.
 pk_status pk_table_load(pk_job* j, const void* keys, const uint32_t* counts, uint64_t n, const pk_params* p) {
   if (!j) return fail(PK_ERR_INVALID, "job is null");
   PK_TRY(check_params(p));
   if (n && (!keys || !counts)) return fail(PK_ERR_INVALID, "keys and counts must not be null");
   if (n >= 0xffffffffull) return fail(PK_ERR_LIMIT, "tables of 2^32-1 rows or more are not supported");
-  j->bsmall_valid = false;  // the loaded table did not come from the table kernel
   const int k = p->k;
   const bool wide = k > 32;
-  const uint64_t* kw = (const uint64_t*)keys;
-  unsigned long long total = 0;
-  for (uint64_t i = 0; i < n; i++) {
-    const unsigned __int128 x = wide ? ((unsigned __int128)kw[2 * i + 1] << 64) | kw[2 * i]
-                                     : (unsigned __int128)kw[i];
-    if (k < 64 && (x >> (2 * k)) != 0) return fail(PK_ERR_INVALID, "row " + std::to_string(i) + " is not a k-mer");
-    if (i) {
-      const unsigned __int128 y = wide ? ((unsigned __int128)kw[2 * i - 1] << 64) | kw[2 * i - 2]
-                                       : (unsigned __int128)kw[i - 1];
-      if (!(y < x)) return fail(PK_ERR_INVALID, "rows must be ascending and unique (row " + std::to_string(i) + ")");
-    }
-    if (counts[i] == 0) return fail(PK_ERR_INVALID, "row " + std::to_string(i) + " has count 0");
-    total += counts[i];
-  }
+  const size_t W = wide ? 16 : 8;
+  // the count histogram is taken while the rows are checked, for the usual -t
+  const int t = p->num_buckets <= 4096 ? p->num_buckets : 0;
   PK_TRY(set_device(j->ctx));
+  unsigned long long chk[2] = {~0ull, 0};
+  DevBuf nk, nc, nh, nx;
+  pk_status s = job_alloc(j, nk, W * (n ? n : 1));
+  if (s == PK_OK) s = job_alloc(j, nc, 4 * (n ? n : 1));
+  if (s == PK_OK) s = job_alloc(j, nh, sizeof(unsigned long long) * (size_t)(t ? t : 1));
+  if (s == PK_OK) s = job_alloc(j, nx, sizeof(chk));
+  const bool on_device = s == PK_OK;
+  auto drop = [&]() {
+    job_free(j, nk);
+    job_free(j, nc);
+    job_free(j, nh);
+    job_free(j, nx);
+  };
+  if (on_device) {
+    auto check = [&]() -> pk_status {
+      PK_CUDA(cudaMemsetAsync(nx.p, 0xff, 8, j->stream));
+      PK_CUDA(cudaMemsetAsync((char*)nx.p + 8, 0, 8, j->stream));
+      if (t) PK_CUDA(cudaMemsetAsync(nh.p, 0, sizeof(unsigned long long) * (size_t)t, j->stream));
+      if (n) {
+        PK_CUDA(cudaMemcpyAsync(nk.p, keys, W * n, cudaMemcpyHostToDevice, j->stream));
+        PK_CUDA(cudaMemcpyAsync(nc.p, counts, 4 * n, cudaMemcpyHostToDevice, j->stream));
+      }
+      PK_CUDA(launch_table_check(nk.p, (const uint32_t*)nc.p, n, k, wide, (unsigned long long*)nx.p, t,
+                                 t ? (unsigned long long*)nh.p : nullptr, j->stream));
+      PK_CUDA(cudaMemcpyAsync(chk, nx.p, sizeof(chk), cudaMemcpyDeviceToHost, j->stream));
+      PK_CUDA(cudaStreamSynchronize(j->stream));
+      return load_rule(chk[0]);
+    };
+    s = check();
+    if (s != PK_OK) {
+      drop();
+      return s;
+    }
+  } else {
+    drop();
+    if (s != PK_ERR_NOMEM) return s;
+    PK_TRY(check_rows_host((const uint64_t*)keys, counts, n, k, chk));
+    PK_TRY(load_rule(chk[0]));
+  }
   for (int i = 0; i < ST_COUNT_; i++) j->ev_rec[i] = false;
+  j->bsmall_valid = false;  // the loaded table did not come from the table kernel
   j->params = *p;
   j->wide = wide;
   j->F = 0;
@@ -600,25 +660,32 @@ pk_status pk_table_load(pk_job* j, const void* keys, const uint32_t* counts, uin
   }
   j->bbits = std::max(2, std::min(bb, std::min(kMaxPartitionBits, 2 * k - 2)));
   const int B = 1 << j->bbits;
-  const size_t W = wide ? 16 : 8;
-  PK_TRY(job_alloc(j, j->tkeys, W * (n ? n : 1)));
-  PK_TRY(job_alloc(j, j->tcounts, 4 * (n ? n : 1)));
+  if (on_device) {
+    std::swap(j->tkeys, nk);
+    std::swap(j->tcounts, nc);
+    if (t) std::swap(j->hist, nh);
+    drop();
+    j->t_hist = t;  // 0: no histogram of this table yet
+  } else {
+    j->t_hist = 0;
+    PK_TRY(job_alloc(j, j->tkeys, W * (n ? n : 1)));
+    PK_TRY(job_alloc(j, j->tcounts, 4 * (n ? n : 1)));
+    if (n) {
+      PK_CUDA(cudaMemcpyAsync(j->tkeys.p, keys, W * n, cudaMemcpyHostToDevice, j->stream));
+      PK_CUDA(cudaMemcpyAsync(j->tcounts.p, counts, 4 * n, cudaMemcpyHostToDevice, j->stream));
+    }
+  }
   PK_TRY(job_alloc(j, j->bstart, sizeof(uint32_t) * (B + 1)));
   PK_TRY(job_alloc(j, j->tu, sizeof(uint32_t) * (size_t)B));
-  if (n) {
-    PK_CUDA(cudaMemcpyAsync(j->tkeys.p, keys, W * n, cudaMemcpyHostToDevice, j->stream));
-    PK_CUDA(cudaMemcpyAsync(j->tcounts.p, counts, 4 * n, cudaMemcpyHostToDevice, j->stream));
-  }
   PK_CUDA(launch_table_bounds(j->tkeys.p, n, j->bbits, k, (uint32_t*)j->bstart.p, (uint32_t*)j->tu.p,
                               wide, j->stream));
   Scalars init{};
   memset(&init, 0, sizeof(init));
   init.n_unique = n;
-  init.n_windows = total;
+  init.n_windows = chk[1];
   *j->h_sc = init;
   PK_CUDA(cudaMemcpyAsync(j->d_sc, j->h_sc, sizeof(Scalars), cudaMemcpyHostToDevice, j->stream));
   PK_CUDA(cudaStreamSynchronize(j->stream));
-  j->t_hist = 0;  // no histogram was fused into a counting pass
   j->dense_valid = false;
   j->stage = 1;
   return PK_OK;
@@ -716,9 +783,9 @@ pk_status pk::cutoff_enqueue(pk_job* j, int t) {
     PK_TRY(sync_scalars(j));
     PK_TRY(job_alloc(j, j->hist2, sizeof(unsigned long long) * (size_t)t));
     PK_CUDA(cudaMemsetAsync(j->hist2.p, 0, sizeof(unsigned long long) * (size_t)t, j->stream));
-    PK_TRY(dense_table(j));
-    PK_CUDA(launch_histogram((const uint32_t*)j->dcounts.p, j->h_sc->n_unique, t,
-                             (unsigned long long*)j->hist2.p, j->stream));
+    PK_CUDA(launch_histogram((const uint32_t*)j->tcounts.p, (const uint32_t*)j->bstart.p,
+                             (const uint32_t*)j->tu.p, 1 << j->bbits, t, (unsigned long long*)j->hist2.p,
+                             j->stream));
     hist = (const unsigned long long*)j->hist2.p;
   }
   mark_begin(j, ST_CUTOFF);

@@ -210,10 +210,16 @@ cudaError_t launch_scatter_fine(const void* in, const uint32_t* cstart, const ui
                                 uint32_t* fcur, void* out, int k, int bbits, int cbits, int wide,
                                 uint32_t* ticket, unsigned long long cap, uint32_t* err, cudaStream_t st);
 cudaError_t launch_bucket_table(const BucketArgs& a, int wide, int grid, cudaStream_t st);
+// checks the rows of a loaded table and histograms their counts below t (hist null: not
+// wanted); chk = {all ones, 0} beforehand, {4 * first bad row + rule, sum of counts} after
+// (rule 0: not a k-mer, 1: not above the row before, 2: count 0)
+cudaError_t launch_table_check(const void* keys, const uint32_t* counts, unsigned long long n, int k, int wide,
+                               unsigned long long* chk, int t, unsigned long long* hist, cudaStream_t st);
 // bstart / tu of a dense ascending table (pk_table_load)
 cudaError_t launch_table_bounds(const void* keys, unsigned long long n, int bbits, int k, uint32_t* bstart,
                                 uint32_t* tu, int wide, cudaStream_t st);
-cudaError_t launch_histogram(const uint32_t* tcounts, unsigned long long u, int t,
+// rows by count below t of the table in its buckets (hist zeroed beforehand)
+cudaError_t launch_histogram(const uint32_t* tcounts, const uint32_t* bstart, const uint32_t* tu, int B, int t,
                              unsigned long long* hist, cudaStream_t st);
 cudaError_t launch_cutoff(const unsigned long long* hist, int t, Scalars* sc, cudaStream_t st);
 cudaError_t launch_filter_kept(const FilterArgs& a, int wide, int grid, cudaStream_t st);
