@@ -731,17 +731,39 @@ __global__ void __launch_bounds__(128) k_cp_apply(Side<KeyT> a, Side<KeyT> b, ui
 //   k_wk_links   every suffix entry's successor: the node its neighbour key names
 //                (find_mnode_exists) and that node's first prefix equal to the first
 //                |S| bases of key + S, resolved for all entries in parallel
-//   k_walk<0>    one thread per begin k-mer (identify_begin_kmers,
+//   k_wk_steps   every wire as one 32-byte record: the suffix it leads through, the
+//                share bounds and where the successor's wires start
+//   k_walk<0>    one warp per begin k-mer (identify_begin_kmers,
 //                src/iterative_compaction.cpp:65-93) runs the depth-first walk over the
-//                links, the current frame in registers and the path's frames on a
-//                bounded stack in HBM; it counts contigs, bases and pieces
+//                records; it counts contigs, bases and pieces
 //   k_walk<1>    the same walk writes each contig's begin key and its pieces (the begin
-//                prefix and every frame's suffix, as arena views)
+//                prefix and every frame's suffix, as arena views), 32 pieces at a time
 //   k_wk_expand  one warp per piece writes its bases (one byte per base)
-struct WFrame {
-  uint32_t node, e0, np;
-  int32_t p, oip, wi, off, rem, share, bpx, bpy, wz, sid;
-  uint32_t lenb;  // contig length before this frame's current suffix
+// A walk is a chain of dependent loads, so a step makes one: its wire's record.  A frame
+// goes on the resume stack only when something of its share is left after the child (a
+// wire that takes the whole share ends its frame, since later wires start past it); the
+// path itself is a second stack that only a contig reads.  45.6k nodes, 463 begins: 1.63 ms
+// a walk; reading wire, entry, link and successor one after the other, and popping every
+// frame of the path after every contig, took 5.50 ms.
+struct WStep {
+  uint64_t xoff;   // the suffix's bases in the arena
+  uint32_t xlen;   // bases, bit 31 = terminal
+  int32_t off;     // the wire's offset in the suffix's visits
+  int32_t cnt;     // its visits
+  uint32_t next;   // first wire of the successor's prefix
+  int32_t n_next;  // its wires; kNoNode / kNoPrefix: no successor
+  uint32_t pad;
+};
+constexpr int32_t kNoNode = -1, kNoPrefix = -2;
+struct WResume {
+  uint32_t base;
+  int32_t n, wi, oip, off, rem;
+  uint32_t d, len;
+};
+struct WPath {
+  uint64_t src;    // the frame's suffix in the arena
+  uint32_t lenb;   // contig length before it
+  uint32_t len;
 };
 struct WPiece {
   uint64_t src;  // arena base offset
@@ -827,133 +849,164 @@ __global__ void __launch_bounds__(256) k_wk_links(Side<KeyT> s, uint32_t n, int 
   }
 }
 
+// The record of every wire slot (unused slots too: their zero wires name suffix 0).
+template <typename KeyT>
+__global__ void __launch_bounds__(256) k_wk_steps(Side<KeyT> s, uint32_t n, const uint2* __restrict__ link,
+                                                  WStep* __restrict__ step) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t e0 = s.eoff[i], e1 = s.eoff[i + 1], np = s.npre[i];
+  for (uint32_t w = e0 + i; w <= e1 + i; w++) {
+    const int3 x = s.wire[w];
+    const uint32_t se = e0 + np + (uint32_t)x.x;
+    WStep r;
+    r.xoff = s.xoff[se];
+    r.xlen = s.xlen[se];
+    r.off = x.y;
+    r.cnt = x.z;
+    r.next = 0;
+    r.n_next = kNoNode;
+    r.pad = 0;
+    if (!(r.xlen & kTerm)) {
+      const uint2 lk = link[se];
+      if (lk.x != ~0u) {
+        r.n_next = kNoPrefix;
+        if (lk.y != ~0u) {
+          const uint32_t f0 = s.eoff[lk.x];
+          const int2 b = s.beg[f0 + lk.y];
+          r.next = f0 + lk.x + (uint32_t)b.x;
+          r.n_next = b.y;
+        }
+      }
+    }
+    step[w] = r;
+  }
+}
+
+__device__ __forceinline__ WStep ld_step(const WStep* __restrict__ p) {
+  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  WStep r;
+  r.xoff = (uint64_t)a.y << 32 | a.x;
+  r.xlen = a.z;
+  r.off = (int32_t)a.w;
+  r.cnt = (int32_t)b.x;
+  r.next = b.y;
+  r.n_next = (int32_t)b.z;
+  r.pad = 0;
+  return r;
+}
+
 template <typename KeyT, int PASS>
 __global__ void __launch_bounds__(128) k_walk(Side<KeyT> s, int L, const uint2* __restrict__ begins, uint32_t nb,
-                                              const uint2* __restrict__ link, WFrame* __restrict__ stk, uint32_t cap,
-                                              uint4* __restrict__ col, const uint4* __restrict__ off,
-                                              uint64_t* __restrict__ ct_off, WPiece* __restrict__ pieces,
-                                              uint8_t* __restrict__ out, uint32_t* err) {
-  // one walk per warp (lane 0): independent walks diverge completely, so they do not
-  // share a warp
+                                              const WStep* __restrict__ step, WResume* __restrict__ resume,
+                                              WPath* __restrict__ path, uint32_t cap, uint4* __restrict__ col,
+                                              const uint4* __restrict__ off, uint64_t* __restrict__ ct_off,
+                                              WPiece* __restrict__ pieces, uint8_t* __restrict__ out,
+                                              uint32_t* err) {
+  // one walk per warp: independent walks diverge completely, so they do not share one.
+  // All lanes step together (same loads); lane 0 stores the frames.
   const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if ((threadIdx.x & 31) != 0 || b >= nb) return;
-  WFrame* st = stk + (uint64_t)b * cap;
+  const uint32_t lane = threadIdx.x & 31;
+  if (b >= nb) return;
+  WResume* rs = resume + (uint64_t)b * cap;
+  WPath* ps = path + (uint64_t)b * cap;
   const uint2 bg = begins[b];
-  const uint32_t be = s.eoff[bg.x] + bg.y;
+  const uint32_t e0 = s.eoff[bg.x], be = e0 + bg.y;
   const uint32_t plen0 = s.xlen[be] & kLenMask;
   uint32_t nct = 0, npc = 0;
   uint64_t nbases = 0;
   uint32_t ci = PASS ? off[b].x : 0u, pc = PASS ? off[b].z : 0u;
   uint64_t bo = PASS ? off[b].y : 0ull;
-  int d = 0;
-  WFrame f;
-  f.node = bg.x;
-  f.e0 = s.eoff[bg.x];
-  f.np = s.npre[bg.x];
-  f.p = (int32_t)bg.y;
-  f.oip = 0;
-  f.wi = 0;
-  f.off = 0;
-  f.rem = s.vis[be];
-  f.share = -1;
-  {
-    const int2 bp = s.beg[f.e0 + f.p];
-    f.bpx = bp.x;
-    f.bpy = bp.y;
-  }
-  f.wz = 0;
-  f.sid = -1;
-  f.lenb = 0;
-  uint32_t len = plen0 + (uint32_t)L;
+  uint32_t d = 0, rp = 0, len = plen0 + (uint32_t)L;
+  const int2 bp = s.beg[be];
+  uint32_t base = e0 + bg.x + (uint32_t)bp.x;
+  int32_t n = bp.y, wi = 0, oip = 0, fo = 0, rem = s.vis[be], fail = 0;
   while (true) {
-    if (f.wi >= f.bpy) {  // this walk is done: back to the parent
-      if (d == 0) break;
-      f = st[--d];
-      f.rem -= f.share;
-      f.share = -1;
-      len = f.lenb;
-      f.off += f.wz;
-      f.wi++;
+    if (wi >= n) {  // this frame is done: back to the nearest one with a share left
+      if (rp == 0) break;
+      rp--;
+      __syncwarp();
+      const uint4 x = reinterpret_cast<const uint4*>(rs + rp)[0], y = reinterpret_cast<const uint4*>(rs + rp)[1];
+      base = x.x;
+      n = (int32_t)x.y;
+      wi = (int32_t)x.z;
+      oip = (int32_t)x.w;
+      fo = (int32_t)y.x;
+      rem = (int32_t)y.y;
+      d = y.z;
+      len = y.w;
       continue;
     }
-    const int3 w = s.wire[f.e0 + f.node + f.bpx + f.wi];
-    if (f.off + w.z <= f.oip || f.off > f.oip + f.rem) {
-      f.off += w.z;
-      f.wi++;
+    const WStep w = ld_step(step + base + wi);
+    if (fo + w.cnt <= oip || fo > oip + rem) {
+      fo += w.cnt;
+      wi++;
       continue;
     }
-    const int oiw = f.oip <= f.off ? 0 : f.oip - f.off;
-    const int next_off = w.y + oiw;
-    const int share = min(f.rem, w.z - oiw);
-    const uint32_t se = f.e0 + f.np + (uint32_t)w.x;
-    const uint32_t xl = s.xlen[se], sl = xl & kLenMask;
-    if (xl & kTerm) {  // a contig: begin prefix, begin key, the frames' suffixes, this one
+    const int oiw = oip <= fo ? 0 : oip - fo;
+    const int next_off = w.off + oiw;
+    const int share = min(rem, w.cnt - oiw);
+    const uint32_t sl = w.xlen & kLenMask;
+    if (w.xlen & kTerm) {  // a contig: begin prefix, begin key, the frames' suffixes, this one
       const uint32_t clen = len + sl;
       if (PASS) {
-        ct_off[ci++] = bo;
-        for (int x = 0; x < L; x++)
-          out[bo + plen0 + x] = (uint8_t)key_bases(s.key[bg.x], L, x, 1);
-        if (plen0) pieces[pc++] = WPiece{s.xoff[be], bo, plen0, 0};
-        for (int q = 0; q < d; q++) {
-          const WFrame& g = st[q];
-          const uint32_t ge = g.e0 + g.np + (uint32_t)g.sid;
-          const uint32_t gl = s.xlen[ge] & kLenMask;
-          if (gl) pieces[pc++] = WPiece{s.xoff[ge], bo + g.lenb, gl, 0};
+        __syncwarp();  // lane 0's path stores before every lane reads them
+        if (lane == 0) ct_off[ci] = bo;
+        ci++;
+        for (uint32_t x = lane; x < (uint32_t)L; x += 32)
+          out[bo + plen0 + x] = (uint8_t)key_bases(s.key[bg.x], L, (int)x, 1);
+        if (plen0) {
+          if (lane == 0) pieces[pc] = WPiece{s.xoff[be], bo, plen0, 0};
+          pc++;
         }
-        if (sl) pieces[pc++] = WPiece{s.xoff[se], bo + len, sl, 0};
+        for (uint32_t q = lane; q < d; q += 32) {
+          const WPath g = ps[q];
+          pieces[pc + q] = WPiece{g.src, bo + g.lenb, g.len, 0};
+        }
+        pc += d;
+        if (sl) {
+          if (lane == 0) pieces[pc] = WPiece{w.xoff, bo + len, sl, 0};
+          pc++;
+        }
         bo += clen;
       } else {
-        npc += (plen0 ? 1u : 0u) + (sl ? 1u : 0u);
-        for (int q = 0; q < d; q++) npc++;
+        npc += (plen0 ? 1u : 0u) + (sl ? 1u : 0u) + d;
       }
       nct++;
       nbases += clen;
-      f.rem -= share;
-      f.off += w.z;
-      f.wi++;
+      rem -= share;
+      fo += w.cnt;
+      wi++;
       continue;
     }
-    const uint2 lk = link[se];
-    if (lk.x == ~0u) {
-      atomicOr(err, CE_TARGET);
+    if (w.n_next == kNoNode) fail = CE_TARGET;
+    else if (w.n_next == kNoPrefix) fail = CE_WALK_PREFIX;
+    else if (share <= 0) fail = CE_WALK_SHARE;
+    else if (len + sl >= kWalkMaxBases) fail = CE_WALK_LONG;
+    else if (d + 1 >= cap) fail = CE_WALK_DEPTH;
+    if (fail) {
+      if (lane == 0) atomicOr(err, (uint32_t)fail);
       break;
     }
-    if (lk.y == ~0u) {
-      atomicOr(err, CE_WALK_PREFIX);
-      break;
+    if (lane == 0) {
+      reinterpret_cast<uint4*>(ps)[d] = make_uint4((uint32_t)w.xoff, (uint32_t)(w.xoff >> 32), len, sl);
+      if (share < rem && wi + 1 < n) {
+        uint4* r = reinterpret_cast<uint4*>(rs + rp);
+        r[0] = make_uint4(base, (uint32_t)n, (uint32_t)(wi + 1), (uint32_t)oip);
+        r[1] = make_uint4((uint32_t)(fo + w.cnt), (uint32_t)(rem - share), d, len);
+      }
     }
-    if (share <= 0) {
-      atomicOr(err, CE_WALK_SHARE);
-      break;
-    }
-    if (len + sl >= kWalkMaxBases) {
-      atomicOr(err, CE_WALK_LONG);
-      break;
-    }
-    if (d + 1 >= (int)cap) {
-      atomicOr(err, CE_WALK_DEPTH);
-      break;
-    }
-    f.share = share;
-    f.sid = w.x;
-    f.wz = w.z;
-    f.lenb = len;
-    st[d++] = f;
+    if (share < rem && wi + 1 < n) rp++;
+    d++;
     len += sl;
-    f.node = lk.x;
-    f.e0 = s.eoff[lk.x];
-    f.np = s.npre[lk.x];
-    f.p = (int32_t)lk.y;
-    f.oip = next_off;
-    f.wi = 0;
-    f.off = 0;
-    f.rem = share;
-    f.share = -1;
-    const int2 bp = s.beg[f.e0 + f.p];
-    f.bpx = bp.x;
-    f.bpy = bp.y;
+    base = w.next;
+    n = w.n_next;
+    oip = next_off;
+    wi = 0;
+    fo = 0;
+    rem = share;
   }
-  if (!PASS) col[b] = make_uint4(nct, (uint32_t)nbases, npc, 0);
+  if (!PASS && lane == 0) col[b] = make_uint4(nct, (uint32_t)nbases, npc, 0);
 }
 
 // one warp per piece: its bases, one byte each
@@ -1022,7 +1075,8 @@ struct CpState {
   };
   DevBuf side[2][NSIDE];
   DevBuf arena, col, off, part, is_id, tkey, tr, tgt, incnt, inoff, fill, inlist, ecol, eoff2, old_of, ct, tot,
-      epos, cpos, ubuf, wk_begins, wk_stack, wk_col, wk_pos, wk_off, wk_out, wk_links, wk_pieces;
+      epos, cpos, ubuf, wk_begins, wk_resume, wk_path, wk_col, wk_pos, wk_off, wk_out, wk_links, wk_steps,
+      wk_pieces;
   uint64_t wk_begins_n = 0, wk_n = 0, wk_bases = 0;
   uint32_t wk_depth = 0;
   bool wk_done = false;
@@ -1256,20 +1310,25 @@ pk_status cp_walk(pk_job* j, CpState& c) {
   const uint64_t B = t.x;
   PK_TRY(cp_alloc(j, c.wk_begins, sizeof(uint2) * (B + 1)));
   PK_TRY(cp_alloc(j, c.wk_links, sizeof(uint2) * (c.E + 1)));
+  PK_TRY(cp_alloc(j, c.wk_steps, sizeof(WStep) * (c.E + n + 1)));
   if (n) {
     pk::note_launch(), k_wk_begins<<<blocks(n, 256), 256, 0, st>>>(a.eoff, a.npre, a.xlen, a.vis, (uint32_t)n, (const uint4*)c.off.p,
                                                 (uint2*)c.wk_begins.p);
     pk::note_launch(), k_wk_links<KeyT><<<blocks(n, 256), 256, 0, st>>>(a, (uint32_t)n, c.L, (const uint64_t*)c.arena.p,
                                                      (uint2*)c.wk_links.p);
+    pk::note_launch(), k_wk_steps<KeyT><<<blocks(n, 256), 256, 0, st>>>(a, (uint32_t)n, (const uint2*)c.wk_links.p,
+                                                                        (WStep*)c.wk_steps.p);
   }
   // frames per walk: 2^26 over all walks, at least 256 and at most 2^20 each
   const uint64_t cap = std::min<uint64_t>(1u << 20, std::max<uint64_t>(256, (1ull << 26) / std::max<uint64_t>(B, 1)));
-  PK_TRY(cp_alloc(j, c.wk_stack, sizeof(WFrame) * cap * std::max<uint64_t>(B, 1)));
+  PK_TRY(cp_alloc(j, c.wk_resume, sizeof(WResume) * cap * std::max<uint64_t>(B, 1)));
+  PK_TRY(cp_alloc(j, c.wk_path, sizeof(WPath) * cap * std::max<uint64_t>(B, 1)));
   PK_TRY(cp_alloc(j, c.wk_col, sizeof(uint4) * (B + 1)));
   PK_TRY(cp_alloc(j, c.wk_pos, sizeof(uint4) * (B + 1)));
   if (B)
     pk::note_launch(), k_walk<KeyT, 0><<<blocks(B * 32, 128), 128, 0, st>>>(a, c.L, (const uint2*)c.wk_begins.p, (uint32_t)B,
-                                                   (const uint2*)c.wk_links.p, (WFrame*)c.wk_stack.p, (uint32_t)cap,
+                                                   (const WStep*)c.wk_steps.p, (WResume*)c.wk_resume.p, (WPath*)c.wk_path.p,
+                                                   (uint32_t)cap,
                                                    (uint4*)c.wk_col.p, nullptr, nullptr, nullptr, nullptr, c.d_err);
   PK_TRY(scan4(j, c, (const uint4*)c.wk_col.p, (uint4*)c.wk_pos.p, B));
   PK_TRY(read_total(j, c, (const uint4*)c.wk_pos.p + B, &t));
@@ -1280,7 +1339,8 @@ pk_status cp_walk(pk_job* j, CpState& c) {
   PK_TRY(cp_alloc(j, c.wk_pieces, sizeof(WPiece) * (NP + 1)));
   if (B)
     pk::note_launch(), k_walk<KeyT, 1><<<blocks(B * 32, 128), 128, 0, st>>>(a, c.L, (const uint2*)c.wk_begins.p, (uint32_t)B,
-                                                   (const uint2*)c.wk_links.p, (WFrame*)c.wk_stack.p, (uint32_t)cap,
+                                                   (const WStep*)c.wk_steps.p, (WResume*)c.wk_resume.p, (WPath*)c.wk_path.p,
+                                                   (uint32_t)cap,
                                                    nullptr, (const uint4*)c.wk_pos.p, (uint64_t*)c.wk_off.p,
                                                    (WPiece*)c.wk_pieces.p, (uint8_t*)c.wk_out.p, c.d_err);
   if (NP)
@@ -1314,8 +1374,8 @@ void pk::cp_free(pk_job* j) {
   DevBuf* rest[] = {&c->arena,  &c->col,      &c->off,    &c->part,   &c->is_id,  &c->tkey,
                     &c->tr,     &c->tgt,      &c->incnt,  &c->inoff,  &c->fill,   &c->inlist,
                     &c->ecol,   &c->eoff2,    &c->old_of, &c->ct,     &c->tot,    &c->epos,
-                    &c->cpos,   &c->ubuf,     &c->wk_begins, &c->wk_stack, &c->wk_col, &c->wk_pos,
-                    &c->wk_off, &c->wk_out, &c->wk_links, &c->wk_pieces};
+                    &c->cpos,   &c->ubuf,     &c->wk_begins, &c->wk_resume, &c->wk_path, &c->wk_col,
+                    &c->wk_pos, &c->wk_off, &c->wk_out, &c->wk_links, &c->wk_steps, &c->wk_pieces};
   for (DevBuf* d : rest)
     if (d->p) {
       cudaFreeAsync(d->p, j->stream);
