@@ -29,7 +29,6 @@ enum : uint32_t {
 
 constexpr int kTileBytes = 65536;   // line-scan tile; chunk boundaries are multiples of it
 constexpr int kSegBytes = 64;       // bytes per thread per extraction step
-constexpr int kBucketThreads = 512;
 constexpr int kMnThreads = 128;
 constexpr int kSmallCounts = 16;    // per-bucket histogram of the table kernel: counts 0..15
 constexpr int kMnCap = 1536;        // items (k-mer records) per macro-node segment on chip
@@ -39,12 +38,14 @@ constexpr int kMnBinMax = 32;       // largest bin ranked within itself (else me
 constexpr int kHistSmem = 1024;     // count-histogram bins kept in shared memory
 constexpr int kBucketStack = 256;   // pending sub-ranges of one bucket
 constexpr int kSplitWays = 4;      // pieces an overflowing sub-range is cut into
+constexpr int kSplitSamples = 256; // distinct keys sampled for the cut
+constexpr int kTableHist = 512;    // count-histogram bins the table kernel keeps on chip
 constexpr int kMaxBucketAttempts = 1 << 16;  // sub-range attempts per bucket before giving up
 constexpr int kCoarseBits = 7;     // pass-1 partition digits (coarse regions)
 constexpr int kMaxPartBits = 18;   // partition digits (table buckets) at most
 constexpr int kHistBits = 15;      // digits the counting pass histograms in shared memory
 constexpr int kSortBinBits = 10;    // top remainder bits of the per-bucket counting sort
-constexpr int kBinMax = 128;        // largest bin sorted by ranking (else radix sort)
+constexpr int kBinMax = 128;        // largest bin sorted by ranking (else bitonic sort)
 // Giant buckets (skewed input: a homopolymer or tandem repeat and its error variants)
 // are first reduced chunk by chunk, by many CTAs, to (key, count) pairs.
 constexpr int kChunkKeys = 32768;                   // keys per chunk of a giant bucket

@@ -77,7 +77,18 @@ struct KeyOps<u128> {
     const uint64_t hi = (uint64_t)(x >> 64);
     return hi ? 127 - __clzll((long long)hi) : 63 - __clzll((long long)(uint64_t)x);
   }
-  __device__ __forceinline__ static u128 cas(u128* p, u128 cmp, u128 val) { return atomicCAS(p, cmp, val); }
+  // p in shared memory (named as such: the compiler need not infer it for a 128-bit atomic)
+  __device__ __forceinline__ static u128 cas(u128* p, u128 cmp, u128 val) {
+    uint64_t lo, hi;
+    asm volatile(
+        "{\n\t.reg .b128 c, v, o;\n\tmov.b128 c, {%3, %4};\n\tmov.b128 v, {%5, %6};\n\t"
+        "atom.shared.cas.b128 o, [%2], c, v;\n\tmov.b128 {%0, %1}, o;\n\t}"
+        : "=l"(lo), "=l"(hi)
+        : "r"((uint32_t)__cvta_generic_to_shared(p)), "l"((uint64_t)cmp), "l"((uint64_t)(cmp >> 64)),
+          "l"((uint64_t)val), "l"((uint64_t)(val >> 64))
+        : "memory");
+    return ((u128)hi << 64) | lo;
+  }
 };
 
 // A key loaded through L2 only (data another CTA of the same kernel wrote).
@@ -1099,24 +1110,39 @@ __global__ void __launch_bounds__(1024) k_bucket_prefix(uint32_t* bstart, int B)
 // ------------------------------------------------------------- per-bucket table ------
 template <typename KeyT>
 struct BucketCfg;
+// Threads, measured with two CTAs on an SM: 64-bit keys 768 (bacterial 1.62 ms; 512 and 1024
+// 1.76 ms), 1024 with giant buckets (whose sub-range passes are one CTA's serial chain:
+// 2.68 against 3.43 ms on the low-complexity reads); 128-bit keys 512, whose four keys in
+// flight need the registers (25 Mbp long-k, 2^18 buckets: 10.9 ms; 768 with two keys in
+// flight 13.7 ms).  Keys loaded ahead: four (64-bit keys with two 1.84, with eight 1.88 ms).
 template <>
 struct BucketCfg<uint64_t> {
-  static constexpr int H = 8192;
+  static constexpr int H = 8192;   // table slots
+  static constexpr int T = 768;    // threads
+  static constexpr int TG = 1024;  // threads when there are giant buckets
+  static constexpr int PF = 4;     // keys loaded per thread before inserting
 };
 template <>
 struct BucketCfg<u128> {
   static constexpr int H = 4096;
+  static constexpr int T = 512;
+  static constexpr int TG = 512;
+  static constexpr int PF = 4;
 };
 
+// Two CTAs fit an SM: for 64-bit keys 115 KB each (96 KB of slots, the sort's order and
+// bins, the histogram and the pending sub-ranges).
 template <typename KeyT>
 struct BucketSmem {
   static constexpr int H = BucketCfg<KeyT>::H;
-  static constexpr int NW = kBucketThreads / 32;
+  static constexpr int BINS = 1 << kSortBinBits;
   static constexpr size_t off_key = 0;
   static constexpr size_t off_cnt = off_key + sizeof(KeyT) * H;
-  static constexpr size_t off_wc = off_cnt + sizeof(uint32_t) * H;
-  static constexpr size_t off_hist = off_wc + sizeof(uint16_t) * NW * 256;
-  static constexpr size_t bytes = off_hist + sizeof(uint32_t) * kHistSmem;
+  static constexpr size_t off_ord = off_cnt + sizeof(uint32_t) * H;      // slot of every sorted element
+  static constexpr size_t off_bin = off_ord + sizeof(uint16_t) * (H / 2);  // sort bins; samples of a split
+  static constexpr size_t off_hist = off_bin + sizeof(uint32_t) * BINS;
+  static constexpr size_t bytes = off_hist + sizeof(uint32_t) * kTableHist;
+  static_assert(sizeof(KeyT) * kSplitSamples <= sizeof(uint32_t) * BINS, "samples share the bins");
 };
 
 // Insert (r, c) into the open-addressing table: 0 = r was present, 1 = r is new,
@@ -1144,6 +1170,12 @@ __device__ __forceinline__ int hash_insert(KeyT* skey, uint32_t* scnt, uint32_t 
   return 2;
 }
 
+// Sort bin of a remainder: the top bits below the sub-range's common prefix.
+template <typename KeyT>
+__device__ __forceinline__ uint32_t sort_bin(KeyT r, int dsh, uint32_t bmask) {
+  return (uint32_t)KeyOps<KeyT>::shr(r, dsh) & bmask;
+}
+
 // One table row, plus its count in the bucket's histogram of small counts (sbsmall, folded
 // into the count histogram when the bucket ends) or in the count histogram (counts below t).
 template <typename KeyT>
@@ -1158,19 +1190,9 @@ __device__ __forceinline__ void emit_row(const BucketArgs& a, KeyT* __restrict__
   if (cnt < (uint32_t)kSmallCounts) {
     atomicAdd(&sbsmall[cnt], 1u);
   } else if (cnt < (uint32_t)a.t) {
-    if (cnt < (uint32_t)kHistSmem) atomicAdd(&shist[cnt], 1u);
+    if (cnt < (uint32_t)kTableHist) atomicAdd(&shist[cnt], 1u);
     else atomicAdd(&a.hist[cnt], 1ull);
   }
-}
-
-// Rows [base+acc, base+acc+u) of a bucket from the sorted on-chip run (sk, sc).
-template <typename KeyT>
-__device__ void write_bucket_rows(const KeyT* sk, const uint32_t* sc, uint32_t u, const BucketArgs& a,
-                                  uint32_t beta, int rem, uint32_t base, uint32_t acc,
-                                  KeyT* __restrict__ tkeys, uint32_t* shist, uint32_t* sbsmall) {
-  const KeyT hi_bits = KeyOps<KeyT>::shl((KeyT)beta, rem);
-  for (uint32_t i = threadIdx.x; i < u; i += kBucketThreads)
-    emit_row<KeyT>(a, tkeys, (unsigned long long)base + acc + i, hi_bits | sk[i], sc[i], shist, sbsmall);
 }
 
 // Chunk items of the giant buckets (one thread per bucket): a bucket of at least
@@ -1194,37 +1216,49 @@ __global__ void __launch_bounds__(256) k_giant_chunks(const uint32_t* __restrict
   gfirst[b] = g0;
 }
 
+// A shared flag as the whole warp sees it: lanes that read it apart could otherwise leave a
+// loop whose warp-wide sum the others still wait in.
+__device__ __forceinline__ bool warp_flag(const uint32_t* f) {
+  return __any_sync(FULLMASK, *(const volatile uint32_t*)f != 0) != 0;
+}
+
+// Empties `slots` slots of the table and the sort bins.
+template <typename KeyT, int T>
+__device__ __forceinline__ void clear_table(KeyT* skey, uint32_t* scnt, uint32_t* bins, uint32_t slots) {
+  for (uint32_t i = threadIdx.x; i < slots; i += T) {
+    skey[i] = ~(KeyT)0;
+    scnt[i] = 0;
+  }
+  for (int i = threadIdx.x; i < (1 << kSortBinBits); i += T) bins[i] = 0;
+}
+
 // One chunk item: keys [cb, cb + kChunkKeys) of a giant bucket are aggregated on chip.
 // When their distinct keys fit half the table they are written back over the chunk's
 // own slots as (remainder, count) pairs -- remainders in slots [cb, cb + u), counts as
 // uint32 from slot cb + kChunkKeys / 2 on -- and chunk_u = u; otherwise the chunk keeps
 // its keys and chunk_u = kChunkRaw.  The bucket item reads the pairs in place of the
-// keys, so a heavy k-mer's copies are summed by many CTAs instead of one.
-template <typename KeyT>
-__device__ __forceinline__ void aggregate_chunk(const BucketArgs& a, KeyT* keys_rw, unsigned long long cb, uint32_t item,
-                                uint32_t beta, KeyT rmask, KeyT* skey, uint32_t* scnt, uint32_t* s_warp,
-                                uint32_t* s_flag, uint32_t* s_cnt) {
+// keys, so a heavy k-mer's copies are summed by many CTAs instead of one.  The table is
+// empty before and after.
+template <typename KeyT, int T>
+__device__ __forceinline__ void aggregate_chunk(const BucketArgs& a, KeyT* keys_rw, unsigned long long cb,
+                                                uint32_t item, uint32_t beta, KeyT rmask, KeyT* skey,
+                                                uint32_t* scnt, uint32_t* s_flag, uint32_t* s_cnt) {
   constexpr int H = BucketCfg<KeyT>::H;
-  constexpr int PF = 4;
+  constexpr int PF = BucketCfg<KeyT>::PF;
   const KeyT EMPTY = ~(KeyT)0;
   const int tid = threadIdx.x, lane = tid & 31;
-  for (uint32_t i = tid; i < (uint32_t)H; i += kBucketThreads) {
-    skey[i] = EMPTY;
-    scnt[i] = 0;
-  }
-  if (tid == 0) {
-    *s_flag = 0;
-    *s_cnt = 0;
-  }
-  __syncthreads();
-  for (uint32_t i0 = 0; i0 < (uint32_t)kChunkKeys; i0 += PF * kBucketThreads) {
-    if (*(volatile uint32_t*)s_flag) break;
+  for (uint32_t i0 = 0; i0 < (uint32_t)kChunkKeys; i0 += PF * T) {
+    if (warp_flag(s_flag)) break;
     KeyT rr[PF];
 #pragma unroll
-    for (int q = 0; q < PF; q++) rr[q] = keys_rw[cb + i0 + q * kBucketThreads + tid] & rmask;
+    for (int q = 0; q < PF; q++) {
+      const uint32_t i = i0 + q * T + tid;
+      rr[q] = i < (uint32_t)kChunkKeys ? keys_rw[cb + i] & rmask : EMPTY;
+    }
     uint32_t fresh = 0;
 #pragma unroll
     for (int q = 0; q < PF; q++) {
+      if (rr[q] == EMPTY) continue;
       const int res = hash_insert<KeyT>(skey, scnt, H - 1, rr[q], 1u);
       if (res == 2) *s_flag = 1;
       fresh += res == 1;
@@ -1234,40 +1268,46 @@ __device__ __forceinline__ void aggregate_chunk(const BucketArgs& a, KeyT* keys_
   }
   __syncthreads();
   const bool raw = *(volatile uint32_t*)s_flag != 0;
-  constexpr int SPT = H / kBucketThreads;
-  KeyT rk[SPT];
-  uint32_t rc[SPT];
-  uint32_t occ = 0;
-#pragma unroll
-  for (int q = 0; q < SPT; q++) {
-    rk[q] = skey[q * kBucketThreads + tid];
-    rc[q] = scnt[q * kBucketThreads + tid];
-    occ += rk[q] != EMPTY;
+  uint32_t u = kChunkRaw;
+  if (!raw) u = *(volatile uint32_t*)s_cnt;
+  __syncthreads();
+  if (tid == 0) {
+    *s_cnt = 0;  // now the write cursor
+    *s_flag = 0;
   }
-  uint32_t u;
-  uint32_t off = block_exclusive_sum(occ, s_warp, u);  // ends with a barrier: every key was read
-  if (!raw && u <= (uint32_t)(H / 2)) {
-    uint32_t* pc = reinterpret_cast<uint32_t*>(keys_rw + cb + kChunkKeys / 2);
-#pragma unroll
-    for (int q = 0; q < SPT; q++) {
-      if (rk[q] != EMPTY) {
-        keys_rw[cb + off] = rk[q];
-        pc[off] = rc[q];
-        off++;
+  __syncthreads();
+  uint32_t* pc = reinterpret_cast<uint32_t*>(keys_rw + cb + kChunkKeys / 2);
+  for (uint32_t i0 = 0; i0 < (uint32_t)H; i0 += T) {
+    const uint32_t i = i0 + tid;
+    const KeyT x = i < (uint32_t)H ? skey[i] : EMPTY;
+    const bool occ = x != EMPTY;
+    const unsigned m = __ballot_sync(FULLMASK, occ);
+    if (!m) continue;
+    uint32_t o = 0;
+    if (lane == 0) o = atomicAdd(s_cnt, (uint32_t)__popc(m));
+    o = __shfl_sync(FULLMASK, o, 0) + __popc(m & lanemask_lt());
+    if (occ) {
+      if (!raw) {
+        keys_rw[cb + o] = x;
+        pc[o] = scnt[i];
       }
+      skey[i] = EMPTY;
+      scnt[i] = 0;
     }
-  } else {
-    u = kChunkRaw;
   }
   if (tid == 0) a.chunk_u[item] = u;
   __threadfence();
   __syncthreads();
-  if (tid == 0) atomicAdd(&a.gdone[beta], 1u);
+  if (tid == 0) {
+    atomicAdd(&a.gdone[beta], 1u);
+    *s_cnt = 0;
+  }
 }
 
 // A giant bucket's item waits (bounded) until its chunk items are done and returns the
 // entries it will read: the chunks' pairs (or keys, where a chunk stayed raw) and the
 // keys after the last chunk.  On expiry it sets ERR_LOOKBACK and *s_fail.
+template <int T>
 __device__ __forceinline__ uint32_t giant_entries(const BucketArgs& a, uint32_t beta, uint32_t n, uint32_t g0,
                                                uint32_t nch, uint32_t* s_warp, uint32_t* s_fail) {
   const int tid = threadIdx.x;
@@ -1285,7 +1325,7 @@ __device__ __forceinline__ uint32_t giant_entries(const BucketArgs& a, uint32_t 
   }
   __syncthreads();
   uint32_t part = 0;
-  for (uint32_t j = tid; j < nch; j += kBucketThreads) {
+  for (uint32_t j = tid; j < nch; j += T) {
     const uint32_t cu = __ldcg(&a.chunk_u[g0 + j]);
     part += cu == kChunkRaw ? (uint32_t)kChunkKeys : cu;
   }
@@ -1297,14 +1337,15 @@ __device__ __forceinline__ uint32_t giant_entries(const BucketArgs& a, uint32_t 
 // One hash pass of a giant bucket's sub-range [lo, hi): chunk by chunk (pairs carry
 // their counts), then the tail keys.  Loads go through L2, as other CTAs wrote the
 // pairs during this kernel.
-template <typename KeyT>
+template <typename KeyT, int T>
 __device__ __forceinline__ void giant_pass(const BucketArgs& a, const KeyT* keys_rw, uint32_t base, uint32_t n,
-                                        uint32_t g0, uint32_t nch, bool whole, KeyT lo, KeyT hi, KeyT rmask,
-                                        KeyT* skey, uint32_t* scnt, uint32_t hmask, uint32_t ulimit,
-                                        uint32_t* s_ovf, uint32_t* s_unew) {
+                                           uint32_t g0, uint32_t nch, bool whole, KeyT lo, KeyT hi, KeyT rmask,
+                                           KeyT* skey, uint32_t* scnt, uint32_t hmask, uint32_t ulimit,
+                                           uint32_t* bins, int dsh, uint32_t bmask, uint32_t* s_ovf,
+                                           uint32_t* s_unew) {
   const int tid = threadIdx.x, lane = tid & 31;
   for (uint32_t j = 0; j <= nch; j++) {
-    if (*(volatile uint32_t*)s_ovf) break;
+    if (warp_flag(s_ovf)) break;
     const unsigned long long cb = (unsigned long long)base + (unsigned long long)j * kChunkKeys;
     uint32_t len = n - nch * (uint32_t)kChunkKeys;
     bool pairs = false;
@@ -1315,12 +1356,15 @@ __device__ __forceinline__ void giant_pass(const BucketArgs& a, const KeyT* keys
     }
     const uint32_t* pc = reinterpret_cast<const uint32_t*>(keys_rw + cb + kChunkKeys / 2);
     uint32_t fresh = 0;
-    for (uint32_t i = tid; i < len; i += kBucketThreads) {
+    for (uint32_t i = tid; i < len; i += T) {
       const KeyT r = ldcg_key(keys_rw + cb + i) & rmask;
       if (whole || (!(r < lo) && r < hi)) {
         const int res = hash_insert<KeyT>(skey, scnt, hmask, r, pairs ? __ldcg(pc + i) : 1u);
         if (res == 2) *s_ovf = 1;
-        fresh += res == 1;
+        if (res == 1) {
+          atomicAdd(&bins[sort_bin<KeyT>(r, dsh, bmask)], 1u);
+          fresh++;
+        }
       }
     }
     fresh = __reduce_add_sync(FULLMASK, fresh);
@@ -1328,34 +1372,75 @@ __device__ __forceinline__ void giant_pass(const BucketArgs& a, const KeyT* keys
   }
 }
 
-// Per bucket: aggregate the bucket's keys into (remainder, count) in an on-chip
-// hash table, radix-sort the distinct remainders and write them as table rows at
-// the bucket's own key range [bstart, bstart + u) ("sparse" table: no inter-bucket
-// dependency).  When the distinct keys of a bucket exceed the on-chip capacity the
-// bucket is counted in 2^slog sub-passes, each taking the keys whose next slog
-// remainder bits equal the sub-pass index (so sub-passes come out in key order).
-template <typename KeyT, bool GIANT>
-__global__ void __launch_bounds__(kBucketThreads, 2) k_bucket_table(BucketArgs a) {
+// Exclusive prefix of the sort bins in place (one barrier inside, one after); *s_crowd is
+// set when a bin holds more than kBinMax elements.
+__device__ __forceinline__ void scan_bins(uint32_t* bins, uint32_t* s_warp, uint32_t* s_crowd) {
+  constexpr int NT = (1 << kSortBinBits) / 4;  // threads that take four bins each
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint4 v = make_uint4(0, 0, 0, 0);
+  uint32_t x = 0, sum = 0;
+  if (tid < NT) {
+    v = reinterpret_cast<const uint4*>(bins)[tid];
+    sum = v.x + v.y + v.z + v.w;
+    if (max(max(v.x, v.y), max(v.z, v.w)) > (uint32_t)kBinMax) *s_crowd = 1;
+    x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULLMASK, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+  }
+  __syncthreads();
+  if (tid < NT) {
+    uint32_t ex = x - sum;
+    for (int w = 0; w < warp; w++) ex += s_warp[w];
+    reinterpret_cast<uint4*>(bins)[tid] = make_uint4(ex, ex + v.x, ex + v.x + v.y, ex + v.x + v.y + v.z);
+  }
+  __syncthreads();
+}
+
+// Per bucket: aggregate the bucket's keys into (remainder, count) in an on-chip hash
+// table, order the distinct remainders and write them as table rows at the bucket's own
+// key range [bstart, bstart + u) ("sparse" table: no inter-bucket dependency).
+// Sub-ranges of the bucket are counted one at a time, in key order.  A sub-range is an
+// interval [lo, hi) of remainders.  The first split guesses from the distinct/keys ratio
+// seen so far; a sub-range whose distinct keys overflow the on-chip table is cut at
+// quantiles of a sample of its distinct keys, so skewed buckets (a heavy k-mer and its
+// error variants) split evenly.
+//
+// The distinct keys never leave their slots: a counting sort by their top bits (its
+// histogram taken as keys are first inserted) orders slot numbers, and each element's
+// rank among its bin, a few keys, gives its row.  Nothing is carried in registers from
+// one phase to the next, so 1536 threads fit an SM, which is what hides the hash table's
+// shared-memory latency; a bucket takes seven barriers, and the slots it emptied are the
+// occupied ones, by the same order.  Bound: issue and shared-memory latency of the
+// insertions.  Bacterial reads (254M keys, 45M distinct): 1.97 -> 1.62 ms against sorting
+// slots held in registers, 512 threads and 17 barriers a bucket.
+template <typename KeyT, bool GIANT, int T>
+__global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
   using SM = BucketSmem<KeyT>;
   constexpr int H = SM::H;
-  constexpr int NW = SM::NW;
+  constexpr int BINS = SM::BINS;
   constexpr int HALF = H / 2;
-  constexpr int RMAX = (HALF + kBucketThreads - 1) / kBucketThreads;  // radix rounds per warp
+  constexpr int PF = BucketCfg<KeyT>::PF;
   extern __shared__ __align__(16) unsigned char smem[];
   KeyT* skey = reinterpret_cast<KeyT*>(smem + SM::off_key);
   uint32_t* scnt = reinterpret_cast<uint32_t*>(smem + SM::off_cnt);
-  uint16_t* wc = reinterpret_cast<uint16_t*>(smem + SM::off_wc);
+  uint16_t* ord = reinterpret_cast<uint16_t*>(smem + SM::off_ord);
+  uint32_t* bins = reinterpret_cast<uint32_t*>(smem + SM::off_bin);
   uint32_t* shist = reinterpret_cast<uint32_t*>(smem + SM::off_hist);
   __shared__ uint32_t s_warp[33];
-  __shared__ uint32_t s_beta, s_ovf, s_fail, s_nb[2], s_unew;
+  __shared__ uint32_t s_tk, s_nb[2], s_ovf, s_fail, s_unew, s_crowd;
   __shared__ int s_sp;
-  __shared__ KeyT s_stk_lo[kBucketStack];  // pending sub-ranges [lo, hi) of the bucket
-  __shared__ KeyT s_stk_hi[kBucketStack];
+  // starts of the pending sub-ranges, the next one last; each ends where the one before it
+  // in the list starts (the first at the end of the remainder range)
+  __shared__ KeyT s_lo[kBucketStack];
   __shared__ KeyT s_split[kSplitWays];
-  __shared__ float s_ratio;
+  __shared__ float s_ratio, s_size;  // expected distinct keys and table slots per key
   __shared__ uint32_t s_bsmall[kSmallCounts];  // the current bucket's rows by small count
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int B = 1 << a.bbits;
   const int rem = 2 * a.k - a.bbits;  // remainder bits below the bucket id
   const KeyT rmask = KeyOps<KeyT>::mask(rem);
@@ -1363,20 +1448,7 @@ __global__ void __launch_bounds__(kBucketThreads, 2) k_bucket_table(BucketArgs a
   const KeyT EMPTY = ~(KeyT)0;
   const KeyT* __restrict__ keys = reinterpret_cast<const KeyT*>(a.keys);
   KeyT* __restrict__ tkeys = reinterpret_cast<KeyT*>(a.tkeys);
-  const int hbins = a.t < kHistSmem ? a.t : kHistSmem;
-  for (int i = tid; i < hbins; i += kBucketThreads) shist[i] = 0;
-  if (tid < kSmallCounts) s_bsmall[tid] = 0;
-  // running distinct/keys ratio of this CTA's buckets; read sets at 20x-80x coverage
-  // with sub-percent errors start near 0.2 (a high guess splits the first buckets
-  // needlessly, a low one costs one overflowing pass)
-  if (tid == 0) s_ratio = 0.2f;
-  const int slog_max = rem < 4 ? rem : 4;  // initial split guess (<= 16 sub-ranges)
 
-  // Work tickets: the chunk items of giant buckets first (tickets [0, nci)), then the
-  // buckets.  A giant bucket waits (bounded) until its chunks are reduced; every chunk
-  // ticket was taken before any bucket ticket, by a CTA that waits on nothing, so the
-  // wait ends.  The next ticket and its bucket's extent are fetched while the current
-  // one is counted.
   // Two instantiations are launched back to back and exactly one of them works: GIANT
   // = false when the partition has no giant bucket (it carries none of their code, so
   // the common case keeps its registers), GIANT = true otherwise, taking the chunk
@@ -1388,142 +1460,143 @@ __global__ void __launch_bounds__(kBucketThreads, 2) k_bucket_table(BucketArgs a
   const uint32_t nt = nci + (uint32_t)B;
   uint32_t* ticket = &a.sc->ticket_bucket;
   KeyT* keys_rw = reinterpret_cast<KeyT*>(a.keys);
+
+  const int hbins = a.t < kTableHist ? a.t : kTableHist;
+  for (int i = tid; i < hbins; i += T) shist[i] = 0;
+  if (tid < kSmallCounts) s_bsmall[tid] = 0;
+  clear_table<KeyT, T>(skey, scnt, bins, H);
+
+  // Work tickets: the chunk items of giant buckets first (tickets [0, nci)), then the
+  // buckets.  A giant bucket waits (bounded) until its chunks are reduced; every chunk
+  // ticket was taken before any bucket ticket, by a CTA that waits on nothing, so the
+  // wait ends.  Thread 0 takes the next ticket when a bucket starts and its extent
+  // once the bucket's keys are in, so neither is waited for between buckets.
   uint32_t next_t = 0, next_base = 0, next_end = 0;
-  auto bucket_of = [&](uint32_t tk) { return tk - nci; };
-  if (tid == 0) {
+  bool have_extent = true;
+  auto take_ticket = [&]() {
     next_t = atomicAdd(ticket, 1u);
+    have_extent = false;
+  };
+  auto take_extent = [&]() {
+    if (have_extent) return;
+    have_extent = true;
     if ((!GIANT || next_t >= nci) && next_t < nt) {
-      const uint32_t b = bucket_of(next_t);
-      next_base = a.bstart[b];
-      next_end = a.bstart[b + 1];
+      next_base = a.bstart[next_t - nci];
+      next_end = a.bstart[next_t - nci + 1];
     }
+  };
+  // thread 0: the next item and its first sub-ranges
+  auto publish = [&]() {
+    take_extent();
+    s_tk = next_t;
+    s_nb[0] = next_base;
+    s_nb[1] = next_end;
+    s_fail = 0;
+    s_ovf = 0;
+    s_unew = 0;
+    s_crowd = 0;
+  };
+  const int slog_max = rem < 4 ? rem : 4;  // initial split guess (<= 16 sub-ranges)
+  auto push_first = [&](uint32_t n_eff) {
+    int slog = 0;
+    while (slog < slog_max && (float)(n_eff >> slog) * s_ratio * 1.2f > (float)HALF) slog++;
+    int sp = 0;
+    for (int j = (1 << slog) - 1; j >= 0; j--) s_lo[sp++] = KeyOps<KeyT>::shl((KeyT)(uint32_t)j, rem - slog);
+    s_sp = sp;
+  };
+  if (tid == 0) {
+    // running distinct/keys ratio of this CTA's buckets; read sets at 20x-80x coverage
+    // with sub-percent errors start near 0.2 (a high guess splits the first buckets
+    // needlessly).  The first bucket's table is sized as if every key were distinct.
+    s_ratio = 0.2f;
+    s_size = 2.5f;
+    take_ticket();
+    publish();
+    if (!GIANT && next_t < nt) push_first(next_end - next_base);
   }
+  __syncthreads();
   while (true) {
-    __syncthreads();
-    if (tid == 0) {
-      s_beta = next_t;
-      s_nb[0] = next_base;
-      s_nb[1] = next_end;
-      if (next_t < nt) {
-        next_t = atomicAdd(ticket, 1u);
-        if ((!GIANT || next_t >= nci) && next_t < nt) {
-          const uint32_t b = bucket_of(next_t);
-          next_base = a.bstart[b];
-          next_end = a.bstart[b + 1];
-        }
-      }
-    }
-    __syncthreads();
-    const uint32_t t = s_beta;
-    if (t >= nt) break;
-    if (GIANT && t < nci) {
+    const uint32_t tk = s_tk;
+    if (tk >= nt) break;
+    if (tid == 0) take_ticket();
+    if (GIANT && tk < nci) {
+      __syncthreads();
       if (tid == 0) {
-        const uint32_t gb = a.chunk_bucket[t];
+        const uint32_t gb = a.chunk_bucket[tk];
         s_nb[0] = gb;
-        s_nb[1] = a.bstart[gb] + (t - a.gfirst[gb]) * (uint32_t)kChunkKeys;
+        s_nb[1] = a.bstart[gb] + (tk - a.gfirst[gb]) * (uint32_t)kChunkKeys;
       }
       __syncthreads();
-      aggregate_chunk<KeyT>(a, keys_rw, s_nb[1], t, s_nb[0], rmask, skey, scnt, s_warp, &s_ovf, &s_unew);
+      aggregate_chunk<KeyT, T>(a, keys_rw, s_nb[1], tk, s_nb[0], rmask, skey, scnt, &s_ovf, &s_unew);
+      __syncthreads();
+      if (tid == 0) publish();
+      __syncthreads();
       continue;
     }
-    const uint32_t beta = bucket_of(t);
+    const uint32_t beta = tk - nci;
     const uint32_t base = s_nb[0];
     const uint32_t n = s_nb[1] - base;
-    if (tid == 0) s_fail = 0;
-    if (n == 0) {
-      if (tid == 0) a.tu[beta] = 0;
-      if (tid < kSmallCounts && a.bsmall) a.bsmall[(size_t)beta * kSmallCounts + tid] = 0;
-      continue;
-    }
     // a giant bucket reads its chunks' pairs (or keys, where a chunk stayed raw) and the
     // keys after its last chunk; n_eff = entries it reads
     const uint32_t g0 = GIANT ? a.gfirst[beta] : 0u;
     const uint32_t nch = GIANT ? a.gcount[beta] : 0u;
-    const uint32_t n_eff = nch ? giant_entries(a, beta, n, g0, nch, s_warp, &s_fail) : n;
-    // Sub-ranges of the bucket are counted one at a time, in key order.  A sub-range
-    // is an interval [lo, hi) of remainders.  The first split guesses from the
-    // distinct/keys ratio seen so far; a sub-range whose distinct keys overflow the
-    // on-chip table is cut at quantiles of a sample of its distinct keys, so skewed
-    // buckets (a heavy k-mer and its error variants) split evenly.
-    int slog = 0;
-    while (slog < slog_max && (float)(n_eff >> slog) * s_ratio * 1.2f > (float)HALF) slog++;
-    if (tid == 0 && s_fail) s_sp = 0;
-    if (tid == 0 && !s_fail) {
-      s_sp = 0;
-      const int psh0 = rem - slog;
-      for (int j = (1 << slog) - 1; j >= 0; j--) {
-        s_stk_lo[s_sp] = KeyOps<KeyT>::shl((KeyT)(uint32_t)j, psh0);
-        s_stk_hi[s_sp] = KeyOps<KeyT>::shl((KeyT)(uint32_t)(j + 1), psh0);
-        s_sp++;
-      }
+    uint32_t n_eff = n;
+    bool failed = false;
+    if (GIANT) {
+      __syncthreads();
+      if (nch) n_eff = giant_entries<T>(a, beta, n, g0, nch, s_warp, &s_fail);
+      failed = s_fail != 0;  // a giant bucket whose chunks did not finish in time
+      if (tid == 0) push_first(n_eff);
+      __syncthreads();
     }
+    if (!GIANT && n == 0) __syncthreads();  // every thread has read this item before the next is published
     uint32_t acc = 0;
     int attempts = 0;
-    __syncthreads();
-    bool failed = s_fail != 0;  // a giant bucket whose chunks did not finish in time
-    while (s_sp > 0) {
-      const KeyT lo = s_stk_lo[s_sp - 1];
-      const KeyT hi = s_stk_hi[s_sp - 1];
-      __syncthreads();
-      if (tid == 0) s_sp--;
+    while (n && !failed) {
+      const int sp = s_sp;
       if (++attempts > kMaxBucketAttempts) { failed = true; break; }
+      const KeyT lo = s_lo[sp - 1];
+      const KeyT hi = sp > 1 ? s_lo[sp - 2] : rtop;
       const bool whole = lo == (KeyT)0 && hi == rtop;
       // bits below the interval's common prefix (all its keys share the bits above)
       const KeyT span = lo ^ (hi - (KeyT)1);
       const int psh = span == (KeyT)0 ? 0 : KeyOps<KeyT>::top_bit(span) + 1;
+      const int dsh = psh < kSortBinBits ? 0 : psh - kSortBinBits;
+      const uint32_t bmask = psh < kSortBinBits ? (1u << psh) - 1u : (uint32_t)BINS - 1u;
       // table sized for the distinct keys expected (2.5x), at least 1024 slots; an
-      // overflow splits the sub-range
+      // overflow of a smaller table than H takes all H, one of H splits the sub-range
       uint32_t Heff = 1024;
       {
-        const float uest = (float)n_eff * s_ratio * 2.5f;
+        const float uest = (float)n_eff * s_size;
         while ((float)Heff < uest && Heff < (uint32_t)H) Heff <<= 1;
         if (!whole) Heff = H;
       }
       const uint32_t hmask = Heff - 1;
-      for (uint32_t i = tid; i < Heff; i += kBucketThreads) {
-        skey[i] = EMPTY;
-        scnt[i] = 0;
-      }
-      // sort bins (counts, then fill cursors) of the distinct remainders: the top
-      // bits below the sub-range's common prefix
-      const int dbits = psh < kSortBinBits ? psh : kSortBinBits;
-      const uint32_t nbins = 1u << dbits;
-      const int dsh = psh - dbits;
-      uint32_t* bh = reinterpret_cast<uint32_t*>(wc);  // [nbins] counts -> offsets
-      uint32_t* bf = bh + (1u << kSortBinBits);        // [nbins] fill
-      for (uint32_t i = tid; i < nbins; i += kBucketThreads) {
-        bh[i] = 0;
-        bf[i] = 0;
-      }
-      if (tid == 0) {
-        s_ovf = 0;
-        s_unew = 0;
-      }
-      __syncthreads();
       // --- hash aggregation of this sub-range; it stops as soon as the distinct keys
-      //     exceed half the table (the sort needs the other half)
-      constexpr int PF = 4;  // keys loaded per thread before inserting
+      //     exceed half the table
       const uint32_t ulimit = Heff / 2;
-      if (nch)
-        giant_pass<KeyT>(a, keys_rw, base, n, g0, nch, whole, lo, hi, rmask, skey, scnt, hmask, ulimit, &s_ovf,
-                         &s_unew);
-      for (uint32_t i0 = 0; i0 < n && !nch; i0 += PF * kBucketThreads) {
-        if (*(volatile uint32_t*)&s_ovf) break;
+      if (GIANT && nch)
+        giant_pass<KeyT, T>(a, keys_rw, base, n, g0, nch, whole, lo, hi, rmask, skey, scnt, hmask, ulimit, bins, dsh,
+                         bmask, &s_ovf, &s_unew);
+      for (uint32_t i0 = 0; i0 < n && !(GIANT && nch); i0 += PF * T) {
+        if (warp_flag(&s_ovf)) break;
         KeyT rr[PF];
 #pragma unroll
         for (int q = 0; q < PF; q++) {
-          const uint32_t i = i0 + q * kBucketThreads + tid;
+          const uint32_t i = i0 + q * T + tid;
           rr[q] = i < n ? (keys[base + i] & rmask) : EMPTY;
         }
         uint32_t fresh = 0;  // distinct keys this thread added in this round
 #pragma unroll
         for (int q = 0; q < PF; q++) {
           const KeyT r = rr[q];
-          const bool v = r != EMPTY && (whole || (!(r < lo) && r < hi));
-          if (v) {
+          if (r != EMPTY && (whole || (!(r < lo) && r < hi))) {
             const int res = hash_insert<KeyT>(skey, scnt, hmask, r, 1u);
             if (res == 2) s_ovf = 1;
-            fresh += res == 1;
+            if (res == 1) {
+              atomicAdd(&bins[sort_bin<KeyT>(r, dsh, bmask)], 1u);
+              fresh++;
+            }
           }
         }
         // the distinct-key count grows once per warp and round (one shared atomic per
@@ -1532,215 +1605,126 @@ __global__ void __launch_bounds__(kBucketThreads, 2) k_bucket_table(BucketArgs a
         if (lane == 0 && fresh && atomicAdd(&s_unew, fresh) + fresh > ulimit) s_ovf = 1;
       }
       __syncthreads();
-      bool ovf = s_ovf != 0;
-      // --- occupied slots into registers, counted, with their sort bins histogrammed;
-      // order is irrelevant here, so slots are read with a stride of one block:
-      // conflict-free shared-memory access
-      constexpr int SPT = H / kBucketThreads;
-      const uint32_t spt = Heff / kBucketThreads;
-      KeyT rk[SPT];
-      uint32_t rc[SPT];
-      uint32_t occ = 0;
-#pragma unroll
-      for (int q = 0; q < SPT; q++) {
-        rk[q] = EMPTY;
-        rc[q] = 0;
-        if ((uint32_t)q < spt) {
-          rk[q] = skey[q * kBucketThreads + tid];
-          rc[q] = scnt[q * kBucketThreads + tid];
-          if (rk[q] != EMPTY) {
-            occ++;
-            if (!ovf) atomicAdd(&bh[(uint32_t)KeyOps<KeyT>::shr(rk[q], dsh) & (nbins - 1)], 1u);
-          }
-        }
-      }
-      uint32_t u;
-      block_exclusive_sum(occ, s_warp, u);
-      if (u > Heff / 2) ovf = true;  // the sort needs a second half
-      if (ovf) {
-        // cut [lo, hi) at quantiles of a sample of the distinct keys in the table
-        // (one per thread: the first occupied slot of its stride)
-        KeyT* samp = reinterpret_cast<KeyT*>(wc);  // kBucketThreads keys
-        KeyT mine = EMPTY;
-#pragma unroll
-        for (int q = SPT - 1; q >= 0; q--)
-          if (rk[q] != EMPTY) mine = rk[q];
-        samp[tid] = mine;
-        const int m = __syncthreads_count(mine != EMPTY);
-        const int ways = m < kSplitWays ? m : kSplitWays;
-        if (ways < 2) {
-          if (tid == 0) s_fail = 1;
-        } else if (mine != EMPTY) {
-          int rank = 0;
-          for (int j = 0; j < kBucketThreads; j++) {
-            const KeyT o = samp[j];
-            rank += (o != EMPTY && o < mine);
-          }
-          // splitter w (1 <= w < ways) is the sample of rank floor(w * m / ways)
-          for (int w = 1; w < ways; w++)
-            if (rank == (w * m) / ways) s_split[w] = mine;
-        }
-        __syncthreads();
-        if (tid == 0 && !s_fail) {
-          if (s_sp + ways > kBucketStack) {
-            s_fail = 1;
-          } else {
-            // push the pieces highest first, so the lowest is counted next
-            KeyT top = hi;
-            for (int w = ways - 1; w >= 1; w--) {
-              s_stk_lo[s_sp] = s_split[w];
-              s_stk_hi[s_sp] = top;
-              top = s_split[w];
-              s_sp++;
+      if (s_ovf) {
+        if (Heff == (uint32_t)H) {
+          // cut [lo, hi) at quantiles of a sample of the distinct keys in the table
+          // (one per sampling thread: the first occupied slot of its stride)
+          KeyT* samp = reinterpret_cast<KeyT*>(bins);
+          KeyT mine = EMPTY;
+          if (tid < kSplitSamples)
+            for (int i = tid; i < H && mine == EMPTY; i += kSplitSamples) mine = skey[i];
+          __syncthreads();  // the bins' last use in this attempt was the insertion
+          if (tid < kSplitSamples) samp[tid] = mine;
+          const int m = __syncthreads_count(mine != EMPTY);
+          const int ways = m < kSplitWays ? m : kSplitWays;
+          if (mine != EMPTY) {
+            int rank = 0;
+            for (int j = 0; j < kSplitSamples; j++) {
+              const KeyT o = samp[j];
+              rank += (o != EMPTY && o < mine);
             }
-            s_stk_lo[s_sp] = lo;
-            s_stk_hi[s_sp] = top;
-            s_sp++;
+            // splitter w (1 <= w < ways) is the sample of rank floor(w * m / ways)
+            for (int w = 1; w < ways; w++)
+              if (rank == (w * m) / ways) s_split[w] = mine;
           }
+          __syncthreads();
+          if (tid == 0) {
+            if (ways < 2 || sp - 1 + ways > kBucketStack) {
+              s_fail = 1;
+            } else {
+              // the pieces take the sub-range's place, highest first, so the lowest is next
+              int o = sp - 1;
+              for (int w = ways - 1; w >= 1; w--) s_lo[o++] = s_split[w];
+              s_lo[o++] = lo;
+              s_sp = o;
+            }
+          }
+          __syncthreads();
+          failed = s_fail != 0;
+        } else if (tid == 0) {
+          s_size = (float)H;  // the same sub-range again, on all H slots
         }
         __syncthreads();
-        if (s_fail) { failed = true; break; }
+        clear_table<KeyT, T>(skey, scnt, bins, Heff);
+        if (tid == 0) {
+          s_ovf = 0;
+          s_unew = 0;
+        }
+        __syncthreads();
         continue;
       }
-      // --- sort the u distinct remainders: bins (top bits below the prefix) are offset
-      //     by a block scan and the slots go from registers straight into their bins;
-      //     each element's rank among its bin (a bin holds a few keys) then gives its
-      //     row, written at once.  A bin above kBinMax falls back to a stable LSD
-      //     radix sort of the binned run.
-      {
-        constexpr int BPT = (1 << kSortBinBits) / kBucketThreads;
-        uint32_t hv[BPT], hs = 0, hm = 0;
-#pragma unroll
-        for (int q = 0; q < BPT; q++) {
-          const uint32_t bi = tid * BPT + q;
-          hv[q] = bi < nbins ? bh[bi] : 0u;
-          hs += hv[q];
-          hm = max(hm, hv[q]);
+      const uint32_t u = s_unew;
+      if (tid == 0) take_extent();
+      // --- order the u distinct remainders: slot numbers go to their bins, in any order
+      scan_bins(bins, s_warp, &s_crowd);
+      for (uint32_t i = tid; i < Heff; i += T) {
+        const KeyT x = skey[i];
+        if (x != EMPTY) ord[atomicAdd(&bins[sort_bin<KeyT>(x, dsh, bmask)], 1u)] = (uint16_t)i;
+      }
+      __syncthreads();  // bins now hold their ends
+      const KeyT hi_bits = KeyOps<KeyT>::shl((KeyT)beta, rem);
+      if (!s_crowd) {
+        // element i of the binned order lands at row b0 + rank, within its bin's rows, so
+        // neighbouring threads store to neighbouring rows
+        for (uint32_t i = tid; i < u; i += T) {
+          const uint32_t slot = ord[i];
+          const KeyT x = skey[slot];
+          const uint32_t bi = sort_bin<KeyT>(x, dsh, bmask);
+          const uint32_t b0 = bi ? bins[bi - 1] : 0u, b1 = bins[bi];
+          uint32_t rank = 0;
+          for (uint32_t j = b0; j < b1; j++) rank += skey[ord[j]] < x;
+          emit_row<KeyT>(a, tkeys, (unsigned long long)base + acc + b0 + rank, hi_bits | x, scnt[slot], shist,
+                         s_bsmall);
         }
-        uint32_t tot;
-        uint32_t ex = block_exclusive_sum(hs, s_warp, tot);
-#pragma unroll
-        for (int q = 0; q < BPT; q++) {
-          const uint32_t bi = tid * BPT + q;
-          if (bi < nbins) bh[bi] = ex;
-          ex += hv[q];
-        }
-        const bool radix = __syncthreads_or(hm > (uint32_t)kBinMax) != 0;
-#pragma unroll
-        for (int q = 0; q < SPT; q++) {
-          if (rk[q] != EMPTY) {
-            const uint32_t bi = (uint32_t)KeyOps<KeyT>::shr(rk[q], dsh) & (nbins - 1);
-            const uint32_t pos = bh[bi] + atomicAdd(&bf[bi], 1u);
-            skey[pos] = rk[q];
-            scnt[pos] = rc[q];
-          }
-        }
+      } else {
+        // a bin above kBinMax: a bitonic sort of the slot numbers by key (0xffff: above all)
+        uint32_t P = 2;
+        while (P < u) P <<= 1;
+        for (uint32_t i = u + tid; i < P; i += T) ord[i] = 0xffffu;
         __syncthreads();
-        if (!radix) {
-          // element i of the binned run lands at row b0 + rank, within its bin's rows,
-          // so neighbouring threads store to neighbouring rows
-          const KeyT hi_bits = KeyOps<KeyT>::shl((KeyT)beta, rem);
-          for (uint32_t i = tid; i < u; i += kBucketThreads) {
-            const KeyT x = skey[i];
-            const uint32_t bi = (uint32_t)KeyOps<KeyT>::shr(x, dsh) & (nbins - 1);
-            const uint32_t b0 = bh[bi], b1 = b0 + bf[bi];
-            uint32_t rank = 0;
-            for (uint32_t j = b0; j < b1; j++) rank += skey[j] < x;
-            emit_row<KeyT>(a, tkeys, (unsigned long long)base + acc + b0 + rank, hi_bits | x, scnt[i], shist,
-                           s_bsmall);
+        for (uint32_t k2 = 2; k2 <= P; k2 <<= 1) {
+          for (uint32_t j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
+            for (uint32_t i = tid; i < P / 2; i += T) {
+              const uint32_t x = 2 * i - (i & (j2 - 1)), y = x | j2;
+              const uint32_t sx = ord[x], sy = ord[y];
+              const KeyT kx = sx == 0xffffu ? EMPTY : skey[sx], ky = sy == 0xffffu ? EMPTY : skey[sy];
+              if ((ky < kx) == ((x & k2) == 0) && kx != ky) {
+                ord[x] = (uint16_t)sy;
+                ord[y] = (uint16_t)sx;
+              }
+            }
+            __syncthreads();
           }
-        } else {
-          // stable LSD radix sort of the binned run in [0, u) through [H/2, H/2 + u)
-          KeyT* sk = skey;
-          uint32_t* sc = scnt;
-          KeyT* dk = skey + Heff / 2;
-          uint32_t* dc = scnt + Heff / 2;
-          const int npass = (psh + 7) / 8;
-          const uint32_t E = (u + NW - 1) / NW;
-          const uint32_t e0 = (uint32_t)warp * E;
-          const uint32_t e1 = min(e0 + E, u);
-          const uint32_t rounds = (E + 31) / 32;
-          for (int pass = 0; pass < npass; pass++) {
-            const int sh = 8 * pass;
-            __syncthreads();
-            for (int i = lane; i < 256; i += 32) wc[warp * 256 + i] = 0;
-            __syncwarp();
-            uint32_t dig[RMAX], offs[RMAX];
-#pragma unroll
-            for (int rr = 0; rr < RMAX; rr++) {
-              dig[rr] = 0;
-              offs[rr] = 0;
-              if ((uint32_t)rr >= rounds) continue;
-              const uint32_t idx = e0 + rr * 32 + lane;
-              const bool v = idx < e1;
-              const uint32_t d = v ? (uint32_t)(KeyOps<KeyT>::shr(sk[idx], sh) & 0xff) : 0u;
-              const unsigned vm = __ballot_sync(FULLMASK, v);
-              uint32_t bse = 0;
-              unsigned peers = 0;
-              if (v) {
-                peers = __match_any_sync(vm, d);
-                if (lane == __ffs(peers) - 1) {
-                  bse = wc[warp * 256 + d];
-                  wc[warp * 256 + d] = (uint16_t)(bse + __popc(peers));
-                }
-              }
-              __syncwarp();
-              const int leader = v ? __ffs(peers) - 1 : lane;
-              bse = __shfl_sync(FULLMASK, bse, leader);
-              dig[rr] = d;
-              offs[rr] = bse + __popc(peers & lanemask_lt());
-            }
-            __syncthreads();
-            {
-              constexpr int PER = (256 * NW) / kBucketThreads;
-              uint32_t vals[PER];
-              uint32_t sum = 0;
-#pragma unroll
-              for (int q = 0; q < PER; q++) {
-                const int e = tid * PER + q;  // e = d * NW + w
-                const int d = e / NW, w = e % NW;
-                vals[q] = wc[w * 256 + d];
-                sum += vals[q];
-              }
-              uint32_t tot2;
-              uint32_t ex2 = block_exclusive_sum(sum, s_warp, tot2);
-#pragma unroll
-              for (int q = 0; q < PER; q++) {
-                const int e = tid * PER + q;
-                const int d = e / NW, w = e % NW;
-                wc[w * 256 + d] = (uint16_t)ex2;
-                ex2 += vals[q];
-              }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int rr = 0; rr < RMAX; rr++) {
-              if ((uint32_t)rr >= rounds) continue;
-              const uint32_t idx = e0 + rr * 32 + lane;
-              if (idx < e1) {
-                const uint32_t pos = wc[warp * 256 + dig[rr]] + offs[rr];
-                dk[pos] = sk[idx];
-                dc[pos] = sc[idx];
-              }
-            }
-            __syncthreads();
-            KeyT* tk = sk; sk = dk; dk = tk;
-            uint32_t* tc = sc; sc = dc; dc = tc;
-          }
-          write_bucket_rows<KeyT>(sk, sc, u, a, beta, rem, base, acc, tkeys, shist, s_bsmall);
+        }
+        for (uint32_t i = tid; i < u; i += T) {
+          const uint32_t slot = ord[i];
+          emit_row<KeyT>(a, tkeys, (unsigned long long)base + acc + i, hi_bits | skey[slot], scnt[slot], shist,
+                         s_bsmall);
         }
       }
       acc += u;
+      __syncthreads();
+      // --- empty the table for the next sub-range or bucket
+      for (uint32_t i = tid; i < u; i += T) {
+        const uint32_t slot = ord[i];
+        skey[slot] = EMPTY;
+        scnt[slot] = 0;
+      }
+      for (int i = tid; i < BINS; i += T) bins[i] = 0;
+      if (sp == 1) break;
+      if (tid == 0) {
+        s_sp = sp - 1;
+        s_unew = 0;
+        s_crowd = 0;
+      }
       __syncthreads();
     }
     if (failed) {
       if (tid == 0) atomicOr(&a.sc->err, ERR_BUCKET);
       acc = 0;
     }
-    __syncthreads();
-    // the bucket's rows by small count: stored for the kept filter and folded into the
-    // count histogram (counts below t); zeroed for the next bucket, whose rows come after
-    // the barrier at the top of the loop
+    // the bucket's rows by small count (every row was emitted before the last barrier):
+    // stored for the kept filter and folded into the count histogram (counts below t)
     if (tid < kSmallCounts) {
       const uint32_t c = s_bsmall[tid];
       if (a.bsmall) a.bsmall[(size_t)beta * kSmallCounts + tid] = c;
@@ -1749,12 +1733,18 @@ __global__ void __launch_bounds__(kBucketThreads, 2) k_bucket_table(BucketArgs a
     }
     if (tid == 0) {
       a.tu[beta] = acc;
-      atomicAdd(&a.sc->n_unique, (unsigned long long)acc);
-      s_ratio = 0.5f * s_ratio + 0.5f * ((float)acc / (float)n_eff);
+      if (n) {
+        atomicAdd(&a.sc->n_unique, (unsigned long long)acc);
+        s_ratio = 0.5f * s_ratio + 0.5f * ((float)acc / (float)n_eff);
+        s_size = 2.5f * s_ratio;
+      }
+      publish();
+      if (!GIANT && next_t < nt) push_first(next_end - next_base);
     }
+    __syncthreads();
   }
   __syncthreads();
-  for (int i = tid; i < hbins; i += kBucketThreads)
+  for (int i = tid; i < hbins; i += T)
     if (shist[i]) atomicAdd(&a.hist[i], (unsigned long long)shist[i]);
 }
 
@@ -2519,20 +2509,22 @@ cudaError_t launch_bucket_offsets(const CountArgs& a, cudaStream_t st) {
 
 template <typename KeyT>
 static cudaError_t launch_bucket_t(const BucketArgs& a, int grid, cudaStream_t st) {
+  using BC = BucketCfg<KeyT>;
   const size_t smem = BucketSmem<KeyT>::bytes;
   static bool attr_set = false;  // a constant, so concurrent first calls agree
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_bucket_table<KeyT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_bucket_table<KeyT, false, BC::T>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_bucket_table<KeyT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = cudaFuncSetAttribute(k_bucket_table<KeyT, true, BC::TG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
   if (grid <= 0) grid = sm_count() * bucket_ctas_per_sm(sizeof(KeyT) == 16);
   // exactly one of the two works (giant buckets present or not); the other returns
-  pk::note_launch(), k_bucket_table<KeyT, false><<<grid, kBucketThreads, smem, st>>>(a);
-  pk::note_launch(), k_bucket_table<KeyT, true><<<grid, kBucketThreads, smem, st>>>(a);
+  pk::note_launch(), k_bucket_table<KeyT, false, BC::T><<<grid, BC::T, smem, st>>>(a);
+  pk::note_launch(), k_bucket_table<KeyT, true, BC::TG><<<grid, BC::TG, smem, st>>>(a);
   return cudaGetLastError();
 }
 
