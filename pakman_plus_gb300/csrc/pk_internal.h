@@ -89,7 +89,9 @@ struct CountArgs {
   // Packed units written by the counting pass and rolled again by the coarse scatter.
   // Unit u (0..3) of kSegBytes-byte segment g (its bytes 16u..16u+15) sits at
   // [u * nseg + g] of the code and bit-2 planes; windows[g] has bit 16u + j set iff the
-  // window whose newest byte is byte j of that unit was counted.
+  // window whose newest byte is byte j of that unit was counted.  The bit-2 plane holds the
+  // segment's sequence bytes; unit 3's word is always written, with bit 1 set when the
+  // segment has any such byte, the other three only then.
   uint32_t* unit_codes;      // 4 x nseg
   uint32_t* unit_nbits;      // 4 x nseg
   unsigned long long* unit_windows;  // nseg

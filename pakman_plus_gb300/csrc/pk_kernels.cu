@@ -316,40 +316,34 @@ __global__ void __launch_bounds__(1024) k_tile_prefix(const uint8_t* __restrict_
 }
 
 // --------------------------------------------------------- k-mer window extraction --
-// 16 input bytes -> 2-bit codes (byte 0 in the top bits), the bit-2 plane of the
-// codes, newline flags and N flags.
+// Four input bytes: their 2-bit codes (byte 0 in the top bits of the low byte), a mask of
+// the bytes equal to a character (bit 7 of each), and such a mask as four bits.
 __device__ __forceinline__ uint32_t pack4_codes(uint32_t w) {
-  return (((w >> 1) & 0x03030303u) * 0x40100401u) >> 24;
+  return ((w >> 1) & 0x03030303u) * 0x40100401u;  // in the top byte
 }
-__device__ __forceinline__ uint32_t pack4_nbits(uint32_t w) {
-  return (((w >> 3) & 0x01010101u) * 0x40100401u) >> 24;
+__device__ __forceinline__ uint32_t zero_bytes(uint32_t x) {
+  return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);
 }
-__device__ __forceinline__ uint32_t flags4(uint32_t eq) {
-  return ((eq & 0x01010101u) * 0x01020408u) >> 24;
+__device__ __forceinline__ uint32_t flags4(uint32_t m) {  // bits 7, 15, 23, 31 -> 0..3
+  return ((m >> 7) * 0x01020408u) >> 24;
 }
-
-struct UnitBits {
-  uint32_t codes;  // base j at bits 2(15-j)+1..2(15-j)
-  uint32_t nbits;  // code bit 2 of byte j at bit 2(15-j)
-  uint32_t nl;     // bit j: byte j is '\n'
-  uint32_t nn;     // bit j: byte j is 'N' or 'n'
-};
-
-__device__ __forceinline__ UnitBits decode_unit(const uint32_t w[4], bool want_n = true) {
-  UnitBits u;
-  u.codes = (pack4_codes(w[0]) << 24) | (pack4_codes(w[1]) << 16) | (pack4_codes(w[2]) << 8) |
-            pack4_codes(w[3]);
-  u.nbits = (pack4_nbits(w[0]) << 24) | (pack4_nbits(w[1]) << 16) | (pack4_nbits(w[2]) << 8) |
-            pack4_nbits(w[3]);
-  u.nl = flags4(__vcmpeq4(w[0], 0x0A0A0A0Au)) | (flags4(__vcmpeq4(w[1], 0x0A0A0A0Au)) << 4) |
-         (flags4(__vcmpeq4(w[2], 0x0A0A0A0Au)) << 8) | (flags4(__vcmpeq4(w[3], 0x0A0A0A0Au)) << 12);
-  u.nn = 0;
-  if (want_n)
-    u.nn = flags4(__vcmpeq4(w[0] | 0x20202020u, 0x6E6E6E6Eu)) |
-           (flags4(__vcmpeq4(w[1] | 0x20202020u, 0x6E6E6E6Eu)) << 4) |
-           (flags4(__vcmpeq4(w[2] | 0x20202020u, 0x6E6E6E6Eu)) << 8) |
-           (flags4(__vcmpeq4(w[3] | 0x20202020u, 0x6E6E6E6Eu)) << 12);
-  return u;
+// a 16-byte unit's four words of such masks as 16 bits
+__device__ __forceinline__ uint32_t flags16(uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+  return flags4(m0) | (flags4(m1) << 4) | (flags4(m2) << 8) | (flags4(m3) << 12);
+}
+// base j's code at bits 2(15-j)+1..2(15-j)
+__device__ __forceinline__ uint32_t unit_codes(const uint32_t w[4]) {
+  const uint32_t hi = __byte_perm(pack4_codes(w[1]), pack4_codes(w[0]), 0x7300);
+  const uint32_t lo = __byte_perm(pack4_codes(w[3]), pack4_codes(w[2]), 0x0073);
+  return (hi & 0xffff0000u) | (lo & 0xffffu);
+}
+// byte flags (bit j) of a unit as its bit-2 plane: byte j at bit 2(15-j)
+__device__ __forceinline__ uint32_t unit_plane(uint32_t flags) {
+  uint32_t x = __brev(flags) >> 16;
+  x = (x | (x << 8)) & 0x00ff00ffu;
+  x = (x | (x << 4)) & 0x0f0f0f0fu;
+  x = (x | (x << 2)) & 0x33333333u;
+  return (x | (x << 1)) & 0x55555555u;
 }
 
 __device__ __forceinline__ void load_unit(const uint8_t* __restrict__ buf, unsigned long long F,
@@ -370,68 +364,58 @@ __device__ __forceinline__ void load_unit(const uint8_t* __restrict__ buf, unsig
   }
 }
 
-// Rolling state: packed 2-bit codes (newest base in bits 0-1 of r0), the bit-2 plane
-// of the codes at each byte's own low-bit position (n*), and a history of "window
-// breakers" (newline, or N under the drop policy), newest at bit 0 of h0.
-struct Roll {
-  uint64_t r0, r1, r2;
-  uint64_t n0, n1, n2;
-  uint64_t h0, h1;
+// What a window of the next segment needs of this one: its units' codes with the bit-2
+// plane folded in (kmer_shift ORs a byte's code bit 2 into the base before it) and the
+// bytes no window may hold.
+struct SegTail {
+  uint32_t w[4];
+  unsigned long long brk;
 };
 
-__device__ __forceinline__ void roll_push(Roll& s, const UnitBits& u, bool drop_n) {
-  s.r2 = (s.r2 << 32) | (s.r1 >> 32);
-  s.r1 = (s.r1 << 32) | (s.r0 >> 32);
-  s.r0 = (s.r0 << 32) | (uint64_t)u.codes;
-  s.n2 = (s.n2 << 32) | (s.n1 >> 32);
-  s.n1 = (s.n1 << 32) | (s.n0 >> 32);
-  s.n0 = (s.n0 << 32) | (uint64_t)u.nbits;
-  uint32_t brk = u.nl | (drop_n ? u.nn : 0u);
-  uint32_t rev = __brev(brk) >> 16;  // byte j -> age 15-j
-  s.h1 = (s.h1 << 16) | (s.h0 >> 48);
-  s.h0 = (s.h0 << 16) | (uint64_t)rev;
+// Codes, line breaks, breakers and bit-2 flags of a 64-byte segment.
+__device__ __forceinline__ void decode_segment(const uint32_t w[4][4], bool drop_n, uint32_t codes[4],
+                                               unsigned long long& nl, unsigned long long& nn,
+                                               unsigned long long& b2) {
+  uint32_t l[4], n[4], t[4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    codes[u] = unit_codes(w[u]);
+    l[u] = flags16(zero_bytes(w[u][0] ^ 0x0A0A0A0Au), zero_bytes(w[u][1] ^ 0x0A0A0A0Au),
+                   zero_bytes(w[u][2] ^ 0x0A0A0A0Au), zero_bytes(w[u][3] ^ 0x0A0A0A0Au));
+    t[u] = flags16((w[u][0] << 4) & 0x80808080u, (w[u][1] << 4) & 0x80808080u, (w[u][2] << 4) & 0x80808080u,
+                   (w[u][3] << 4) & 0x80808080u);
+    n[u] = 0;
+    if (drop_n)
+      n[u] = flags16(zero_bytes((w[u][0] | 0x20202020u) ^ 0x6E6E6E6Eu),
+                     zero_bytes((w[u][1] | 0x20202020u) ^ 0x6E6E6E6Eu),
+                     zero_bytes((w[u][2] | 0x20202020u) ^ 0x6E6E6E6Eu),
+                     zero_bytes((w[u][3] | 0x20202020u) ^ 0x6E6E6E6Eu));
+  }
+  nl = (unsigned long long)(l[0] | (l[1] << 16)) | ((unsigned long long)(l[2] | (l[3] << 16)) << 32);
+  nn = (unsigned long long)(n[0] | (n[1] << 16)) | ((unsigned long long)(n[2] | (n[3] << 16)) << 32);
+  b2 = (unsigned long long)(t[0] | (t[1] << 16)) | ((unsigned long long)(t[2] | (t[3] << 16)) << 32);
 }
 
-// The same roll from a packed unit (the coarse scatter: the counting pass already
-// decided which windows count, so no breaker history is kept).
-__device__ __forceinline__ void roll_push_codes(Roll& s, uint32_t codes, uint32_t nbits) {
-  s.r2 = (s.r2 << 32) | (s.r1 >> 32);
-  s.r1 = (s.r1 << 32) | (s.r0 >> 32);
-  s.r0 = (s.r0 << 32) | (uint64_t)codes;
-  s.n2 = (s.n2 << 32) | (s.n1 >> 32);
-  s.n1 = (s.n1 << 32) | (s.n0 >> 32);
-  s.n0 = (s.n0 << 32) | (uint64_t)nbits;
+// Bits [shift, shift + 64) of the 192-bit string c2:c1:c0 (shift < 128).
+__device__ __forceinline__ unsigned long long bits64(uint64_t c0, uint64_t c1, uint64_t c2, int shift) {
+  const uint64_t a = shift < 64 ? c0 : c1, b = shift < 64 ? c1 : c2;
+  const int t = shift & 63;
+  return t ? (a >> t) | (b << (64 - t)) : a;
 }
 
-// The k-mer whose newest byte has age sh/2: kmer_shift ORs a byte's code bit 2 into
-// the previous base's low bit, so only bytes inside the window (age >= sh/2)
-// contribute their bit-2 plane, shifted up by one base.
+// The k-mer whose newest byte has age sh/2 (sh = 0, 2, .., 30), codes alone.
 template <typename KeyT>
-__device__ __forceinline__ KeyT window_key(const Roll& s, int sh, const KeyT kmask);
-
+__device__ __forceinline__ KeyT window_codes(uint64_t r0, uint64_t r1, uint64_t r2, int sh);
 template <>
-__device__ __forceinline__ uint64_t window_key<uint64_t>(const Roll& s, int sh, const uint64_t kmask) {
-  uint64_t x = sh ? ((s.r0 >> sh) | (s.r1 << (64 - sh))) : s.r0;
-  uint64_t n = sh ? ((s.n0 >> sh) | (s.n1 << (64 - sh))) : s.n0;
-  return (x | (n << 2)) & kmask;
+__device__ __forceinline__ uint64_t window_codes<uint64_t>(uint64_t r0, uint64_t r1, uint64_t, int sh) {
+  const uint32_t lo = __funnelshift_r((uint32_t)r0, (uint32_t)(r0 >> 32), sh);
+  const uint32_t hi = __funnelshift_r((uint32_t)(r0 >> 32), (uint32_t)r1, sh);
+  return (uint64_t)hi << 32 | lo;
 }
-
 template <>
-__device__ __forceinline__ u128 window_key<u128>(const Roll& s, int sh, const u128 kmask) {
-  uint64_t lo = sh ? ((s.r0 >> sh) | (s.r1 << (64 - sh))) : s.r0;
-  uint64_t hi = sh ? ((s.r1 >> sh) | (s.r2 << (64 - sh))) : s.r1;
-  uint64_t nlo = sh ? ((s.n0 >> sh) | (s.n1 << (64 - sh))) : s.n0;
-  uint64_t nhi = sh ? ((s.n1 >> sh) | (s.n2 << (64 - sh))) : s.n1;
-  const u128 x = ((u128)hi << 64) | lo;
-  const u128 n = ((u128)nhi << 64) | nlo;
-  return (x | (n << 2)) & kmask;
-}
-
-// window of ages [a, a+k) holds no breaker
-__device__ __forceinline__ bool window_clear(const Roll& s, int a, int k) {
-  uint64_t lo = a ? ((s.h0 >> a) | (s.h1 << (64 - a))) : s.h0;
-  uint64_t m = k >= 64 ? ~0ull : ((1ull << k) - 1ull);
-  return (lo & m) == 0;
+__device__ __forceinline__ u128 window_codes<u128>(uint64_t r0, uint64_t r1, uint64_t r2, int sh) {
+  const uint64_t lo = window_codes<uint64_t>(r0, r1, 0, sh), hi = window_codes<uint64_t>(r1, r2, 0, sh);
+  return ((u128)hi << 64) | lo;
 }
 
 // Reference record-start rule: a sequence line ending at `pos` (a newline) must be
@@ -450,16 +434,6 @@ __device__ void check_record_start(const uint8_t* __restrict__ buf, unsigned lon
   if (counts) atomicOr(err, ERR_FORMAT);
 }
 
-// Bucket of the window whose newest byte has age sh/2, for 64-bit keys whose bucket
-// digits lie in the high word of the key (shift = 2k - digits >= 34): only the high words
-// of the code and bit-2 planes are funnel-shifted.  The bit-2 plane's carry from the low
-// word lands in bits 0-1 of the high word, below the digits.
-__device__ __forceinline__ uint32_t window_bucket_hi(const Roll& s, int sh, int shift_hi, uint32_t hmask) {
-  const uint32_t xh = __funnelshift_r((uint32_t)(s.r0 >> 32), (uint32_t)s.r1, sh);
-  const uint32_t nh = __funnelshift_r((uint32_t)(s.n0 >> 32), (uint32_t)s.n1, sh);
-  return ((xh | (nh << 2)) >> shift_hi) & hmask;
-}
-
 template <typename KeyT>
 __device__ __forceinline__ void guarded_store(KeyT* __restrict__ out, uint32_t idx, KeyT v,
                                               unsigned long long cap, uint32_t* err) {
@@ -467,218 +441,250 @@ __device__ __forceinline__ void guarded_store(KeyT* __restrict__ out, uint32_t i
   else atomicOr(err, ERR_BOUNDS);
 }
 
-// Counting-pass threads: 1024 for 64-bit keys (more warps hide the decode's latency),
-// 512 for 128-bit keys (whose windows need twice the registers)
-template <typename KeyT>
-struct CountCfg {
-  static constexpr int T = sizeof(KeyT) == 8 ? 1024 : 512;
-};
-
-// Counting pass: per chunk, the bucket histogram of its windows (FASTB: the bucket is
-// taken from the high words alone, see window_bucket_hi).
-template <typename KeyT, bool FASTB>
-__global__ void __launch_bounds__(CountCfg<KeyT>::T, 1)
-k_extract(CountArgs a) {
-  constexpr int NT = CountCfg<KeyT>::T;
+// Counting pass: per chunk, the bucket histogram of its windows, and the packed units that
+// the coarse scatter rolls.  A thread takes a 64-byte segment; 1024 threads a CTA, one CTA
+// per SM (its histogram holds up to 2^15 bins).
+//
+// Bound: issue.  So whole segments are decided at once, in 64-bit masks: line parity is a
+// prefix XOR of the line breaks, the windows that hold a breaker are the breakers smeared
+// over k - 1 bytes (the run before the segment comes from its left neighbour by shuffle,
+// not by decoding 64 bytes again), and what is left is one bit per window.  A window's
+// bucket is a funnel shift of the segment's codes aligned to the bucket digits: the digits
+// start at key bit 2 or above, and a byte outside the window can only reach key bit 0.
+// Bit-2 planes are built only for segments whose sequence bytes have such a bit (N, '\r').
+// Bacterial reads (407 MB): 0.66 -> 0.37 ms against testing every window by itself; 25 Mbp
+// long-k (1.05 GB, k = 63): 2.93 -> 1.02 ms.  The histogram's shared-memory atomics are
+// about half of what is left.
+constexpr int kCountT = 1024;
+template <bool WIDE>
+__global__ void __launch_bounds__(kCountT, 1) k_extract(CountArgs a) {
+  constexpr int NW = kCountT / 32;
   extern __shared__ uint32_t s_bins[];
-  __shared__ uint32_t s_wpar[NT / 32];
-  __shared__ uint32_t s_red[NT / 32];
+  __shared__ uint32_t s_wpar[NW];
+  __shared__ SegTail s_tail[NW];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int NW = NT / 32;
   const int B = 1 << a.bbits;
   const int k = a.k;
-  const int shift = 2 * k - a.bbits;
-  const KeyT kmask = KeyOps<KeyT>::mask(2 * k);
+  const int shift = 2 * k - a.bbits;  // >= 2
+  const uint32_t hmask = (uint32_t)(B - 1) << 2;  // byte offset of a bin
   const bool drop_n = a.drop_n != 0;
   const uint8_t* __restrict__ buf = a.fasta;
   const unsigned long long F = a.F;
   const unsigned long long s0 = a.sc->s0;
   const int c = blockIdx.x;
 
-  for (int i = tid; i < B; i += NT) s_bins[i] = 0;
+  for (int i = tid; i < B; i += kCountT) s_bins[i] = 0;
   __syncthreads();
 
   const unsigned long long c0 = (unsigned long long)c * a.chunk;
   const unsigned long long c1 = min(c0 + a.chunk, F);
   uint32_t local = 0;
-  const int warm_units = (k - 1 + 15) / 16;
   if (c0 < c1 && s0 < F) {
     uint32_t carry = (a.tile_nl[c0 / kTileBytes] ^ a.sc->nl_before_s0) & 1u;
-    for (unsigned long long base = c0; base < c1; base += (unsigned long long)NT * kSegBytes) {
+    for (unsigned long long base = c0; base < c1; base += (unsigned long long)kCountT * kSegBytes) {
       const unsigned long long seg = base + (unsigned long long)tid * kSegBytes;
       const bool active = seg < c1;
-      uint32_t w[4][4];
-      uint32_t nlc = 0;
+      // the segment before warp 0's first: the last one of the previous step, or decoded
+      // from memory at the chunk's start
+      SegTail before;
+      before.w[0] = before.w[1] = before.w[2] = before.w[3] = 0;
+      before.brk = 0;
+      if (tid == 0) {
+        if (base > c0) {
+          before = s_tail[NW - 1];
+        } else if (seg >= kSegBytes) {
+          uint32_t w[4][4], codes[4];
+          unsigned long long nl, nn, b2;
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        unsigned long long p = seg + 16ull * u;
-        if (active && p < c1) {
-          load_unit(buf, F, p, w[u]);
+          for (int u = 0; u < 4; u++) load_unit(buf, F, seg - kSegBytes + 16ull * u, w[u]);
+          decode_segment(w, drop_n, codes, nl, nn, b2);
+          before.brk = nl | nn;
+          uint32_t up = 0;
 #pragma unroll
-          for (int i = 0; i < 4; i++) nlc += __popc(__vcmpeq4(w[u][i], 0x0A0A0A0Au)) >> 3;
-        } else {
-          w[u][0] = w[u][1] = w[u][2] = w[u][3] = 0;
-        }
-      }
-      // parity of the line count at the segment start (block XOR-scan)
-      const unsigned bal = __ballot_sync(FULLMASK, nlc & 1u);
-      if (lane == 0) s_wpar[warp] = __popc(bal) & 1u;
-      __syncthreads();
-      uint32_t wp = 0, tot = 0;
-#pragma unroll
-      for (int i = 0; i < NW; i++) {
-        uint32_t x = s_wpar[i];
-        tot ^= x;
-        if (i < warp) wp ^= x;
-      }
-      __syncthreads();
-      uint32_t pin = carry ^ wp ^ (__popc(bal & lanemask_lt()) & 1u);
-      carry ^= tot;
-      if (!active) continue;
-
-      Roll s;
-      s.r0 = s.r1 = s.r2 = 0;
-      s.n0 = s.n1 = s.n2 = 0;
-      s.h0 = s.h1 = 0;
-      for (int u = warm_units; u >= 1; u--) {
-        long long p = (long long)seg - 16ll * u;
-        if (p < 0) continue;
-        uint32_t ww[4];
-        load_unit(buf, F, (unsigned long long)p, ww);
-        roll_push(s, decode_unit(ww, drop_n), drop_n);
-      }
-      const unsigned long long g = seg / kSegBytes;
-      unsigned long long counted = 0;  // windows counted, bit 16u + j
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const unsigned long long p = seg + 16ull * u;
-        if (p >= c1) break;
-        const UnitBits ub = decode_unit(w[u], drop_n);
-        roll_push(s, ub, drop_n);
-        a.unit_codes[u * a.nseg + g] = ub.codes;
-        a.unit_nbits[u * a.nseg + g] = ub.nbits;
-        // line parity per byte: exclusive prefix XOR of the newline bits
-        uint32_t x = ub.nl;
-        x ^= x << 1; x ^= x << 2; x ^= x << 4; x ^= x << 8;
-        uint32_t ex = (x << 1) & 0xffffu;
-        uint32_t odd = (pin ? ~ex : ex) & 0xffffu;
-        pin ^= __popc(ub.nl) & 1u;
-        uint32_t in = 0xffffu;
-        if (p + 16 > F) in &= (1u << (uint32_t)(F - p)) - 1u;
-        if (p < s0) in &= s0 - p >= 16 ? 0u : ~((1u << (uint32_t)(s0 - p)) - 1u);
-        {
-          uint32_t ends = ub.nl & odd & in;  // newlines that end sequence lines
-          while (ends) {
-            int q = __ffs(ends) - 1;
-            ends &= ends - 1;
-            // the byte after the newline, read from memory (it is in L1): picking it out of
-            // w by a run-time index would keep w in local memory for the whole loop
-            const uint8_t next = p + q + 1 < F ? __ldg(buf + p + q + 1) : (uint8_t)'>';
-            check_record_start(buf, F, a.lmer_m, p + q, next, &a.sc->err);
+          for (int u = 3; u >= 0; u--) {
+            const uint32_t n = unit_plane((uint32_t)(b2 >> (16 * u)) & 0xffffu);
+            before.w[u] = codes[u] | (n << 2) | up;
+            up = n >> 30;
           }
         }
-        uint32_t v = odd & in & ~ub.nl;
-        if (!v) continue;
-        // all 16 windows of this unit span ages [0, k+15)
-        const bool all_clear =
-            k + 15 <= 64 ? window_clear(s, 0, k + 15)
-                         : (s.h0 == 0 && (s.h1 & ((1ull << (k + 15 - 64)) - 1ull)) == 0);
+      }
+      uint32_t w[4][4];
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-          if (!((v >> j) & 1u)) continue;
-          const int age = 15 - j;
-          if (!all_clear && !window_clear(s, age, k)) continue;
-          uint32_t beta;
-          if (FASTB) beta = window_bucket_hi(s, 2 * age, shift - 32, (uint32_t)(B - 1));
-          else beta = (uint32_t)(window_key<KeyT>(s, 2 * age, kmask) >> shift);
-          atomicAdd(&s_bins[beta], 1u);
-          local++;
-          counted |= 1ull << (16 * u + j);
+      for (int u = 0; u < 4; u++) {
+        if (active) load_unit(buf, F, seg + 16ull * u, w[u]);
+        else w[u][0] = w[u][1] = w[u][2] = w[u][3] = 0;
+      }
+      uint32_t codes[4];
+      unsigned long long nl, nn, b2;
+      decode_segment(w, drop_n, codes, nl, nn, b2);
+      // parity of the line count at the segment start (block XOR-scan)
+      const unsigned bal = __ballot_sync(FULLMASK, __popcll(nl) & 1);
+      if (lane == 0) s_wpar[warp] = __popc(bal) & 1u;
+      __syncthreads();
+      const unsigned wpar = __ballot_sync(FULLMASK, s_wpar[lane] != 0);
+      const uint32_t pin = (carry ^ __popc(wpar & ((1u << warp) - 1u)) ^ __popc(bal & lanemask_lt())) & 1u;
+      carry ^= __popc(wpar) & 1u;
+      // sequence bytes: odd lines, from the first '>' on, inside the buffer
+      unsigned long long x = nl;
+      x ^= x << 1; x ^= x << 2; x ^= x << 4; x ^= x << 8; x ^= x << 16; x ^= x << 32;
+      unsigned long long in = (x << 1) ^ (pin ? ~0ull : 0ull);
+      if (seg + kSegBytes > F) in &= active ? (1ull << (F - seg)) - 1ull : 0ull;
+      if (seg < s0) in &= s0 - seg >= kSegBytes ? 0ull : ~0ull << (s0 - seg);
+      // code bit 2 of sequence bytes, folded into the codes
+      const unsigned long long n2 = b2 & in & ~nl;
+      SegTail t;
+#pragma unroll
+      for (int u = 0; u < 4; u++) t.w[u] = codes[u];
+      t.brk = nl | nn;
+      const unsigned long long g = seg / kSegBytes;
+      uint32_t flag = 0, up = 0;
+      if (n2) {
+        flag = 2;
+#pragma unroll
+        for (int u = 3; u >= 0; u--) {
+          const uint32_t n = unit_plane((uint32_t)(n2 >> (16 * u)) & 0xffffu);
+          t.w[u] |= (n << 2) | up;
+          up = n >> 30;
+          if (active) a.unit_nbits[u * a.nseg + g] = u == 3 ? n | flag : n;
         }
       }
+      if (lane == 31) s_tail[warp] = t;
+      __syncthreads();
+      SegTail pv;
+#pragma unroll
+      for (int u = 0; u < 4; u++) pv.w[u] = WIDE || u >= 2 ? __shfl_up_sync(FULLMASK, t.w[u], 1) : 0u;
+      pv.brk = __shfl_up_sync(FULLMASK, t.brk, 1);
+      // the first unit's top bit reaches back into the neighbour's last base: below the digits
+      // of any window that ends in the neighbour, inside those that end here
+      if (lane == 0) pv = warp ? s_tail[warp - 1] : before;
+      if (!active) continue;
+      pv.w[3] |= up;
+      // windows without a breaker: none among the k - 1 bytes before the newest, or at it
+      unsigned long long bad = t.brk;
+      {
+        int cov = 1;
+        while (2 * cov <= k) {
+          bad |= bad << cov;
+          cov *= 2;
+        }
+        if (cov < k) bad |= bad << (k - cov);
+      }
+      const int run = pv.brk ? __clzll((long long)pv.brk) : kSegBytes;  // clean bytes before the segment
+      unsigned long long counted = ~bad & in;
+      if (run < k - 1) counted &= ~0ull << (k - 1 - run);
       a.unit_windows[g] = counted;
+      if (!n2) a.unit_nbits[3 * a.nseg + g] = 0;
+      {
+        unsigned long long ends = nl & in;  // newlines that end sequence lines
+        while (ends) {
+          const int q = __ffsll((long long)ends) - 1;
+          ends &= ends - 1;
+          // the byte after the newline, read from memory (it is in L1)
+          const unsigned long long p = seg + q;
+          const uint8_t next = p + 1 < F ? __ldg(buf + p + 1) : (uint8_t)'>';
+          check_record_start(buf, F, a.lmer_m, p, next, &a.sc->err);
+        }
+      }
+      local += __popcll(counted);
+      uint64_t r0 = (uint64_t)pv.w[2] << 32 | pv.w[3], r1 = (uint64_t)pv.w[0] << 32 | pv.w[1], r2 = 0;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        a.unit_codes[u * a.nseg + g] = codes[u];
+        if (WIDE) r2 = (r2 << 32) | (r1 >> 32);
+        r1 = (r1 << 32) | (r0 >> 32);
+        r0 = (r0 << 32) | t.w[u];
+        const uint32_t v = (uint32_t)(counted >> (16 * u)) & 0xffffu;
+        if (!v) continue;
+        // the unit's windows aligned so that age 0's bucket digits start at bit 2
+        const unsigned long long q = bits64(r0, r1, r2, shift - 2);
+        const uint32_t qlo = (uint32_t)q, qhi = (uint32_t)(q >> 32);
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+          if ((v >> j) & 1u) {
+            const uint32_t o = __funnelshift_r(qlo, qhi, 2 * (15 - j)) & hmask;
+            atomicAdd(reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(s_bins) + o), 1u);
+          }
+        }
+      }
     }
   }
   __syncthreads();
-  {
-    for (int i = tid; i < B; i += NT) a.counts[(size_t)c * B + i] = s_bins[i];
-    uint32_t x = local;
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(FULLMASK, x, o);
-    if (lane == 0) s_red[warp] = x;
-    __syncthreads();
-    if (tid == 0) {
-      unsigned long long tsum = 0;
-      for (int i = 0; i < NW; i++) tsum += s_red[i];
-      if (tsum) atomicAdd(&a.sc->n_windows, tsum);
-    }
+  for (int i = tid; i < B; i += kCountT) a.counts[(size_t)c * B + i] = s_bins[i];
+  local = __reduce_add_sync(FULLMASK, local);
+  if (lane == 0) s_wpar[warp] = local;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t n = __reduce_add_sync(FULLMASK, s_wpar[lane]);
+    if (lane == 0 && n) atomicAdd(&a.sc->n_windows, (unsigned long long)n);
   }
 }
 
 // ----------------------------------------------------- two-pass partition of keys ---
 // Pass 1 (k_scatter_coarse): roll the k-mers of a chunk again and append each key to a
-// shared-memory ring of its coarse bucket (leading kCoarseBits bits); full 128-byte
+// shared-memory ring of its coarse bucket (leading kCoarseBits bits); whole 128-byte
 // lines are flushed by warps to the chunk's segment of the coarse region, so global
-// stores are whole lines instead of scattered 8/16-byte writes.
+// stores are lines instead of scattered 8/16-byte writes.
 template <typename KeyT>
 struct CoarseCfg {
   static constexpr int C = 1 << kCoarseBits;               // coarse buckets
   static constexpr int R = sizeof(KeyT) == 8 ? 128 : 64;    // ring slots per bucket
   static constexpr int FU = 128 / (int)sizeof(KeyT);        // keys per 128-byte line
-  // threads: 1024 for 64-bit keys (the ring inserts and flushes are issue-bound and
-  // gain from the extra warps), 512 for 128-bit keys (whose rings hold half the slots)
-  static constexpr int T = sizeof(KeyT) == 8 ? 1024 : 512;
-  // window positions per batch (T * BP keys between flushes): an average ring takes
-  // about 80 of its 128 slots per batch for 64-bit keys and 35 of its 64 for 128-bit
-  // keys (a ring that overflows sends its extra keys straight to global memory); flushing
-  // every 8 positions instead cost 1.01 against 0.91 ms on the bacterial workload and
-  // 5.09 against 4.29 ms on half the long-k workload
-  static constexpr int BP = 16;
+  // Rings are flushed after every BP window positions of a thread, when an average ring
+  // has taken about 80 of its 128 slots (64-bit keys) or 40 of its 64 (128-bit keys); a
+  // ring that overflows sends its extra keys straight to global memory.  64-bit keys every
+  // 8 positions instead: 0.84 against 0.73 ms (bacterial); 128-bit keys with 512 threads and
+  // 16 positions: 3.27 against 2.70 ms (25 Mbp long-k).
+  static constexpr int T = 1024;
+  static constexpr int BP = sizeof(KeyT) == 8 ? 16 : 8;
   static constexpr size_t smem = sizeof(KeyT) * C * R;
 };
 
+// Writes the rings' keys out up to the last whole 128-byte line of the output (all of
+// them at the end) and moves what is left to the front, so that a ring's next key goes to
+// slot s_w[b] and s_g[b] is where slot 0 belongs.
 template <typename KeyT>
-__device__ __forceinline__ void coarse_flush(KeyT* ring, uint32_t* w, uint32_t* f, const uint32_t* g,
-                                             KeyT* __restrict__ out, bool final_flush,
-                                             unsigned long long cap, uint32_t* err) {
+__device__ __forceinline__ void coarse_flush(KeyT* ring, uint32_t* w, uint32_t* g, KeyT* __restrict__ out,
+                                             bool final_flush, unsigned long long cap, uint32_t* err) {
   using CF = CoarseCfg<KeyT>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NW = CF::T / 32;
   for (int b = warp; b < CF::C; b += NW) {
-    const uint32_t W = w[b];
-    uint32_t Fv = f[b];
+    const uint32_t W = w[b], gb = g[b];
     KeyT* rb = ring + b * CF::R;
-    const uint32_t gb = g[b];
-    if (W - Fv > (uint32_t)CF::R) {
-      // the ring overflowed this batch: keys past Fv+R went straight to global memory
-      for (uint32_t x = lane; x < (uint32_t)CF::R; x += 32)
-        guarded_store(out, gb + Fv + x, rb[(Fv + x) & (CF::R - 1)], cap, err);
-      Fv = W;
-    } else {
-      while (W - Fv >= 32) {
-        guarded_store(out, gb + Fv + lane, rb[(Fv + lane) & (CF::R - 1)], cap, err);
-        Fv += 32;
-      }
-      if (W - Fv >= (uint32_t)CF::FU) {
-        if (lane < CF::FU) guarded_store(out, gb + Fv + lane, rb[(Fv + lane) & (CF::R - 1)], cap, err);
-        Fv += CF::FU;
-      }
-      if (final_flush && W > Fv) {
-        if ((uint32_t)lane < W - Fv) guarded_store(out, gb + Fv + lane, rb[(Fv + lane) & (CF::R - 1)], cap, err);
-        Fv = W;
+    uint32_t n = W, left = 0;
+    if (W > (uint32_t)CF::R) {
+      n = CF::R;  // the ring overflowed: the keys past it went straight to global memory
+    } else if (!final_flush) {
+      left = min(W, (gb + W) & (uint32_t)(CF::FU - 1));
+      n = W - left;
+    }
+    for (uint32_t x = lane; x < n; x += 32) guarded_store(out, gb + x, rb[x], cap, err);
+    if (n) {
+      KeyT keep = 0;
+      if ((uint32_t)lane < left) keep = rb[n + lane];
+      __syncwarp();
+      if ((uint32_t)lane < left) rb[lane] = keep;
+      if (lane == 0) {
+        w[b] = left;
+        g[b] = gb + (W - left);
       }
     }
-    __syncwarp();
-    if (lane == 0) f[b] = Fv;
   }
 }
 
+// Bound: the shared-memory atomic and ring store of every key.  A window is two funnel
+// shifts of the codes (four for 128-bit keys), its coarse bucket one more of the codes
+// aligned to the bucket digits; rings start at slot 0 after every flush, which ends at a
+// whole line of the output, so an append needs no ring position.  Bacterial reads: 0.91 ->
+// 0.73 ms against rolling both planes for every window; 25 Mbp long-k: 4.21 -> 2.70 ms.
 template <typename KeyT>
 __global__ void __launch_bounds__(CoarseCfg<KeyT>::T, 1)
 k_scatter_coarse(CountArgs a, const uint32_t* __restrict__ coff, KeyT* __restrict__ out) {
   using CF = CoarseCfg<KeyT>;
+  constexpr bool WIDE = sizeof(KeyT) == 16;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   KeyT* ring = reinterpret_cast<KeyT*>(smem_raw);
-  __shared__ uint32_t s_w[CF::C], s_f[CF::C], s_g[CF::C];
+  __shared__ uint32_t s_w[CF::C], s_g[CF::C];
   const int tid = threadIdx.x;
   const int k = a.k;
   const int cshift = 2 * k - a.cbits;  // coarse bucket = leading cbits bits
@@ -689,14 +695,17 @@ k_scatter_coarse(CountArgs a, const uint32_t* __restrict__ coff, KeyT* __restric
   const int Cn = 1 << a.cbits;
   for (int i = tid; i < CF::C; i += CF::T) {
     s_w[i] = 0;
-    s_f[i] = 0;
     s_g[i] = i < Cn ? coff[(size_t)c * Cn + i] : 0;
   }
   __syncthreads();
   const unsigned long long c0 = (unsigned long long)c * a.chunk;
   const unsigned long long c1 = min(c0 + a.chunk, F);
-  const int warm_units = (k - 1 + 15) / 16;  // <= 4 (k <= 64): all in the previous segment
   const unsigned long long nseg = a.nseg;
+  auto append = [&](KeyT key, uint32_t b) {
+    const uint32_t pos = atomicAdd(&s_w[b], 1u);
+    if (pos < (uint32_t)CF::R) ring[b * CF::R + pos] = key;
+    else guarded_store(out, s_g[b] + pos, key, a.n_keys, &a.sc->err);
+  };
   if (c0 < c1 && s0 < F) {
     for (unsigned long long base = c0; base < c1; base += (unsigned long long)CF::T * kSegBytes) {
       const unsigned long long seg = base + (unsigned long long)tid * kSegBytes;
@@ -704,50 +713,72 @@ k_scatter_coarse(CountArgs a, const uint32_t* __restrict__ coff, KeyT* __restric
       const unsigned long long g = seg / kSegBytes;
       // the counting pass's packed units: codes, bit-2 plane and the windows it counted
       // (no FASTA decode, no line parity, no window checks here)
-      Roll s;
-      s.r0 = s.r1 = s.r2 = 0;
-      s.n0 = s.n1 = s.n2 = 0;
-      s.h0 = s.h1 = 0;
+      uint32_t cd[4] = {0, 0, 0, 0};
       unsigned long long counted = 0;
+      uint64_t r0 = 0, r1 = 0, r2 = 0;
+      uint32_t own = 0, left = 0;  // unit 3's bit-2 words of this segment and the one before
       if (active) {
         counted = __ldg(a.unit_windows + g);
-        if (g > 0)
-          for (int wu = warm_units; wu >= 1; wu--) {
-            const unsigned long long q = (unsigned long long)(4 - wu) * nseg + g - 1;
-            roll_push_codes(s, __ldg(a.unit_codes + q), __ldg(a.unit_nbits + q));
-          }
+        own = __ldg(a.unit_nbits + 3 * nseg + g);
+#pragma unroll
+        for (int u = 0; u < 4; u++) cd[u] = __ldg(a.unit_codes + u * nseg + g);
+        if (g > 0) {
+          r0 = (uint64_t)__ldg(a.unit_codes + 2 * nseg + g - 1) << 32 | __ldg(a.unit_codes + 3 * nseg + g - 1);
+          if (WIDE) r1 = (uint64_t)__ldg(a.unit_codes + g - 1) << 32 | __ldg(a.unit_codes + nseg + g - 1);
+          left = __ldg(a.unit_nbits + 3 * nseg + g - 1);
+        }
+      }
+      // bit-2 planes are folded into the codes, each byte's bit into the base before it;
+      // a window then takes the low bit of its newest base from the plain codes, as the
+      // byte after it is not its own
+      const bool fold = __any_sync(FULLMASK, own | left);
+      if (left) {
+        const uint64_t m0 = (uint64_t)__ldg(a.unit_nbits + 2 * nseg + g - 1) << 32 | (left & 0x55555555u);
+        r0 |= m0 << 2;
+        if (WIDE) {
+          const uint64_t m1 = (uint64_t)__ldg(a.unit_nbits + g - 1) << 32 | __ldg(a.unit_nbits + nseg + g - 1);
+          r1 |= (m1 << 2) | (m0 >> 62);
+        }
       }
 #pragma unroll
       for (int u = 0; u < 4; u++) {
-        const bool live = active && seg + 16ull * u < c1;
-        uint32_t v = 0;
-        if (live) {
-          const unsigned long long q = (unsigned long long)u * nseg + g;
-          roll_push_codes(s, __ldg(a.unit_codes + q), __ldg(a.unit_nbits + q));
-          v = (uint32_t)(counted >> (16 * u)) & 0xffffu;
-        }
+        const uint32_t v = (uint32_t)(counted >> (16 * u)) & 0xffffu;
+        if (WIDE) r2 = (r2 << 32) | (r1 >> 32);
+        r1 = (r1 << 32) | (r0 >> 32);
+        r0 = (r0 << 32) | cd[u];
+        if (own) r0 |= (uint64_t)(u == 3 ? own & 0x55555555u : __ldg(a.unit_nbits + u * nseg + g)) << 2;
+        const unsigned long long q = bits64(r0, r1, r2, cshift);
+        const uint32_t qlo = (uint32_t)q, qhi = (uint32_t)(q >> 32);
 #pragma unroll
-        for (int half = 0; half < 16 / CF::BP; half++) {
+        for (int part = 0; part < 16 / CF::BP; part++) {
+          if (!fold) {
 #pragma unroll
-          for (int jj = 0; jj < CF::BP; jj++) {
-            const int j = half * CF::BP + jj;
-            if (!((v >> j) & 1u)) continue;
-            const int age = 15 - j;
-            const KeyT key = window_key<KeyT>(s, 2 * age, kmask);
-            const uint32_t b = (uint32_t)(key >> cshift);
-            const uint32_t pos = atomicAdd(&s_w[b], 1u);
-            if (pos - s_f[b] < (uint32_t)CF::R) ring[b * CF::R + (pos & (CF::R - 1))] = key;
-            else guarded_store(out, s_g[b] + pos, key, a.n_keys, &a.sc->err);
+            for (int jj = 0; jj < CF::BP; jj++) {
+              const int j = part * CF::BP + jj, sh = 2 * (15 - j);
+              if ((v >> j) & 1u)
+                append(window_codes<KeyT>(r0, r1, r2, sh) & kmask,
+                       __funnelshift_r(qlo, qhi, sh) & (uint32_t)(Cn - 1));
+            }
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < CF::BP; jj++) {
+              const int j = part * CF::BP + jj, sh = 2 * (15 - j);
+              if ((v >> j) & 1u) {
+                const KeyT key = window_codes<KeyT>(r0, r1, r2, sh) & kmask;
+                append((key & ~(KeyT)1) | (KeyT)((cd[u] >> sh) & 1u),
+                       __funnelshift_r(qlo, qhi, sh) & (uint32_t)(Cn - 1));
+              }
+            }
           }
           __syncthreads();
-          coarse_flush<KeyT>(ring, s_w, s_f, s_g, out, false, a.n_keys, &a.sc->err);
+          coarse_flush<KeyT>(ring, s_w, s_g, out, false, a.n_keys, &a.sc->err);
           __syncthreads();
         }
       }
     }
   }
   __syncthreads();
-  coarse_flush<KeyT>(ring, s_w, s_f, s_g, out, true, a.n_keys, &a.sc->err);
+  coarse_flush<KeyT>(ring, s_w, s_g, out, true, a.n_keys, &a.sc->err);
 }
 
 // Coarse offsets: coff[c][g] = start of chunk c's segment in coarse region g (the
@@ -2391,28 +2422,24 @@ cudaError_t launch_line_scan(const CountArgs& a, cudaStream_t st) {
   return launch_tile_prefix(a, st);
 }
 
-template <typename KeyT, bool FASTB>
+template <bool WIDE>
 static cudaError_t launch_extract_t(const CountArgs& a, cudaStream_t st) {
   const size_t smem = sizeof(uint32_t) << a.bbits;
   // the attribute is shared by every thread launching this kernel, so it is always
   // set to the largest histogram (15 partition digits), never to this launch's size
   static bool attr_set = false;  // same value from every thread, so a race is benign
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_extract<KeyT, FASTB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_extract<WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(sizeof(uint32_t) << kHistBits));
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  pk::note_launch(), k_extract<KeyT, FASTB><<<a.grid, CountCfg<KeyT>::T, smem, st>>>(a);
+  pk::note_launch(), k_extract<WIDE><<<a.grid, kCountT, smem, st>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_bucket_count(const CountArgs& a, int wide, cudaStream_t st) {
-  if (wide) return launch_extract_t<u128, false>(a, st);
-  // bucket digits in the key's high word: the 32-bit bucket path
-  if (2 * a.k - a.bbits >= 34) return launch_extract_t<uint64_t, true>(a, st);
-  return launch_extract_t<uint64_t, false>(a, st);
+  return wide ? launch_extract_t<true>(a, st) : launch_extract_t<false>(a, st);
 }
 
 template <typename KeyT>
