@@ -330,19 +330,43 @@ pk_status pk::check_params(const pk_params* p) {
   return PK_OK;
 }
 
-// Partition digits: the leading key bits that pick a bucket, sized so an average
-// bucket holds a few thousand keys (the per-bucket kernel counts a bucket on chip).
-// The keys reach their buckets in two passes (kCoarseBits coarse regions, then fine
-// buckets inside each region), so the digit count is not tied to L2 capacity.
-int pk::auto_bucket_bits(uint64_t F, int k, int wide) {
-  // keys per bucket aimed at: large enough to amortise the per-bucket work of the
-  // table and macro-node kernels, small enough that a bucket's distinct keys usually
-  // fit one on-chip hash table (8192 64-bit or 4096 128-bit slots at load <= 1/2)
-  const double per_bucket = wide ? 3000.0 : 16000.0;
-  const double est = 0.62 * (double)F;               // k-mer windows per byte, 100 bp reads, k=32
+// Partition digits: the leading key bits that pick a bucket.  The keys reach their buckets
+// in two passes (kCoarseBits coarse regions, then fine buckets inside each region), so the
+// digit count is not tied to L2 capacity.
+//
+// Keys per bucket aimed at, by how many buckets that makes.  Many: large enough to amortise
+// the per-bucket work of the table and macro-node kernels, small enough that a bucket's
+// distinct keys fit half an on-chip hash table (8192 64-bit or 4096 128-bit slots).  Fewer
+// than about a thousand: smaller, so that every SM has buckets; a handful: a few hundred.
+// Stage sums measured at the neighbours of each choice (us; digits): 20.7k windows 4: 132,
+// 6: 130, 8: 151 (two digits, one bucket per 5200 keys: 266 before); 1.7M 8: 203, 9: 195, 10:
+// 204; 3.5M 9: 249, 10: 241, 11: 247; 13.8M 10: 504, 11: 464, 12: 488; 83M 12: 2036, 13: 1683,
+// 14: 1874; 254M 13: 6450, 14: 5310, 15: 5870; 128-bit keys, 1.9M 9: 273, 10: 264, 12: 295;
+// 15M 11: 1285, 12: 895, 13: 959; 70M 13: 3744, 14: 2937, 15: 3356; 568M 17: 28900, 18: 32400.
+static int partition_bits(double n, int k, int wide) {
   int b = 2;
-  while (b < kMaxPartitionBits && est / (double)(1u << b) > per_bucket) b++;
+  while (b < kMaxPartitionBits) {
+    const double most = b < 6 ? 350.0 : wide ? (b < 10 ? 2000.0 : 4500.0)
+                                             : (b < 10 ? 3500.0 : b < 12 ? 9000.0 : b < 14 ? 10500.0 : 16000.0);
+    if (n / (double)(1u << b) <= most) break;
+    b++;
+  }
   return std::max(2, std::min(b, 2 * k - 2));
+}
+
+// The digits for an input whose windows are not counted yet: windows per byte of 100 bp
+// reads at k = 32 and of 100-150 bp reads at k = 63.
+int pk::auto_bucket_bits(uint64_t F, int k, int wide) {
+  return partition_bits((wide ? 0.45 : 0.62) * (double)F, k, wide);
+}
+
+// The digits the counting pass histograms when the partition's own follow from its window
+// count: enough for long reads (0.85 windows per byte) where a digit more is cheap, as many
+// as the histogram holds at most.
+static int hist_bits(uint64_t F, int k, int wide) {
+  int b = partition_bits(0.62 * (double)F, k, wide);
+  if (b < 14) b = std::max(b, std::min(14, partition_bits(0.85 * (double)F, k, wide)));
+  return std::min(b, kHistBits);
 }
 
 static pk_status table_impl(pk_job* j, uint64_t N, int t);
@@ -357,13 +381,15 @@ pk_status pk::count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_pa
   j->wired = false;
   j->compacted = false;
   const int W = j->wide ? 16 : 8;
+  // automatic digits follow from the window count, which the counting pass takes with hb
+  // digits first (graph mode knows no counts)
+  const bool by_count = !p->bucket_bits && !j->graph_mode;
   const int bb = p->bucket_bits ? std::min(p->bucket_bits, std::min(kMaxPartitionBits, 2 * k - 2))
                                 : auto_bucket_bits(n, k, j->wide);
   j->bbits = std::max(2, bb);
-  const int B = 1 << j->bbits;
   // the counting pass histograms at most kHistBits digits; deeper partitions get their
   // fine bucket sizes from a count over the coarse regions (k_fine_count)
-  const int hb = std::min(j->bbits, kHistBits);
+  const int hb = by_count ? hist_bits(n, k, j->wide) : std::min(j->bbits, kHistBits);
   const int HB = 1 << hb;
   const uint64_t ntiles = (n + kTileBytes - 1) / kTileBytes;
   int grid = (int)std::min<uint64_t>((uint64_t)thread_sms(j->ctx->sms), std::max<uint64_t>(ntiles, 1));
@@ -380,9 +406,8 @@ pk_status pk::count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_pa
   // 16 input bytes)
   const uint64_t nseg = (n + kSegBytes - 1) / kSegBytes;
   PK_TRY(job_alloc(j, j->units, (size_t)40 * nseg));
-  PK_TRY(job_alloc(j, j->bstart, sizeof(uint32_t) * (B + 1)));
-  if (hb < j->bbits) PK_TRY(job_alloc(j, j->hstart, sizeof(uint32_t) * (HB + 1)));
-  uint32_t* hstart = (uint32_t*)(hb < j->bbits ? j->hstart.p : j->bstart.p);
+  PK_TRY(job_alloc(j, j->hstart, sizeof(uint32_t) * (HB + 1)));
+  uint32_t* hstart = (uint32_t*)j->hstart.p;
   if (!j->graph_mode && !j->lines_ready) {
     Scalars init{};
     memset(&init, 0, sizeof(init));
@@ -398,7 +423,6 @@ pk_status pk::count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_pa
   a.lmer_m = std::min(k, p->lmer_length);
   a.drop_n = p->drop_n ? 1 : 0;
   a.bbits = hb;
-  a.cbits = std::min(j->bbits, kCoarseBits);
   a.grid = grid;
   a.chunk = chunk;
   a.tile_nl = (uint32_t*)j->tile_nl.p;
@@ -434,6 +458,14 @@ pk_status pk::count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_pa
   if (N >= (1ull << 32) - 1)
     return fail(PK_ERR_LIMIT, "more than 2^32-2 k-mer windows in one job; split the input");
   j->N = N;
+  if (by_count) {
+    j->bbits = partition_bits((double)N, k, j->wide);
+    // a digit or two short of the target costs less than a count over the coarse regions
+    if (hb < kHistBits) j->bbits = std::min(j->bbits, hb);
+  }
+  const int B = 1 << j->bbits;
+  a.cbits = std::min(j->bbits, kCoarseBits);
+  PK_TRY(job_alloc(j, j->bstart, sizeof(uint32_t) * (B + 1)));
   PK_TRY(job_alloc(j, j->keys, (size_t)W * N));
   a.n_keys = N;
   PK_TRY(job_alloc(j, j->tkeys, (size_t)W * N));
@@ -452,11 +484,11 @@ pk_status pk::count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_pa
   PK_TRY(job_alloc(j, j->cstart, sizeof(uint32_t) * (Cn + 1)));
   PK_TRY(job_alloc(j, j->slice_start, sizeof(uint32_t) * (Cn + 1)));
   PK_TRY(job_alloc(j, j->fcur, sizeof(uint32_t) * (size_t)B));
-  const bool two_pass = a.cbits < a.bbits;
+  const bool two_pass = a.cbits < j->bbits;
   mark_begin(j, ST_SCATTER);
-  PK_CUDA(launch_coarse_offsets(a, (uint32_t*)j->coff.p, (uint32_t*)j->cstart.p,
+  PK_CUDA(launch_coarse_offsets(a, j->bbits, (uint32_t*)j->coff.p, (uint32_t*)j->cstart.p,
                                 (uint32_t*)j->slice_start.p, fine_slice_keys(j->wide, j->bbits - a.cbits),
-                                j->stream));
+                                (uint32_t*)j->bstart.p, (uint32_t*)j->fcur.p, j->stream));
   PK_CUDA(launch_scatter_coarse(a, (const uint32_t*)j->coff.p, two_pass ? j->tkeys.p : j->keys.p,
                                 j->wide, j->stream));
   mark_end(j, ST_SCATTER);
@@ -469,10 +501,9 @@ pk_status pk::count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_pa
                                 (uint32_t*)j->bstart.p, k, j->bbits, a.cbits, j->wide, &j->d_sc->ticket_fcount,
                                 j->stream));
       PK_CUDA(launch_prefix((uint32_t*)j->bstart.p, B, j->stream));
+      PK_CUDA(cudaMemcpyAsync(j->fcur.p, j->bstart.p, sizeof(uint32_t) * (size_t)B, cudaMemcpyDeviceToDevice,
+                              j->stream));
     }
-    PK_CUDA(cudaMemcpyAsync(j->fcur.p, j->bstart.p, sizeof(uint32_t) * (size_t)B, cudaMemcpyDeviceToDevice,
-                            j->stream));
-    PK_CUDA(cudaMemsetAsync(&j->d_sc->ticket_fine, 0, sizeof(uint32_t), j->stream));
     PK_CUDA(launch_scatter_fine(j->tkeys.p, (const uint32_t*)j->cstart.p, (const uint32_t*)j->slice_start.p,
                                 (uint32_t*)j->fcur.p, j->keys.p, k, j->bbits, a.cbits, j->wide,
                                 &j->d_sc->ticket_fine, N, &j->d_sc->err, j->stream));
@@ -486,20 +517,24 @@ static pk_status table_impl(pk_job* j, uint64_t N, int t) {
   const int k = j->params.k;
   const int B = 1 << j->bbits;
   mark_begin(j, ST_TABLE);
-  // giant buckets are reduced chunk by chunk first (chunk items ahead of the buckets)
-  PK_TRY(job_alloc(j, j->gfirst, sizeof(uint32_t) * (size_t)B));
-  PK_TRY(job_alloc(j, j->gcount, sizeof(uint32_t) * (size_t)B));
-  PK_TRY(job_alloc(j, j->gdone, sizeof(uint32_t) * (size_t)B));
-  PK_TRY(job_alloc(j, j->chunk_bucket, sizeof(uint32_t) * (size_t)(N / kChunkKeys + 1)));
-  PK_TRY(job_alloc(j, j->chunk_u, sizeof(uint32_t) * (size_t)(N / kChunkKeys + 1)));
-  PK_CUDA(launch_giant_chunks((const uint32_t*)j->bstart.p, j->bbits, (uint32_t*)j->gfirst.p,
-                              (uint32_t*)j->gcount.p, (uint32_t*)j->chunk_bucket.p, (uint32_t*)j->gdone.p,
-                              j->d_sc, j->stream));
+  // giant buckets are reduced chunk by chunk first (chunk items ahead of the buckets);
+  // fewer windows than a giant bucket's keys hold none
+  const bool giants = N >= kGiantKeys;
+  if (giants) {
+    PK_TRY(job_alloc(j, j->gfirst, sizeof(uint32_t) * (size_t)B));
+    PK_TRY(job_alloc(j, j->gcount, sizeof(uint32_t) * (size_t)B));
+    PK_TRY(job_alloc(j, j->gdone, sizeof(uint32_t) * (size_t)B));
+    PK_TRY(job_alloc(j, j->chunk_bucket, sizeof(uint32_t) * (size_t)(N / kChunkKeys + 1)));
+    PK_TRY(job_alloc(j, j->chunk_u, sizeof(uint32_t) * (size_t)(N / kChunkKeys + 1)));
+    PK_CUDA(launch_giant_chunks((const uint32_t*)j->bstart.p, j->bbits, (uint32_t*)j->gfirst.p,
+                                (uint32_t*)j->gcount.p, (uint32_t*)j->chunk_bucket.p, (uint32_t*)j->gdone.p,
+                                j->d_sc, j->stream));
+  }
   PK_TRY(job_alloc(j, j->bsmall, sizeof(uint32_t) * kSmallCounts * (size_t)B));
   BucketArgs b{};
   b.keys = j->keys.p;
   b.bsmall = (uint32_t*)j->bsmall.p;
-  b.gfirst = (const uint32_t*)j->gfirst.p;
+  b.gfirst = giants ? (const uint32_t*)j->gfirst.p : nullptr;
   b.gcount = (const uint32_t*)j->gcount.p;
   b.chunk_bucket = (const uint32_t*)j->chunk_bucket.p;
   b.gdone = (uint32_t*)j->gdone.p;

@@ -783,35 +783,54 @@ k_scatter_coarse(CountArgs a, const uint32_t* __restrict__ coff, KeyT* __restric
 
 // Coarse offsets: coff[c][g] = start of chunk c's segment in coarse region g (the
 // coarse region is the union of its fine buckets' regions); cstart[g] = region start;
-// slice_start[g] = first pass-2 slice of region g.
+// slice_start[g] = first pass-2 slice of region g.  The counting pass's histogram has 2^hbits
+// bins; where that is the partition's 2^pbits buckets or more, their starts and the fine
+// scatter's cursors are picked out of its prefix here too.
 __global__ void __launch_bounds__(256) k_coarse_offsets(const uint32_t* __restrict__ counts,
-                                                        const uint32_t* __restrict__ bstart, int grid,
-                                                        int bbits, int cbits, uint32_t* coff,
-                                                        uint32_t* cstart, uint32_t* slice_start,
-                                                        int slice_keys) {
+                                                        const uint32_t* __restrict__ hstart, int hbits, int pbits,
+                                                        int cbits, uint32_t* coff, uint32_t* cstart,
+                                                        uint32_t* slice_start, int slice_keys,
+                                                        uint32_t* __restrict__ bstart,
+                                                        uint32_t* __restrict__ fcur, Scalars* sc) {
   __shared__ uint32_t s_c[1 << kCoarseBits];
+  __shared__ uint32_t s_warp[33];
   const int c = blockIdx.x;
-  const int B = 1 << bbits, Cn = 1 << cbits, fb = bbits - cbits;
-  // a warp sums the 2^fb fine buckets of one coarse region at a time
+  const int Cn = 1 << cbits, fb = hbits - cbits;
+  // a warp sums the 2^fb histogram bins of one coarse region at a time
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int g = warp; g < Cn; g += nw) {
     uint32_t sum = 0;
-    for (int i = lane; i < (1 << fb); i += 32) sum += counts[(size_t)c * B + ((size_t)g << fb) + i];
+    for (int i = lane; i < (1 << fb); i += 32) sum += counts[((size_t)c << hbits) + ((size_t)g << fb) + i];
     sum = __reduce_add_sync(FULLMASK, sum);
     if (lane == 0) s_c[g] = sum;
   }
   __syncthreads();
-  for (int g = threadIdx.x; g < Cn; g += blockDim.x) coff[(size_t)c * Cn + g] = bstart[g << fb] + s_c[g];
-  if (c == 0 && threadIdx.x == 0) {
-    uint32_t acc = 0;
-    for (int g = 0; g < Cn; g++) {
-      cstart[g] = bstart[g << fb];
-      slice_start[g] = acc;
-      const uint32_t n = bstart[(g + 1) << fb] - bstart[g << fb];
-      acc += (n + slice_keys - 1) / slice_keys;
+  for (int g = threadIdx.x; g < Cn; g += blockDim.x) coff[(size_t)c * Cn + g] = hstart[g << fb] + s_c[g];
+  if (pbits <= hbits) {
+    const int B = 1 << pbits, d = hbits - pbits;
+    for (int i = c * blockDim.x + threadIdx.x; i <= B; i += gridDim.x * blockDim.x) {
+      const uint32_t v = hstart[i << d];
+      bstart[i] = v;
+      if (i < B) fcur[i] = v;
     }
-    cstart[Cn] = bstart[B];
-    slice_start[Cn] = acc;
+  }
+  if (c == 0) {
+    static_assert((1 << kCoarseBits) <= 256, "one region per thread");
+    const int g = threadIdx.x;
+    uint32_t s = 0, e = 0;
+    if (g < Cn) {
+      s = hstart[g << fb];
+      e = hstart[(g + 1) << fb];
+      cstart[g] = s;
+      if (g == Cn - 1) cstart[Cn] = e;
+    }
+    uint32_t tot;
+    const uint32_t first = block_exclusive_sum((e - s + slice_keys - 1) / slice_keys, s_warp, tot);
+    if (g < Cn) slice_start[g] = first;
+    if (g == 0) {
+      slice_start[Cn] = tot;
+      sc->ticket_fine = 0;
+    }
   }
 }
 
@@ -2461,11 +2480,11 @@ cudaError_t launch_scatter_coarse(const CountArgs& a, const uint32_t* coff, void
               : launch_coarse_t<uint64_t>(a, coff, reinterpret_cast<uint64_t*>(out), st);
 }
 
-cudaError_t launch_coarse_offsets(const CountArgs& a, uint32_t* coff, uint32_t* cstart,
-                                  uint32_t* slice_start, int slice_keys, cudaStream_t st) {
-  const int sk = slice_keys;
-  pk::note_launch(), k_coarse_offsets<<<a.grid, 256, 0, st>>>(a.counts, a.bstart, a.grid, a.bbits, a.cbits, coff, cstart,
-                                           slice_start, sk);
+cudaError_t launch_coarse_offsets(const CountArgs& a, int pbits, uint32_t* coff, uint32_t* cstart,
+                                  uint32_t* slice_start, int slice_keys, uint32_t* bstart, uint32_t* fcur,
+                                  cudaStream_t st) {
+  pk::note_launch(), k_coarse_offsets<<<a.grid, 256, 0, st>>>(a.counts, a.bstart, a.bbits, pbits, a.cbits, coff, cstart,
+                                                              slice_start, slice_keys, bstart, fcur, a.sc);
   return cudaGetLastError();
 }
 
@@ -2551,7 +2570,7 @@ static cudaError_t launch_bucket_t(const BucketArgs& a, int grid, cudaStream_t s
   if (grid <= 0) grid = sm_count() * bucket_ctas_per_sm(sizeof(KeyT) == 16);
   // exactly one of the two works (giant buckets present or not); the other returns
   pk::note_launch(), k_bucket_table<KeyT, false, BC::T><<<grid, BC::T, smem, st>>>(a);
-  pk::note_launch(), k_bucket_table<KeyT, true, BC::TG><<<grid, BC::TG, smem, st>>>(a);
+  if (a.gfirst) pk::note_launch(), k_bucket_table<KeyT, true, BC::TG><<<grid, BC::TG, smem, st>>>(a);
   return cudaGetLastError();
 }
 
