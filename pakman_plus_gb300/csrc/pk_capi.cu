@@ -823,6 +823,7 @@ pk_status pk::cutoff_enqueue(pk_job* j, int t) {
                              j->stream));
     hist = (const unsigned long long*)j->hist2.p;
   }
+  j->cut_max = (uint32_t)std::max(1, t - 1);
   mark_begin(j, ST_CUTOFF);
   PK_CUDA(launch_cutoff(hist, t, j->d_sc, j->stream));
   mark_end(j, ST_CUTOFF);
@@ -858,15 +859,19 @@ pk_status pk::mn_enqueue(pk_job* j, uint32_t min_count, uint64_t kept_bound) {
   PK_TRY(job_alloc(j, j->kstart, sizeof(uint32_t) * B));
   PK_TRY(job_alloc(j, j->kcount, sizeof(uint32_t) * B));
   PK_TRY(job_alloc(j, j->ksub, sizeof(uint32_t) * 3 * (size_t)B));
-  PK_TRY(job_alloc(j, j->flags_f, sizeof(unsigned long long) * B));
+  const size_t fflags = sizeof(unsigned long long) * (((size_t)B + 255) / 256);
+  PK_TRY(job_alloc(j, j->flags_f, fflags));
   PK_TRY(job_alloc(j, j->nkeys, W * cap));
   PK_TRY(job_alloc(j, j->nsuf, 16 * cap));
   PK_TRY(job_alloc(j, j->npre, 16 * cap));
-  PK_TRY(job_alloc(j, j->flags_m, sizeof(unsigned long long) * B));
-  PK_CUDA(cudaMemsetAsync(j->flags_f.p, 0, sizeof(unsigned long long) * B, j->stream));
-  PK_CUDA(cudaMemsetAsync(j->flags_m.p, 0, sizeof(unsigned long long) * B, j->stream));
+  // the macro-node kernel's look-back words, and its list of big units behind them
+  const size_t mflags = sizeof(unsigned long long) * mn_flag_words(j->bbits);
+  PK_TRY(job_alloc(j, j->flags_m, mflags + sizeof(uint32_t) * (size_t)B));
+  PK_CUDA(cudaMemsetAsync(j->flags_f.p, 0, fflags, j->stream));
+  PK_CUDA(cudaMemsetAsync(j->flags_m.p, 0, mflags, j->stream));
   PK_CUDA(cudaMemsetAsync(&j->d_sc->ticket_mn, 0, sizeof(uint32_t), j->stream));
   PK_CUDA(cudaMemsetAsync(&j->d_sc->ticket_filter, 0, sizeof(uint32_t), j->stream));
+  PK_CUDA(cudaMemsetAsync(&j->d_sc->n_big, 0, sizeof(uint32_t), j->stream));
   PK_CUDA(cudaMemsetAsync(&j->d_sc->n_nodes, 0, sizeof(unsigned long long), j->stream));
   PK_CUDA(cudaMemsetAsync(&j->d_sc->n_kept_rows, 0, sizeof(unsigned long long), j->stream));
   if (min_count) PK_CUDA(cudaMemcpyAsync(&j->d_sc->cutoff, &min_count, sizeof(uint32_t), cudaMemcpyHostToDevice, j->stream));
@@ -890,7 +895,8 @@ pk_status pk::mn_enqueue(pk_job* j, uint32_t min_count, uint64_t kept_bound) {
   f.spin_limit = (int)j->wait_limit;
   f.sc = j->d_sc;
   mark_begin(j, ST_FILTER);
-  PK_CUDA(launch_filter_kept(f, j->wide, 0, j->stream));
+  const uint32_t cut_max = min_count ? min_count : j->cut_max;
+  PK_CUDA(launch_filter_kept(f, j->wide, !f.bsmall || cut_max > (uint32_t)kSmallCounts, j->stream));
   mark_end(j, ST_FILTER);
   MnArgs m{};
   m.kkeys = j->kkeys.p;
@@ -899,6 +905,7 @@ pk_status pk::mn_enqueue(pk_job* j, uint32_t min_count, uint64_t kept_bound) {
   m.kcount = (const uint32_t*)j->kcount.p;
   m.ksub = (const uint32_t*)j->ksub.p;
   m.flags = (unsigned long long*)j->flags_m.p;
+  m.big = (uint32_t*)((char*)j->flags_m.p + mflags);
   m.nkeys = j->nkeys.p;
   m.nsuf = (uint32_t*)j->nsuf.p;
   m.npre = (uint32_t*)j->npre.p;
@@ -906,16 +913,13 @@ pk_status pk::mn_enqueue(pk_job* j, uint32_t min_count, uint64_t kept_bound) {
   m.kcap = kcap;
   m.k = j->params.k;
   m.bbits = j->bbits;
-  // node units of about 1000 kept rows: each unit merges up to 2V / units rows
+  // node units of up to 1000 rows where the partition is that fine (each merges 2V / units
+  // of them on average, half from each side; a joined unit holds kMnJoin a side)
   {
-    const double units = std::max(1.0, 2.0 * (double)kept_bound / 1000.0);
-    int ub = 0;
-    while ((double)(1u << ub) < units && ub < 30) ub++;
-    int level = (j->bbits - ub) / 2;
-    if (level < 1) level = 0;
-    if (j->params.mn_units > 0) level = j->params.mn_units - 1;
-    if (2 * level > j->bbits) level = j->bbits / 2;
-    m.level = level;
+    int x = 0;
+    while (x < j->bbits && 2.0 * (double)kept_bound / (double)(1u << (j->bbits - x - 1)) <= 1000.0) x++;
+    if (j->params.mn_units > 0) x = std::min(2 * (j->params.mn_units - 1), j->bbits & ~1);
+    m.xbits = x;
   }
   m.spin_limit = (int)j->wait_limit;
   m.withhold_unit = j->withhold_unit;

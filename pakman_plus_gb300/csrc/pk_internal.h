@@ -29,10 +29,12 @@ enum : uint32_t {
 
 constexpr int kTileBytes = 65536;   // line-scan tile; chunk boundaries are multiples of it
 constexpr int kSegBytes = 64;       // bytes per thread per extraction step
-constexpr int kMnThreads = 128;
+constexpr int kMnThreads = 256;
+constexpr int kMnCap = 1568;        // items per segment of a sorted unit
+constexpr int kMnFit = kMnCap - 16; // rows per segment before ties; both sides of a joined unit
+constexpr int kMnJoin = 768;        // items a side of a joined macro-node unit
 constexpr int kSmallCounts = 16;    // per-bucket histogram of the table kernel: counts 0..15
-constexpr int kMnCap = 1536;        // items (k-mer records) per macro-node segment on chip
-constexpr int kMnBinBits = 8;       // counting-sort bins of a macro-node segment
+constexpr int kMnBinBits = 9;       // counting-sort bins of a macro-node segment
 constexpr int kMnBins = 1 << kMnBinBits;
 constexpr int kMnBinMax = 32;       // largest bin ranked within itself (else merge ranks)
 constexpr int kHistSmem = 1024;     // count-histogram bins kept in shared memory
@@ -65,6 +67,7 @@ struct Scalars {                    // device-side scalars of one job
   uint32_t ticket_fine;
   uint32_t ticket_fcount;
   uint32_t n_chunk_items;           // chunk items of giant buckets (table kernel)
+  uint32_t n_big;                   // macro-node units of more than one segment
   unsigned long long n_unique;      // U
   unsigned long long n_kept;        // V
   unsigned long long n_nodes;       // M
@@ -128,7 +131,7 @@ struct FilterArgs {
   const uint32_t* tcounts;
   const uint32_t* bstart;
   const uint32_t* tu;
-  unsigned long long* flags; // 2^bbits look-back words (zeroed)
+  unsigned long long* flags; // look-back words of the offsets, one per 256 buckets (zeroed)
   void* kkeys;               // kept keys out
   uint32_t* kcounts;         // kept counts out
   uint32_t* kstart;          // 2^bbits
@@ -151,7 +154,8 @@ struct MnArgs {
   const uint32_t* kstart;
   const uint32_t* kcount;
   const uint32_t* ksub;
-  unsigned long long* flags; // 2^bbits look-back words (zeroed)
+  unsigned long long* flags; // mn_flag_words(bbits) look-back words (zeroed)
+  uint32_t* big;             // 2^bbits: the units of more than one segment
   void* nkeys;               // node keys out (capacity cap)
   uint32_t* nsuf;            // 4 * cap
   uint32_t* npre;            // 4 * cap
@@ -159,7 +163,7 @@ struct MnArgs {
   unsigned long long kcap;   // kept rows the kept buffers hold
   int k;
   int bbits;
-  int level;                 // node units cover 4^level table buckets (0: one bucket, split)
+  int xbits;                 // node units cover 2^xbits table buckets' node keys
   int spin_limit;            // polls of a bounded wait before it gives up (0: default)
   int withhold_unit;         // a unit that publishes no look-back word (-1: none; tests of
                              // the bounded waits)
@@ -228,7 +232,9 @@ cudaError_t launch_table_bounds(const void* keys, unsigned long long n, int bbit
 cudaError_t launch_histogram(const uint32_t* tcounts, const uint32_t* bstart, const uint32_t* tu, int B, int t,
                              unsigned long long* hist, cudaStream_t st);
 cudaError_t launch_cutoff(const unsigned long long* hist, int t, Scalars* sc, cudaStream_t st);
-cudaError_t launch_filter_kept(const FilterArgs& a, int wide, int grid, cudaStream_t st);
+// count_rows: the cutoff may be above what the small-count histograms tell, or there are none
+cudaError_t launch_filter_kept(const FilterArgs& a, int wide, bool count_rows, cudaStream_t st);
+size_t mn_flag_words(int bbits);  // look-back words of the macro-node kernel
 cudaError_t launch_macro_nodes(const MnArgs& a, int wide, int grid, cudaStream_t st);
 // Dense copy of the sparse table (doff: exclusive prefix of tu, computed by
 // launch_row_offsets).  packed != null writes KmerPairs records instead of arrays.

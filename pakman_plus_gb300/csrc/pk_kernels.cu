@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "pk_internal.h"
@@ -106,14 +107,15 @@ __device__ __forceinline__ unsigned lanemask_lt() {
   return r;
 }
 
-__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+// Look-back words carry all their data themselves: relaxed accesses, coherent in the device.
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
   unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 
-__device__ __forceinline__ void st_release(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
@@ -136,14 +138,25 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
   return v;
 }
 
-// Exclusive prefix of `flags[0..idx)`, computed by a whole warp (all 32 lanes call it
-// and all get the sum).  Each step reads the 32 nearest unread predecessors at once
-// (lane 0 = nearest): it stops at the nearest inclusive word, otherwise adds the
-// aggregates up to the first word still unpublished and moves past them.  Waiting on
-// an unpublished word is bounded: on expiry the error bit is set and the partial sum
-// is returned.
-__device__ unsigned long long lookback_exclusive(unsigned long long* flags, int idx, uint32_t* err,
-                                                int limit) {
+// Waits a little before a look-back word is read again; false when the wait has run out
+// (the error bit is set).
+__device__ __forceinline__ bool lookback_wait(int& spins, int max_spins, uint32_t* err) {
+  if (++spins >= max_spins) {
+    if ((threadIdx.x & 31) == 0) atomicOr(err, ERR_LOOKBACK);
+    return false;
+  }
+  __nanosleep(spins < 64 ? 32 : 256);
+  return true;
+}
+
+// Sum over the words before `idx` of a look-back sequence, by a whole warp (all 32 lanes
+// call it and all get the sum).  read(j, value) gives word j's state: 0 unpublished, 1 an
+// aggregate, 2 an inclusive prefix.  Each step reads the 32 nearest unread predecessors
+// (lane 0 = nearest): it stops at the nearest inclusive word, otherwise adds the aggregates
+// up to the first word still unpublished and moves past them.  Waiting is bounded: on
+// expiry the partial sum is returned.
+template <typename Read>
+__device__ __forceinline__ unsigned long long lookback_exclusive(int idx, uint32_t* err, int limit, Read&& read) {
   const int max_spins = spin_limit(limit);
   const int lane = threadIdx.x & 31;
   unsigned long long sum = 0;
@@ -151,29 +164,71 @@ __device__ unsigned long long lookback_exclusive(unsigned long long* flags, int 
   int spins = 0;
   while (top >= 0) {
     const int j = top - lane;
-    const unsigned long long f = j >= 0 ? ld_acquire(&flags[j]) : kLbIncl;  // below 0: inclusive 0
-    const unsigned st = (unsigned)(f >> 62);
+    unsigned long long v = 0;
+    const unsigned st = j >= 0 ? read(j, v) : 2u;  // below 0: inclusive 0
     const unsigned waiting = __ballot_sync(FULLMASK, st == 0);
     const unsigned incl = __ballot_sync(FULLMASK, st == 2);
     const int first_wait = waiting ? __ffs(waiting) - 1 : 32;
     const int first_incl = incl ? __ffs(incl) - 1 : 32;
-    if (first_incl < first_wait) {
-      sum += warp_sum_u64(lane <= first_incl ? (f & kLbVal) : 0ull);
-      return sum;
-    }
+    if (first_incl < first_wait) return sum + warp_sum_u64(lane <= first_incl ? v : 0ull);
     if (first_wait > 0) {
-      sum += warp_sum_u64(lane < first_wait ? (f & kLbVal) : 0ull);
+      sum += warp_sum_u64(lane < first_wait ? v : 0ull);
       top -= first_wait;
       spins = 0;
       continue;
     }
-    if (++spins >= max_spins) {
-      if (lane == 0) atomicOr(err, ERR_LOOKBACK);
-      return sum;
-    }
-    __nanosleep(spins < 64 ? 32 : 256);
+    if (!lookback_wait(spins, max_spins, err)) return sum;
   }
   return sum;
+}
+
+// Look-back in two levels, for sequences with hundreds of units in flight: a unit publishes
+// its value in its own word and adds it to its group of 32; it reads the words before it in
+// its group, and looks back over groups (complete ones count as aggregates; the group's
+// last unit publishes the inclusive prefix).  Looking back over single units, every unit
+// read hundreds of words that all the others were reading too.  (Eight words a lane and
+// step instead of one made that worse, 0.37 to 0.91 ms for 8.6M nodes: the reads of the
+// same lines are the cost, not their number in a row.)  The words: unit (units), then per
+// group the sum (count of published units in bits 48 up) and the inclusive prefix; all zero
+// beforehand.
+struct GroupFlags {
+  unsigned long long *unit, *sum, *incl;
+  __device__ GroupFlags(unsigned long long* words, uint32_t units)
+      : unit(words), sum(words + units), incl(sum + (units + 31) / 32) {}
+};
+
+__device__ __forceinline__ void group_publish(const GroupFlags& w, uint32_t u, unsigned long long mine) {
+  st_relaxed(&w.unit[u], kLbAgg | mine);
+  atomicAdd(&w.sum[u >> 5], (1ull << 48) | mine);
+}
+
+// The sum before unit u.  Its own value is published first, or waited for where another CTA
+// publishes it (`mine` = ~0); `publish` false keeps it from the successors (fault injection).
+__device__ unsigned long long group_lookback(const GroupFlags& w, uint32_t u, unsigned long long mine,
+                                             bool publish, uint32_t* err, int limit) {
+  const int lane = threadIdx.x & 31, max_spins = spin_limit(limit);
+  const uint32_t g = u >> 5, i = u & 31;
+  const bool own = mine != ~0ull;
+  if (lane == 0 && publish && own) group_publish(w, u, mine);
+  __syncwarp();
+  unsigned long long f = 0;
+  int spins = 0;
+  while (true) {
+    const bool wanted = (uint32_t)lane < i || ((uint32_t)lane == i && !own);
+    f = wanted ? ld_relaxed(&w.unit[32 * g + lane]) : kLbAgg;
+    if (__all_sync(FULLMASK, f != 0)) break;
+    if (!lookback_wait(spins, max_spins, err)) return 0;
+  }
+  if (!own) mine = __shfl_sync(FULLMASK, f, i) & kLbVal;
+  const unsigned long long before = warp_sum_u64((uint32_t)lane < i ? f & kLbVal : 0ull);
+  const unsigned long long ex = before + lookback_exclusive((int)g, err, limit, [&](int j, unsigned long long& v) {
+    const unsigned long long p = ld_relaxed(&w.incl[j]), s = ld_relaxed(&w.sum[j]);
+    const bool inclusive = (p >> 62) == 2;
+    v = inclusive ? p & kLbVal : s & ((1ull << 48) - 1);
+    return inclusive ? 2u : (s >> 48) == 32 ? 1u : 0u;
+  });
+  if (lane == 0 && publish && i == 31) st_relaxed(&w.incl[g], kLbIncl | (ex + mine));
+  return ex;
 }
 
 // Block-wide exclusive sum over `nthreads` (multiple of 32, <= 1024) threads.
@@ -1885,14 +1940,45 @@ __global__ void __launch_bounds__(1024) k_cutoff(const unsigned long long* __res
 
 // ----------------------------------------------------------------- macro-nodes -------
 template <typename KeyT>
-struct MnSmem {
-  static constexpr size_t off_key = 0;
-  static constexpr size_t off_cnt = off_key + sizeof(KeyT) * kMnCap;
-  static constexpr size_t off_tag = off_cnt + sizeof(uint32_t) * kMnCap;
-  static constexpr size_t off_ord = off_tag + sizeof(uint8_t) * kMnCap;
-  static constexpr size_t off_nid = off_ord + sizeof(uint16_t) * kMnCap;
-  static constexpr size_t bytes = off_nid + sizeof(uint16_t) * kMnCap;
+struct MnCfg;
+template <>
+struct MnCfg<uint64_t> {  // with 256 threads; 128 and 192 threads were 5 to 20 % slower
+  static constexpr int CTAS = 6;  // CTAs per SM
 };
+template <>
+struct MnCfg<u128> {
+  static constexpr int CTAS = 5;
+};
+
+template <typename KeyT>
+struct MnSmem {
+  static constexpr int CAP = kMnCap;
+  static constexpr size_t off_key = 0;
+  static constexpr size_t off_cnt = off_key + sizeof(KeyT) * CAP;
+  static constexpr size_t off_bin = off_cnt + sizeof(uint32_t) * CAP;
+  static constexpr size_t off_ord = off_bin + sizeof(uint16_t) * CAP;
+  static constexpr size_t merge_bytes = off_ord + sizeof(uint16_t) * CAP;
+  // joined units: node rows, suffix-side node keys, first suffix item of every bin
+  static constexpr size_t off_rows = 0;
+  static constexpr size_t off_pkey = off_rows + 32 * (kMnJoin + 32);
+  static constexpr size_t off_start = off_pkey + sizeof(KeyT) * kMnJoin;
+  static constexpr size_t join_bytes = (off_start + sizeof(uint16_t) * (kMnBins + 1) + 15) / 16 * 16;
+  static constexpr size_t bytes = merge_bytes > join_bytes ? merge_bytes : join_bytes;
+  static_assert(CAP <= 2048, "item numbers have 11 bits");
+};
+
+__device__ __forceinline__ uint64_t shfl_xor_key(uint64_t x, int o) {
+  return __shfl_xor_sync(FULLMASK, (unsigned long long)x, o);
+}
+__device__ __forceinline__ u128 shfl_xor_key(u128 x, int o) {
+  return ((u128)shfl_xor_key((uint64_t)(x >> 64), o) << 64) | shfl_xor_key((uint64_t)x, o);
+}
+__device__ __forceinline__ uint64_t shfl_key(uint64_t x, int l) {
+  return __shfl_sync(FULLMASK, (unsigned long long)x, l);
+}
+__device__ __forceinline__ u128 shfl_key(u128 x, int l) {
+  return ((u128)shfl_key((uint64_t)(x >> 64), l) << 64) | shfl_key((uint64_t)x, l);
+}
 
 template <typename KeyT>
 __device__ __forceinline__ uint32_t lower_bound_s(const KeyT* k, uint32_t lo, uint32_t hi, KeyT x) {
@@ -1932,52 +2018,102 @@ __device__ __forceinline__ uint32_t kept_group(const FilterArgs& a, uint32_t q, 
   return m;
 }
 
+// Kept rows (count >= cutoff) of every table bucket by reading its counts, one warp per
+// bucket: where the table kernel's histogram of small counts does not tell (a cutoff above
+// it, or a table that did not come from that kernel).
+__device__ __forceinline__ bool small_counts_tell(const FilterArgs& a, uint32_t cut) {
+  return a.bsmall && cut <= (uint32_t)kSmallCounts;
+}
+
+__global__ void __launch_bounds__(256) k_kept_count(FilterArgs a) {
+  const uint32_t cut = a.sc->cutoff;
+  if (small_counts_tell(a, cut)) return;
+  const int lane = threadIdx.x & 31;
+  const uint32_t B = 1u << a.bbits, warps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < B; b += warps) {
+    const uint32_t r0 = a.bstart[b], e = r0 + a.tu[b];
+    uint32_t v = 0;
+    for (uint32_t g = r0 & ~3u; g < e; g += 128) {
+      uint32_t c[4];
+      v += __popc(kept_group(a, g + 4 * lane, r0, e, cut, c));
+    }
+    v = __reduce_add_sync(FULLMASK, v);
+    if (lane == 0) a.kcount[b] = v;
+  }
+}
+
+// Kept rows and their prefix over the buckets, one bucket per thread: a bucket keeps its
+// rows minus those counted fewer than cutoff times.  One look-back per 256 buckets, where
+// one per bucket inside the filter cost it 0.20 against 0.17 ms (bacterial) and 1.21
+// against 0.82 ms (46M kept 63-mers), offsets included.
+constexpr int kKeptT = 256;
+__global__ void __launch_bounds__(kKeptT) k_kept_offsets(FilterArgs a) {
+  __shared__ uint32_t s_warp[33];
+  __shared__ uint32_t s_tile;
+  __shared__ unsigned long long s_before;
+  const uint32_t cut = a.sc->cutoff;
+  const uint32_t B = 1u << a.bbits, tiles = (B + kKeptT - 1) / kKeptT;
+  if (threadIdx.x == 0) s_tile = atomicAdd(&a.sc->ticket_filter, 1u);
+  __syncthreads();
+  const uint32_t tile = s_tile, b = tile * kKeptT + threadIdx.x;
+  uint32_t v = 0;
+  if (b < B) {
+    if (small_counts_tell(a, cut)) {
+      uint32_t below = 0;
+      const uint4* h = reinterpret_cast<const uint4*>(a.bsmall + (size_t)b * kSmallCounts);
+      for (uint32_t q = 0; 4 * q < cut; q++) {  // counts 4q .. 4q + 3 (no row counts 0)
+        const uint4 c = h[q];
+        below += (4 * q > 0 ? c.x : 0u) + (4 * q + 1 < cut ? c.y : 0u) + (4 * q + 2 < cut ? c.z : 0u) +
+                 (4 * q + 3 < cut ? c.w : 0u);
+      }
+      v = a.tu[b] - below;
+    } else {
+      v = a.kcount[b];
+    }
+  }
+  uint32_t tot;
+  const uint32_t ex = block_exclusive_sum(v, s_warp, tot);
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) st_relaxed(&a.flags[tile], (tile ? kLbAgg : kLbIncl) | (unsigned long long)tot);
+    __syncwarp();
+    const unsigned long long before = lookback_exclusive((int)tile, &a.sc->err, a.spin_limit,
+                                                         [&](int j, unsigned long long& x) {
+      const unsigned long long f = ld_relaxed(&a.flags[j]);
+      x = f & kLbVal;
+      return (unsigned)(f >> 62);
+    });
+    if (threadIdx.x == 0) {
+      if (tile) st_relaxed(&a.flags[tile], kLbIncl | (before + tot));
+      s_before = before;
+      if (tile == tiles - 1) a.sc->n_kept_rows = before + tot;
+    }
+  }
+  __syncthreads();
+  if (b < B) {
+    a.kstart[b] = (uint32_t)s_before + ex;
+    a.kcount[b] = v;
+  }
+}
+
 // Kept rows (count >= cutoff) of every table bucket, written densely in key order --
-// the k-mers construct_kmer_histogram hands to macro-node construction.  Per bucket:
-// kstart (first kept row), kcount, and ksub (kept rows whose next two key bits are
-// < 1, 2, 3).  Bucket offsets come from a decoupled look-back (every bucket publishes
-// its aggregate before waiting).
+// the k-mers construct_kmer_histogram hands to macro-node construction -- from the bucket's
+// offset (kstart) on, and ksub (kept rows whose next two key bits are < 1, 2, 3).
+// One warp per table bucket, with no waits between buckets.  Lane l takes the rows
+// [g + 4l, g + 4l + 4) of each 128-row step, with g aligned to four rows, so one 16-byte load
+// brings its four counts and lane order is row order.
 template <typename KeyT>
 __global__ void __launch_bounds__(256) k_filter_kept(FilterArgs a) {
-  // one warp per table bucket: no block-wide barriers.  Lane l takes the rows
-  // [g + 4l, g + 4l + 4) of each 128-row step, with g aligned to four rows, so one
-  // 16-byte load brings its four counts and lane order is row order.
   const int lane = threadIdx.x & 31;
-  const int B = 1 << a.bbits;
+  const uint32_t B = 1u << a.bbits, warps = gridDim.x * (blockDim.x >> 5);
   const int rem = 2 * a.k - a.bbits;
   const uint32_t cut = a.sc->cutoff;
   const KeyT* __restrict__ tkeys = reinterpret_cast<const KeyT*>(a.tkeys);
   KeyT* __restrict__ kkeys = reinterpret_cast<KeyT*>(a.kkeys);
-  while (true) {
-    uint32_t beta = 0;
-    if (lane == 0) beta = atomicAdd(&a.sc->ticket_filter, 1u);
-    beta = __shfl_sync(FULLMASK, beta, 0);
-    if (beta >= (uint32_t)B) break;
+  for (uint32_t beta = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; beta < B; beta += warps) {
     const uint32_t r0 = a.bstart[beta], e = r0 + a.tu[beta];
-    const uint32_t g0 = r0 & ~3u;
-    uint32_t v = 0;
-    if (a.bsmall && cut <= (uint32_t)kSmallCounts) {
-      // kept rows = the bucket's rows minus those counted fewer than cut times
-      uint32_t below = (lane >= 1 && (uint32_t)lane < cut) ? a.bsmall[(size_t)beta * kSmallCounts + lane] : 0u;
-      below = __reduce_add_sync(FULLMASK, below);
-      v = (e - r0) - below;
-    } else {
-      for (uint32_t g = g0; g < e; g += 128) {
-        uint32_t c[4];
-        v += __popc(kept_group(a, g + 4 * lane, r0, e, cut, c));
-      }
-      v = __reduce_add_sync(FULLMASK, v);
-    }
-    if (lane == 0) st_release(&a.flags[beta], kLbAgg | (unsigned long long)v);
-    __syncwarp();
-    unsigned long long K = lookback_exclusive(a.flags, (int)beta, &a.sc->err, a.spin_limit);
-    if (lane == 0) {
-      st_release(&a.flags[beta], kLbIncl | (K + v));
-      if (beta == (uint32_t)B - 1) a.sc->n_kept_rows = K + v;
-    }
-    uint32_t pos = (uint32_t)K;
+    uint32_t pos = a.kstart[beta];
     uint32_t dl0 = 0, dl1 = 0, dl2 = 0;
-    for (uint32_t g = g0; g < e; g += 128) {
+    for (uint32_t g = r0 & ~3u; g < e; g += 128) {
       const uint32_t q = g + 4 * lane;
       uint32_t c[4];
       const uint32_t m = kept_group(a, q, r0, e, cut, c);
@@ -2011,8 +2147,6 @@ __global__ void __launch_bounds__(256) k_filter_kept(FilterArgs a) {
     dl1 = __reduce_add_sync(FULLMASK, dl1);
     dl2 = __reduce_add_sync(FULLMASK, dl2);
     if (lane == 0) {
-      a.kstart[beta] = (uint32_t)K;
-      a.kcount[beta] = v;
       a.ksub[3 * beta + 0] = dl0;
       a.ksub[3 * beta + 1] = dl0 + dl1;
       a.ksub[3 * beta + 2] = dl0 + dl1 + dl2;
@@ -2040,290 +2174,512 @@ __device__ uint32_t upper_bound_rows(const KeyT* __restrict__ kk, uint32_t lo, u
   return lo;
 }
 
-// Per (k-1)-mer bucket: the suffix-side stream (kept rows of table bucket beta, node =
-// x >> 2, extension = last base) and four prefix-side streams (kept rows of the table
-// buckets whose remaining bits continue with beta, node = x & SUCC_MASK, extension =
-// first base f) are each sorted by node key; merged they give the bucket's
-// macro-nodes in key order.  A bucket larger than kMnCap rows is processed in
-// segments split at node-key pivots.
+// Rows of stream st (0: suffix side, 1 + f: prefix side of first base f) of node unit beta,
+// the node keys whose top bbits - x bits are beta: stream 0 is the kept rows of table
+// buckets [beta << x, (beta + 1) << x); stream 1 + f the kept rows whose leading base is f
+// and whose next bits are beta -- whole table buckets when x >= 2, else the half or quarter
+// of one bucket that its next-digit offsets mark.  Contiguous kept rows each.
+__device__ __forceinline__ void mn_extent(const MnArgs& a, uint32_t beta, int st, uint32_t& r0, uint32_t& r1) {
+  const int x = a.xbits;
+  if (st == 0) {
+    const uint32_t b0 = beta << x, b1 = b0 + (1u << x) - 1;
+    r0 = a.kstart[b0];
+    r1 = a.kstart[b1] + a.kcount[b1];
+    return;
+  }
+  const uint32_t lead = (uint32_t)(st - 1) << (a.bbits - 2);
+  if (x >= 2) {
+    const uint32_t b0 = lead | (beta << (x - 2)), b1 = b0 + (1u << (x - 2)) - 1;
+    r0 = a.kstart[b0];
+    r1 = a.kstart[b1] + a.kcount[b1];
+    return;
+  }
+  const int part = 2 - x;  // bits of beta below the bucket's own
+  const uint32_t bp = lead | (beta >> part);
+  const uint32_t d0 = (beta & ((1u << part) - 1u)) << x, d1 = d0 + (1u << x);  // of four digits
+  const uint32_t b0 = a.kstart[bp];
+  r0 = b0 + (d0 ? a.ksub[3 * bp + d0 - 1] : 0u);
+  r1 = b0 + (d1 == 4 ? a.kcount[bp] : a.ksub[3 * bp + d1 - 1]);
+}
+
+// Units of more rows than one segment holds: counted ahead of all others, by the first
+// tickets of the macro-node kernel, so that no other unit waits for a long one.
+__device__ __forceinline__ bool mn_big(uint32_t rows, uint32_t fit) { return rows > fit; }
+__global__ void __launch_bounds__(256) k_mn_big(MnArgs a, uint32_t fit) {
+  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= 1u << (a.bbits - a.xbits)) return;
+  uint32_t rows = 0;
+  for (int st = 0; st < 5; st++) {
+    uint32_t r0, r1;
+    mn_extent(a, u, st, r0, r1);
+    if (r1 <= a.kcap && r0 <= r1) rows += r1 - r0;
+  }
+  if (mn_big(rows, fit)) a.big[atomicAdd(&a.sc->n_big, 1u)] = u;
+}
+
+// Per node unit: the suffix-side stream (node = x >> 2, extension = last base) and four
+// prefix-side streams (node = x & SUCC_MASK, extension = first base) are each sorted by node
+// key; merged they give the unit's macro-nodes in key order.  A unit larger than CAP
+// rows is processed in segments split at node-key pivots.
+//
+// Units whose prefix-side items nearly all find their node on the suffix side are joined by
+// lookup (see below); the others are sorted.  There a counting sort on the bits below the unit's
+// prefix orders item numbers; an item's rank among its bin (two or three items) is its
+// place.  Node heads are ballots, and the thread of a head collects its node's up to eight
+// items and stores the node's three rows whole.
+//
+// Bound: the wait for the units before (without it 8.6M nodes take 0.21 ms and 46M 63-mer
+// nodes 1.5 ms).  Bacterial nodes (8.6M): 0.39 -> 0.23 ms, 46M nodes of 63-mers 6.95 ->
+// 3.54 ms, against sorting every unit, assembling nodes by 4-byte stores into zeroed rows
+// and looking back over single units.
 template <typename KeyT>
-__global__ void __launch_bounds__(kMnThreads, 8) k_macro_nodes(MnArgs a) {
+__global__ void __launch_bounds__(kMnThreads, MnCfg<KeyT>::CTAS) k_macro_nodes(MnArgs a) {
   using SM = MnSmem<KeyT>;
+  constexpr int T = kMnThreads, NW = T / 32, CAP = kMnCap, NCH = CAP / 32, JCH = kMnJoin / 32;
+  static_assert(JCH <= NCH && JCH <= 32, "a joined unit's chunks");
   extern __shared__ __align__(16) unsigned char smem[];
   KeyT* ikey = reinterpret_cast<KeyT*>(smem + SM::off_key);
   uint32_t* icnt = reinterpret_cast<uint32_t*>(smem + SM::off_cnt);
-  uint8_t* itag = reinterpret_cast<uint8_t*>(smem + SM::off_tag);
-  uint16_t* ord = reinterpret_cast<uint16_t*>(smem + SM::off_ord);
-  uint16_t* nid = reinterpret_cast<uint16_t*>(smem + SM::off_nid);
+  // item numbers (low 11 bits) and tags (0-3: suffix by last base, 4-7: prefix by first)
+  uint16_t* binned = reinterpret_cast<uint16_t*>(smem + SM::off_bin);  // in bin order
+  uint16_t* ord = reinterpret_cast<uint16_t*>(smem + SM::off_ord);     // in node order
   __shared__ uint32_t s_warp[33];
-  __shared__ uint32_t s_beta, s_off[6], s_cur[5], s_end[5], s_segend[5], s_beg[5], s_last;
+  __shared__ uint32_t s_off[6], s_cur[5], s_end[5], s_segend[5], s_ncur[5], s_nend[5], s_nbeta, s_ntask;
+  __shared__ uint32_t s_last, s_nodes;
   __shared__ unsigned long long s_NO;
-  // counting-sort bins of a segment: offset (low 16 bits) and fill (high 16 bits)
-  __shared__ uint32_t s_bin[kMnBins];
+  __shared__ uint32_t s_bin[kMnBins];  // offset (low 16 bits) and fill (high 16 bits)
+  __shared__ uint32_t s_head[NCH], s_first[NCH];  // per 32 positions: head ballot, heads before
+  // a joined unit's items whose node has no suffix side
+  __shared__ uint32_t s_extra, s_xcnt[32];
+  __shared__ KeyT s_xkey[32];
+  __shared__ uint8_t s_xf[32];
 
-  const int tid = threadIdx.x;
-  const int Bu = 1 << (a.bbits - 2 * a.level);  // node units
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ubits = a.bbits - a.xbits;
+  const uint32_t Bu = 1u << ubits;  // node units
   const int k = a.k;
   const int nb = 2 * (k - 1);
   const KeyT succ_mask = KeyOps<KeyT>::mask(nb);
   const KeyT KINF = ~(KeyT)0;  // above every (k-1)-mer key
   const KeyT* __restrict__ kk = reinterpret_cast<const KeyT*>(a.kkeys);
   KeyT* __restrict__ nkeys = reinterpret_cast<KeyT*>(a.nkeys);
-  constexpr uint32_t CAP = kMnCap - 16;  // rows per segment before ties
-  // every node key of a unit shares its top pbits bits; the sort bins are the next
+  constexpr uint32_t FIT = kMnFit;  // rows per segment before ties
+  // every node key of a unit shares its top ubits bits; the sort bins are the next
   // (at most kMnBinBits) bits
-  const int pbits = a.bbits - 2 * a.level;
-  const int rbits = nb - pbits > 0 ? nb - pbits : 0;
+  const int rbits = nb - ubits > 0 ? nb - ubits : 0;
   const int dbits = rbits < kMnBinBits ? rbits : kMnBinBits;
   const int bsh = rbits - dbits;
   const uint32_t bmask = (1u << dbits) - 1u;
 
-  // kept rows beyond the kept buffers were not written: nothing to merge (every CTA
-  // reads the same flag, so all of them leave)
-  if (tid == 0) s_beta = (a.sc->err & ERR_BOUNDS) ? 1u : 0u;
-  // merge positions start in range, so even runs that break the sorted-input contract
-  // only ever index the segment arrays
-  for (int i = tid; i < kMnCap; i += kMnThreads) ord[i] = 0;
+  // kept rows beyond the kept buffers, or without a place, were not written: nothing to
+  // merge.  (A wait that runs out in this kernel sets the flag too; the units left are taken
+  // by the CTAs that run.)
+  if (tid == 0) s_nbeta = a.sc->err & (ERR_BOUNDS | ERR_LOOKBACK);
   __syncthreads();
-  if (s_beta) return;
+  if (s_nbeta) return;
+  __syncthreads();
+
+  // the next ticket's unit and extents, by one warp: first the big units' counts, then
+  // every unit in order
+  const uint32_t nbig = a.sc->n_big;
+  auto take_unit = [&]() {
+    uint32_t t = 0;
+    __syncwarp();
+    if (lane == 0) t = atomicAdd(&a.sc->ticket_mn, 1u);
+    t = __shfl_sync(FULLMASK, t, 0);
+    const uint32_t u = t < nbig ? a.big[t] : t - nbig;
+    uint32_t r0 = 0, r1 = 0;
+    if (u < Bu && lane < 5) {
+      mn_extent(a, u, lane, r0, r1);
+      if (r1 > a.kcap || r0 > r1) {  // never read past the kept rows
+        atomicOr(&a.sc->err, ERR_BOUNDS);
+        r0 = r1 = 0;
+      }
+    }
+    if (lane < 5) {
+      s_ncur[lane] = r0;
+      s_nend[lane] = r1;
+    }
+    if (lane == 0) {
+      s_nbeta = u;
+      s_ntask = t < nbig;
+    }
+  };
+  if (warp == NW - 1) take_unit();
+  __syncthreads();
 
   while (true) {
-    __syncthreads();
-    if (tid == 0) s_beta = atomicAdd(&a.sc->ticket_mn, 1u);
-    __syncthreads();
-    const uint32_t beta = s_beta;
-    if (beta >= (uint32_t)Bu) break;
-    if (tid == 0) {
-      if (a.level == 0) {
-        // node bucket = table bucket: suffix stream = the bucket's kept rows, prefix
-        // streams = the part of bucket (f, beta >> 2) whose next two bits are beta & 3
-        s_cur[0] = a.kstart[beta];
-        s_end[0] = a.kstart[beta] + a.kcount[beta];
-        for (int f = 0; f < 4; f++) {
-          const uint32_t bp = ((uint32_t)f << (a.bbits - 2)) | (beta >> 2);
-          const uint32_t d = beta & 3;
-          const uint32_t b0 = a.kstart[bp];
-          s_cur[f + 1] = b0 + (d == 0 ? 0u : a.ksub[3 * bp + d - 1]);
-          s_end[f + 1] = b0 + (d == 3 ? a.kcount[bp] : a.ksub[3 * bp + d]);
-        }
-      } else {
-        // node unit = the node keys whose top bbits - 2 level bits are beta: suffix
-        // stream = table buckets [beta << 2L, (beta + 1) << 2L), prefix stream f =
-        // table buckets (f, beta, any 2L - 2 bits) -- contiguous kept rows each
-        const int L2 = 2 * a.level;
-        const uint32_t s0b = beta << L2, s1b = s0b + (1u << L2) - 1;
-        s_cur[0] = a.kstart[s0b];
-        s_end[0] = a.kstart[s1b] + a.kcount[s1b];
-        for (int f = 0; f < 4; f++) {
-          const uint32_t p0 = ((uint32_t)f << (a.bbits - 2)) | (beta << (L2 - 2));
-          const uint32_t p1 = p0 + (1u << (L2 - 2)) - 1;
-          s_cur[f + 1] = a.kstart[p0];
-          s_end[f + 1] = a.kstart[p1] + a.kcount[p1];
+    const uint32_t beta = s_nbeta;
+    if (beta >= Bu) break;
+    // ---- joined units: almost every node has a suffix side (a k-mer starts with it), and
+    //      the suffix-side stream is those nodes in order.  Each prefix-side item looks its
+    //      node up there, so nothing has to be sorted but the few items whose node has no
+    //      suffix side (up to 32; dead ends of the graph).
+    const uint32_t c0 = s_ncur[0], n0 = s_nend[0] - c0;
+    const uint32_t p1 = s_nend[1] - s_ncur[1], p2 = p1 + s_nend[2] - s_ncur[2], p3 = p2 + s_nend[3] - s_ncur[3],
+                   np = p3 + s_nend[4] - s_ncur[4];
+    if (n0 > 0 && n0 <= (uint32_t)kMnJoin && np <= (uint32_t)kMnJoin) {
+      constexpr int IT = kMnJoin / T;
+      uint32_t* rows = reinterpret_cast<uint32_t*>(smem + SM::off_rows);
+      KeyT* pkey = reinterpret_cast<KeyT*>(smem + SM::off_pkey);
+      uint16_t* start = reinterpret_cast<uint16_t*>(smem + SM::off_start);
+      uint32_t scnt[IT], pcnt[IT], pfirst[IT], sbase = 0;  // sbase: last bases, two bits each
+      KeyT py[IT];
+#pragma unroll
+      for (int q = 0; q < IT; q++) {  // prefix side: node key, count, first base
+        const uint32_t i = q * T + tid;
+        py[q] = 0;
+        pcnt[q] = pfirst[q] = 0;
+        if (i < np) {
+          const int st = (i >= p1) + (i >= p2) + (i >= p3);
+          const uint32_t row = s_ncur[st + 1] + (i - (st == 0 ? 0u : st == 1 ? p1 : st == 2 ? p2 : p3));
+          py[q] = kk[row] & succ_mask;
+          pcnt[q] = a.kcounts[row];
+          pfirst[q] = st;
         }
       }
-      for (int st = 0; st < 5; st++)
-        if (s_end[st] > a.kcap || s_cur[st] > s_end[st]) {  // never read past the kept rows
-          atomicOr(&a.sc->err, ERR_BOUNDS);
-          s_cur[st] = s_end[st] = 0;
+#pragma unroll
+      for (int q = 0; q < IT; q++) {  // suffix side: heads, and the first item of every bin
+        const uint32_t i = q * T + tid;
+        bool head = false;
+        scnt[q] = 0;
+        if (i < n0) {
+          const KeyT x = kk[c0 + i], y = x >> 2;
+          scnt[q] = a.kcounts[c0 + i];
+          sbase |= (uint32_t)(x & 3) << (2 * q);
+          pkey[i] = y;
+          uint32_t b = 0;  // bins below the item's that no item before it is in or above
+          head = i == 0;
+          if (i) {
+            const KeyT z = kk[c0 + i - 1] >> 2;
+            head = !(z == y);
+            b = ((uint32_t)KeyOps<KeyT>::shr(z, bsh) & bmask) + 1;
+          }
+          const uint32_t mine = (uint32_t)KeyOps<KeyT>::shr(y, bsh) & bmask;
+          for (; b <= mine; b++) start[b] = (uint16_t)i;
+          if (i == n0 - 1)
+            for (b = mine + 1; b <= bmask + 1; b++) start[b] = (uint16_t)n0;
         }
+        const unsigned m = __ballot_sync(FULLMASK, head);
+        if (lane == 0) s_head[q * NW + warp] = m;
+      }
+      for (uint32_t i = tid; i < 2 * (n0 + 32); i += T) reinterpret_cast<uint4*>(rows)[i] = make_uint4(0, 0, 0, 0);
+      if (tid == 0) s_extra = 0;
+      __syncthreads();
+      uint32_t at[IT];
+#pragma unroll
+      for (int q = 0; q < IT; q++) {
+        at[q] = n0;
+        if (q * T + tid < np) {
+          const uint32_t b = (uint32_t)KeyOps<KeyT>::shr(py[q], bsh) & bmask;
+          for (uint32_t i = start[b], e = min((uint32_t)start[b + 1], n0); i < e; i++)
+            if (pkey[i] == py[q]) {
+              at[q] = i;
+              break;
+            }
+          if (at[q] == n0) {  // a node of its own
+            const uint32_t x = atomicAdd(&s_extra, 1u);
+            if (x < 32) {
+              s_xkey[x] = py[q];
+              s_xcnt[x] = pcnt[q];
+              s_xf[x] = (uint8_t)pfirst[q];
+            }
+          }
+        }
+      }
+      __syncthreads();
+      const uint32_t E = s_extra;
+      if (E <= 32) {
+        // heads before every 32 suffix items (lane c of each warp holds chunk c)
+        const uint32_t mask = lane < JCH ? s_head[lane] : 0u;
+        uint32_t inc = __popc(mask);
+#pragma unroll
+        for (int o = 1; o < JCH; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(FULLMASK, inc, o);
+          if (lane >= o) inc += y;
+        }
+        const uint32_t heads = __shfl_sync(FULLMASK, inc, JCH - 1);
+        auto heads_to = [&](uint32_t i) {  // heads among suffix items [0, i] (all lanes call it)
+          const uint32_t ch = min(i >> 5, (uint32_t)JCH - 1u);
+          const uint32_t m = __shfl_sync(FULLMASK, mask, ch), to = __shfl_sync(FULLMASK, inc, ch) - __popc(m);
+          return to + __popc(m & ((2u << (i & 31)) - 1u));
+        };
+        // nodes that only prefix-side items name, one item per lane: the first of each key,
+        // the heads below it and its rank among them
+        uint32_t xheads = 0, xrank = 0;
+        unsigned xfirst = 0;
+        KeyT xk = 0;
+        if (E) {
+          const bool have = (uint32_t)lane < E;
+          xk = have ? s_xkey[lane] : KINF;
+          bool dup = false;
+          for (uint32_t j = 0; j < E; j++) {
+            const KeyT o = shfl_key(xk, j);  // every lane takes part
+            dup |= j < (uint32_t)lane && o == xk;
+          }
+          xfirst = __ballot_sync(FULLMASK, have && !dup);
+          for (uint32_t j = 0; j < E; j++) {
+            const KeyT o = shfl_key(xk, j);
+            xrank += ((xfirst >> j) & 1u) != 0 && o < xk ? 1u : 0u;
+          }
+          uint32_t i = 0;
+          if (have) {
+            i = start[(uint32_t)KeyOps<KeyT>::shr(xk, bsh) & bmask];
+            while (i < n0 && pkey[i] < xk) i++;
+          }
+          const uint32_t h = heads_to(i ? i - 1 : 0u);
+          xheads = i ? h : 0u;
+        }
+        const uint32_t nodes = heads + __popc(xfirst);
+        auto place = [&](uint32_t h) {  // node of the head of rank h (all lanes call it)
+          uint32_t n = h;
+          for (uint32_t j = 0; j < E; j++) {
+            const uint32_t o = __shfl_sync(FULLMASK, xheads, j);
+            n += ((xfirst >> j) & 1u) != 0 && o <= h ? 1u : 0u;
+          }
+          return n;
+        };
+        if (warp == 0) {
+          const unsigned long long ex = group_lookback(GroupFlags(a.flags, Bu), beta, nodes,
+                                                       (int)beta != a.withhold_unit, &a.sc->err, a.spin_limit);
+          if (lane == 0) s_NO = ex;
+          if ((uint32_t)lane < E) rows[8 * (xheads + xrank) + 4 + s_xf[lane]] = s_xcnt[lane];
+        }
+        uint32_t node[IT];
+#pragma unroll
+        for (int q = 0; q < IT; q++) {
+          const uint32_t i = q * T + tid;
+          node[q] = place(heads_to(i) - 1u);
+          if (i < n0) rows[8 * node[q] + ((sbase >> (2 * q)) & 3u)] = scnt[q];
+          const uint32_t t = place(heads_to(at[q]) - 1u);
+          if (i < np && at[q] < n0) rows[8 * t + 4 + pfirst[q]] = pcnt[q];
+        }
+        __syncthreads();
+        const unsigned long long q0 = s_NO;
+        if (warp == NW - 1) take_unit();
+        if (q0 + nodes <= a.cap) {
+#pragma unroll
+          for (int q = 0; q < IT; q++) {
+            const uint32_t i = q * T + tid;
+            if (i < n0 && ((s_head[i >> 5] >> (i & 31)) & 1u)) nkeys[q0 + node[q]] = pkey[i];
+          }
+          if (warp == 0 && ((xfirst >> lane) & 1u)) nkeys[q0 + xheads + xrank] = xk;
+          for (uint32_t i = tid; i < 2 * nodes; i += T)
+            reinterpret_cast<uint4*>(i & 1 ? a.npre : a.nsuf)[q0 + (i >> 1)] = reinterpret_cast<const uint4*>(rows)[i];
+        } else if (tid == 0) {
+          atomicOr(&a.sc->err, ERR_MN_CAPACITY);
+        }
+        if (tid == 0 && beta == Bu - 1) a.sc->n_nodes = q0 + nodes;
+        __syncthreads();
+        continue;
+      }
     }
-    if (tid == 0)
-      for (int st = 0; st < 5; st++) s_beg[st] = s_cur[st];
-    __syncthreads();
-    // A bucket that fits one segment is merged, counted and written in one pass.  A
-    // larger one is first merged to count its nodes (so its aggregate is published
-    // before any wait and later buckets do not queue behind it), then merged again
-    // and written.
-    bool counting = false;
-    unsigned long long NO = 0, total = 0;
-    for (int pass = 0; pass < 2; pass++) {
-      bool first = true;
-      unsigned long long done_nodes = 0;
-      while (true) {
-        // ---- choose this segment's rows: everything left, or rows up to a pivot key
-        if (tid == 0) {
-          uint32_t rows = 0;
-          for (int st = 0; st < 5; st++) rows += s_end[st] - s_cur[st];
+    // ---- sorted units, in segments: a count task only counts its nodes (and publishes
+    //      them), a big unit's place is known before its segments are written, and a unit of
+    //      one segment looks for its place once that is counted
+    const bool task = s_ntask != 0;
+    const bool big = mn_big(n0 + np, FIT);
+    if (tid < 5) {
+      s_cur[tid] = s_ncur[tid];
+      s_end[tid] = s_nend[tid];
+    }
+    if (big && !task && warp == 0) {
+      const unsigned long long ex = group_lookback(GroupFlags(a.flags, Bu), beta, ~0ull,
+                                                   (int)beta != a.withhold_unit, &a.sc->err, a.spin_limit);
+      if (lane == 0) s_NO = ex;
+    }
+    unsigned long long NO = 0, done_nodes = 0;
+    while (true) {
+      // ---- choose this segment's rows: everything left, or rows up to a pivot key;
+      //      lane st of warp 0 handles stream st
+      if (warp == 0) {
+        __syncwarp();
+        const uint32_t c0 = lane < 5 ? s_cur[lane] : 0u, c1 = lane < 5 ? s_end[lane] : 0u;
+        const uint32_t rows = __reduce_add_sync(FULLMASK, c1 - c0);
+        uint32_t e = c1;
+        if (rows > FIT) {
           KeyT piv = KINF;
-          if (rows > CAP) {
-            const float frac = 0.9f * (float)CAP / (float)rows;
-            for (int st = 0; st < 5; st++) {
-              const uint32_t take = (uint32_t)((float)(s_end[st] - s_cur[st]) * frac);
-              if (take >= 1) {
-                const KeyT kx = node_key(kk, s_cur[st] + take - 1, st, succ_mask);
-                if (kx < piv) piv = kx;
-              }
-            }
+          const uint32_t take = (uint32_t)((float)(c1 - c0) * (0.9f * (float)FIT / (float)rows));
+          if (take >= 1) piv = node_key(kk, c0 + take - 1, lane, succ_mask);
+          for (int o = 4; o > 0; o >>= 1) {  // the least of lanes 0..4 (the others hold KINF)
+            const KeyT y = shfl_xor_key(piv, o);
+            if (y < piv) piv = y;
           }
-          s_last = 1;
-          for (int st = 0; st < 5; st++) {
-            s_segend[st] = piv == KINF ? s_end[st]
-                                       : upper_bound_rows(kk, s_cur[st], s_end[st], st, succ_mask, piv);
-            if (s_segend[st] != s_end[st]) s_last = 0;
-          }
-          uint32_t o = 0;
-          for (int st = 0; st < 5; st++) {
-            s_off[st] = o;
-            o += s_segend[st] - s_cur[st];
-          }
-          s_off[5] = o;
+          piv = shfl_key(piv, 0);
+          if (lane < 5 && piv != KINF) e = upper_bound_rows(kk, c0, c1, lane, succ_mask, piv);
         }
-        __syncthreads();
-        const bool last = s_last != 0;
-        if (pass == 0 && first && !last) counting = true;
-        uint32_t mm = s_off[5];
-        if (mm > (uint32_t)kMnCap) {  // cannot happen with CAP-sized segments
-          if (tid == 0) atomicOr(&a.sc->err, ERR_MN_CAPACITY);
-          mm = 0;
-        }
-        // ---- gather the five sorted runs
-        for (uint32_t i = tid; i < mm; i += kMnThreads) {
-          int st = 0;
-          while (i >= s_off[st + 1]) st++;
-          const uint32_t row = s_cur[st] + (i - s_off[st]);
-          const KeyT x = kk[row];
-          ikey[i] = st == 0 ? (x >> 2) : (x & succ_mask);
-          itag[i] = (uint8_t)(st == 0 ? (uint32_t)(x & 3) : (uint32_t)(3 + st));
-          icnt[i] = a.kcounts[row];
-        }
-        __syncthreads();
-        // ---- order of the items by node key, ties by run and then position (the stable
-        //      merge of the five runs): a counting sort on the key bits below the unit's
-        //      common prefix, then each item's rank among its bin, which holds a few items.
-        //      A crowded bin falls back to merge ranks across the runs.
-        for (int b = tid; b < kMnBins; b += kMnThreads) s_bin[b] = 0;
-        __syncthreads();
-        for (uint32_t i = tid; i < mm; i += kMnThreads)
-          atomicAdd(&s_bin[(uint32_t)KeyOps<KeyT>::shr(ikey[i], bsh) & bmask], 1u);
-        __syncthreads();
-        {
-          constexpr int BPT = kMnBins / kMnThreads;
-          uint32_t hv[BPT], hs = 0, hm = 0;
+        const unsigned more = __ballot_sync(FULLMASK, e != c1);
+        uint32_t inc = e - c0;
 #pragma unroll
-          for (int q = 0; q < BPT; q++) {
-            hv[q] = s_bin[tid * BPT + q];
-            hs += hv[q];
-            hm = max(hm, hv[q]);
-          }
-          uint32_t tot;
-          uint32_t ex = block_exclusive_sum(hs, s_warp, tot);
-#pragma unroll
-          for (int q = 0; q < BPT; q++) {
-            s_bin[tid * BPT + q] = ex;
-            ex += hv[q];
-          }
-          const bool crowded = __syncthreads_or(hm > (uint32_t)kMnBinMax) != 0;
-          if (!crowded) {
-            uint16_t* binned = nid;  // scratch until the node ids are computed
-            for (uint32_t i = tid; i < mm; i += kMnThreads) {
-              const uint32_t o = atomicAdd(&s_bin[(uint32_t)KeyOps<KeyT>::shr(ikey[i], bsh) & bmask], 1u << 16);
-              binned[(o & 0xffffu) + (o >> 16)] = (uint16_t)i;
-            }
-            __syncthreads();
-            for (uint32_t p = tid; p < mm; p += kMnThreads) {
-              const uint32_t i = binned[p];
-              const KeyT x = ikey[i];
-              const uint32_t o = s_bin[(uint32_t)KeyOps<KeyT>::shr(x, bsh) & bmask];
-              const uint32_t b0 = o & 0xffffu, b1 = b0 + (o >> 16);
-              uint32_t rank = 0;
-              for (uint32_t j = b0; j < b1; j++) {
-                const uint32_t ij = binned[j];
-                const KeyT y = ikey[ij];
-                rank += (y < x || (!(x < y) && ij < i)) ? 1u : 0u;
-              }
-              ord[b0 + rank] = (uint16_t)i;
-            }
-          } else {
-            for (uint32_t i = tid; i < mm; i += kMnThreads) {
-              int st = 0;
-              while (i >= s_off[st + 1]) st++;
-              const KeyT x = ikey[i];
-              uint32_t rank = i - s_off[st];
-              for (int b = 0; b < 5; b++) {
-                if (b == st) continue;
-                const uint32_t lo = s_off[b], hi = s_off[b + 1];
-                rank += (b < st ? upper_bound_s(ikey, lo, hi, x) : lower_bound_s(ikey, lo, hi, x)) - lo;
-              }
-              ord[rank] = (uint16_t)i;
-            }
-          }
+        for (int o = 1; o < 8; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(FULLMASK, inc, o);
+          if (lane >= o) inc += y;
         }
-        __syncthreads();
-        // ---- node boundaries and node index per merged position: each thread takes
-        //      a contiguous run of positions, so one block scan serves the segment
-        uint32_t nodes = 0;
-        {
-          const uint32_t per = (mm + kMnThreads - 1) / kMnThreads;
-          const uint32_t r0 = min(mm, tid * per), r1 = min(mm, r0 + per);
-          uint32_t cnt = 0;
-          for (uint32_t r = r0; r < r1; r++) cnt += (r == 0) || !(ikey[ord[r - 1]] == ikey[ord[r]]);
-          uint32_t tot;
-          uint32_t run = block_exclusive_sum(cnt, s_warp, tot);
-          for (uint32_t r = r0; r < r1; r++) {
-            run += (r == 0) || !(ikey[ord[r - 1]] == ikey[ord[r]]);
-            nid[r] = (uint16_t)(run - 1);
-          }
-          nodes = tot;
+        if (lane < 5) {
+          s_segend[lane] = e;
+          s_off[lane + 1] = inc;
         }
-        __syncthreads();  // nid is read across threads below
-        if (!counting) {
-          // ---- node offset: decoupled look-back over node buckets
-          if (first) {
-            if (tid < 32) {  // warp 0 looks back
-              const unsigned long long mine = pass == 0 ? nodes : total;
-              // a withheld unit (bounded-wait tests) publishes nothing: its successors'
-              // waits run out and report ERR_LOOKBACK
-              const bool publish = (int)beta != a.withhold_unit;
-              if (tid == 0 && publish) st_release(&a.flags[beta], kLbAgg | mine);
-              __syncwarp();
-              const unsigned long long ex = lookback_exclusive(a.flags, (int)beta, &a.sc->err, a.spin_limit);
-              if (tid == 0) {
-                if (publish) st_release(&a.flags[beta], kLbIncl | (ex + mine));
-                s_NO = ex;
-              }
-            }
-            __syncthreads();
-            NO = s_NO;
-          }
-          const unsigned long long q0 = NO + done_nodes;
-          if (q0 + nodes <= a.cap) {
-            for (uint32_t r = tid; r < mm; r += kMnThreads) {
-              if (r == 0 || nid[r] != nid[r - 1]) {
-                const unsigned long long q = q0 + nid[r];
-                nkeys[q] = ikey[ord[r]];
-                reinterpret_cast<uint4*>(a.nsuf)[q] = make_uint4(0, 0, 0, 0);
-                reinterpret_cast<uint4*>(a.npre)[q] = make_uint4(0, 0, 0, 0);
-              }
-            }
-            __syncthreads();
-            for (uint32_t r = tid; r < mm; r += kMnThreads) {
-              const uint32_t i = ord[r];
-              const unsigned long long q = q0 + nid[r];
-              const uint32_t tg = itag[i];
-              if (tg < 4) a.nsuf[4 * q + tg] = icnt[i];
-              else a.npre[4 * q + (tg - 4)] = icnt[i];
-            }
-          } else if (tid == 0) {
-            atomicOr(&a.sc->err, ERR_MN_CAPACITY);
-          }
+        if (lane == 0) {
+          s_off[0] = 0;
+          s_last = more == 0;
         }
-        done_nodes += nodes;
-        first = false;
-        __syncthreads();
-        if (tid == 0)
-          for (int st = 0; st < 5; st++) s_cur[st] = s_segend[st];
-        __syncthreads();
-        if (last) break;
       }
-      total = done_nodes;
-      if (!counting) break;
-      // counted: rewind and write
-      counting = false;
-      if (tid == 0)
-        for (int st = 0; st < 5; st++) s_cur[st] = s_beg[st];
+      for (int b = tid; b < kMnBins; b += T) s_bin[b] = 0;
+      __syncthreads();
+      const bool last = s_last != 0;
+      uint32_t mm = s_off[5];
+      if (mm > (uint32_t)CAP) {  // cannot happen with FIT-sized segments
+        if (tid == 0) atomicOr(&a.sc->err, ERR_MN_CAPACITY);
+        mm = 0;
+      }
+      // ---- gather the five sorted runs, counted by sort bin
+      const uint32_t o1 = s_off[1], o2 = s_off[2], o3 = s_off[3], o4 = s_off[4];
+      for (uint32_t i = tid; i < mm; i += T) {
+        const int st = (i >= o1) + (i >= o2) + (i >= o3) + (i >= o4);
+        const uint32_t row = s_cur[st] + (i - s_off[st]);
+        const KeyT x = kk[row];
+        const KeyT y = st == 0 ? (x >> 2) : (x & succ_mask);
+        ikey[i] = y;
+        icnt[i] = a.kcounts[row];
+        ord[i] = (uint16_t)(i | ((st == 0 ? (uint32_t)(x & 3) : (uint32_t)(3 + st)) << 11));
+        atomicAdd(&s_bin[(uint32_t)KeyOps<KeyT>::shr(y, bsh) & bmask], 1u);
+      }
+      __syncthreads();
+      // ---- order of the items by node key, ties by run and then position (the stable
+      //      merge of the five runs)
+      {
+        constexpr int BPT = (kMnBins + T - 1) / T;
+        uint32_t hv[BPT], hs = 0, hm = 0;
+#pragma unroll
+        for (int q = 0; q < BPT; q++) {
+          const int bi = tid * BPT + q;
+          hv[q] = bi < kMnBins ? s_bin[bi] : 0u;
+          hs += hv[q];
+          hm = max(hm, hv[q]);
+        }
+        uint32_t tot;
+        uint32_t ex = block_exclusive_sum(hs, s_warp, tot);
+#pragma unroll
+        for (int q = 0; q < BPT; q++) {
+          const int bi = tid * BPT + q;
+          if (bi < kMnBins) s_bin[bi] = ex;
+          ex += hv[q];
+        }
+        const bool crowded = __syncthreads_or(hm > (uint32_t)kMnBinMax) != 0;
+        if (!crowded) {
+          for (uint32_t i = tid; i < mm; i += T) {
+            const uint32_t o = atomicAdd(&s_bin[(uint32_t)KeyOps<KeyT>::shr(ikey[i], bsh) & bmask], 1u << 16);
+            binned[(o & 0xffffu) + (o >> 16)] = ord[i];
+          }
+          __syncthreads();
+          for (uint32_t p = tid; p < mm; p += T) {
+            const uint32_t v = binned[p], i = v & 2047u;
+            const KeyT x = ikey[i];
+            const uint32_t o = s_bin[(uint32_t)KeyOps<KeyT>::shr(x, bsh) & bmask];
+            const uint32_t b0 = o & 0xffffu, b1 = b0 + (o >> 16);
+            uint32_t rank = 0;
+            for (uint32_t j = b0; j < b1; j++) {
+              const uint32_t ij = binned[j] & 2047u;
+              const KeyT y = ikey[ij];
+              rank += (y < x || (!(x < y) && ij < i)) ? 1u : 0u;
+            }
+            ord[b0 + rank] = (uint16_t)v;
+          }
+        } else {
+          // a crowded bin: merge ranks across the runs
+          for (uint32_t i = tid; i < mm; i += T) binned[i] = ord[i];
+          __syncthreads();
+          for (uint32_t i = tid; i < mm; i += T) {
+            const int st = (i >= o1) + (i >= o2) + (i >= o3) + (i >= o4);
+            const KeyT x = ikey[i];
+            uint32_t rank = i - s_off[st];
+            for (int b = 0; b < 5; b++) {
+              if (b == st) continue;
+              const uint32_t lo = s_off[b], hi = s_off[b + 1];
+              rank += (b < st ? upper_bound_s(ikey, lo, hi, x) : lower_bound_s(ikey, lo, hi, x)) - lo;
+            }
+            ord[rank] = binned[i];
+          }
+        }
+      }
+      __syncthreads();
+      // ---- node heads: one ballot per 32 positions
+      const uint32_t nch = (mm + 31) / 32;
+      for (uint32_t ch = warp; ch < nch; ch += NW) {
+        const uint32_t r = 32 * ch + lane;
+        bool head = false;
+        if (r < mm) head = r == 0 || !(ikey[ord[r - 1] & 2047u] == ikey[ord[r] & 2047u]);
+        const unsigned m = __ballot_sync(FULLMASK, head);
+        if (lane == 0) s_head[ch] = m;
+      }
+      __syncthreads();
+      if (warp == 0) {  // heads before each 32 positions, and the unit's place
+        uint32_t run = 0;
+        for (uint32_t c0 = 0; c0 < nch; c0 += 32) {
+          const uint32_t n = c0 + lane < nch ? __popc(s_head[c0 + lane]) : 0u;
+          uint32_t inc = n;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULLMASK, inc, o);
+            if (lane >= o) inc += y;
+          }
+          if (c0 + lane < nch) s_first[c0 + lane] = run + inc - n;
+          run += __shfl_sync(FULLMASK, inc, 31);
+        }
+        if (lane == 0) s_nodes = run;
+        if (!big) {
+          // A withheld unit (bounded-wait tests) publishes nothing: its successors' waits
+          // run out and report ERR_LOOKBACK.
+          const unsigned long long ex = group_lookback(GroupFlags(a.flags, Bu), beta, run,
+                                                       (int)beta != a.withhold_unit, &a.sc->err, a.spin_limit);
+          if (lane == 0) s_NO = ex;
+        }
+      }
+      __syncthreads();
+      const uint32_t nodes = s_nodes;
+      // the unit's place is published: the next one is taken while this one is written
+      if (last && warp == NW - 1) take_unit();
+      if (!task) {
+        NO = s_NO;
+        const unsigned long long q0 = NO + done_nodes;
+        if (q0 + nodes <= a.cap) {
+          for (uint32_t ch = warp; ch < nch; ch += NW) {
+            const uint32_t m = s_head[ch];
+            if (!((m >> lane) & 1u)) continue;
+            uint32_t r = 32 * ch + lane;
+            const unsigned long long q = q0 + s_first[ch] + __popc(m & lanemask_lt());
+            uint32_t v = ord[r];
+            nkeys[q] = ikey[v & 2047u];
+            uint32_t c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            do {
+              const uint32_t n = icnt[v & 2047u], tag = v >> 11;
+#pragma unroll
+              for (int e = 0; e < 8; e++)
+                if (tag == (uint32_t)e) c[e] = n;
+              r++;
+              if (r >= mm || ((s_head[r >> 5] >> (r & 31)) & 1u)) break;
+              v = ord[r];
+            } while (true);
+            reinterpret_cast<uint4*>(a.nsuf)[q] = make_uint4(c[0], c[1], c[2], c[3]);
+            reinterpret_cast<uint4*>(a.npre)[q] = make_uint4(c[4], c[5], c[6], c[7]);
+          }
+        } else if (tid == 0) {
+          atomicOr(&a.sc->err, ERR_MN_CAPACITY);
+        }
+      }
+      done_nodes += nodes;
+      __syncthreads();
+      if (last) break;
+      if (tid < 5) s_cur[tid] = s_segend[tid];
       __syncthreads();
     }
-    if (tid == 0 && beta == (uint32_t)Bu - 1) a.sc->n_nodes = NO + total;
+    if (tid == 0) {
+      if (task) {
+        if ((int)beta != a.withhold_unit) group_publish(GroupFlags(a.flags, Bu), beta, done_nodes);
+      } else if (beta == Bu - 1) {
+        a.sc->n_nodes = NO + done_nodes;
+      }
+    }
   }
 }
 
@@ -2420,7 +2776,7 @@ size_t bucket_smem_bytes(int wide) {
 }
 size_t mn_smem_bytes(int wide) { return wide ? MnSmem<u128>::bytes : MnSmem<uint64_t>::bytes; }
 int bucket_ctas_per_sm(int) { return 2; }
-int mn_ctas_per_sm(int wide) { return wide ? 5 : 8; }
+int mn_ctas_per_sm(int wide) { return wide ? MnCfg<u128>::CTAS : MnCfg<uint64_t>::CTAS; }
 
 cudaError_t launch_line_tiles(const uint8_t* buf, unsigned long long F, uint32_t* tile_nl, Scalars* sc,
                               unsigned long long tile0, unsigned long long ntiles, cudaStream_t st) {
@@ -2597,15 +2953,22 @@ cudaError_t launch_cutoff(const unsigned long long* hist, int t, Scalars* sc, cu
   return cudaGetLastError();
 }
 
+size_t mn_flag_words(int bbits) {
+  return (size_t)(1u << bbits) + 2 * (((size_t)(1u << bbits) + 31) / 32);
+}
+
 template <typename KeyT>
-static cudaError_t launch_filter_t(const FilterArgs& a, int grid, cudaStream_t st) {
-  if (grid <= 0) grid = sm_count() * 8;
+static cudaError_t launch_filter_t(const FilterArgs& a, bool count_rows, cudaStream_t st) {
+  const int B = 1 << a.bbits;
+  const int most = sm_count() * 8, grid = std::min((B + 7) / 8, most);
+  if (count_rows) pk::note_launch(), k_kept_count<<<grid, 256, 0, st>>>(a);
+  pk::note_launch(), k_kept_offsets<<<(B + kKeptT - 1) / kKeptT, kKeptT, 0, st>>>(a);
   pk::note_launch(), k_filter_kept<KeyT><<<grid, 256, 0, st>>>(a);
   return cudaGetLastError();
 }
 
-cudaError_t launch_filter_kept(const FilterArgs& a, int wide, int grid, cudaStream_t st) {
-  return wide ? launch_filter_t<u128>(a, grid, st) : launch_filter_t<uint64_t>(a, grid, st);
+cudaError_t launch_filter_kept(const FilterArgs& a, int wide, bool count_rows, cudaStream_t st) {
+  return wide ? launch_filter_t<u128>(a, count_rows, st) : launch_filter_t<uint64_t>(a, count_rows, st);
 }
 
 template <typename KeyT>
@@ -2618,6 +2981,8 @@ static cudaError_t launch_mn_t(const MnArgs& a, int grid, cudaStream_t st) {
     attr_set = true;
   }
   if (grid <= 0) grid = sm_count() * mn_ctas_per_sm(sizeof(KeyT) == 16);
+  const unsigned units = 1u << (a.bbits - a.xbits);
+  pk::note_launch(), k_mn_big<<<(units + 255) / 256, 256, 0, st>>>(a, kMnFit);
   pk::note_launch(), k_macro_nodes<KeyT><<<grid, kMnThreads, smem, st>>>(a);
   return cudaGetLastError();
 }

@@ -76,6 +76,7 @@ struct pk_job {
   uint64_t F = 0, N = 0;
   int t_hist = 0;
   int stage = 0;  // 0 none, 1 counted, 2 cutoff, 3 macro-nodes
+  uint32_t cut_max = 0;  // the last cutoff is at most this (its -t less one)
   uint64_t mn_cap = 0;
   pk::Scalars* d_sc = nullptr;
   pk::Scalars* h_sc = nullptr;  // pinned mirror
