@@ -152,11 +152,10 @@ pk_status presize(pk_job* j, uint64_t fmax, int k, int bbits, int t, int sms) {
   PK_TRY(job_alloc(j, j->kstart, 4 * (size_t)B));
   PK_TRY(job_alloc(j, j->kcount, 4 * (size_t)B));
   PK_TRY(job_alloc(j, j->ksub, 12 * (size_t)B));
-  PK_TRY(job_alloc(j, j->flags_f, 8 * (((size_t)B + 255) / 256)));
   PK_TRY(job_alloc(j, j->nkeys, W * 2 * vcap));
   PK_TRY(job_alloc(j, j->nsuf, 16 * 2 * vcap));
   PK_TRY(job_alloc(j, j->npre, 16 * 2 * vcap));
-  PK_TRY(job_alloc(j, j->flags_m, 8 * mn_flag_words(bbits) + 4 * (size_t)B));
+  PK_TRY(job_alloc(j, j->flags_m, 8 * (((size_t)B + 255) / 256 + mn_flag_words(bbits)) + 4 * (size_t)B));
   PK_TRY(job_alloc(j, j->gfirst, 4 * (size_t)B));
   PK_TRY(job_alloc(j, j->gcount, 4 * (size_t)B));
   PK_TRY(job_alloc(j, j->chunk_bucket, 4 * (fmax / kChunkKeys + 1)));

@@ -3,12 +3,14 @@
 // sequence of the counting -> cutoff -> macro-node path.  No CPU fallback: every
 // result comes from the kernels in pk_kernels.cu.
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
 
 #include <algorithm>
 #include <atomic>
+#include <iterator>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -38,48 +40,98 @@ pk_status pk::set_device(pk_ctx* c) {
   return PK_OK;
 }
 
+// ------------------------------------------------------------ device blocks -----
+static void* cache_take(pk_ctx* c, size_t bytes, size_t* block) {
+  std::lock_guard<std::mutex> lk(c->cache_mu);
+  auto it = c->cache.lower_bound(bytes);
+  if (it == c->cache.end() || it->first > std::max(bytes + bytes / 8, bytes + 65536)) return nullptr;
+  void* p = it->second;
+  *block = it->first;
+  c->cached -= it->first;
+  c->cache.erase(it);
+  return p;
+}
+
+// Frees cached blocks, largest first, until at most `keep` bytes are cached.
+static void cache_trim(pk_ctx* c, uint64_t keep) {
+  std::lock_guard<std::mutex> lk(c->cache_mu);
+  while (!c->cache.empty() && c->cached > keep) {
+    auto it = std::prev(c->cache.end());
+    cudaFree(it->second);  // idle: nothing to wait for
+    c->cached -= it->first;
+    c->cache.erase(it);
+  }
+}
+
+static void cache_put(pk_ctx* c, DevBuf& b) {
+  if (b.p) {
+    c->used -= b.bytes;
+    uint64_t keep = c->cache_limit;
+    if (c->budget) keep = std::min<uint64_t>(keep, c->budget - std::min<uint64_t>(c->budget, c->used.load()));
+    bool room;
+    {
+      std::lock_guard<std::mutex> lk(c->cache_mu);
+      room = c->cached + b.block <= keep;
+      if (room) {
+        c->cache.emplace(b.block, b.p);
+        c->cached += b.block;
+      }
+    }
+    if (!room) cudaFree(b.p);
+  }
+  b = DevBuf{};
+}
+
 pk_status pk::job_alloc(pk_job* j, DevBuf& b, size_t bytes) {
   if (b.p && b.bytes >= bytes) return PK_OK;
   if (j->graph_mode) return fail(PK_ERR_STATE, "batch buffers are smaller than a set needs");
-  if (b.p) {
-    PK_CUDA(cudaFreeAsync(b.p, j->stream));
-    j->ctx->used -= b.bytes;
-    b.p = nullptr;
-    b.bytes = 0;
-  }
+  job_free(j, b);
+  pk_ctx* c = j->ctx;
   if (bytes == 0) bytes = 16;
   bytes = (bytes + 255) & ~(size_t)255;
-  uint64_t now = j->ctx->used.fetch_add(bytes) + bytes;
-  if (j->ctx->budget && now > j->ctx->budget) {
-    j->ctx->used -= bytes;
+  uint64_t now = c->used.fetch_add(bytes) + bytes;
+  if (c->budget && now > c->budget) {
+    c->used -= bytes;
     return fail(PK_ERR_NOMEM, "HBM budget exceeded: need " + std::to_string(bytes) + " more bytes, " +
-                                  std::to_string(now - bytes) + " of " + std::to_string(j->ctx->budget) +
+                                  std::to_string(now - bytes) + " of " + std::to_string(c->budget) +
                                   " in use");
   }
-  cudaError_t e = cudaMallocFromPoolAsync(&b.p, bytes, j->ctx->pool, j->stream);
-  if (e != cudaSuccess) {
-    j->ctx->used -= bytes;
-    b.p = nullptr;
-    return fail(PK_ERR_NOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
+  size_t block = bytes;
+  void* p = cache_take(c, bytes, &block);
+  if (!p) {
+    if (c->budget) cache_trim(c, c->budget - now);  // what is in use and what is kept stay within it
+    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, c->pool, j->stream);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      cache_trim(c, 0);
+      e = cudaMallocFromPoolAsync(&p, bytes, c->pool, j->stream);
+    }
+    if (e != cudaSuccess) {
+      c->used -= bytes;
+      return fail(PK_ERR_NOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
+    }
   }
+  b.p = p;
   b.bytes = bytes;
+  b.block = block;
   return PK_OK;
 }
 
-static void job_free(pk_job* j, DevBuf& b) {
+void pk::job_free(pk_job* j, DevBuf& b) {
   if (b.p) {
     cudaFreeAsync(b.p, j->stream);
     j->ctx->used -= b.bytes;
   }
-  b.p = nullptr;
-  b.bytes = 0;
+  b = DevBuf{};
 }
+
+void pk::job_free_idle(pk_job* j, DevBuf& b) { cache_put(j->ctx, b); }
 
 int pk::job_buffers(pk_job* j, DevBuf** out, int cap) {
   DevBuf* all[] = {&j->fasta, &j->tile_nl, &j->counts, &j->bstart, &j->hstart, &j->keys,  &j->tkeys,
                    &j->tcounts, &j->tu,    &j->flags_m, &j->hist,  &j->hist2,
                    &j->nkeys,  &j->nsuf,   &j->npre,    &j->packed,  &j->doff,  &j->dkeys,
-                   &j->dcounts, &j->flags_f, &j->kkeys, &j->kcounts, &j->kstart, &j->kcount,
+                   &j->dcounts, &j->kkeys, &j->kcounts, &j->kstart, &j->kcount,
                    &j->ksub,  &j->coff,    &j->cstart,  &j->slice_start, &j->fcur, &j->wiring,
                    &j->gfirst, &j->gcount, &j->chunk_bucket, &j->gdone,
                    &j->chunk_u, &j->acc_keys[0], &j->acc_keys[1], &j->acc_counts[0], &j->acc_counts[1],
@@ -92,7 +144,11 @@ int pk::job_buffers(pk_job* j, DevBuf** out, int cap) {
 void pk::job_free_all(pk_job* j) {
   DevBuf* all[64];
   const int n = job_buffers(j, all, 64);
-  for (int i = 0; i < n; i++) job_free(j, *all[i]);
+  const bool idle = cudaStreamSynchronize(j->stream) == cudaSuccess;
+  for (int i = 0; i < n; i++) {
+    if (idle) job_free_idle(j, *all[i]);
+    else job_free(j, *all[i]);
+  }
   j->bsmall_valid = false;
   cp_free(j);
   j->compacted = false;
@@ -181,6 +237,9 @@ pk_status pk_ctx_create(int device, uint64_t budget, pk_ctx** out) {
   uint64_t thr = ~0ull;
   cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &thr);
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
+  size_t mem_free = 0, mem_total = 0;
+  if (cudaMemGetInfo(&mem_free, &mem_total) != cudaSuccess) cudaGetLastError();
+  c->cache_limit = mem_total / 8;
   *out = c;
   return PK_OK;
 }
@@ -189,6 +248,7 @@ void pk_ctx_destroy(pk_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   cudaDeviceSynchronize();
+  cache_trim(c, 0);
   if (c->pool) cudaMemPoolDestroy(c->pool);
   delete c;
 }
@@ -235,7 +295,6 @@ pk_status pk_job_create(pk_ctx* c, void* stream, pk_job** out) {
 void pk_job_destroy(pk_job* j) {
   if (!j) return;
   cudaSetDevice(j->ctx->device);
-  cudaStreamSynchronize(j->stream);
   job_free_all(j);
   cudaStreamSynchronize(j->stream);
   for (int i = 0; i < ST_COUNT_; i++) {
@@ -369,6 +428,9 @@ static int hist_bits(uint64_t F, int k, int wide) {
   return std::min(b, kHistBits);
 }
 
+static const char* kFormatError =
+    "a FASTA record start is not '>' (one '>' header line and one sequence line per record expected)";
+
 static pk_status table_impl(pk_job* j, uint64_t N, int t);
 
 // Stages 1-5: device FASTA -> sorted (k-mer, count) table, resident.
@@ -378,12 +440,14 @@ pk_status pk::count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_pa
   j->wide = k > 32;
   j->F = n;
   j->stage = 0;
+  j->sc_fresh = false;
   j->wired = false;
   j->compacted = false;
   const int W = j->wide ? 16 : 8;
   // automatic digits follow from the window count, which the counting pass takes with hb
-  // digits first (graph mode knows no counts)
-  const bool by_count = !p->bucket_bits && !j->graph_mode;
+  // digits first (graph mode and small runs know no counts)
+  const bool waits = !j->graph_mode && !j->no_wait;
+  const bool by_count = !p->bucket_bits && waits;
   const int bb = p->bucket_bits ? std::min(p->bucket_bits, std::min(kMaxPartitionBits, 2 * k - 2))
                                 : auto_bucket_bits(n, k, j->wide);
   j->bbits = std::max(2, bb);
@@ -445,14 +509,12 @@ pk_status pk::count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_pa
   PK_CUDA(launch_bucket_offsets(a, j->stream));
   mark_end(j, ST_OFFSETS);
   // the key buffer is sized by the exact window count (graph mode: by the bound the
-  // caller sized its buffers for)
-  uint64_t N = j->ncap;
-  if (!j->graph_mode) {
+  // caller sized its buffers for; small runs: no more windows than bytes)
+  uint64_t N = j->graph_mode ? j->ncap : n;
+  if (waits) {
     PK_CUDA(cudaMemcpyAsync(j->h_sc, j->d_sc, sizeof(Scalars), cudaMemcpyDeviceToHost, j->stream));
     PK_CUDA(cudaStreamSynchronize(j->stream));
-    if (j->h_sc->err & ERR_FORMAT)
-      return fail(PK_ERR_FORMAT, "a FASTA record start is not '>' (one '>' header line and one "
-                                 "sequence line per record expected)");
+    if (j->h_sc->err & ERR_FORMAT) return fail(PK_ERR_FORMAT, kFormatError);
     N = j->h_sc->n_windows;
   }
   if (N >= (1ull << 32) - 1)
@@ -649,11 +711,11 @@ pk_status pk_table_load(pk_job* j, const void* keys, const uint32_t* counts, uin
   if (s == PK_OK) s = job_alloc(j, nh, sizeof(unsigned long long) * (size_t)(t ? t : 1));
   if (s == PK_OK) s = job_alloc(j, nx, sizeof(chk));
   const bool on_device = s == PK_OK;
-  auto drop = [&]() {
-    job_free(j, nk);
-    job_free(j, nc);
-    job_free(j, nh);
-    job_free(j, nx);
+  auto drop = [&](bool idle) {
+    for (DevBuf* b : {&nk, &nc, &nh, &nx}) {
+      if (idle) job_free_idle(j, *b);
+      else job_free(j, *b);
+    }
   };
   if (on_device) {
     auto check = [&]() -> pk_status {
@@ -672,11 +734,11 @@ pk_status pk_table_load(pk_job* j, const void* keys, const uint32_t* counts, uin
     };
     s = check();
     if (s != PK_OK) {
-      drop();
+      drop(false);
       return s;
     }
   } else {
-    drop();
+    drop(false);
     if (s != PK_ERR_NOMEM) return s;
     PK_TRY(check_rows_host((const uint64_t*)keys, counts, n, k, chk));
     PK_TRY(load_rule(chk[0]));
@@ -699,7 +761,7 @@ pk_status pk_table_load(pk_job* j, const void* keys, const uint32_t* counts, uin
     std::swap(j->tkeys, nk);
     std::swap(j->tcounts, nc);
     if (t) std::swap(j->hist, nh);
-    drop();
+    drop(true);  // check() waited for the stream
     j->t_hist = t;  // 0: no histogram of this table yet
   } else {
     j->t_hist = 0;
@@ -721,16 +783,22 @@ pk_status pk_table_load(pk_job* j, const void* keys, const uint32_t* counts, uin
   *j->h_sc = init;
   PK_CUDA(cudaMemcpyAsync(j->d_sc, j->h_sc, sizeof(Scalars), cudaMemcpyHostToDevice, j->stream));
   PK_CUDA(cudaStreamSynchronize(j->stream));
+  j->sc_fresh = true;
   j->dense_valid = false;
   j->stage = 1;
   return PK_OK;
 }
 
+// The scalars as the enqueued work leaves them (the stream is idle afterwards unless more
+// was enqueued that does not touch them).
 pk_status pk::sync_scalars(pk_job* j) {
-  PK_CUDA(cudaMemcpyAsync(j->h_sc, j->d_sc, sizeof(Scalars), cudaMemcpyDeviceToHost, j->stream));
-  PK_CUDA(cudaStreamSynchronize(j->stream));
+  if (!j->sc_fresh) {
+    PK_CUDA(cudaMemcpyAsync(j->h_sc, j->d_sc, sizeof(Scalars), cudaMemcpyDeviceToHost, j->stream));
+    PK_CUDA(cudaStreamSynchronize(j->stream));
+    j->sc_fresh = true;
+  }
   const uint32_t err = j->h_sc->err;
-  if (err & ERR_FORMAT) return fail(PK_ERR_FORMAT, "a FASTA record start is not '>'");
+  if (err & ERR_FORMAT) return fail(PK_ERR_FORMAT, kFormatError);
   if (err & ERR_LOOKBACK) return fail(PK_ERR_DEVICE, "a bounded look-back wait expired");
   if (err & ERR_BUCKET) return fail(PK_ERR_DEVICE, "a bucket could not be split to fit on chip");
   if (err & ERR_MN_CAPACITY) return fail(PK_ERR_DEVICE, "a macro-node segment exceeded on-chip capacity");
@@ -794,7 +862,7 @@ pk_status pk_copy_table_packed(pk_job* j, void* pairs, uint64_t cap) {
                               nullptr, j->packed.p, j->stream));
   PK_CUDA(cudaMemcpyAsync(pairs, j->packed.p, rec * u, cudaMemcpyDeviceToHost, j->stream));
   PK_CUDA(cudaStreamSynchronize(j->stream));
-  job_free(j, j->packed);
+  job_free_idle(j, j->packed);
   return PK_OK;
 }
 
@@ -824,6 +892,7 @@ pk_status pk::cutoff_enqueue(pk_job* j, int t) {
     hist = (const unsigned long long*)j->hist2.p;
   }
   j->cut_max = (uint32_t)std::max(1, t - 1);
+  j->sc_fresh = false;
   mark_begin(j, ST_CUTOFF);
   PK_CUDA(launch_cutoff(hist, t, j->d_sc, j->stream));
   mark_end(j, ST_CUTOFF);
@@ -859,21 +928,17 @@ pk_status pk::mn_enqueue(pk_job* j, uint32_t min_count, uint64_t kept_bound) {
   PK_TRY(job_alloc(j, j->kstart, sizeof(uint32_t) * B));
   PK_TRY(job_alloc(j, j->kcount, sizeof(uint32_t) * B));
   PK_TRY(job_alloc(j, j->ksub, sizeof(uint32_t) * 3 * (size_t)B));
-  const size_t fflags = sizeof(unsigned long long) * (((size_t)B + 255) / 256);
-  PK_TRY(job_alloc(j, j->flags_f, fflags));
   PK_TRY(job_alloc(j, j->nkeys, W * cap));
   PK_TRY(job_alloc(j, j->nsuf, 16 * cap));
   PK_TRY(job_alloc(j, j->npre, 16 * cap));
-  // the macro-node kernel's look-back words, and its list of big units behind them
+  // look-back words of the kept offsets and of the macro-node kernel, zeroed together, and
+  // that kernel's list of big units behind them
+  const size_t fflags = sizeof(unsigned long long) * (((size_t)B + 255) / 256);
   const size_t mflags = sizeof(unsigned long long) * mn_flag_words(j->bbits);
-  PK_TRY(job_alloc(j, j->flags_m, mflags + sizeof(uint32_t) * (size_t)B));
-  PK_CUDA(cudaMemsetAsync(j->flags_f.p, 0, fflags, j->stream));
-  PK_CUDA(cudaMemsetAsync(j->flags_m.p, 0, mflags, j->stream));
-  PK_CUDA(cudaMemsetAsync(&j->d_sc->ticket_mn, 0, sizeof(uint32_t), j->stream));
-  PK_CUDA(cudaMemsetAsync(&j->d_sc->ticket_filter, 0, sizeof(uint32_t), j->stream));
-  PK_CUDA(cudaMemsetAsync(&j->d_sc->n_big, 0, sizeof(uint32_t), j->stream));
-  PK_CUDA(cudaMemsetAsync(&j->d_sc->n_nodes, 0, sizeof(unsigned long long), j->stream));
-  PK_CUDA(cudaMemsetAsync(&j->d_sc->n_kept_rows, 0, sizeof(unsigned long long), j->stream));
+  PK_TRY(job_alloc(j, j->flags_m, fflags + mflags + sizeof(uint32_t) * (size_t)B));
+  PK_CUDA(cudaMemsetAsync(j->flags_m.p, 0, fflags + mflags, j->stream));
+  j->sc_fresh = false;
+  PK_CUDA(cudaMemsetAsync(&j->d_sc->mn_begin, 0, offsetof(Scalars, mn_end) - offsetof(Scalars, mn_begin), j->stream));
   if (min_count) PK_CUDA(cudaMemcpyAsync(&j->d_sc->cutoff, &min_count, sizeof(uint32_t), cudaMemcpyHostToDevice, j->stream));
   j->mn_cap = cap;
   FilterArgs f{};
@@ -881,7 +946,7 @@ pk_status pk::mn_enqueue(pk_job* j, uint32_t min_count, uint64_t kept_bound) {
   f.tcounts = (const uint32_t*)j->tcounts.p;
   f.bstart = (const uint32_t*)j->bstart.p;
   f.tu = (const uint32_t*)j->tu.p;
-  f.flags = (unsigned long long*)j->flags_f.p;
+  f.flags = (unsigned long long*)j->flags_m.p;
   f.kkeys = j->kkeys.p;
   f.kcounts = (uint32_t*)j->kcounts.p;
   f.kstart = (uint32_t*)j->kstart.p;
@@ -904,8 +969,8 @@ pk_status pk::mn_enqueue(pk_job* j, uint32_t min_count, uint64_t kept_bound) {
   m.kstart = (const uint32_t*)j->kstart.p;
   m.kcount = (const uint32_t*)j->kcount.p;
   m.ksub = (const uint32_t*)j->ksub.p;
-  m.flags = (unsigned long long*)j->flags_m.p;
-  m.big = (uint32_t*)((char*)j->flags_m.p + mflags);
+  m.flags = (unsigned long long*)((char*)j->flags_m.p + fflags);
+  m.big = (uint32_t*)((char*)j->flags_m.p + fflags + mflags);
   m.nkeys = j->nkeys.p;
   m.nsuf = (uint32_t*)j->nsuf.p;
   m.npre = (uint32_t*)j->npre.p;
@@ -1019,26 +1084,51 @@ pk_status pk_summary_get(pk_job* j, pk_summary* o) {
   return PK_OK;
 }
 
+static pk_status empty_after_cutoff(pk_job* j) {
+  return fail(PK_ERR_EMPTY, "no k-mer reaches the cutoff " + std::to_string(j->h_sc->cutoff) +
+                                "; macro-node construction cannot proceed");
+}
+
 static pk_status run_rest(pk_job* j, const pk_params* p, pk_summary* out) {
   PK_TRY(cutoff_enqueue(j, p->num_buckets));
-  PK_TRY(sync_scalars(j));
-  if (j->h_sc->n_kept == 0) {
-    if (out) pk_summary_get(j, out);
-    return fail(PK_ERR_EMPTY, "no k-mer reaches the cutoff " + std::to_string(j->h_sc->cutoff) +
-                                  "; macro-node construction cannot proceed");
+  uint64_t kept = j->N;  // small runs: no more kept k-mers than windows
+  if (!j->no_wait) {
+    PK_TRY(sync_scalars(j));
+    kept = j->h_sc->n_kept;
+    if (kept == 0) {
+      if (out) pk_summary_get(j, out);
+      return empty_after_cutoff(j);
+    }
   }
-  PK_TRY(mn_enqueue(j, 0, j->h_sc->n_kept));
-  if (out) return pk_summary_get(j, out);
-  return sync_scalars(j);
+  PK_TRY(mn_enqueue(j, 0, kept));
+  const pk_status s = sync_scalars(j);
+  if (s == PK_ERR_FORMAT && j->no_wait) j->stage = 0;  // as when the count is waited for
+  PK_TRY(s);
+  if (j->no_wait && j->h_sc->n_kept == 0) {
+    j->stage = 2;
+    if (out) pk_summary_get(j, out);
+    return empty_after_cutoff(j);
+  }
+  return out ? pk_summary_get(j, out) : PK_OK;
+}
+
+// The whole path.  Small inputs (whose buffers are small at their bounds too) run without
+// waiting for the window count and the kept count in between: a wait is 10 us of the 150 or
+// so that they take.  Not with a budget, which counts exact sizes.
+constexpr uint64_t kSmallRun = 1ull << 20;
+static pk_status run_all(pk_job* j, const void* fasta, uint64_t n, const pk_params* p, pk_summary* out, bool host) {
+  if (!j) return fail(PK_ERR_INVALID, "job is null");
+  j->no_wait = p && n <= kSmallRun && p->chunking != 1 && j->ctx->budget == 0;
+  pk_status s = host ? pk_count(j, (const char*)fasta, n, p) : pk_count_device(j, fasta, n, p);
+  if (s == PK_OK) s = run_rest(j, p, out);
+  j->no_wait = false;
+  return s;
 }
 
 pk_status pk_run(pk_job* j, const char* fasta, uint64_t n, const pk_params* p, pk_summary* out) {
-  PK_TRY(pk_count(j, fasta, n, p));
-  return run_rest(j, p, out);
+  return run_all(j, fasta, n, p, out, true);
 }
 
 pk_status pk_run_device(pk_job* j, const void* d_fasta, uint64_t n, const pk_params* p, pk_summary* out) {
-  PK_TRY(pk_count_device(j, d_fasta, n, p));
-  return run_rest(j, p, out);
+  return run_all(j, d_fasta, n, p, out, false);
 }
-

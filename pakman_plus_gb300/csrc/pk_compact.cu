@@ -1103,10 +1103,7 @@ pk_status cp_grow(pk_job* j, DevBuf& b, size_t bytes, size_t keep) {
   DevBuf nb;
   PK_TRY(job_alloc(j, nb, bytes));
   if (keep && b.p) PK_CUDA(cudaMemcpyAsync(nb.p, b.p, keep, cudaMemcpyDeviceToDevice, j->stream));
-  if (b.p) {
-    cudaFreeAsync(b.p, j->stream);
-    j->ctx->used -= b.bytes;
-  }
+  job_free(j, b);
   b = nb;
   return PK_OK;
 }
@@ -1363,25 +1360,19 @@ pk_status cp_walk(pk_job* j, CpState& c) {
 void pk::cp_free(pk_job* j) {
   CpState* c = j->cp;
   if (!c) return;
+  const bool idle = cudaStreamSynchronize(j->stream) == cudaSuccess;
+  auto drop = [&](DevBuf& d) {
+    if (idle) job_free_idle(j, d);
+    else job_free(j, d);
+  };
   for (int s = 0; s < 2; s++)
-    for (int b = 0; b < CpState::NSIDE; b++) {
-      DevBuf& d = c->side[s][b];
-      if (d.p) {
-        cudaFreeAsync(d.p, j->stream);
-        j->ctx->used -= d.bytes;
-      }
-    }
+    for (int b = 0; b < CpState::NSIDE; b++) drop(c->side[s][b]);
   DevBuf* rest[] = {&c->arena,  &c->col,      &c->off,    &c->part,   &c->is_id,  &c->tkey,
                     &c->tr,     &c->tgt,      &c->incnt,  &c->inoff,  &c->fill,   &c->inlist,
                     &c->ecol,   &c->eoff2,    &c->old_of, &c->ct,     &c->tot,    &c->epos,
                     &c->cpos,   &c->ubuf,     &c->wk_begins, &c->wk_resume, &c->wk_path, &c->wk_col,
                     &c->wk_pos, &c->wk_off, &c->wk_out, &c->wk_links, &c->wk_steps, &c->wk_pieces};
-  for (DevBuf* d : rest)
-    if (d->p) {
-      cudaFreeAsync(d->p, j->stream);
-      j->ctx->used -= d->bytes;
-    }
-  cudaStreamSynchronize(j->stream);
+  for (DevBuf* d : rest) drop(*d);
   if (c->d_err) cudaFree(c->d_err);
   if (c->h_tot) cudaFreeHost(c->h_tot);
   delete c;

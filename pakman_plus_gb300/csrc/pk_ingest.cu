@@ -168,6 +168,7 @@ pk_status stream_and_count(pk_job* j, Fd& f, const char* path, uint64_t off, uin
   memset(&init, 0, sizeof(init));
   init.s0 = ~0ull;
   *j->h_sc = init;
+  j->sc_fresh = false;
   PK_CUDA(cudaMemcpyAsync(j->d_sc, j->h_sc, sizeof(Scalars), cudaMemcpyHostToDevice, j->stream));
 
   mark_begin(j, ST_H2D);

@@ -61,17 +61,20 @@ struct Scalars {                    // device-side scalars of one job
   uint32_t nl_before_s0;            // newlines in [0, s0)
   uint32_t err;                     // ERR_* bits
   uint32_t ticket_bucket;           // work tickets
-  uint32_t ticket_mn;
   uint32_t cutoff;                  // histogram cutoff
-  uint32_t ticket_filter;
   uint32_t ticket_fine;
   uint32_t ticket_fcount;
   uint32_t n_chunk_items;           // chunk items of giant buckets (table kernel)
-  uint32_t n_big;                   // macro-node units of more than one segment
   unsigned long long n_unique;      // U
   unsigned long long n_kept;        // V
+  // zeroed together before macro-nodes are built
+  unsigned long long mn_begin[0];
   unsigned long long n_nodes;       // M
-  unsigned long long n_kept_rows;   // V as counted by the filter
+  unsigned long long n_kept_rows;   // V as counted by the kept offsets
+  uint32_t ticket_mn;
+  uint32_t ticket_filter;
+  uint32_t n_big;                   // macro-node units of more than one segment
+  uint32_t mn_end[0];
 };
 
 struct CountArgs {

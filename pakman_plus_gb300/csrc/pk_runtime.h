@@ -7,6 +7,8 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <map>
+#include <mutex>
 #include <string>
 
 #include "../../include/pakman_gb300.h"
@@ -33,11 +35,20 @@ struct pk_ctx {
   std::atomic<uint64_t> used{0};
   cudaMemPool_t pool = nullptr;
   int sms = 0;
+  // Idle device blocks (no work in flight uses them) for the next job's buffers: an
+  // allocation from the pool takes 0.1 ms and more in a process with dozens of streams, and
+  // a job takes about thirty.  At most cache_limit bytes, and with a budget no more than it
+  // leaves; given back when an allocation fails and with the context.
+  std::mutex cache_mu;
+  std::multimap<size_t, void*> cache;
+  uint64_t cached = 0;
+  uint64_t cache_limit = 0;
 };
 
 struct DevBuf {
   void* p = nullptr;
-  size_t bytes = 0;
+  size_t bytes = 0;  // usable and charged to the budget
+  size_t block = 0;  // of the device block (at most an eighth or 64 KB more)
 };
 
 enum Stage {
@@ -77,11 +88,14 @@ struct pk_job {
   int t_hist = 0;
   int stage = 0;  // 0 none, 1 counted, 2 cutoff, 3 macro-nodes
   uint32_t cut_max = 0;  // the last cutoff is at most this (its -t less one)
+  bool sc_fresh = false; // h_sc is d_sc as the enqueued work leaves it, and the stream is idle
+  // pk_run of a small input: buffers sized by bounds instead of counts read back in between
+  bool no_wait = false;
   uint64_t mn_cap = 0;
   pk::Scalars* d_sc = nullptr;
   pk::Scalars* h_sc = nullptr;  // pinned mirror
   DevBuf fasta, tile_nl, counts, bstart, hstart, keys, tkeys, tcounts, tu, flags_m, hist, hist2,
-      nkeys, nsuf, npre, packed, doff, dkeys, dcounts, flags_f, kkeys, kcounts, kstart, kcount, ksub,
+      nkeys, nsuf, npre, packed, doff, dkeys, dcounts, kkeys, kcounts, kstart, kcount, ksub,
       coff, cstart, slice_start, fcur, wiring, gfirst, gcount, chunk_bucket, gdone, chunk_u,
       units,   // packed units of the counting pass, rolled again by the coarse scatter
       bsmall;  // rows of each table bucket by count below kSmallCounts (the table kernel's)
@@ -120,7 +134,10 @@ struct pk_job {
 namespace pk {
 pk_status set_device(pk_ctx* c);
 pk_status job_alloc(pk_job* j, DevBuf& b, size_t bytes);
-void job_free_all(pk_job* j);
+// releases a buffer that the stream may still use (stream-ordered), or one that is idle
+void job_free(pk_job* j, DevBuf& b);
+void job_free_idle(pk_job* j, DevBuf& b);
+void job_free_all(pk_job* j);  // waits for the job's stream
 void cp_free(pk_job* j);  // the compaction state, if any
 pk_status check_params(const pk_params* p);
 int auto_bucket_bits(uint64_t F, int k, int wide);
