@@ -284,8 +284,57 @@ __device__ void block_or_and(KeyT& x_or, KeyT& x_and, KeyT* s_red) {
   __syncthreads();
 }
 
+// Four input bytes: their 2-bit codes (byte 0 in the top bits of the low byte), a mask of
+// the bytes equal to a character (bit 7 of each), and such a mask as four bits.
+__device__ __forceinline__ uint32_t pack4_codes(uint32_t w) {
+  return ((w >> 1) & 0x03030303u) * 0x40100401u;  // in the top byte
+}
+__device__ __forceinline__ uint32_t zero_bytes(uint32_t x) {
+  return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);
+}
+__device__ __forceinline__ uint32_t flags4(uint32_t m) {  // bits 7, 15, 23, 31 -> 0..3
+  return ((m >> 7) * 0x01020408u) >> 24;
+}
+// a 16-byte unit's four words of such masks as 16 bits
+__device__ __forceinline__ uint32_t flags16(uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+  return flags4(m0) | (flags4(m1) << 4) | (flags4(m2) << 8) | (flags4(m3) << 12);
+}
+// base j's code at bits 2(15-j)+1..2(15-j)
+__device__ __forceinline__ uint32_t unit_codes(const uint32_t w[4]) {
+  const uint32_t hi = __byte_perm(pack4_codes(w[1]), pack4_codes(w[0]), 0x7300);
+  const uint32_t lo = __byte_perm(pack4_codes(w[3]), pack4_codes(w[2]), 0x0073);
+  return (hi & 0xffff0000u) | (lo & 0xffffu);
+}
+// byte flags (bit j) of a unit as its bit-2 plane: byte j at bit 2(15-j)
+__device__ __forceinline__ uint32_t unit_plane(uint32_t flags) {
+  uint32_t x = __brev(flags) >> 16;
+  x = (x | (x << 8)) & 0x00ff00ffu;
+  x = (x | (x << 4)) & 0x0f0f0f0fu;
+  x = (x | (x << 2)) & 0x33333333u;
+  return (x | (x << 1)) & 0x55555555u;
+}
+
+__device__ __forceinline__ void load_unit(const uint8_t* __restrict__ buf, unsigned long long F,
+                                          unsigned long long p, uint32_t w[4]) {
+  if (p + 16 <= F) {
+    uint4 v = __ldg(reinterpret_cast<const uint4*>(buf + p));
+    w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      uint32_t x = 0;
+      for (int b = 0; b < 4; b++) {
+        unsigned long long q = p + 4 * i + b;
+        if (q < F) x |= (uint32_t)buf[q] << (8 * b);
+      }
+      w[i] = x;
+    }
+  }
+}
+
 // ------------------------------------------------------------- line scan (k_line_scan) -
-// Newlines per 64 KB tile, the first '>' and the number of '>' bytes.
+// Newlines per 64 KB tile, the first '>' and the number of '>' bytes.  Bound: the read;
+// 407 MB in 95 us (4.3 TB/s) with four loads in flight a thread, 127 us with one.
 __global__ void __launch_bounds__(256) k_line_scan(const uint8_t* __restrict__ buf,
                                                    unsigned long long F, uint32_t* tile_nl,
                                                    Scalars* sc, unsigned long long tile0) {
@@ -294,28 +343,38 @@ __global__ void __launch_bounds__(256) k_line_scan(const uint8_t* __restrict__ b
   const unsigned long long t1 = min(t0 + (unsigned long long)kTileBytes, F);
   uint32_t nl = 0, gt = 0;
   unsigned long long first = ~0ull;
-  for (unsigned long long p = t0 + 16ull * threadIdx.x; p < t1; p += 16ull * blockDim.x) {
-    uint32_t w[4];
-    if (p + 16 <= F) {
-      uint4 v = __ldg(reinterpret_cast<const uint4*>(buf + p));
-      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    } else {
-      for (int i = 0; i < 4; i++) {
-        uint32_t x = 0;
-        for (int b = 0; b < 4; b++) {
-          unsigned long long q = p + 4 * i + b;
-          if (q < F) x |= (uint32_t)buf[q] << (8 * b);
-        }
-        w[i] = x;
-      }
-    }
+  auto scan = [&](const uint32_t w[4], unsigned long long p) {
+    uint32_t g[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      nl += __popc(__vcmpeq4(w[i], 0x0A0A0A0Au)) >> 3;
-      uint32_t g = __vcmpeq4(w[i], 0x3E3E3E3Eu);
-      // a zero byte past F never compares equal to '>'
-      gt += __popc(g) >> 3;
-      if (g && first == ~0ull) first = p + 4 * i + (__ffs(g) - 1) / 8;
+      nl += __popc(zero_bytes(w[i] ^ 0x0A0A0A0Au));
+      g[i] = zero_bytes(w[i] ^ 0x3E3E3E3Eu);
+      gt += __popc(g[i]);
+    }
+    if (first == ~0ull && (g[0] | g[1] | g[2] | g[3])) {
+#pragma unroll
+      for (int i = 3; i >= 0; i--)
+        if (g[i]) first = p + 4 * i + (__ffs(g[i]) - 1) / 8;
+    }
+  };
+  if (t1 - t0 == kTileBytes) {  // whole tiles: four 16-byte loads in flight a thread
+    const uint4* __restrict__ v = reinterpret_cast<const uint4*>(buf + t0) + threadIdx.x;
+#pragma unroll 1
+    for (int o = 0; o < kTileBytes / 16; o += 1024) {
+      uint4 x[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) x[q] = __ldg(v + o + 256 * q);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const uint32_t w[4] = {x[q].x, x[q].y, x[q].z, x[q].w};
+        scan(w, t0 + 16ull * (o + 256 * q + threadIdx.x));
+      }
+    }
+  } else {
+    for (unsigned long long p = t0 + 16ull * threadIdx.x; p < t1; p += 16ull * blockDim.x) {
+      uint32_t w[4];
+      load_unit(buf, F, p, w);  // a zero byte past F is neither '\n' nor '>'
+      scan(w, p);
     }
   }
   __shared__ uint32_t s_nl[8], s_gt[8];
@@ -371,54 +430,6 @@ __global__ void __launch_bounds__(1024) k_tile_prefix(const uint8_t* __restrict_
 }
 
 // --------------------------------------------------------- k-mer window extraction --
-// Four input bytes: their 2-bit codes (byte 0 in the top bits of the low byte), a mask of
-// the bytes equal to a character (bit 7 of each), and such a mask as four bits.
-__device__ __forceinline__ uint32_t pack4_codes(uint32_t w) {
-  return ((w >> 1) & 0x03030303u) * 0x40100401u;  // in the top byte
-}
-__device__ __forceinline__ uint32_t zero_bytes(uint32_t x) {
-  return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);
-}
-__device__ __forceinline__ uint32_t flags4(uint32_t m) {  // bits 7, 15, 23, 31 -> 0..3
-  return ((m >> 7) * 0x01020408u) >> 24;
-}
-// a 16-byte unit's four words of such masks as 16 bits
-__device__ __forceinline__ uint32_t flags16(uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
-  return flags4(m0) | (flags4(m1) << 4) | (flags4(m2) << 8) | (flags4(m3) << 12);
-}
-// base j's code at bits 2(15-j)+1..2(15-j)
-__device__ __forceinline__ uint32_t unit_codes(const uint32_t w[4]) {
-  const uint32_t hi = __byte_perm(pack4_codes(w[1]), pack4_codes(w[0]), 0x7300);
-  const uint32_t lo = __byte_perm(pack4_codes(w[3]), pack4_codes(w[2]), 0x0073);
-  return (hi & 0xffff0000u) | (lo & 0xffffu);
-}
-// byte flags (bit j) of a unit as its bit-2 plane: byte j at bit 2(15-j)
-__device__ __forceinline__ uint32_t unit_plane(uint32_t flags) {
-  uint32_t x = __brev(flags) >> 16;
-  x = (x | (x << 8)) & 0x00ff00ffu;
-  x = (x | (x << 4)) & 0x0f0f0f0fu;
-  x = (x | (x << 2)) & 0x33333333u;
-  return (x | (x << 1)) & 0x55555555u;
-}
-
-__device__ __forceinline__ void load_unit(const uint8_t* __restrict__ buf, unsigned long long F,
-                                          unsigned long long p, uint32_t w[4]) {
-  if (p + 16 <= F) {
-    uint4 v = __ldg(reinterpret_cast<const uint4*>(buf + p));
-    w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      uint32_t x = 0;
-      for (int b = 0; b < 4; b++) {
-        unsigned long long q = p + 4 * i + b;
-        if (q < F) x |= (uint32_t)buf[q] << (8 * b);
-      }
-      w[i] = x;
-    }
-  }
-}
-
 // What a window of the next segment needs of this one: its units' codes with the bit-2
 // plane folded in (kmer_shift ORs a byte's code bit 2 into the base before it) and the
 // bytes no window may hold.
@@ -890,10 +901,13 @@ __global__ void __launch_bounds__(256) k_coarse_offsets(const uint32_t* __restri
 }
 
 // Pass 2 (k_scatter_fine): a slice of a coarse region (in chunk order) is counted by
-// fine bucket in shared memory; one atomic per (slice, fine bucket) reserves a run in
-// the bucket's region and every key goes to its run at a shared-memory-atomic rank.
-// Keys stay in registers, so the CTA needs only three small tables and many CTAs fit
-// an SM to hide the load latency.
+// fine bucket in shared memory, which also gives every key its rank in its bucket; one
+// atomic per (slice, fine bucket) reserves a run in the bucket's region; the slice is staged
+// by bucket and stored in runs.  Keys stay in registers between the two.  Bound: latency
+// between its barriers, at 63 to 66 % of the copy bandwidth.  Bacterial reads (254M keys):
+// 1.02 -> 0.91 ms against a second atomic per key for its rank and a binary search in
+// global memory for every slice's region.  One CTA of 1024 threads an SM: 0.98 ms; the next
+// slice's ticket taken ahead: no change.
 template <typename KeyT>
 struct FineCfg {
   static constexpr int T = 512;                             // threads
@@ -913,36 +927,46 @@ __global__ void __launch_bounds__(512, 2) k_scatter_fine(const KeyT* __restrict_
   using FC = FineCfg<KeyT>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   KeyT* stage = reinterpret_cast<KeyT*>(smem_raw);  // the slice grouped by fine bucket
-  __shared__ uint32_t s_hist[FC::FBMAX], s_loff[FC::FBMAX], s_goff[FC::FBMAX], s_fill[FC::FBMAX];
+  // per fine bucket: keys, first staged key, and what takes a staged position to its place
+  __shared__ uint32_t s_hist[FC::FBMAX], s_loff[FC::FBMAX], s_move[FC::FBMAX];
   __shared__ uint32_t s_warp[33];
   __shared__ uint32_t s_slice, s_g;
+  // the region tables live in shared memory: a slice finds its region with one read a lane
+  __shared__ uint32_t s_ss[(1 << kCoarseBits) + 1], s_cs[(1 << kCoarseBits) + 1];
   const int tid = threadIdx.x;
   const int Cn = 1 << cbits, fb = bbits - cbits, FB = 1 << fb;
   const int fshift = 2 * k - bbits;
+  const uint32_t fmask = (uint32_t)(FB - 1);
+  for (int i = tid; i <= Cn; i += FC::T) {
+    s_ss[i] = slice_start[i];
+    s_cs[i] = cstart[i];
+  }
+  for (int i = tid; i < FB; i += FC::T) s_hist[i] = 0;
   const uint32_t nslices = slice_start[Cn];
   while (true) {
     __syncthreads();
-    if (tid == 0) {
-      s_slice = atomicAdd(ticket, 1u);
-      if (s_slice < nslices) {
-        int lo = 0, hi = Cn - 1;  // last g with slice_start[g] <= slice
-        while (lo < hi) {
-          int mid = (lo + hi + 1) >> 1;
-          if (slice_start[mid] <= s_slice) lo = mid; else hi = mid - 1;
-        }
-        s_g = lo;
+    if (tid < 32) {
+      uint32_t sl = 0;
+      if (tid == 0) sl = atomicAdd(ticket, 1u);
+      sl = __shfl_sync(FULLMASK, sl, 0);
+      uint32_t below = 0;  // regions that start at or before the slice
+      for (int i = tid; i < Cn; i += 32) below += s_ss[i] <= sl ? 1u : 0u;
+      below = __reduce_add_sync(FULLMASK, below);
+      if (tid == 0) {
+        s_slice = sl;
+        s_g = below - 1;
       }
     }
-    for (int i = tid; i < FB; i += FC::T) { s_hist[i] = 0; s_fill[i] = 0; }
     __syncthreads();
     const uint32_t sl = s_slice;
     if (sl >= nslices) break;
     const uint32_t g = s_g;
-    const uint32_t r0 = cstart[g] + (sl - slice_start[g]) * FC::S;
-    const uint32_t r1 = min(r0 + (uint32_t)FC::S, cstart[g + 1]);
+    const uint32_t r0 = s_cs[g] + (sl - s_ss[g]) * FC::S;
+    const uint32_t r1 = min(r0 + (uint32_t)FC::S, s_cs[g + 1]);
     const uint32_t m = r1 - r0;
     KeyT xs[FC::PT];
-    uint32_t fs[FC::PT];
+    uint32_t rank[FC::PT / 2];  // a key's rank in its fine bucket, two to a word (a slice has
+                                // at most 8192 keys)
 #pragma unroll
     for (int q = 0; q < FC::PT; q++) {
       const uint32_t i = q * FC::T + tid;
@@ -951,8 +975,10 @@ __global__ void __launch_bounds__(512, 2) k_scatter_fine(const KeyT* __restrict_
 #pragma unroll
     for (int q = 0; q < FC::PT; q++) {
       const uint32_t i = q * FC::T + tid;
-      fs[q] = (uint32_t)(xs[q] >> fshift) & (uint32_t)(FB - 1);
-      if (i < m) atomicAdd(&s_hist[fs[q]], 1u);
+      uint32_t r = 0;
+      if (i < m) r = atomicAdd(&s_hist[(uint32_t)(xs[q] >> fshift) & fmask], 1u);
+      if (q & 1) rank[q / 2] |= r << 16;
+      else rank[q / 2] = r;
     }
     __syncthreads();
     {
@@ -963,7 +989,11 @@ __global__ void __launch_bounds__(512, 2) k_scatter_fine(const KeyT* __restrict_
       uint32_t hv[FPT], sum = 0;
 #pragma unroll
       for (int q = 0; q < FPT; q++) {
-        hv[q] = (q < per && f0 + q < FB) ? s_hist[f0 + q] : 0u;
+        hv[q] = 0u;
+        if (q < per && f0 + q < FB) {
+          hv[q] = s_hist[f0 + q];
+          s_hist[f0 + q] = 0;  // for the next slice
+        }
         sum += hv[q];
       }
       uint32_t tot;
@@ -972,7 +1002,7 @@ __global__ void __launch_bounds__(512, 2) k_scatter_fine(const KeyT* __restrict_
       for (int q = 0; q < FPT; q++) {
         if (q < per && f0 + q < FB) {
           s_loff[f0 + q] = ex;
-          s_goff[f0 + q] = hv[q] ? atomicAdd(&fcur[(g << fb) + f0 + q], hv[q]) : 0u;
+          s_move[f0 + q] = hv[q] ? atomicAdd(&fcur[(g << fb) + f0 + q], hv[q]) - ex : 0u;
           ex += hv[q];
         }
       }
@@ -981,14 +1011,16 @@ __global__ void __launch_bounds__(512, 2) k_scatter_fine(const KeyT* __restrict_
 #pragma unroll
     for (int q = 0; q < FC::PT; q++) {
       const uint32_t i = q * FC::T + tid;
-      if (i < m) stage[s_loff[fs[q]] + atomicAdd(&s_fill[fs[q]], 1u)] = xs[q];
+      if (i < m) {
+        const uint32_t r = (q & 1) ? rank[q / 2] >> 16 : rank[q / 2] & 0xffffu;
+        stage[s_loff[(uint32_t)(xs[q] >> fshift) & fmask] + r] = xs[q];
+      }
     }
     __syncthreads();
     // runs of one fine bucket are contiguous in `stage` and in `out`: coalesced stores
     for (uint32_t i = tid; i < m; i += FC::T) {
       const KeyT x = stage[i];
-      const uint32_t f = (uint32_t)(x >> fshift) & (uint32_t)(FB - 1);
-      guarded_store(out, s_goff[f] + (i - s_loff[f]), x, cap, err);
+      guarded_store(out, s_move[(uint32_t)(x >> fshift) & fmask] + i, x, cap, err);
     }
   }
 }
@@ -1116,7 +1148,8 @@ int fine_slice_keys(int wide, int fb) {
 
 // Fine bucket sizes when the partition has more digits than the counting pass's
 // histogram: slices of each coarse region are counted by their fine digits in shared
-// memory and added to bcount[(g << fb) + f].
+// memory and added to bcount[(g << fb) + f].  Bound: reading the keys; a thread keeps eight
+// loads in flight (one at a time took 2.43 ms for 568M 128-bit keys).
 template <typename KeyT>
 __global__ void __launch_bounds__(512, 2) k_fine_count(const KeyT* __restrict__ in,
                                                    const uint32_t* __restrict__ cstart,
@@ -1124,43 +1157,53 @@ __global__ void __launch_bounds__(512, 2) k_fine_count(const KeyT* __restrict__ 
                                                    uint32_t* bcount, int k, int bbits, int cbits,
                                                    uint32_t* ticket, uint32_t slice_keys) {
   using FC = FineCfg<KeyT>;
+  constexpr int T = 512, PF = 8;
   __shared__ uint32_t s_hist[FC::FBMAX];
   __shared__ uint32_t s_slice, s_g;
   const int tid = threadIdx.x;
   const int Cn = 1 << cbits, fb = bbits - cbits, FB = 1 << fb;
   const int fshift = 2 * k - bbits;
-  // the region tables live in shared memory: the slice -> region search of every slice
-  // reads no global memory
+  // the region tables live in shared memory: a slice finds its region with one read a lane
   __shared__ uint32_t s_ss[(1 << kCoarseBits) + 1], s_cs[(1 << kCoarseBits) + 1];
-  for (int i = tid; i <= Cn; i += (int)blockDim.x) {
+  for (int i = tid; i <= Cn; i += T) {
     s_ss[i] = slice_start[i];
     s_cs[i] = cstart[i];
   }
   const uint32_t nslices = slice_start[Cn];
   while (true) {
     __syncthreads();
-    if (tid == 0) {
-      s_slice = atomicAdd(ticket, 1u);
-      if (s_slice < nslices) {
-        int lo = 0, hi = Cn - 1;  // last g with slice_start[g] <= slice
-        while (lo < hi) {
-          int mid = (lo + hi + 1) >> 1;
-          if (s_ss[mid] <= s_slice) lo = mid; else hi = mid - 1;
-        }
-        s_g = lo;
+    if (tid < 32) {
+      uint32_t sl = 0;
+      if (tid == 0) sl = atomicAdd(ticket, 1u);
+      sl = __shfl_sync(FULLMASK, sl, 0);
+      uint32_t below = 0;  // regions that start at or before the slice
+      for (int i = tid; i < Cn; i += 32) below += s_ss[i] <= sl ? 1u : 0u;
+      below = __reduce_add_sync(FULLMASK, below);
+      if (tid == 0) {
+        s_slice = sl;
+        s_g = below - 1;
       }
     }
-    for (int i = tid; i < FB; i += (int)blockDim.x) s_hist[i] = 0;
+    for (int i = tid; i < FB; i += T) s_hist[i] = 0;
     __syncthreads();
     const uint32_t sl = s_slice;
     if (sl >= nslices) break;
     const uint32_t g = s_g;
     const uint32_t r0 = s_cs[g] + (sl - s_ss[g]) * slice_keys;
-    const uint32_t r1 = min(r0 + slice_keys, s_cs[g + 1]);
-    for (uint32_t i = r0 + tid; i < r1; i += blockDim.x)
-      atomicAdd(&s_hist[(uint32_t)(in[i] >> fshift) & (uint32_t)(FB - 1)], 1u);
+    const uint32_t m = min(slice_keys, s_cs[g + 1] - r0);
+    for (uint32_t i0 = 0; i0 < m; i0 += PF * T) {
+      uint32_t f[PF];
+#pragma unroll
+      for (int q = 0; q < PF; q++) {
+        const uint32_t i = i0 + q * T + tid;
+        f[q] = i < m ? (uint32_t)(in[r0 + i] >> fshift) & (uint32_t)(FB - 1) : ~0u;
+      }
+#pragma unroll
+      for (int q = 0; q < PF; q++)
+        if (f[q] != ~0u) atomicAdd(&s_hist[f[q]], 1u);
+    }
     __syncthreads();
-    for (int f = tid; f < FB; f += (int)blockDim.x)
+    for (int f = tid; f < FB; f += T)
       if (s_hist[f]) atomicAdd(&bcount[((uint32_t)g << fb) + f], s_hist[f]);
   }
 }
@@ -1193,23 +1236,33 @@ __global__ void __launch_bounds__(256) k_col_prefix(uint32_t* counts, int grid, 
   }
 }
 
-// Exclusive prefix of bstart[0..B) in place, bstart[B] = total.  One block: each
-// thread sums a contiguous run of ceil(B / 1024) entries, one block scan gives the run
-// offsets, and each thread writes its run (B up to 2^18).
+// Exclusive prefix of bstart[0..B) in place, bstart[B] = total.  One CTA, 16384 entries a
+// step: four 16-byte loads a thread and one block scan (B a power of two up to 2^18; a run of
+// B / 1024 entries a thread, one after the other, took 140 us at 2^17).
 __global__ void __launch_bounds__(1024) k_bucket_prefix(uint32_t* bstart, int B) {
   __shared__ uint32_t s_warp[33];
-  const int per = (B + (int)blockDim.x - 1) / (int)blockDim.x;
-  const int b0 = min(B, (int)threadIdx.x * per), b1 = min(B, b0 + per);
-  uint32_t sum = 0;
-  for (int b = b0; b < b1; b++) sum += bstart[b];
-  uint32_t tot;
-  uint32_t run = block_exclusive_sum(sum, s_warp, tot);
-  for (int b = b0; b < b1; b++) {
-    const uint32_t v = bstart[b];
-    bstart[b] = run;
-    run += v;
+  uint4* v4 = reinterpret_cast<uint4*>(bstart);  // B is 4 or more
+  uint32_t carry = 0;
+  for (int base = 0; base < B; base += 16 * 1024) {
+    const int i0 = base / 4 + 4 * (int)threadIdx.x;
+    uint4 v[4];
+    uint32_t sum = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      v[q] = 4 * (i0 + q) < B ? v4[i0 + q] : make_uint4(0, 0, 0, 0);
+      sum += v[q].x + v[q].y + v[q].z + v[q].w;
+    }
+    uint32_t tot;
+    uint32_t run = carry + block_exclusive_sum(sum, s_warp, tot);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint4 o = make_uint4(run, run + v[q].x, run + v[q].x + v[q].y, run + v[q].x + v[q].y + v[q].z);
+      run = o.w + v[q].w;
+      if (4 * (i0 + q) < B) v4[i0 + q] = o;
+    }
+    carry += tot;
   }
-  if (threadIdx.x == 0) bstart[B] = tot;
+  if (threadIdx.x == 0) bstart[B] = carry;
 }
 
 // ------------------------------------------------------------- per-bucket table ------
