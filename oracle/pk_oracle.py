@@ -26,9 +26,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 BUILD = os.path.join(HERE, "_build")
 REF_OUT = os.path.join(HERE, "_ref")
 LIB = os.path.join(BUILD, "libpk_oracle.so")
-# The reference source tree: $PAKMAN_REFERENCE, else where this project's build
-# container mounts it.  Absent on machines that only run the prebuilt oracle.
+# The reference source tree: $PAKMAN_REFERENCE, else its usual mount point.  Absent on
+# machines that only run the prebuilt oracle; an empty mount point counts as absent.
 REFERENCE_TREE = os.environ.get("PAKMAN_REFERENCE", "/root/reference")
+if os.path.isdir(REFERENCE_TREE) and not os.listdir(REFERENCE_TREE):
+    REFERENCE_TREE = ""
 
 PKO_OK, PKO_EFORMAT, PKO_EARG, PKO_ENOMEM, PKO_EEMPTY = 0, -1, -2, -3, -4
 
