@@ -161,6 +161,7 @@ pk_status presize(pk_job* j, uint64_t fmax, int k, int bbits, int t, int sms) {
   PK_TRY(job_alloc(j, j->chunk_bucket, 4 * (fmax / kChunkKeys + 1)));
   PK_TRY(job_alloc(j, j->gdone, 4 * (size_t)B));
   PK_TRY(job_alloc(j, j->chunk_u, 4 * (fmax / kChunkKeys + 1)));
+  PK_TRY(job_alloc(j, j->gpart, giant_part_bytes(fmax)));
   return PK_OK;
 }
 

@@ -134,7 +134,7 @@ int pk::job_buffers(pk_job* j, DevBuf** out, int cap) {
                    &j->dcounts, &j->kkeys, &j->kcounts, &j->kstart, &j->kcount,
                    &j->ksub,  &j->coff,    &j->cstart,  &j->slice_start, &j->fcur, &j->wiring,
                    &j->gfirst, &j->gcount, &j->chunk_bucket, &j->gdone,
-                   &j->chunk_u, &j->acc_keys[0], &j->acc_keys[1], &j->acc_counts[0], &j->acc_counts[1],
+                   &j->chunk_u, &j->gpart, &j->acc_keys[0], &j->acc_keys[1], &j->acc_counts[0], &j->acc_counts[1],
                    &j->merge_keys, &j->merge_counts, &j->merge_part, &j->units, &j->bsmall};
   const int n = (int)(sizeof(all) / sizeof(all[0]));
   for (int i = 0; i < n && i < cap; i++) out[i] = all[i];
@@ -588,9 +588,7 @@ static pk_status table_impl(pk_job* j, uint64_t N, int t) {
     PK_TRY(job_alloc(j, j->gdone, sizeof(uint32_t) * (size_t)B));
     PK_TRY(job_alloc(j, j->chunk_bucket, sizeof(uint32_t) * (size_t)(N / kChunkKeys + 1)));
     PK_TRY(job_alloc(j, j->chunk_u, sizeof(uint32_t) * (size_t)(N / kChunkKeys + 1)));
-    PK_CUDA(launch_giant_chunks((const uint32_t*)j->bstart.p, j->bbits, (uint32_t*)j->gfirst.p,
-                                (uint32_t*)j->gcount.p, (uint32_t*)j->chunk_bucket.p, (uint32_t*)j->gdone.p,
-                                j->d_sc, j->stream));
+    PK_TRY(job_alloc(j, j->gpart, giant_part_bytes(N)));
   }
   PK_TRY(job_alloc(j, j->bsmall, sizeof(uint32_t) * kSmallCounts * (size_t)B));
   BucketArgs b{};
@@ -601,6 +599,12 @@ static pk_status table_impl(pk_job* j, uint64_t N, int t) {
   b.chunk_bucket = (const uint32_t*)j->chunk_bucket.p;
   b.gdone = (uint32_t*)j->gdone.p;
   b.chunk_u = (uint32_t*)j->chunk_u.p;
+  uint32_t* glist = nullptr;
+  if (giants) {
+    b.gpart = (unsigned long long*)j->gpart.p;
+    glist = (uint32_t*)(b.gpart + (size_t)kGiantParts * (N / kGiantKeys + 1));
+  }
+  b.glist = glist;
   b.bstart = (const uint32_t*)j->bstart.p;
   b.tkeys = j->tkeys.p;
   b.tcounts = (uint32_t*)j->tcounts.p;
@@ -612,6 +616,9 @@ static pk_status table_impl(pk_job* j, uint64_t N, int t) {
   b.cap = N;
   b.spin_limit = (int)j->wait_limit;
   b.sc = j->d_sc;
+  if (giants)
+    PK_CUDA(launch_giant_chunks(b, (uint32_t*)j->gfirst.p, (uint32_t*)j->gcount.p, (uint32_t*)j->chunk_bucket.p,
+                                glist, j->stream));
   PK_CUDA(launch_bucket_table(b, j->wide, j->table_ctas > 0 ? j->table_ctas * thread_sms(j->ctx->sms) : 0, j->stream));
   mark_end(j, ST_TABLE);
   j->bsmall_valid = true;

@@ -52,6 +52,7 @@ constexpr int kBinMax = 128;        // largest bin sorted by ranking (else biton
 // are first reduced chunk by chunk, by many CTAs, to (key, count) pairs.
 constexpr int kChunkKeys = 32768;                   // keys per chunk of a giant bucket
 constexpr uint32_t kGiantKeys = 16u * kChunkKeys;   // a bucket this large is giant
+constexpr int kGiantParts = 16;                     // work items that count one giant bucket
 constexpr uint32_t kChunkRaw = 0xffffffffu;         // chunk left as keys (too many distinct)
 
 struct Scalars {                    // device-side scalars of one job
@@ -65,6 +66,7 @@ struct Scalars {                    // device-side scalars of one job
   uint32_t ticket_fine;
   uint32_t ticket_fcount;
   uint32_t n_chunk_items;           // chunk items of giant buckets (table kernel)
+  uint32_t n_giants;                // giant buckets
   unsigned long long n_unique;      // U
   unsigned long long n_kept;        // V
   // zeroed together before macro-nodes are built
@@ -123,6 +125,9 @@ struct BucketArgs {
   const uint32_t* chunk_bucket;  // per chunk item: its bucket
   uint32_t* gdone;           // 2^bbits: chunk items of the bucket finished
   uint32_t* chunk_u;         // per chunk item: pairs it left, or kChunkRaw
+  // per giant bucket kGiantParts look-back words (rows up to the part's end), and its bucket
+  unsigned long long* gpart;
+  const uint32_t* glist;
   uint32_t* bsmall;          // kSmallCounts x 2^bbits: rows of each bucket by count < kSmallCounts
   int spin_limit;            // polls of a bounded wait before it gives up (0: default)
   Scalars* sc;
@@ -189,9 +194,11 @@ int thread_sms(int device_sms);
 cudaError_t launch_line_scan(const CountArgs& a, cudaStream_t st);
 // chunk items of the giant buckets (n_b >= kGiantKeys): floor(n_b / kChunkKeys)
 // consecutive items each, from gfirst[b], gcount[b] of them; chunk_bucket maps an item
-// to its bucket; sc->n_chunk_items = all items; gdone = 0
-cudaError_t launch_giant_chunks(const uint32_t* bstart, int bbits, uint32_t* gfirst, uint32_t* gcount,
-                                uint32_t* chunk_bucket, uint32_t* gdone, Scalars* sc, cudaStream_t st);
+// to its bucket; sc->n_chunk_items = all items; sc->n_giants and glist: the buckets; gdone,
+// gpart and the giants' rows of bsmall = 0
+cudaError_t launch_giant_chunks(const BucketArgs& a, uint32_t* gfirst, uint32_t* gcount, uint32_t* chunk_bucket,
+                                uint32_t* glist, cudaStream_t st);
+size_t giant_part_bytes(unsigned long long keys);  // gpart, then glist
 // the line scan in two halves: per-tile newline counts for tiles [tile0, tile0 + ntiles)
 // (any order, any number of launches), then the prefix over all tiles
 cudaError_t launch_line_tiles(const uint8_t* buf, unsigned long long F, uint32_t* tile_nl, Scalars* sc,

@@ -1356,10 +1356,14 @@ __device__ __forceinline__ void emit_row(const BucketArgs& a, KeyT* __restrict__
 // Chunk items of the giant buckets (one thread per bucket): a bucket of at least
 // kGiantKeys keys reserves floor(n / kChunkKeys) consecutive chunk items, gfirst[b] the
 // first and gcount[b] how many, and marks them as its own in chunk_bucket; the number
-// of chunk items ends in sc->n_chunk_items (zero beforehand); gdone = 0.
+// of chunk items ends in sc->n_chunk_items (zero beforehand); gdone = 0.  Its kGiantParts
+// part items find it in glist; their look-back words and its small-count histogram, which
+// they add to, are zeroed.
 __global__ void __launch_bounds__(256) k_giant_chunks(const uint32_t* __restrict__ bstart, int B,
                                                       uint32_t* gfirst, uint32_t* gcount,
-                                                      uint32_t* chunk_bucket, uint32_t* gdone, Scalars* sc) {
+                                                      uint32_t* chunk_bucket, uint32_t* gdone,
+                                                      unsigned long long* gpart, uint32_t* glist,
+                                                      uint32_t* bsmall, Scalars* sc) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   const uint32_t n = bstart[b + 1] - bstart[b];
@@ -1370,6 +1374,10 @@ __global__ void __launch_bounds__(256) k_giant_chunks(const uint32_t* __restrict
   if (c) {
     g0 = atomicAdd(&sc->n_chunk_items, c);
     for (uint32_t i = 0; i < c; i++) chunk_bucket[g0 + i] = (uint32_t)b;
+    const uint32_t g = atomicAdd(&sc->n_giants, 1u);
+    glist[g] = (uint32_t)b;
+    for (int i = 0; i < kGiantParts; i++) gpart[(size_t)kGiantParts * g + i] = 0;
+    for (int i = 0; i < kSmallCounts; i++) bsmall[(size_t)b * kSmallCounts + i] = 0;
   }
   gfirst[b] = g0;
 }
@@ -1462,12 +1470,13 @@ __device__ __forceinline__ void aggregate_chunk(const BucketArgs& a, KeyT* keys_
   }
 }
 
-// A giant bucket's item waits (bounded) until its chunk items are done and returns the
+// A giant bucket's part waits (bounded) until the bucket's chunk items are done and returns the
 // entries it will read: the chunks' pairs (or keys, where a chunk stayed raw) and the
-// keys after the last chunk.  On expiry it sets ERR_LOOKBACK and *s_fail.
+// keys after the last chunk; `raws` tells whether any chunk stayed raw.  On expiry it sets
+// ERR_LOOKBACK and *s_fail.
 template <int T>
 __device__ __forceinline__ uint32_t giant_entries(const BucketArgs& a, uint32_t beta, uint32_t n, uint32_t g0,
-                                               uint32_t nch, uint32_t* s_warp, uint32_t* s_fail) {
+                                               uint32_t nch, uint32_t* s_warp, uint32_t* s_fail, bool& raws) {
   const int tid = threadIdx.x;
   if (tid == 0) {
     int spins = 0;
@@ -1483,50 +1492,124 @@ __device__ __forceinline__ uint32_t giant_entries(const BucketArgs& a, uint32_t 
   }
   __syncthreads();
   uint32_t part = 0;
+  bool raw = false;
   for (uint32_t j = tid; j < nch; j += T) {
     const uint32_t cu = __ldcg(&a.chunk_u[g0 + j]);
+    raw |= cu == kChunkRaw;
     part += cu == kChunkRaw ? (uint32_t)kChunkKeys : cu;
   }
+  raws = __syncthreads_or(raw) != 0;
   uint32_t tot;
   block_exclusive_sum(part, s_warp, tot);
   return tot + (n - nch * (uint32_t)kChunkKeys);
 }
 
-// One hash pass of a giant bucket's sub-range [lo, hi): chunk by chunk (pairs carry
-// their counts), then the tail keys.  Loads go through L2, as other CTAs wrote the
-// pairs during this kernel.
+// The remainder range [lo, hi) of part `part` of a giant bucket, by thread 0's view in *s_lo
+// and *s_end: quantiles of kSplitSamples of the entries that its parts read.  Every part
+// takes the same sample and so the same quantiles; equal ones leave parts empty.  A bucket
+// with few entries is its first part's alone.  `samp`: kSplitSamples keys, barriers inside.
+// One CTA that made every pass over a giant bucket, 16 equal ranges first, took 2.6 of the
+// 3.26 ms of the low-complexity reads (36M windows, buckets of up to 5.7M); with the parts on
+// as many CTAs the whole path takes 0.92 ms (1.55 ms with quicker passes of one CTA).
+template <typename KeyT>
+__device__ __forceinline__ void giant_range(const BucketArgs& a, const KeyT* keys_rw, uint32_t base, uint32_t n_eff,
+                                            uint32_t g0, uint32_t nch, uint32_t part, KeyT rmask, KeyT rtop,
+                                            KeyT* samp, KeyT* s_lo, KeyT* s_end) {
+  static_assert(kSplitSamples % kGiantParts == 0, "quantiles are samples");
+  constexpr uint32_t PER = kSplitSamples / kGiantParts;
+  const uint32_t tid = threadIdx.x;
+  if (n_eff <= (uint32_t)BucketCfg<KeyT>::H / 2) {
+    if (tid == 0) {
+      *s_lo = (KeyT)0;
+      *s_end = part ? (KeyT)0 : rtop;
+    }
+    __syncthreads();
+    return;
+  }
+  KeyT mine = 0;
+  if (tid < (uint32_t)kSplitSamples) {
+    const uint32_t j = (uint32_t)(((unsigned long long)tid * nch) / kSplitSamples);
+    const uint32_t len = min(__ldcg(&a.chunk_u[g0 + j]), (uint32_t)kChunkKeys);  // raw: all of them
+    const uint32_t e = len ? (tid * 2654435761u >> 8) % len : 0u;
+    mine = ldcg_key(keys_rw + ((unsigned long long)base + (unsigned long long)j * kChunkKeys + e)) & rmask;
+    samp[tid] = mine;
+  }
+  if (tid == 0) {
+    *s_lo = (KeyT)0;
+    *s_end = rtop;
+  }
+  __syncthreads();
+  if (tid < (uint32_t)kSplitSamples) {
+    uint32_t rank = 0;
+    for (uint32_t j = 0; j < (uint32_t)kSplitSamples; j++) {
+      const KeyT o = samp[j];
+      rank += (o < mine || (o == mine && j < tid)) ? 1u : 0u;
+    }
+    if (part && rank == part * PER) *s_lo = mine;
+    if (rank == (part + 1) * PER) *s_end = mine;  // never reached by the last part
+  }
+  __syncthreads();
+  if (tid < (uint32_t)kSplitSamples) samp[tid] = 0;  // the sort bins again
+  __syncthreads();
+}
+
+// One hash pass of a giant bucket's sub-range [lo, hi): every warp takes whole chunks of
+// pairs (their counts are read only inside the sub-range), then the CTA reads the chunks that
+// stayed raw (`raws`: there are any) and the tail keys together.  Loads go through L2, as
+// other CTAs wrote the pairs during this kernel: four in flight a thread.
 template <typename KeyT, int T>
 __device__ __forceinline__ void giant_pass(const BucketArgs& a, const KeyT* keys_rw, uint32_t base, uint32_t n,
-                                           uint32_t g0, uint32_t nch, bool whole, KeyT lo, KeyT hi, KeyT rmask,
-                                           KeyT* skey, uint32_t* scnt, uint32_t hmask, uint32_t ulimit,
+                                           uint32_t g0, uint32_t nch, bool raws, bool whole, KeyT lo, KeyT hi,
+                                           KeyT rmask, KeyT* skey, uint32_t* scnt, uint32_t hmask, uint32_t ulimit,
                                            uint32_t* bins, int dsh, uint32_t bmask, uint32_t* s_ovf,
                                            uint32_t* s_unew) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (uint32_t j = 0; j <= nch; j++) {
-    if (warp_flag(s_ovf)) break;
-    const unsigned long long cb = (unsigned long long)base + (unsigned long long)j * kChunkKeys;
-    uint32_t len = n - nch * (uint32_t)kChunkKeys;
-    bool pairs = false;
-    if (j < nch) {
-      const uint32_t cu = __ldcg(&a.chunk_u[g0 + j]);
-      pairs = cu != kChunkRaw;
-      len = pairs ? cu : (uint32_t)kChunkKeys;
-    }
+  constexpr int GP = 4;  // loads in flight
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // entries [i, len) of the chunk at cb, `step` apart, GP at a time
+  auto read = [&](unsigned long long cb, uint32_t i0, uint32_t len, uint32_t step, bool pairs) {
     const uint32_t* pc = reinterpret_cast<const uint32_t*>(keys_rw + cb + kChunkKeys / 2);
+    KeyT r[GP];
+    uint32_t c[GP];
+#pragma unroll
+    for (int q = 0; q < GP; q++) {
+      const uint32_t i = i0 + q * step;
+      r[q] = i < len ? ldcg_key(keys_rw + cb + i) & rmask : ~(KeyT)0;
+    }
+#pragma unroll
+    for (int q = 0; q < GP; q++) {
+      const bool in = r[q] != ~(KeyT)0 && (whole || (!(r[q] < lo) && r[q] < hi));
+      c[q] = in ? 1u : 0u;
+      if (in && pairs) c[q] = __ldcg(pc + i0 + q * step);
+    }
     uint32_t fresh = 0;
-    for (uint32_t i = tid; i < len; i += T) {
-      const KeyT r = ldcg_key(keys_rw + cb + i) & rmask;
-      if (whole || (!(r < lo) && r < hi)) {
-        const int res = hash_insert<KeyT>(skey, scnt, hmask, r, pairs ? __ldcg(pc + i) : 1u);
-        if (res == 2) *s_ovf = 1;
-        if (res == 1) {
-          atomicAdd(&bins[sort_bin<KeyT>(r, dsh, bmask)], 1u);
-          fresh++;
-        }
+#pragma unroll
+    for (int q = 0; q < GP; q++) {
+      if (!c[q]) continue;
+      const int res = hash_insert<KeyT>(skey, scnt, hmask, r[q], c[q]);
+      if (res == 2) *s_ovf = 1;
+      if (res == 1) {
+        atomicAdd(&bins[sort_bin<KeyT>(r[q], dsh, bmask)], 1u);
+        fresh++;
       }
     }
     fresh = __reduce_add_sync(FULLMASK, fresh);
     if (lane == 0 && fresh && atomicAdd(s_unew, fresh) + fresh > ulimit) *s_ovf = 1;
+  };
+  for (uint32_t j = warp; j < nch; j += T / 32) {
+    const uint32_t len = __ldcg(&a.chunk_u[g0 + j]);
+    if (len == kChunkRaw) continue;
+    for (uint32_t i0 = 0; i0 < len; i0 += 32 * GP) {
+      if (warp_flag(s_ovf)) break;
+      read((unsigned long long)base + (unsigned long long)j * kChunkKeys, i0 + lane, len, 32, true);
+    }
+  }
+  for (uint32_t j = raws ? 0 : nch; j <= nch; j++) {
+    if (j < nch && __ldcg(&a.chunk_u[g0 + j]) != kChunkRaw) continue;
+    const uint32_t len = j < nch ? (uint32_t)kChunkKeys : n - nch * (uint32_t)kChunkKeys;
+    for (uint32_t i0 = 0; i0 < len; i0 += GP * T) {
+      if (warp_flag(s_ovf)) break;
+      read((unsigned long long)base + (unsigned long long)j * kChunkKeys, i0 + tid, len, T, false);
+    }
   }
 }
 
@@ -1595,6 +1678,8 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
   // in the list starts (the first at the end of the remainder range)
   __shared__ KeyT s_lo[kBucketStack];
   __shared__ KeyT s_split[kSplitWays];
+  __shared__ KeyT s_end;       // end of a giant bucket's part
+  __shared__ uint32_t s_before;  // rows of the parts before it
   __shared__ float s_ratio, s_size;  // expected distinct keys and table slots per key
   __shared__ uint32_t s_bsmall[kSmallCounts];  // the current bucket's rows by small count
 
@@ -1615,7 +1700,8 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
   const uint32_t ng = a.gfirst ? a.sc->n_chunk_items : 0u;
   if ((ng != 0) != GIANT) return;
   const uint32_t nci = GIANT ? ng : 0u;
-  const uint32_t nt = nci + (uint32_t)B;
+  const uint32_t first_bucket = GIANT ? nci + kGiantParts * a.sc->n_giants : 0u;
+  const uint32_t nt = first_bucket + (uint32_t)B;
   uint32_t* ticket = &a.sc->ticket_bucket;
   KeyT* keys_rw = reinterpret_cast<KeyT*>(a.keys);
 
@@ -1624,10 +1710,10 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
   if (tid < kSmallCounts) s_bsmall[tid] = 0;
   clear_table<KeyT, T>(skey, scnt, bins, H);
 
-  // Work tickets: the chunk items of giant buckets first (tickets [0, nci)), then the
-  // buckets.  A giant bucket waits (bounded) until its chunks are reduced; every chunk
-  // ticket was taken before any bucket ticket, by a CTA that waits on nothing, so the
-  // wait ends.  Thread 0 takes the next ticket when a bucket starts and its extent
+  // Work tickets: the chunk items of giant buckets first (tickets [0, nci)), then their
+  // parts, then the other buckets.  A part waits (bounded) until its bucket's chunks are
+  // reduced, and before it writes rows until the parts before it have counted theirs: items
+  // of earlier tickets, held by CTAs that wait on still earlier ones, so the waits end.  Thread 0 takes the next ticket when a bucket starts and its extent
   // once the bucket's keys are in, so neither is waited for between buckets.
   uint32_t next_t = 0, next_base = 0, next_end = 0;
   bool have_extent = true;
@@ -1638,9 +1724,9 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
   auto take_extent = [&]() {
     if (have_extent) return;
     have_extent = true;
-    if ((!GIANT || next_t >= nci) && next_t < nt) {
-      next_base = a.bstart[next_t - nci];
-      next_end = a.bstart[next_t - nci + 1];
+    if ((!GIANT || next_t >= first_bucket) && next_t < nt) {
+      next_base = a.bstart[next_t - first_bucket];
+      next_end = a.bstart[next_t - first_bucket + 1];
     }
   };
   // thread 0: the next item and its first sub-ranges
@@ -1691,30 +1777,72 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
       __syncthreads();
       continue;
     }
-    const uint32_t beta = tk - nci;
-    const uint32_t base = s_nb[0];
-    const uint32_t n = s_nb[1] - base;
-    // a giant bucket reads its chunks' pairs (or keys, where a chunk stayed raw) and the
-    // keys after its last chunk; n_eff = entries it reads
-    const uint32_t g0 = GIANT ? a.gfirst[beta] : 0u;
+    // a giant bucket is counted by its parts, one remainder range each; a part reads the
+    // chunks' pairs (or keys, where a chunk stayed raw) and the keys after the last chunk;
+    // n_eff = entries it reads
+    const bool part = GIANT && tk < first_bucket;
+    const uint32_t item = tk - nci;  // of a part: its place in gpart
+    const uint32_t beta = part ? a.glist[item / kGiantParts] : tk - first_bucket;
+    const uint32_t base = part ? a.bstart[beta] : s_nb[0];
+    const uint32_t all = (part ? a.bstart[beta + 1] : s_nb[1]) - base;
+    const uint32_t g0 = part ? a.gfirst[beta] : 0u;
     const uint32_t nch = GIANT ? a.gcount[beta] : 0u;
+    const bool elsewhere = GIANT && !part && nch;  // counted by its parts
+    uint32_t n = elsewhere ? 0u : all;
     uint32_t n_eff = n;
-    bool failed = false;
+    bool failed = false, raws = false;
     if (GIANT) {
       __syncthreads();
-      if (nch) n_eff = giant_entries<T>(a, beta, n, g0, nch, s_warp, &s_fail);
+      if (part) n_eff = giant_entries<T>(a, beta, n, g0, nch, s_warp, &s_fail, raws);
       failed = s_fail != 0;  // a giant bucket whose chunks did not finish in time
-      if (tid == 0) push_first(n_eff);
+      if (part && !failed) {
+        giant_range<KeyT>(a, keys_rw, base, n_eff, g0, nch, item % kGiantParts, rmask, rtop,
+                          reinterpret_cast<KeyT*>(bins), &s_lo[0], &s_end);
+        if (s_lo[0] == s_end) n = 0;
+      }
+      if (tid == 0) {
+        if (part) {
+          s_sp = 1;
+        } else {
+          s_end = rtop;
+          push_first(n_eff);
+        }
+      }
       __syncthreads();
     }
     if (!GIANT && n == 0) __syncthreads();  // every thread has read this item before the next is published
-    uint32_t acc = 0;
+    uint32_t acc = 0, before = 0;  // rows written so far; of a part, those before it
+    bool placed = !part;
+    // a part's first row follows the parts before it; the rows up to its own end (`rows` of
+    // its own, when it is known to end with them) are published for the parts after it
+    unsigned long long* const word = part ? a.gpart + item : nullptr;
+    auto place = [&]() {
+      if (tid == 0) {
+        unsigned long long w = kLbIncl;
+        if (item % kGiantParts) {
+          int spins = 0;
+          const int max_spins = spin_limit(a.spin_limit);
+          while ((w = ld_relaxed(word - 1)) == 0) {
+            if (++spins >= max_spins) {
+              atomicOr(&a.sc->err, ERR_LOOKBACK);
+              break;
+            }
+            __nanosleep(spins < 64 ? 32 : 256);
+          }
+        }
+        s_before = (uint32_t)(w & kLbVal);
+      }
+      __syncthreads();
+      before = s_before;
+      acc = before;
+      placed = true;
+    };
     int attempts = 0;
     while (n && !failed) {
       const int sp = s_sp;
       if (++attempts > kMaxBucketAttempts) { failed = true; break; }
       const KeyT lo = s_lo[sp - 1];
-      const KeyT hi = sp > 1 ? s_lo[sp - 2] : rtop;
+      const KeyT hi = sp > 1 ? s_lo[sp - 2] : GIANT ? s_end : rtop;
       const bool whole = lo == (KeyT)0 && hi == rtop;
       // bits below the interval's common prefix (all its keys share the bits above)
       const KeyT span = lo ^ (hi - (KeyT)1);
@@ -1733,10 +1861,10 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
       // --- hash aggregation of this sub-range; it stops as soon as the distinct keys
       //     exceed half the table
       const uint32_t ulimit = Heff / 2;
-      if (GIANT && nch)
-        giant_pass<KeyT, T>(a, keys_rw, base, n, g0, nch, whole, lo, hi, rmask, skey, scnt, hmask, ulimit, bins, dsh,
-                         bmask, &s_ovf, &s_unew);
-      for (uint32_t i0 = 0; i0 < n && !(GIANT && nch); i0 += PF * T) {
+      if (GIANT && part)
+        giant_pass<KeyT, T>(a, keys_rw, base, n, g0, nch, raws, whole, lo, hi, rmask, skey, scnt, hmask, ulimit, bins,
+                            dsh, bmask, &s_ovf, &s_unew);
+      for (uint32_t i0 = 0; i0 < n && !(GIANT && part); i0 += PF * T) {
         if (warp_flag(&s_ovf)) break;
         KeyT rr[PF];
 #pragma unroll
@@ -1813,6 +1941,8 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
       }
       const uint32_t u = s_unew;
       if (tid == 0) take_extent();
+      if (GIANT && !placed) place();
+      if (GIANT && part && sp == 1 && tid == 0) st_relaxed(word, kLbIncl | (acc + u));
       // --- order the u distinct remainders: slot numbers go to their bins, in any order
       scan_bins(bins, s_warp, &s_crowd);
       for (uint32_t i = tid; i < Heff; i += T) {
@@ -1877,23 +2007,34 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
       }
       __syncthreads();
     }
+    if (GIANT && part && (failed || n == 0)) {  // nothing was published yet
+      if (!placed) place();
+      if (tid == 0) st_relaxed(word, kLbIncl | acc);
+    }
     if (failed) {
       if (tid == 0) atomicOr(&a.sc->err, ERR_BUCKET);
       acc = 0;
+      before = 0;
     }
     // the bucket's rows by small count (every row was emitted before the last barrier):
     // stored for the kept filter and folded into the count histogram (counts below t)
     if (tid < kSmallCounts) {
       const uint32_t c = s_bsmall[tid];
-      if (a.bsmall) a.bsmall[(size_t)beta * kSmallCounts + tid] = c;
+      uint32_t* bs = a.bsmall + (size_t)beta * kSmallCounts + tid;
+      if (part) {
+        if (c) atomicAdd(bs, c);
+      } else if (a.bsmall && !elsewhere) {
+        *bs = c;
+      }
       if (c && tid < a.t) atomicAdd(&shist[tid], c);
       s_bsmall[tid] = 0;
     }
     if (tid == 0) {
-      a.tu[beta] = acc;
+      // of a giant bucket the last part knows all rows
+      if (!elsewhere && (!part || item % kGiantParts == kGiantParts - 1)) a.tu[beta] = acc;
       if (n) {
-        atomicAdd(&a.sc->n_unique, (unsigned long long)acc);
-        s_ratio = 0.5f * s_ratio + 0.5f * ((float)acc / (float)n_eff);
+        atomicAdd(&a.sc->n_unique, (unsigned long long)(acc - before));
+        if (!part) s_ratio = 0.5f * s_ratio + 0.5f * ((float)acc / (float)n_eff);
         s_size = 2.5f * s_ratio;
       }
       publish();
@@ -2987,11 +3128,16 @@ cudaError_t launch_bucket_table(const BucketArgs& a, int wide, int grid, cudaStr
   return wide ? launch_bucket_t<u128>(a, grid, st) : launch_bucket_t<uint64_t>(a, grid, st);
 }
 
-cudaError_t launch_giant_chunks(const uint32_t* bstart, int bbits, uint32_t* gfirst, uint32_t* gcount,
-                                uint32_t* chunk_bucket, uint32_t* gdone, Scalars* sc, cudaStream_t st) {
-  const int B = 1 << bbits;
-  pk::note_launch(), k_giant_chunks<<<(B + 255) / 256, 256, 0, st>>>(bstart, B, gfirst, gcount, chunk_bucket, gdone, sc);
+cudaError_t launch_giant_chunks(const BucketArgs& a, uint32_t* gfirst, uint32_t* gcount, uint32_t* chunk_bucket,
+                                uint32_t* glist, cudaStream_t st) {
+  const int B = 1 << a.bbits;
+  pk::note_launch(), k_giant_chunks<<<(B + 255) / 256, 256, 0, st>>>(a.bstart, B, gfirst, gcount, chunk_bucket, a.gdone,
+                                                                    a.gpart, glist, a.bsmall, a.sc);
   return cudaGetLastError();
+}
+
+size_t giant_part_bytes(unsigned long long keys) {
+  return (keys / kGiantKeys + 1) * (kGiantParts * sizeof(unsigned long long) + sizeof(uint32_t));
 }
 
 cudaError_t launch_histogram(const uint32_t* tcounts, const uint32_t* bstart, const uint32_t* tu, int B, int t,

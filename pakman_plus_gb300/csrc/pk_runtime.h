@@ -96,7 +96,7 @@ struct pk_job {
   pk::Scalars* h_sc = nullptr;  // pinned mirror
   DevBuf fasta, tile_nl, counts, bstart, hstart, keys, tkeys, tcounts, tu, flags_m, hist, hist2,
       nkeys, nsuf, npre, packed, doff, dkeys, dcounts, kkeys, kcounts, kstart, kcount, ksub,
-      coff, cstart, slice_start, fcur, wiring, gfirst, gcount, chunk_bucket, gdone, chunk_u,
+      coff, cstart, slice_start, fcur, wiring, gfirst, gcount, chunk_bucket, gdone, chunk_u, gpart,
       units,   // packed units of the counting pass, rolled again by the coarse scatter
       bsmall;  // rows of each table bucket by count below kSmallCounts (the table kernel's)
   bool bsmall_valid = false;  // bsmall describes the current table
