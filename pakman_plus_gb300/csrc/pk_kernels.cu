@@ -2423,9 +2423,11 @@ __global__ void __launch_bounds__(256) k_mn_big(MnArgs a, uint32_t fit) {
 // items and stores the node's three rows whole.
 //
 // Bound: the wait for the units before (without it 8.6M nodes take 0.21 ms and 46M 63-mer
-// nodes 1.5 ms).  Bacterial nodes (8.6M): 0.39 -> 0.23 ms, 46M nodes of 63-mers 6.95 ->
-// 3.54 ms, against sorting every unit, assembling nodes by 4-byte stores into zeroed rows
-// and looking back over single units.
+// nodes 1.5 ms): all units in flight wait for the slowest of them, so a lookup is a binary
+// search in its bin.  Scanning the bin, a unit of repeats took up to 48 thousand cycles
+// against 14 thousand on average, and the 46M nodes 3.54 instead of 2.2 ms.  Bacterial nodes
+// (8.6M): 0.39 -> 0.23 ms, 46M nodes of 63-mers 6.95 -> 3.54 ms, against sorting every unit,
+// assembling nodes by 4-byte stores into zeroed rows and looking back over single units.
 template <typename KeyT>
 __global__ void __launch_bounds__(kMnThreads, MnCfg<KeyT>::CTAS) k_macro_nodes(MnArgs a) {
   using SM = MnSmem<KeyT>;
@@ -2566,11 +2568,8 @@ __global__ void __launch_bounds__(kMnThreads, MnCfg<KeyT>::CTAS) k_macro_nodes(M
         at[q] = n0;
         if (q * T + tid < np) {
           const uint32_t b = (uint32_t)KeyOps<KeyT>::shr(py[q], bsh) & bmask;
-          for (uint32_t i = start[b], e = min((uint32_t)start[b + 1], n0); i < e; i++)
-            if (pkey[i] == py[q]) {
-              at[q] = i;
-              break;
-            }
+          const uint32_t i = lower_bound_s(pkey, start[b], start[b + 1], py[q]);
+          if (i < n0 && pkey[i] == py[q]) at[q] = i;
           if (at[q] == n0) {  // a node of its own
             const uint32_t x = atomicAdd(&s_extra, 1u);
             if (x < 32) {
@@ -2618,8 +2617,8 @@ __global__ void __launch_bounds__(kMnThreads, MnCfg<KeyT>::CTAS) k_macro_nodes(M
           }
           uint32_t i = 0;
           if (have) {
-            i = start[(uint32_t)KeyOps<KeyT>::shr(xk, bsh) & bmask];
-            while (i < n0 && pkey[i] < xk) i++;
+            const uint32_t b = (uint32_t)KeyOps<KeyT>::shr(xk, bsh) & bmask;
+            i = lower_bound_s(pkey, start[b], start[b + 1], xk);
           }
           const uint32_t h = heads_to(i ? i - 1 : 0u);
           xheads = i ? h : 0u;
