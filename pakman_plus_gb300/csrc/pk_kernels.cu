@@ -908,23 +908,28 @@ __global__ void __launch_bounds__(256) k_coarse_offsets(const uint32_t* __restri
 // 1.02 -> 0.91 ms against a second atomic per key for its rank and a binary search in
 // global memory for every slice's region.  One CTA of 1024 threads an SM: 0.98 ms; the next
 // slice's ticket taken ahead: no change.
-template <typename KeyT>
+// FEW: up to 2^kFewFine fine buckets, where slices of a quarter still give runs of 16 (64-bit)
+// or 8 keys: six CTAs an SM instead of two wait at their barriers at other times.  Bacterial
+// reads (2^14 buckets, 2^7 fine): 0.90 -> 0.77 ms; three CTAs of 4096-key slices 0.80 ms, of
+// 8192 1.28 ms (they spill).  With 2^10 fine buckets 4096-key slices lose (25 Mbp long-k path
+// 22.6 -> 26.0 ms).
+constexpr int kFewFine = 7;
+template <typename KeyT, bool FEW>
 struct FineCfg {
-  static constexpr int T = 512;                             // threads
-  static constexpr int PT = sizeof(KeyT) == 8 ? 16 : 8;      // keys per thread
-  static constexpr int S = T * PT;                          // keys per slice (64 KB)
-  static constexpr int FBMAX = 1 << (kMaxPartBits - kCoarseBits);  // fine buckets per coarse
+  static constexpr int T = FEW ? 256 : 512;                  // threads
+  static constexpr int CTAS = FEW ? 6 : 2;                   // CTAs per SM
+  static constexpr int PT = (FEW ? 64 : 128) / (int)sizeof(KeyT);  // keys per thread
+  static constexpr int S = T * PT;                           // keys per slice (16 or 64 KB)
+  static constexpr int FBMAX = 1 << (FEW ? kFewFine : kMaxPartBits - kCoarseBits);  // fine buckets per coarse
   static constexpr size_t smem = sizeof(KeyT) * S;
 };
 
-template <typename KeyT>
-__global__ void __launch_bounds__(512, 2) k_scatter_fine(const KeyT* __restrict__ in,
-                                                        const uint32_t* __restrict__ cstart,
-                                                        const uint32_t* __restrict__ slice_start,
-                                                        uint32_t* fcur, KeyT* __restrict__ out,
-                                                        int k, int bbits, int cbits, uint32_t* ticket,
-                                                        unsigned long long cap, uint32_t* err) {
-  using FC = FineCfg<KeyT>;
+template <typename KeyT, bool FEW>
+__global__ void __launch_bounds__(FineCfg<KeyT, FEW>::T, FineCfg<KeyT, FEW>::CTAS)
+k_scatter_fine(const KeyT* __restrict__ in, const uint32_t* __restrict__ cstart,
+               const uint32_t* __restrict__ slice_start, uint32_t* fcur, KeyT* __restrict__ out, int k, int bbits,
+               int cbits, uint32_t* ticket, unsigned long long cap, uint32_t* err) {
+  using FC = FineCfg<KeyT, FEW>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   KeyT* stage = reinterpret_cast<KeyT*>(smem_raw);  // the slice grouped by fine bucket
   // per fine bucket: keys, first staged key, and what takes a staged position to its place
@@ -1045,7 +1050,7 @@ __global__ void __launch_bounds__(1024, 1) k_scatter_fine_big(const KeyT* __rest
                                                              int k, int bbits, int cbits, uint32_t* ticket,
                                                              unsigned long long cap, uint32_t* err) {
   using FC = FineBigCfg<KeyT>;
-  constexpr int FBMAX = FineCfg<KeyT>::FBMAX;
+  constexpr int FBMAX = FineCfg<KeyT, false>::FBMAX;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   KeyT* stage = reinterpret_cast<KeyT*>(smem_raw);
   __shared__ uint32_t s_hist[FBMAX], s_loff[FBMAX], s_goff[FBMAX], s_fill[FBMAX];
@@ -1143,7 +1148,8 @@ __global__ void __launch_bounds__(1024, 1) k_scatter_fine_big(const KeyT* __rest
 
 int fine_slice_keys(int wide, int fb) {
   if (fb >= 11) return wide ? FineBigCfg<u128>::S : FineBigCfg<uint64_t>::S;
-  return wide ? FineCfg<u128>::S : FineCfg<uint64_t>::S;
+  if (fb <= kFewFine) return wide ? FineCfg<u128, true>::S : FineCfg<uint64_t, true>::S;
+  return wide ? FineCfg<u128, false>::S : FineCfg<uint64_t, false>::S;
 }
 
 // Fine bucket sizes when the partition has more digits than the counting pass's
@@ -1156,7 +1162,7 @@ __global__ void __launch_bounds__(512, 2) k_fine_count(const KeyT* __restrict__ 
                                                    const uint32_t* __restrict__ slice_start,
                                                    uint32_t* bcount, int k, int bbits, int cbits,
                                                    uint32_t* ticket, uint32_t slice_keys) {
-  using FC = FineCfg<KeyT>;
+  using FC = FineCfg<KeyT, false>;
   constexpr int T = 512, PF = 8;
   __shared__ uint32_t s_hist[FC::FBMAX];
   __shared__ uint32_t s_slice, s_g;
@@ -3037,17 +3043,27 @@ cudaError_t launch_coarse_offsets(const CountArgs& a, int pbits, uint32_t* coff,
   return cudaGetLastError();
 }
 
+template <typename KeyT, bool FEW>
+static cudaError_t launch_fine_n(const KeyT* in, const uint32_t* cstart, const uint32_t* slice_start,
+                                 uint32_t* fcur, KeyT* out, int k, int bbits, int cbits, uint32_t* ticket,
+                                 unsigned long long cap, uint32_t* err, cudaStream_t st) {
+  using FC = FineCfg<KeyT, FEW>;
+  static bool attr_set = false;  // a constant, so concurrent first calls agree
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(k_scatter_fine<KeyT, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)FC::smem);
+    if (e != cudaSuccess) return e;
+    attr_set = true;
+  }
+  pk::note_launch(), k_scatter_fine<KeyT, FEW><<<sm_count() * FC::CTAS, FC::T, FC::smem, st>>>(
+      in, cstart, slice_start, fcur, out, k, bbits, cbits, ticket, cap, err);
+  return cudaGetLastError();
+}
+
 template <typename KeyT>
 static cudaError_t launch_fine_t(const KeyT* in, const uint32_t* cstart, const uint32_t* slice_start,
                                  uint32_t* fcur, KeyT* out, int k, int bbits, int cbits, uint32_t* ticket,
                                  unsigned long long cap, uint32_t* err, cudaStream_t st) {
-  const size_t smem = FineCfg<KeyT>::smem;
-  static bool attr_set = false;  // a constant, so concurrent first calls agree
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_scatter_fine<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
   if (bbits - cbits >= 11) {
     const size_t bsmem = FineBigCfg<KeyT>::smem;
     static bool big_attr_set = false;
@@ -3061,9 +3077,10 @@ static cudaError_t launch_fine_t(const KeyT* in, const uint32_t* cstart, const u
                                                                              bbits, cbits, ticket, cap, err);
     return cudaGetLastError();
   }
-  pk::note_launch(), k_scatter_fine<KeyT><<<sm_count() * 2, FineCfg<KeyT>::T, smem, st>>>(in, cstart, slice_start, fcur, out,
-                                                                        k, bbits, cbits, ticket, cap, err);
-  return cudaGetLastError();
+  return bbits - cbits <= kFewFine ? launch_fine_n<KeyT, true>(in, cstart, slice_start, fcur, out, k, bbits, cbits, ticket,
+                                                              cap, err, st)
+                                   : launch_fine_n<KeyT, false>(in, cstart, slice_start, fcur, out, k, bbits, cbits,
+                                                               ticket, cap, err, st);
 }
 
 cudaError_t launch_scatter_fine(const void* in, const uint32_t* cstart, const uint32_t* slice_start,
