@@ -43,6 +43,7 @@
 #include "pk_internal.h"
 #include "pk_runtime.h"
 #include "pk_stdsort.cuh"
+#include "pk_wire.cuh"
 
 using namespace pk;
 
@@ -68,6 +69,7 @@ enum : uint32_t {
   CE_WALK_DEPTH = 256u,  // a walk went deeper than its stack
 };
 constexpr uint32_t kWalkMaxBases = 500000;  // src/walk.cpp:285
+constexpr uint64_t kWalkRecords = 1u << 22;  // pieces that the counting walk records at most
 
 struct Tr {            // one TransferNode (src/merge_mn.cpp:483-525)
   uint64_t w;          // arena base offset of W = P + K + S
@@ -352,75 +354,122 @@ __device__ __forceinline__ int32_t visit_of(int32_t c, int32_t cov) {  // (int)c
   return q;
 }
 
+// One thread per node ranks its two lists in registers, wires them as setup_wiring does a
+// first time and stages what its entries need in shared memory; then the CTA writes its nodes'
+// entries and wire slots, contiguous runs, one after the other.  Bound: HBM, by the entries
+// it writes.  4.0M nodes: 620 us with the lists in local memory and every thread storing its
+// own entries, 284 us so.
+constexpr int kInitT = 128;                // nodes per CTA
+constexpr int kInitE = 10;                 // entries of a node at most
 template <typename KeyT>
-__global__ void k_cp_init(const KeyT* __restrict__ nkeys, const uint4* __restrict__ nsuf,
-                          const uint4* __restrict__ npre, uint32_t m, int L, int32_t cov,
-                          const uint4* __restrict__ col, Side<KeyT> s, uint32_t* err) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > m) return;
-  if (i == m) {
-    s.eoff[m] = col[m].x;
-    return;
+__global__ void __launch_bounds__(kInitT) k_cp_init(const KeyT* __restrict__ nkeys, const uint4* __restrict__ nsuf,
+                                                    const uint4* __restrict__ npre, uint32_t m, int L, int32_t cov,
+                                                    const uint4* __restrict__ col, Side<KeyT> s, uint32_t* err) {
+  __shared__ int32_t s_wire[3 * kInitT * (kInitE + 1)];
+  __shared__ int32_t s_cnt[kInitT * kInitE], s_vis[kInitT * kInitE];
+  __shared__ uint16_t s_beg[kInitT * kInitE];  // first wire (low byte) and wires
+  __shared__ uint8_t s_node[kInitT * kInitE], s_what[kInitT * kInitE];  // base; bit 2: terminal, bit 3: suffix
+  __shared__ int32_t s_sv[kInitT * 5], s_pv[kInitT * 5];  // visits in rank order
+  __shared__ KeyT s_key[kInitT];
+  const uint32_t tid = threadIdx.x, i0 = blockIdx.x * kInitT, i = i0 + tid, i1 = min(i0 + kInitT, m);
+  const uint32_t E0 = col[i0].x, M = col[i1].x - E0;  // the CTA's entries
+  const uint32_t words = 3 * (M + (i1 - i0));
+  for (uint32_t w = tid; w < words; w += kInitT) s_wire[w] = 0;
+  for (uint32_t e = tid; e < M; e += kInitT) s_beg[e] = 0;
+  if (i == m) s.eoff[m] = col[m].x;
+  __syncthreads();
+  if (i < i1) {
+    const KeyT key = nkeys[i];
+    const uint4 s4 = nsuf[i], p4 = npre[i];
+    const uint32_t sraw[4] = {s4.x, s4.y, s4.z, s4.w}, praw[4] = {p4.x, p4.y, p4.z, p4.w};
+    const uint32_t e0 = col[i].x, le = e0 - E0;
+    int32_t sv[5], pv[5];
+    int ns = 1, np = 1, sc = 0, pc = 0;
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      sv[b] = sraw[b] ? visit_of((int32_t)sraw[b], cov) : 0;
+      pv[b] = praw[b] ? visit_of((int32_t)praw[b], cov) : 0;
+      ns += sraw[b] != 0;
+      np += praw[b] != 0;
+      sc += sv[b];
+      pc += pv[b];
+    }
+    sv[4] = max(pc - sc, 0);
+    pv[4] = max(sc - pc, 0);
+    s_key[tid] = key;
+    s.key[i] = key;
+    s.eoff[i] = e0;
+    s.npre[i] = (uint32_t)np;
+    uint32_t e = le;
+    auto put = [&](uint32_t what, int32_t c, int32_t v) {
+      s_node[e] = (uint8_t)tid;
+      s_what[e] = (uint8_t)what;
+      s_cnt[e] = c;
+      s_vis[e] = v;
+      e++;
+    };
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+      if (praw[b]) put(b, (int32_t)praw[b], pv[b]);
+    put(4, 1, pv[4]);
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+      if (sraw[b]) put(8 + b, (int32_t)sraw[b], sv[b]);
+    put(12, 1, sv[4]);
+    int32_t* svis = s_sv + 5 * tid;
+    int32_t* pvis = s_pv + 5 * tid;
+    const uint32_t sids = wire_rank(sraw, sv, svis), pids = wire_rank(praw, pv, pvis);
+    if (sc + sv[4] != pc + pv[4]) {
+      atomicOr(err, CE_BALANCE);
+    } else {
+      // the ranked lists are consumed front to back: a suffix's offset is what has been
+      // taken from it so far, and a prefix's wires are consecutive
+      int32_t* wire = s_wire + 3 * (le + tid);
+      const int nw = np + ns + 1;
+      int leftover = sc + sv[4];
+      int top_p = 0, top_s = 0, var_p = 0, var_s = 0, wi = 0, first = 0;
+      while (leftover > 0) {
+        if (top_p >= np || top_s >= ns || wi >= nw) {
+          atomicOr(err, CE_BOUNDS);
+          break;
+        }
+        const int32_t pcur = pvis[top_p], scur = svis[top_s];
+        const int c = min(pcur - var_p, scur - var_s);
+        wire[3 * wi + 0] = (int32_t)((sids >> (4 * top_s)) & 15u);
+        wire[3 * wi + 1] = var_s;
+        wire[3 * wi + 2] = c;
+        wi++;
+        leftover -= c;
+        var_p += c;
+        var_s += c;
+        if (var_p == pcur) {
+          s_beg[le + ((pids >> (4 * top_p)) & 15u)] = (uint16_t)(first | (wi - first) << 8);
+          first = wi;
+          var_p = 0;
+          top_p++;
+        }
+        if (var_s == scur) {
+          var_s = 0;
+          top_s++;
+        }
+      }
+    }
   }
-  const KeyT key = nkeys[i];
-  const uint32_t e0 = col[i].x;
-  s.eoff[i] = e0;
-  const uint32_t sc4[4] = {nsuf[i].x, nsuf[i].y, nsuf[i].z, nsuf[i].w};
-  const uint32_t pc4[4] = {npre[i].x, npre[i].y, npre[i].z, npre[i].w};
-  int32_t pcnt[5], pvis[5], scnt[5], svis[5];
-  bool pempty[5], sempty[5];
-  int np = 0, ns = 0;
+  __syncthreads();
   const KeyT lmask = low_mask<KeyT>(L);
-  uint32_t e = e0;
-  for (int b = 0; b < 4; b++)
-    if (pc4[b]) {
-      pcnt[np] = (int32_t)pc4[b];
-      pvis[np] = visit_of(pcnt[np], cov);
-      pempty[np] = false;
-      s.xoff[e] = (uint64_t)b;  // the arena's first word holds A, C, T, G
-      s.xlen[e] = 1;
-      s.nbr[e] = ((KeyT)b << (2 * (L - 1))) | (key >> 2);
-      e++;
-      np++;
-    }
-  pcnt[np] = -1;
-  pvis[np] = -1;
-  pempty[np] = true;
-  s.xoff[e] = 0;
-  s.xlen[e] = kTerm;
-  s.nbr[e] = 0;
-  e++;
-  np++;
-  for (int b = 0; b < 4; b++)
-    if (sc4[b]) {
-      scnt[ns] = (int32_t)sc4[b];
-      svis[ns] = visit_of(scnt[ns], cov);
-      sempty[ns] = false;
-      s.xoff[e] = (uint64_t)b;
-      s.xlen[e] = 1;
-      s.nbr[e] = ((key << 2) | (KeyT)b) & lmask;
-      e++;
-      ns++;
-    }
-  scnt[ns] = -1;
-  svis[ns] = -1;
-  sempty[ns] = true;
-  s.xoff[e] = 0;
-  s.xlen[e] = kTerm;
-  s.nbr[e] = 0;
-  ns++;
-  s.key[i] = key;
-  s.npre[i] = (uint32_t)np;
-  setup_wiring(np, pcnt, pvis, pempty, ns, scnt, svis, sempty, s.wire + e0 + i, s.beg + e0, err);
-  for (int q = 0; q < np; q++) {
-    s.cnt[e0 + q] = pcnt[q];
-    s.vis[e0 + q] = pvis[q];
+  for (uint32_t j = tid; j < M; j += kInitT) {
+    const uint32_t what = s_what[j], b = what & 3u, d = E0 + j;
+    const KeyT key = s_key[s_node[j]];
+    const bool term = (what & 4u) != 0;
+    s.xoff[d] = (uint64_t)b;  // the arena's first word holds A, C, T, G
+    s.xlen[d] = term ? kTerm : 1u;
+    s.nbr[d] = term ? (KeyT)0 : (what & 8u) ? ((key << 2) | (KeyT)b) & lmask : ((KeyT)b << (2 * (L - 1))) | (key >> 2);
+    s.cnt[d] = s_cnt[j];
+    s.vis[d] = s_vis[j];
+    s.beg[d] = make_int2(s_beg[j] & 0xff, s_beg[j] >> 8);
   }
-  for (int q = 0; q < ns; q++) {
-    s.cnt[e0 + np + q] = scnt[q];
-    s.vis[e0 + np + q] = svis[q];
-    s.beg[e0 + np + q] = make_int2(0, 0);
-  }
+  int32_t* wout = reinterpret_cast<int32_t*>(s.wire + E0 + i0);
+  for (uint32_t w = tid; w < words; w += kInitT) wout[w] = s_wire[w];
 }
 
 // ------------------------------------------------------------------ round --------
@@ -735,15 +784,17 @@ __global__ void __launch_bounds__(128) k_cp_apply(Side<KeyT> a, Side<KeyT> b, ui
 //                share bounds and where the successor's wires start
 //   k_walk<0>    one warp per begin k-mer (identify_begin_kmers,
 //                src/iterative_compaction.cpp:65-93) runs the depth-first walk over the
-//                records; it counts contigs, bases and pieces
-//   k_walk<1>    the same walk writes each contig's begin key and its pieces (the begin
-//                prefix and every frame's suffix, as arena views), 32 pieces at a time
+//                records; it counts contigs, bases and pieces, and records each contig and
+//                its pieces (the begin prefix and every frame's suffix, as arena views, 32
+//                at a time) while there is room for them
+//   k_wk_contigs each recorded contig's place and the bases of its begin key
+//   k_walk<1>    where there was no room, the same walk again writes contigs and pieces
 //   k_wk_expand  one warp per piece writes its bases (one byte per base)
 // A walk is a chain of dependent loads, so a step makes one: its wire's record.  A frame
 // goes on the resume stack only when something of its share is left after the child (a
 // wire that takes the whole share ends its frame, since later wires start past it); the
 // path itself is a second stack that only a contig reads.  45.6k nodes, 463 begins: 1.63 ms
-// a walk; reading wire, entry, link and successor one after the other, and popping every
+// for counting and writing walk, 0.99 ms for one that records; reading wire, entry, link and successor one after the other, and popping every
 // frame of the path after every contig, took 5.50 ms.
 struct WStep {
   uint64_t xoff;   // the suffix's bases in the arena
@@ -767,8 +818,13 @@ struct WPath {
 };
 struct WPiece {
   uint64_t src;  // arena base offset
-  uint64_t dst;  // output byte offset
-  uint32_t len, pad;
+  uint64_t dst;  // output byte offset, after that of walk `walk` where the walks' are given
+  uint32_t len, walk;
+};
+struct WContig {   // a contig that k_walk<0> recorded
+  uint64_t dst;    // output byte offset after its walk's
+  uint32_t walk;
+  uint32_t index;  // among its walk's contigs
 };
 
 __global__ void k_wk_begin_count(const uint32_t* __restrict__ eoff, const uint32_t* __restrict__ npre,
@@ -902,7 +958,8 @@ __global__ void __launch_bounds__(128) k_walk(Side<KeyT> s, int L, const uint2* 
                                               WPath* __restrict__ path, uint32_t cap, uint4* __restrict__ col,
                                               const uint4* __restrict__ off, uint64_t* __restrict__ ct_off,
                                               WPiece* __restrict__ pieces, uint8_t* __restrict__ out,
-                                              uint32_t* err) {
+                                              WContig* __restrict__ contigs, uint32_t ccap, uint32_t pcap,
+                                              unsigned long long* recorded, uint32_t* err) {
   // one walk per warp: independent walks diverge completely, so they do not share one.
   // All lanes step together (same loads); lane 0 stores the frames.
   const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -915,6 +972,7 @@ __global__ void __launch_bounds__(128) k_walk(Side<KeyT> s, int L, const uint2* 
   const uint32_t plen0 = s.xlen[be] & kLenMask;
   uint32_t nct = 0, npc = 0;
   uint64_t nbases = 0;
+  bool room = true;
   uint32_t ci = PASS ? off[b].x : 0u, pc = PASS ? off[b].z : 0u;
   uint64_t bo = PASS ? off[b].y : 0ull;
   uint32_t d = 0, rp = 0, len = plen0 + (uint32_t)L;
@@ -970,7 +1028,32 @@ __global__ void __launch_bounds__(128) k_walk(Side<KeyT> s, int L, const uint2* 
         }
         bo += clen;
       } else {
-        npc += (plen0 ? 1u : 0u) + (sl ? 1u : 0u) + d;
+        const uint32_t m = (plen0 ? 1u : 0u) + (sl ? 1u : 0u) + d;
+        npc += m;
+        if (room) {  // records, in any order: the first walk that finds no room is the sign to walk again
+          unsigned long long c0 = 0, p0 = 0;
+          __syncwarp();  // lane 0's path stores before every lane reads them
+          if (lane == 0) {
+            c0 = atomicAdd(recorded, 1ull);
+            p0 = atomicAdd(recorded + 1, (unsigned long long)m);
+          }
+          c0 = __shfl_sync(~0u, c0, 0);
+          p0 = __shfl_sync(~0u, p0, 0);
+          room = c0 < ccap && p0 + m <= pcap;
+          if (room) {
+            WPiece* to = pieces + p0;
+            if (lane == 0) {
+              contigs[c0] = WContig{nbases, b, nct};
+              if (plen0) to[0] = WPiece{s.xoff[be], nbases, plen0, b};
+              if (sl) to[m - 1] = WPiece{w.xoff, nbases + len, sl, b};
+            }
+            if (plen0) to++;
+            for (uint32_t q = lane; q < d; q += 32) {
+              const WPath g = ps[q];
+              to[q] = WPiece{g.src, nbases + g.lenb, g.len, b};
+            }
+          }
+        }
       }
       nct++;
       nbases += clen;
@@ -1010,12 +1093,32 @@ __global__ void __launch_bounds__(128) k_walk(Side<KeyT> s, int L, const uint2* 
 }
 
 // one warp per piece: its bases, one byte each
+// (off: the walks' output offsets that the pieces' are relative to, or null)
 __global__ void k_wk_expand(const WPiece* __restrict__ pieces, uint32_t np, const uint64_t* __restrict__ ar,
-                            uint8_t* __restrict__ out) {
+                            const uint4* __restrict__ off, uint8_t* __restrict__ out) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= np) return;
   const WPiece pc = pieces[w];
-  for (uint32_t i = lane; i < pc.len; i += 32) out[pc.dst + i] = (uint8_t)(ar_get(ar, pc.src + i) >> 62);
+  uint8_t* o = out + pc.dst + (off ? off[pc.walk].y : 0u);
+  for (uint32_t i = lane; i < pc.len; i += 32) o[i] = (uint8_t)(ar_get(ar, pc.src + i) >> 62);
+}
+
+// one warp per recorded contig: its place among all contigs and its begin key's bases
+template <typename KeyT>
+__global__ void __launch_bounds__(256) k_wk_contigs(Side<KeyT> s, int L, const uint2* __restrict__ begins,
+                                                    const WContig* __restrict__ contigs, uint32_t nc,
+                                                    const uint4* __restrict__ off, uint64_t* __restrict__ ct_off,
+                                                    uint8_t* __restrict__ out) {
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= nc) return;
+  const WContig c = contigs[w];
+  const uint4 o = off[c.walk];
+  const uint2 bg = begins[c.walk];
+  const uint64_t bo = o.y + c.dst;
+  const uint32_t plen0 = s.xlen[s.eoff[bg.x] + bg.y] & kLenMask;
+  if (lane == 0) ct_off[o.x + c.index] = bo;
+  for (uint32_t x = lane; x < (uint32_t)L; x += 32)
+    out[bo + plen0 + x] = (uint8_t)key_bases(s.key[bg.x], L, (int)x, 1);
 }
 
 // ------------------------------------------------------------- copy-out ---------
@@ -1076,7 +1179,7 @@ struct CpState {
   DevBuf side[2][NSIDE];
   DevBuf arena, col, off, part, is_id, tkey, tr, tgt, incnt, inoff, fill, inlist, ecol, eoff2, old_of, ct, tot,
       epos, cpos, ubuf, wk_begins, wk_resume, wk_path, wk_col, wk_pos, wk_off, wk_out, wk_links, wk_steps,
-      wk_pieces;
+      wk_pieces, wk_contigs;
   uint64_t wk_begins_n = 0, wk_n = 0, wk_bases = 0;
   uint32_t wk_depth = 0;
   bool wk_done = false;
@@ -1192,7 +1295,7 @@ pk_status cp_init(pk_job* j, CpState& c, int32_t cov) {
   PK_CUDA(cudaMemsetAsync(c.arena.p, 0, 16, j->stream));
   PK_CUDA(cudaMemcpyAsync(c.arena.p, &w0, 8, cudaMemcpyHostToDevice, j->stream));
   c.arena_words = 1;
-  pk::note_launch(), k_cp_init<KeyT><<<blocks(m + 1, 128), 128, 0, j->stream>>>((const KeyT*)j->nkeys.p, (const uint4*)j->nsuf.p,
+  pk::note_launch(), k_cp_init<KeyT><<<blocks(m + 1, kInitT), kInitT, 0, j->stream>>>((const KeyT*)j->nkeys.p, (const uint4*)j->nsuf.p,
                                                               (const uint4*)j->npre.p, (uint32_t)m, c.L, cov,
                                                               (const uint4*)c.off.p, side_of<KeyT>(c, 0), c.d_err);
   PK_CUDA(cudaGetLastError());
@@ -1322,27 +1425,40 @@ pk_status cp_walk(pk_job* j, CpState& c) {
   PK_TRY(cp_alloc(j, c.wk_path, sizeof(WPath) * cap * std::max<uint64_t>(B, 1)));
   PK_TRY(cp_alloc(j, c.wk_col, sizeof(uint4) * (B + 1)));
   PK_TRY(cp_alloc(j, c.wk_pos, sizeof(uint4) * (B + 1)));
+  // room for the contigs and pieces that the counting walk records: walks of a compacted map
+  // visit most wires a few times at most
+  const uint64_t pcap = std::min<uint64_t>(kWalkRecords, 2 * (c.E + n) + 1024), ccap = pcap / 4;
+  PK_TRY(cp_alloc(j, c.wk_pieces, sizeof(WPiece) * pcap));
+  PK_TRY(cp_alloc(j, c.wk_contigs, sizeof(WContig) * ccap));
+  PK_TRY(cp_alloc(j, c.tot, 2 * sizeof(unsigned long long)));
+  PK_CUDA(cudaMemsetAsync(c.tot.p, 0, 2 * sizeof(unsigned long long), st));
   if (B)
-    pk::note_launch(), k_walk<KeyT, 0><<<blocks(B * 32, 128), 128, 0, st>>>(a, c.L, (const uint2*)c.wk_begins.p, (uint32_t)B,
-                                                   (const WStep*)c.wk_steps.p, (WResume*)c.wk_resume.p, (WPath*)c.wk_path.p,
-                                                   (uint32_t)cap,
-                                                   (uint4*)c.wk_col.p, nullptr, nullptr, nullptr, nullptr, c.d_err);
+    pk::note_launch(), k_walk<KeyT, 0><<<blocks(B * 32, 128), 128, 0, st>>>(
+        a, c.L, (const uint2*)c.wk_begins.p, (uint32_t)B, (const WStep*)c.wk_steps.p, (WResume*)c.wk_resume.p,
+        (WPath*)c.wk_path.p, (uint32_t)cap, (uint4*)c.wk_col.p, nullptr, nullptr, (WPiece*)c.wk_pieces.p, nullptr,
+        (WContig*)c.wk_contigs.p, (uint32_t)ccap, (uint32_t)pcap, (unsigned long long*)c.tot.p, c.d_err);
   PK_TRY(scan4(j, c, (const uint4*)c.wk_col.p, (uint4*)c.wk_pos.p, B));
   PK_TRY(read_total(j, c, (const uint4*)c.wk_pos.p + B, &t));
   PK_TRY(check_err(c));
   const uint64_t NC = t.x, NB = t.y, NP = t.z;
   PK_TRY(cp_alloc(j, c.wk_off, 8 * (NC + 1)));
   PK_TRY(cp_alloc(j, c.wk_out, NB + 1));
-  PK_TRY(cp_alloc(j, c.wk_pieces, sizeof(WPiece) * (NP + 1)));
-  if (B)
-    pk::note_launch(), k_walk<KeyT, 1><<<blocks(B * 32, 128), 128, 0, st>>>(a, c.L, (const uint2*)c.wk_begins.p, (uint32_t)B,
-                                                   (const WStep*)c.wk_steps.p, (WResume*)c.wk_resume.p, (WPath*)c.wk_path.p,
-                                                   (uint32_t)cap,
-                                                   nullptr, (const uint4*)c.wk_pos.p, (uint64_t*)c.wk_off.p,
-                                                   (WPiece*)c.wk_pieces.p, (uint8_t*)c.wk_out.p, c.d_err);
+  const bool recorded = NC <= ccap && NP <= pcap;
+  if (recorded && NC) {
+    pk::note_launch(), k_wk_contigs<KeyT><<<blocks(NC * 32, 256), 256, 0, st>>>(
+        a, c.L, (const uint2*)c.wk_begins.p, (const WContig*)c.wk_contigs.p, (uint32_t)NC, (const uint4*)c.wk_pos.p,
+        (uint64_t*)c.wk_off.p, (uint8_t*)c.wk_out.p);
+  } else if (!recorded) {
+    PK_TRY(cp_alloc(j, c.wk_pieces, sizeof(WPiece) * (NP + 1)));
+    pk::note_launch(), k_walk<KeyT, 1><<<blocks(B * 32, 128), 128, 0, st>>>(
+        a, c.L, (const uint2*)c.wk_begins.p, (uint32_t)B, (const WStep*)c.wk_steps.p, (WResume*)c.wk_resume.p,
+        (WPath*)c.wk_path.p, (uint32_t)cap, nullptr, (const uint4*)c.wk_pos.p, (uint64_t*)c.wk_off.p,
+        (WPiece*)c.wk_pieces.p, (uint8_t*)c.wk_out.p, nullptr, 0u, 0u, nullptr, c.d_err);
+  }
   if (NP)
-    pk::note_launch(), k_wk_expand<<<blocks(NP * 32, 256), 256, 0, st>>>((const WPiece*)c.wk_pieces.p, (uint32_t)NP,
-                                                       (const uint64_t*)c.arena.p, (uint8_t*)c.wk_out.p);
+    pk::note_launch(), k_wk_expand<<<blocks(NP * 32, 256), 256, 0, st>>>(
+        (const WPiece*)c.wk_pieces.p, (uint32_t)NP, (const uint64_t*)c.arena.p,
+        recorded ? (const uint4*)c.wk_pos.p : nullptr, (uint8_t*)c.wk_out.p);
   PK_CUDA(cudaMemcpyAsync((uint64_t*)c.wk_off.p + NC, &NB, 8, cudaMemcpyHostToDevice, st));
   PK_CUDA(cudaGetLastError());
   PK_TRY(read_total(j, c, (const uint4*)c.wk_pos.p + B, &t));
@@ -1371,7 +1487,8 @@ void pk::cp_free(pk_job* j) {
                     &c->tr,     &c->tgt,      &c->incnt,  &c->inoff,  &c->fill,   &c->inlist,
                     &c->ecol,   &c->eoff2,    &c->old_of, &c->ct,     &c->tot,    &c->epos,
                     &c->cpos,   &c->ubuf,     &c->wk_begins, &c->wk_resume, &c->wk_path, &c->wk_col,
-                    &c->wk_pos, &c->wk_off, &c->wk_out, &c->wk_links, &c->wk_steps, &c->wk_pieces};
+                    &c->wk_pos, &c->wk_off, &c->wk_out, &c->wk_links, &c->wk_steps, &c->wk_pieces,
+                    &c->wk_contigs};
   for (DevBuf* d : rest) drop(*d);
   if (c->d_err) cudaFree(c->d_err);
   if (c->h_tot) cudaFreeHost(c->h_tot);

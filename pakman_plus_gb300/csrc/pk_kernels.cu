@@ -26,6 +26,7 @@
 #include <atomic>
 
 #include "pk_internal.h"
+#include "pk_wire.cuh"
 
 namespace pk {
 
@@ -3345,30 +3346,6 @@ namespace pk {
 // 1970 us.  128 nodes a CTA: a multiple of 16 bytes of rows, eight CTAs' rows on an SM.
 constexpr int kWireT = 128;                            // nodes per CTA
 constexpr int kWireW = (int)(sizeof(WireRow) / 4);     // words of a row (42)
-
-// Ranks of a side's five slots (four base codes and the terminal entry) among the present
-// ones; their visits land in vis[rank] and the list positions of the ranked entries come
-// back four bits each.
-__device__ __forceinline__ uint32_t wire_rank(const uint32_t raw[4], const int32_t v[5], int32_t* vis) {
-  uint32_t pos = 0, ids = 0;  // pos: present slots so far
-#pragma unroll
-  for (int e = 0; e < 5; e++) {
-    if (e < 4 && !raw[e]) continue;
-    const int32_t ce = e < 4 ? (int32_t)raw[e] : 1;
-    uint32_t rank = 0;
-#pragma unroll
-    for (int o = 0; o < 5; o++) {
-      if (o == e || (o < 4 && !raw[o])) continue;
-      const int32_t co = o < 4 ? (int32_t)raw[o] : 1;
-      const bool same = v[o] == v[e] && co == ce;
-      rank += (v[o] > v[e] || (v[o] == v[e] && co > ce) || (same && o < e)) ? 1u : 0u;
-    }
-    vis[rank] = v[e];
-    ids |= pos << (4 * rank);
-    pos++;
-  }
-  return ids;
-}
 
 __global__ void __launch_bounds__(kWireT, 8) k_wire(const uint4* __restrict__ nsuf, const uint4* __restrict__ npre,
                                                     unsigned long long m, int coverage,
