@@ -303,6 +303,8 @@ void pk_job_destroy(pk_job* j) {
   }
   if (j->d_sc) cudaFree(j->d_sc);
   if (j->h_sc) cudaFreeHost(j->h_sc);
+  if (j->cp_dev) cudaFree(j->cp_dev);
+  if (j->cp_host) cudaFreeHost(j->cp_host);
   for (int i = 0; i < pk_job::kIngestBufs; i++) {
     if (j->ing_host[i]) cudaFreeHost(j->ing_host[i]);
     if (j->ing_ev[i]) cudaEventDestroy(j->ing_ev[i]);

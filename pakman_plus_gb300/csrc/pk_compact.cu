@@ -261,50 +261,68 @@ __device__ bool setup_wiring(int np, int32_t* pcnt, int32_t* pvis, const bool* p
 __device__ __forceinline__ uint4 operator+(uint4 a, uint4 b) {
   return make_uint4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
-__device__ __forceinline__ uint4 shfl_up4(uint4 v, int d) {
+__device__ __forceinline__ uint4 operator-(uint4 a, uint4 b) {
+  return make_uint4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w);
+}
+__device__ __forceinline__ uint4 shfl_up_v(uint4 v, int d) {
   return make_uint4(__shfl_up_sync(~0u, v.x, d), __shfl_up_sync(~0u, v.y, d), __shfl_up_sync(~0u, v.z, d),
                     __shfl_up_sync(~0u, v.w, d));
 }
+__device__ __forceinline__ uint32_t shfl_up_v(uint32_t v, int d) { return __shfl_up_sync(~0u, v, d); }
+__device__ __forceinline__ uint4 as_uint4(uint4 v) { return v; }
+__device__ __forceinline__ uint4 as_uint4(uint32_t v) { return make_uint4(v, 0, 0, 0); }
 
-// exclusive block scan of one uint4 per thread (kScanT threads); returns the total too
-__device__ uint4 block_scan4(uint4 v, uint4* s_w, uint4& total) {
+// An exclusive scan as its readers see it: sums within a tile, and before every tile.  A
+// round's scans are read once or twice, so adding the two there costs less than a pass over
+// the array.
+template <typename V>
+struct Scanned {
+  const V* v;
+  const V* part;
+  uint32_t n;
+  __device__ __forceinline__ V at(uint32_t i) const { return i < n ? v[i] + part[i / kScanTile] : v[n]; }
+};
+
+// exclusive block scan of one value per thread (kScanT threads); returns the total too
+template <typename V>
+__device__ V block_scan(V v, V* s_w, V& total) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint4 inc = v;
+  V inc = v;
   for (int d = 1; d < 32; d <<= 1) {
-    const uint4 o = shfl_up4(inc, d);
+    const V o = shfl_up_v(inc, d);
     if (lane >= d) inc = inc + o;
   }
   if (lane == 31) s_w[wid] = inc;
   __syncthreads();
   if (wid == 0) {
-    uint4 x = lane < (kScanT / 32) ? s_w[lane] : make_uint4(0, 0, 0, 0);
+    V x = lane < (kScanT / 32) ? s_w[lane] : V{};
     for (int d = 1; d < 32; d <<= 1) {
-      const uint4 o = shfl_up4(x, d);
+      const V o = shfl_up_v(x, d);
       if (lane >= d) x = x + o;
     }
     s_w[lane] = x;  // inclusive over warps
   }
   __syncthreads();
   total = s_w[kScanT / 32 - 1];
-  const uint4 before = wid ? s_w[wid - 1] : make_uint4(0, 0, 0, 0);
-  const uint4 ex = inc + make_uint4(0u - v.x, 0u - v.y, 0u - v.z, 0u - v.w);
+  const V before = wid ? s_w[wid - 1] : V{};
   __syncthreads();
-  return before + ex;
+  return before + (inc - v);
 }
 
 // pass 1: tile-local exclusive scan into out, tile totals into part
-__global__ void __launch_bounds__(kScanT) k_scan_tiles(const uint4* __restrict__ in, uint4* __restrict__ out,
-                                                      uint4* __restrict__ part, uint32_t n) {
-  __shared__ uint4 s_w[32];
+template <typename V>
+__global__ void __launch_bounds__(kScanT) k_scan_tiles(const V* __restrict__ in, V* __restrict__ out,
+                                                      V* __restrict__ part, uint32_t n) {
+  __shared__ V s_w[32];
   const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanPer;
-  uint4 v[kScanPer], sum = make_uint4(0, 0, 0, 0);
+  V v[kScanPer], sum = V{};
 #pragma unroll
   for (int q = 0; q < kScanPer; q++) {
-    v[q] = base + q < n ? in[base + q] : make_uint4(0, 0, 0, 0);
+    v[q] = base + q < n ? in[base + q] : V{};
     sum = sum + v[q];
   }
-  uint4 tot;
-  uint4 ex = block_scan4(sum, s_w, tot);
+  V tot;
+  V ex = block_scan(sum, s_w, tot);
 #pragma unroll
   for (int q = 0; q < kScanPer; q++) {
     if (base + q < n) out[base + q] = ex;
@@ -313,20 +331,25 @@ __global__ void __launch_bounds__(kScanT) k_scan_tiles(const uint4* __restrict__
   if (threadIdx.x == 0) part[blockIdx.x] = tot;
 }
 
-// pass 2: one CTA scans the tile totals (any count) and writes the grand total to out[n]
-__global__ void __launch_bounds__(kScanT) k_scan_parts(uint4* __restrict__ part, uint32_t nparts,
-                                                      uint4* __restrict__ out, uint32_t n) {
-  __shared__ uint4 s_w[32];
-  uint4 carry = make_uint4(0, 0, 0, 0);
+// pass 2: one CTA scans the tile totals (any count) and writes the grand total to out[n] and
+// *total
+template <typename V>
+__global__ void __launch_bounds__(kScanT) k_scan_parts(V* __restrict__ part, uint32_t nparts,
+                                                      V* __restrict__ out, uint32_t n, uint4* __restrict__ total) {
+  __shared__ V s_w[32];
+  V carry = V{};
   for (uint32_t b = 0; b < nparts; b += kScanT) {
     const uint32_t i = b + threadIdx.x;
-    const uint4 v = i < nparts ? part[i] : make_uint4(0, 0, 0, 0);
-    uint4 tot;
-    const uint4 ex = block_scan4(v, s_w, tot);
+    const V v = i < nparts ? part[i] : V{};
+    V tot;
+    const V ex = block_scan(v, s_w, tot);
     if (i < nparts) part[i] = carry + ex;
     carry = carry + tot;
   }
-  if (threadIdx.x == 0) out[n] = carry;
+  if (threadIdx.x == 0) {
+    out[n] = carry;
+    *total = as_uint4(carry);
+  }
 }
 
 __global__ void k_scan_add(uint4* __restrict__ out, const uint4* __restrict__ part, uint32_t n) {
@@ -528,7 +551,7 @@ __global__ void __launch_bounds__(256) k_cp_mark(Side<KeyT> s, uint32_t n, int L
 }
 
 template <typename KeyT>
-__global__ void __launch_bounds__(256) k_cp_emit(Side<KeyT> s, uint32_t n, int L, const uint4* __restrict__ off,
+__global__ void __launch_bounds__(256) k_cp_emit(Side<KeyT> s, uint32_t n, int L, Scanned<uint4> off,
                                                  const uint8_t* __restrict__ is_id, uint64_t* __restrict__ ar,
                                                  uint64_t ar_word0, uint64_t ar_cap_words, KeyT* __restrict__ tkey,
                                                  Tr* __restrict__ tr, Ct* __restrict__ ct, uint64_t ct0,
@@ -537,7 +560,7 @@ __global__ void __launch_bounds__(256) k_cp_emit(Side<KeyT> s, uint32_t n, int L
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const KeyT key = s.key[i];
-  const uint4 o = off[i];
+  const uint4 o = off.at(i);
   if (!is_id[i]) {
     nkey[o.w] = key;
     old_of[o.w] = i;
@@ -572,7 +595,7 @@ __global__ void __launch_bounds__(256) k_cp_emit(Side<KeyT> s, uint32_t n, int L
 
 template <typename KeyT>
 __global__ void k_cp_resolve(const KeyT* __restrict__ tkey, uint32_t T, const KeyT* __restrict__ nkey, uint32_t n,
-                             uint32_t* __restrict__ tgt, uint4* __restrict__ incnt, uint32_t* err) {
+                             uint32_t* __restrict__ tgt, uint32_t* __restrict__ incnt, uint32_t* err) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   const KeyT k = tkey[t];
@@ -588,16 +611,16 @@ __global__ void k_cp_resolve(const KeyT* __restrict__ tkey, uint32_t T, const Ke
     return;
   }
   tgt[t] = lo;
-  atomicAdd(&incnt[lo].x, 1u);
+  atomicAdd(&incnt[lo], 1u);
 }
 
-__global__ void k_cp_fill(const uint32_t* __restrict__ tgt, uint32_t T, const uint4* __restrict__ inoff,
+__global__ void k_cp_fill(const uint32_t* __restrict__ tgt, uint32_t T, Scanned<uint32_t> inoff,
                           uint32_t* __restrict__ fill, uint32_t* __restrict__ inlist) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   const uint32_t g = tgt[t];
   if (g == ~0u) return;
-  inlist[inoff[g].x + atomicAdd(&fill[g], 1u)] = t;
+  inlist[inoff.at(g) + atomicAdd(&fill[g], 1u)] = t;
 }
 
 // A list entry during the replay: an old entry (>= 0) or incoming transfer t (-1 - t).
@@ -610,26 +633,27 @@ struct Replay {
 template <typename KeyT, int PASS>
 __global__ void __launch_bounds__(128) k_cp_apply(Side<KeyT> a, Side<KeyT> b, uint32_t n, int L,
                                                   const uint32_t* __restrict__ old_of,
-                                                  const uint4* __restrict__ inoff, uint32_t* __restrict__ inlist,
+                                                  Scanned<uint32_t> inoff, uint32_t* __restrict__ inlist,
                                                   const Tr* __restrict__ tr, const uint64_t* __restrict__ ar,
-                                                  uint4* __restrict__ ecol, uint32_t* err) {
+                                                  uint32_t* __restrict__ ecol, Scanned<uint32_t> eoff,
+                                                  uint32_t* err) {
   const uint32_t ni = blockIdx.x * blockDim.x + threadIdx.x;
   if (ni > n) return;
   if (PASS == 1 && ni == n) {
-    b.eoff[n] = ecol[n].x;
+    b.eoff[n] = eoff.at(n);
     return;
   }
   if (ni == n) return;
-  if (PASS == 1) b.eoff[ni] = ecol[ni].x;
+  const uint32_t d0 = PASS == 1 ? eoff.at(ni) : 0u;
+  if (PASS == 1) b.eoff[ni] = d0;
   const uint32_t i = old_of[ni];
   const uint32_t e0 = a.eoff[i], e1 = a.eoff[i + 1], np0 = a.npre[i];
-  const uint32_t q0 = inoff[ni].x, q1 = inoff[ni + 1].x;
+  const uint32_t q0 = inoff.at(ni), q1 = inoff.at(ni + 1);
   if (q0 == q1) {  // untouched: entries, begin slots and wires carry over
     if (PASS == 0) {
-      ecol[ni] = make_uint4(e1 - e0, 0, 0, 0);
+      ecol[ni] = e1 - e0;
       return;
     }
-    const uint32_t d0 = ecol[ni].x;
     b.npre[ni] = np0;
     for (uint32_t e = e0; e < e1; e++) {
       const uint32_t d = d0 + (e - e0);
@@ -659,7 +683,7 @@ __global__ void __launch_bounds__(128) k_cp_apply(Side<KeyT> a, Side<KeyT> b, ui
   r.ns = (int)(e1 - e0 - np0);
   if (r.np > kMaxList || r.ns > kMaxList) {
     atomicOr(err, CE_LIST);
-    if (PASS == 0) ecol[ni] = make_uint4(e1 - e0, 0, 0, 0);
+    if (PASS == 0) ecol[ni] = e1 - e0;
     return;
   }
   for (int q = 0; q < r.np; q++) r.pre[q] = (int)(e0 + q);
@@ -715,15 +739,14 @@ __global__ void __launch_bounds__(128) k_cp_apply(Side<KeyT> a, Side<KeyT> b, ui
   }
   if (over) {
     atomicOr(err, CE_LIST);
-    if (PASS == 0) ecol[ni] = make_uint4(e1 - e0, 0, 0, 0);
+    if (PASS == 0) ecol[ni] = e1 - e0;
     return;
   }
   if (PASS == 0) {
-    ecol[ni] = make_uint4((uint32_t)(r.np + r.ns), 0, 0, 0);
+    ecol[ni] = (uint32_t)(r.np + r.ns);
     return;
   }
   // write the lists, then re-wire
-  const uint32_t d0 = ecol[ni].x;
   int32_t pcnt[kMaxList], pvis[kMaxList], scnt[kMaxList], svis[kMaxList];
   bool pempty[kMaxList], sempty[kMaxList];
   for (int side = 0; side < 2; side++) {
@@ -1177,7 +1200,7 @@ struct CpState {
     KEY, EOFF, NPRE, XOFF, XLEN, CNT, VIS, NBR, BEG, WIRE, NSIDE
   };
   DevBuf side[2][NSIDE];
-  DevBuf arena, col, off, part, is_id, tkey, tr, tgt, incnt, inoff, fill, inlist, ecol, eoff2, old_of, ct, tot,
+  DevBuf arena, col, off, part, in_part, is_id, tkey, tr, tgt, incnt, inoff, fill, inlist, ecol, eoff2, old_of, ct, tot,
       epos, cpos, ubuf, wk_begins, wk_resume, wk_path, wk_col, wk_pos, wk_off, wk_out, wk_links, wk_steps,
       wk_pieces, wk_contigs;
   uint64_t wk_begins_n = 0, wk_n = 0, wk_bases = 0;
@@ -1190,8 +1213,8 @@ struct CpState {
   int L = 0;
   bool wide = false;
   bool done = false;
-  uint32_t* d_err = nullptr;
-  uint4* h_tot = nullptr;  // pinned
+  uint32_t* d_err = nullptr;  // error bits, and from word 4 the last scan's four totals
+  uint4* h_tot = nullptr;     // their pinned mirror; both belong to the job
 };
 
 }  // namespace pk
@@ -1236,28 +1259,39 @@ pk_status alloc_side(pk_job* j, CpState& c, int s, uint64_t n, uint64_t E) {
   return PK_OK;
 }
 
-// exclusive scan of n uint4 (in place allowed: in == out is not; out holds n+1)
-pk_status scan4(pk_job* j, CpState& c, const uint4* in, uint4* out, uint64_t n) {
+// Exclusive scan of n values by tiles (out holds n + 1, not in place): *r reads it.  The
+// total goes to the report that read_total reads.
+template <typename V>
+pk_status scan(pk_job* j, CpState& c, const V* in, V* out, DevBuf& parts, uint64_t n, Scanned<V>* r) {
   const uint32_t tiles = (uint32_t)((n + kScanTile - 1) / kScanTile);
-  PK_TRY(cp_alloc(j, c.part, sizeof(uint4) * (tiles + 1)));
-  uint4* part = (uint4*)c.part.p;
-  if (tiles) pk::note_launch(), k_scan_tiles<<<tiles, kScanT, 0, j->stream>>>(in, out, part, (uint32_t)n);
-  pk::note_launch(), k_scan_parts<<<1, kScanT, 0, j->stream>>>(part, tiles, out, (uint32_t)n);
-  if (n) pk::note_launch(), k_scan_add<<<(uint32_t)((n + 255) / 256), 256, 0, j->stream>>>(out, part, (uint32_t)n);
+  PK_TRY(cp_alloc(j, parts, sizeof(V) * (tiles + 1)));
+  V* part = (V*)parts.p;
+  if (tiles) pk::note_launch(), k_scan_tiles<V><<<tiles, kScanT, 0, j->stream>>>(in, out, part, (uint32_t)n);
+  pk::note_launch(), k_scan_parts<V><<<1, kScanT, 0, j->stream>>>(part, tiles, out, (uint32_t)n, (uint4*)(c.d_err + 4));
+  PK_CUDA(cudaGetLastError());
+  if (r) *r = Scanned<V>{out, part, (uint32_t)n};
+  return PK_OK;
+}
+
+// the same of uint4, added up in place
+pk_status scan4(pk_job* j, CpState& c, const uint4* in, uint4* out, uint64_t n) {
+  PK_TRY(scan<uint4>(j, c, in, out, c.part, n, nullptr));
+  if (n)
+    pk::note_launch(), k_scan_add<<<(uint32_t)((n + 255) / 256), 256, 0, j->stream>>>(out, (const uint4*)c.part.p, (uint32_t)n);
   PK_CUDA(cudaGetLastError());
   return PK_OK;
 }
 
-pk_status read_total(pk_job* j, CpState& c, const uint4* at, uint4* out) {
-  PK_CUDA(cudaMemcpyAsync(c.h_tot, at, sizeof(uint4), cudaMemcpyDeviceToHost, j->stream));
-  PK_CUDA(cudaMemcpyAsync(c.h_tot + 1, c.d_err, 4, cudaMemcpyDeviceToHost, j->stream));
+// waits for the stream: the last scan's total, and the error bits for check_err
+pk_status read_total(pk_job* j, CpState& c, uint4* out) {
+  PK_CUDA(cudaMemcpyAsync(c.h_tot, c.d_err, 2 * sizeof(uint4), cudaMemcpyDeviceToHost, j->stream));
   PK_CUDA(cudaStreamSynchronize(j->stream));
-  *out = c.h_tot[0];
+  *out = c.h_tot[1];
   return PK_OK;
 }
 
 pk_status check_err(CpState& c) {
-  const uint32_t e = c.h_tot[1].x;
+  const uint32_t e = c.h_tot[0].x;
   if (!e) return PK_OK;
   std::string m = "compaction: ";
   if (e & CE_LIST) m += "a prefix or suffix list grew past 32 entries; ";
@@ -1283,7 +1317,7 @@ pk_status cp_init(pk_job* j, CpState& c, int32_t cov) {
                                                                   (uint32_t)m, (uint4*)c.col.p);
   PK_TRY(scan4(j, c, (const uint4*)c.col.p, (uint4*)c.off.p, m));
   uint4 tot;
-  PK_TRY(read_total(j, c, (const uint4*)c.off.p + m, &tot));
+  PK_TRY(read_total(j, c, &tot));
   c.n = m;
   c.E = tot.x;
   c.cur = 0;
@@ -1312,9 +1346,10 @@ pk_status cp_round(pk_job* j, CpState& c) {
   PK_TRY(cp_alloc(j, c.off, sizeof(uint4) * (n + 1)));
   PK_TRY(cp_alloc(j, c.is_id, n + 1));
   pk::note_launch(), k_cp_mark<KeyT><<<blocks(n, 256), 256, 0, j->stream>>>(a, (uint32_t)n, c.L, (uint4*)c.col.p, (uint8_t*)c.is_id.p);
-  PK_TRY(scan4(j, c, (const uint4*)c.col.p, (uint4*)c.off.p, n));
+  Scanned<uint4> off{};
+  PK_TRY(scan<uint4>(j, c, (const uint4*)c.col.p, (uint4*)c.off.p, c.part, n, &off));
   uint4 tot;
-  PK_TRY(read_total(j, c, (const uint4*)c.off.p + n, &tot));
+  PK_TRY(read_total(j, c, &tot));
   PK_TRY(check_err(c));
   const uint64_t T = tot.x, C = tot.y, WB = tot.z, n2 = tot.w;
   // capacities: transfers, contigs (kept across rounds), arena (kept), next side
@@ -1337,35 +1372,36 @@ pk_status cp_round(pk_job* j, CpState& c) {
   PK_TRY(cp_alloc(j, c.old_of, 4 * (n2 + 1)));
   Side<KeyT> b = side_of<KeyT>(c, nb);
   pk::note_launch(), k_cp_emit<KeyT><<<blocks(n, 256), 256, 0, j->stream>>>(
-      a, (uint32_t)n, c.L, (const uint4*)c.off.p, (const uint8_t*)c.is_id.p, (uint64_t*)c.arena.p, c.arena_words,
+      a, (uint32_t)n, c.L, off, (const uint8_t*)c.is_id.p, (uint64_t*)c.arena.p, c.arena_words,
       c.arena_cap, (KeyT*)c.tkey.p, (Tr*)c.tr.p, (Ct*)c.ct.p, c.C, b.key, (uint32_t*)c.old_of.p, c.d_err);
   PK_CUDA(cudaGetLastError());
-  PK_TRY(cp_alloc(j, c.incnt, sizeof(uint4) * (n2 + 1)));
-  PK_TRY(cp_alloc(j, c.inoff, sizeof(uint4) * (n2 + 1)));
+  PK_TRY(cp_alloc(j, c.incnt, 4 * (n2 + 1)));
+  PK_TRY(cp_alloc(j, c.inoff, 4 * (n2 + 1)));
   PK_TRY(cp_alloc(j, c.fill, 4 * (n2 + 1)));
-  PK_TRY(cp_alloc(j, c.ecol, sizeof(uint4) * (n2 + 1)));
-  PK_TRY(cp_alloc(j, c.eoff2, sizeof(uint4) * (n2 + 1)));
-  PK_CUDA(cudaMemsetAsync(c.incnt.p, 0, sizeof(uint4) * (n2 + 1), j->stream));
+  PK_TRY(cp_alloc(j, c.ecol, 4 * (n2 + 1)));
+  PK_TRY(cp_alloc(j, c.eoff2, 4 * (n2 + 1)));
+  PK_CUDA(cudaMemsetAsync(c.incnt.p, 0, 4 * (n2 + 1), j->stream));
   PK_CUDA(cudaMemsetAsync(c.fill.p, 0, 4 * (n2 + 1), j->stream));
   if (T)
     pk::note_launch(), k_cp_resolve<KeyT><<<blocks(T, 256), 256, 0, j->stream>>>((const KeyT*)c.tkey.p, (uint32_t)T, b.key,
-                                                               (uint32_t)n2, (uint32_t*)c.tgt.p, (uint4*)c.incnt.p,
+                                                               (uint32_t)n2, (uint32_t*)c.tgt.p, (uint32_t*)c.incnt.p,
                                                                c.d_err);
-  PK_TRY(scan4(j, c, (const uint4*)c.incnt.p, (uint4*)c.inoff.p, n2));
+  Scanned<uint32_t> inoff{}, eoff{};
+  PK_TRY(scan<uint32_t>(j, c, (const uint32_t*)c.incnt.p, (uint32_t*)c.inoff.p, c.in_part, n2, &inoff));
   if (T)
     pk::note_launch(), k_cp_fill<<<blocks(T, 256), 256, 0, j->stream>>>((const uint32_t*)c.tgt.p, (uint32_t)T,
-                                                     (const uint4*)c.inoff.p, (uint32_t*)c.fill.p,
+                                                     inoff, (uint32_t*)c.fill.p,
                                                      (uint32_t*)c.inlist.p);
   pk::note_launch(), k_cp_apply<KeyT, 0><<<blocks(n2 + 1, 128), 128, 0, j->stream>>>(
-      a, b, (uint32_t)n2, c.L, (const uint32_t*)c.old_of.p, (const uint4*)c.inoff.p, (uint32_t*)c.inlist.p,
-      (const Tr*)c.tr.p, (const uint64_t*)c.arena.p, (uint4*)c.ecol.p, c.d_err);
-  PK_TRY(scan4(j, c, (const uint4*)c.ecol.p, (uint4*)c.eoff2.p, n2));
+      a, b, (uint32_t)n2, c.L, (const uint32_t*)c.old_of.p, inoff, (uint32_t*)c.inlist.p,
+      (const Tr*)c.tr.p, (const uint64_t*)c.arena.p, (uint32_t*)c.ecol.p, eoff, c.d_err);
+  PK_TRY(scan<uint32_t>(j, c, (const uint32_t*)c.ecol.p, (uint32_t*)c.eoff2.p, c.part, n2, &eoff));
   pk::note_launch(), k_cp_apply<KeyT, 1><<<blocks(n2 + 1, 128), 128, 0, j->stream>>>(
-      a, b, (uint32_t)n2, c.L, (const uint32_t*)c.old_of.p, (const uint4*)c.inoff.p, (uint32_t*)c.inlist.p,
-      (const Tr*)c.tr.p, (const uint64_t*)c.arena.p, (uint4*)c.eoff2.p, c.d_err);
+      a, b, (uint32_t)n2, c.L, (const uint32_t*)c.old_of.p, inoff, (uint32_t*)c.inlist.p,
+      (const Tr*)c.tr.p, (const uint64_t*)c.arena.p, nullptr, eoff, c.d_err);
   PK_CUDA(cudaGetLastError());
   uint4 etot;
-  PK_TRY(read_total(j, c, (const uint4*)c.eoff2.p + n2, &etot));
+  PK_TRY(read_total(j, c, &etot));
   PK_TRY(check_err(c));
   c.arena_words += WB;
   c.C += C;
@@ -1385,10 +1421,10 @@ pk_status cp_finish(pk_job* j, CpState& c) {
   if (c.E) pk::note_launch(), k_cp_lengths<<<blocks(c.E, 256), 256, 0, j->stream>>>(a.xlen, (uint32_t)c.E, (uint4*)c.col.p);
   PK_TRY(scan4(j, c, (const uint4*)c.col.p, (uint4*)c.epos.p, c.E));
   uint4 t1, t2;
-  PK_TRY(read_total(j, c, (const uint4*)c.epos.p + c.E, &t1));
+  PK_TRY(read_total(j, c, &t1));
   if (c.C) pk::note_launch(), k_cp_ct_lengths<<<blocks(c.C, 256), 256, 0, j->stream>>>((const Ct*)c.ct.p, (uint32_t)c.C, (uint4*)c.col.p);
   PK_TRY(scan4(j, c, (const uint4*)c.col.p, (uint4*)c.cpos.p, c.C));
-  PK_TRY(read_total(j, c, (const uint4*)c.cpos.p + c.C, &t2));
+  PK_TRY(read_total(j, c, &t2));
   PK_TRY(check_err(c));
   c.ext_bases = t1.x;
   c.ct_bases = t2.x;
@@ -1406,7 +1442,7 @@ pk_status cp_walk(pk_job* j, CpState& c) {
   if (n) pk::note_launch(), k_wk_begin_count<<<blocks(n, 256), 256, 0, st>>>(a.eoff, a.npre, a.xlen, a.vis, (uint32_t)n, (uint4*)c.col.p);
   PK_TRY(scan4(j, c, (const uint4*)c.col.p, (uint4*)c.off.p, n));
   uint4 t;
-  PK_TRY(read_total(j, c, (const uint4*)c.off.p + n, &t));
+  PK_TRY(read_total(j, c, &t));
   const uint64_t B = t.x;
   PK_TRY(cp_alloc(j, c.wk_begins, sizeof(uint2) * (B + 1)));
   PK_TRY(cp_alloc(j, c.wk_links, sizeof(uint2) * (c.E + 1)));
@@ -1438,7 +1474,7 @@ pk_status cp_walk(pk_job* j, CpState& c) {
         (WPath*)c.wk_path.p, (uint32_t)cap, (uint4*)c.wk_col.p, nullptr, nullptr, (WPiece*)c.wk_pieces.p, nullptr,
         (WContig*)c.wk_contigs.p, (uint32_t)ccap, (uint32_t)pcap, (unsigned long long*)c.tot.p, c.d_err);
   PK_TRY(scan4(j, c, (const uint4*)c.wk_col.p, (uint4*)c.wk_pos.p, B));
-  PK_TRY(read_total(j, c, (const uint4*)c.wk_pos.p + B, &t));
+  PK_TRY(read_total(j, c, &t));
   PK_TRY(check_err(c));
   const uint64_t NC = t.x, NB = t.y, NP = t.z;
   PK_TRY(cp_alloc(j, c.wk_off, 8 * (NC + 1)));
@@ -1461,7 +1497,7 @@ pk_status cp_walk(pk_job* j, CpState& c) {
         recorded ? (const uint4*)c.wk_pos.p : nullptr, (uint8_t*)c.wk_out.p);
   PK_CUDA(cudaMemcpyAsync((uint64_t*)c.wk_off.p + NC, &NB, 8, cudaMemcpyHostToDevice, st));
   PK_CUDA(cudaGetLastError());
-  PK_TRY(read_total(j, c, (const uint4*)c.wk_pos.p + B, &t));
+  PK_TRY(read_total(j, c, &t));
   PK_TRY(check_err(c));
   c.wk_begins_n = B;
   c.wk_n = NC;
@@ -1483,15 +1519,13 @@ void pk::cp_free(pk_job* j) {
   };
   for (int s = 0; s < 2; s++)
     for (int b = 0; b < CpState::NSIDE; b++) drop(c->side[s][b]);
-  DevBuf* rest[] = {&c->arena,  &c->col,      &c->off,    &c->part,   &c->is_id,  &c->tkey,
+  DevBuf* rest[] = {&c->arena,  &c->col,      &c->off,    &c->part,   &c->in_part, &c->is_id,  &c->tkey,
                     &c->tr,     &c->tgt,      &c->incnt,  &c->inoff,  &c->fill,   &c->inlist,
                     &c->ecol,   &c->eoff2,    &c->old_of, &c->ct,     &c->tot,    &c->epos,
                     &c->cpos,   &c->ubuf,     &c->wk_begins, &c->wk_resume, &c->wk_path, &c->wk_col,
                     &c->wk_pos, &c->wk_off, &c->wk_out, &c->wk_links, &c->wk_steps, &c->wk_pieces,
                     &c->wk_contigs};
   for (DevBuf* d : rest) drop(*d);
-  if (c->d_err) cudaFree(c->d_err);
-  if (c->h_tot) cudaFreeHost(c->h_tot);
   delete c;
   j->cp = nullptr;
 }
@@ -1521,9 +1555,11 @@ extern "C" pk_status pk_compact(pk_job* j, uint64_t threshold, int32_t coverage,
   CpState& c = *j->cp;
   c.wide = j->wide != 0;
   c.L = j->params.k - 1;
-  PK_CUDA(cudaMalloc(&c.d_err, 16));
-  PK_CUDA(cudaMemsetAsync(c.d_err, 0, 16, j->stream));
-  PK_CUDA(cudaHostAlloc(&c.h_tot, 2 * sizeof(uint4), cudaHostAllocDefault));
+  if (!j->cp_dev) PK_CUDA(cudaMalloc(&j->cp_dev, 2 * sizeof(uint4)));
+  if (!j->cp_host) PK_CUDA(cudaHostAlloc(&j->cp_host, 2 * sizeof(uint4), cudaHostAllocDefault));
+  c.d_err = (uint32_t*)j->cp_dev;
+  c.h_tot = (uint4*)j->cp_host;
+  PK_CUDA(cudaMemsetAsync(c.d_err, 0, 2 * sizeof(uint4), j->stream));
   mark_begin(j, ST_COMPACT);
   pk_status s = c.wide ? cp_init<u128>(j, c, cov) : cp_init<uint64_t>(j, c, cov);
   while (s == PK_OK && c.n > threshold) {

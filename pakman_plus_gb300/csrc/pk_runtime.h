@@ -106,6 +106,7 @@ struct pk_job {
   bool dense_valid = false;
   bool wired = false;  // wiring matches the current macro-nodes
   pk::CpState* cp = nullptr;
+  void *cp_dev = nullptr, *cp_host = nullptr;  // the compaction's error and total words
   bool compacted = false;  // the compaction state matches the current macro-nodes
   bool timing = false;
   // launch shapes chosen by the batch autotuner (0: the defaults): counting/scatter chunks
