@@ -1276,8 +1276,8 @@ __global__ void __launch_bounds__(1024) k_bucket_prefix(uint32_t* bstart, int B)
 template <typename KeyT>
 struct BucketCfg;
 // Threads, measured with two CTAs on an SM: 64-bit keys 768 (bacterial 1.62 ms; 512 and 1024
-// 1.76 ms), 1024 with giant buckets (whose sub-range passes are one CTA's serial chain:
-// 2.68 against 3.43 ms on the low-complexity reads); 128-bit keys 512, whose four keys in
+// 1.76 ms), 1024 with giant buckets (low-complexity reads: whole path 0.91 against
+// 0.99 ms); 128-bit keys 512, whose four keys in
 // flight need the registers (25 Mbp long-k, 2^18 buckets: 10.9 ms; 768 with two keys in
 // flight 13.7 ms).  Keys loaded ahead: four (64-bit keys with two 1.84, with eight 1.88 ms).
 template <>
@@ -1620,6 +1620,16 @@ __device__ __forceinline__ void giant_pass(const BucketArgs& a, const KeyT* keys
   }
 }
 
+// Asks for the keys [p, q) in L2 (whole 16-byte units of them, at most a megabyte).
+template <typename KeyT>
+__device__ __forceinline__ void prefetch_l2(const KeyT* p, const KeyT* q) {
+  const unsigned long long a = ((unsigned long long)__cvta_generic_to_global(p) + 15) & ~15ull;
+  const unsigned long long b = (unsigned long long)__cvta_generic_to_global(q) & ~15ull;
+  if (a >= b) return;
+  const uint32_t n = (uint32_t)min(b - a, 1ull << 20);
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(n) : "memory");
+}
+
 // Exclusive prefix of the sort bins in place (one barrier inside, one after); *s_crowd is
 // set when a bin holds more than kBinMax elements.
 __device__ __forceinline__ void scan_bins(uint32_t* bins, uint32_t* s_warp, uint32_t* s_crowd) {
@@ -1664,7 +1674,9 @@ __device__ __forceinline__ void scan_bins(uint32_t* bins, uint32_t* s_warp, uint
 // shared-memory latency; a bucket takes seven barriers, and the slots it emptied are the
 // occupied ones, by the same order.  Bound: issue and shared-memory latency of the
 // insertions.  Bacterial reads (254M keys, 45M distinct): 1.97 -> 1.62 ms against sorting
-// slots held in registers, 512 threads and 17 barriers a bucket.
+// slots held in registers, 512 threads and 17 barriers a bucket.  The next bucket's keys are
+// asked for in L2 while this one's rows are ordered (64-bit keys: whole path 4.19 -> 4.15 ms;
+// 128-bit keys: no change; asked for a bucket earlier: less).
 template <typename KeyT, bool GIANT, int T>
 __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
   using SM = BucketSmem<KeyT>;
@@ -1947,7 +1959,10 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
         continue;
       }
       const uint32_t u = s_unew;
-      if (tid == 0) take_extent();
+      if (tid == 0) {
+        take_extent();
+        if (sizeof(KeyT) == 8 && next_t >= first_bucket && next_t < nt) prefetch_l2(keys + next_base, keys + next_end);
+      }
       if (GIANT && !placed) place();
       if (GIANT && part && sp == 1 && tid == 0) st_relaxed(word, kLbIncl | (acc + u));
       // --- order the u distinct remainders: slot numbers go to their bins, in any order
