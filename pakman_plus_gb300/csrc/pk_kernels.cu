@@ -2523,7 +2523,7 @@ __global__ void __launch_bounds__(kMnThreads, MnCfg<KeyT>::CTAS) k_macro_nodes(M
   __syncthreads();
 
   // the next ticket's unit and extents, by one warp: first the big units' counts, then
-  // every unit in order
+  // every unit in order.  Its rows are asked for in L2 (bacterial path 4.137 -> 4.114 ms)
   const uint32_t nbig = a.sc->n_big;
   auto take_unit = [&]() {
     uint32_t t = 0;
@@ -2540,6 +2540,8 @@ __global__ void __launch_bounds__(kMnThreads, MnCfg<KeyT>::CTAS) k_macro_nodes(M
       }
     }
     if (lane < 5) {
+      prefetch_l2(kk + r0, kk + r1);
+      prefetch_l2(a.kcounts + r0, a.kcounts + r1);
       s_ncur[lane] = r0;
       s_nend[lane] = r1;
     }
