@@ -2319,9 +2319,10 @@ __global__ void __launch_bounds__(kKeptT) k_kept_offsets(FilterArgs a) {
 // brings its four counts and lane order is row order.  Bound: the wait for its loads, counts
 // and then keys; the next step's counts are under way while this step's keys are waited for:
 // 1 Mbp, 30x, whole path 0.748 -> 0.722 ms; bacterial 4.15 -> 4.13 ms (eight rows a lane: 0.736
-// and 4.12 ms).
+// and 4.12 ms).  Six CTAs an SM: bacterial 4.105 -> 4.092 ms against the five that its 48
+// registers would leave; eight 4.103 ms.
 template <typename KeyT>
-__global__ void __launch_bounds__(256) k_filter_kept(FilterArgs a) {
+__global__ void __launch_bounds__(256, 6) k_filter_kept(FilterArgs a) {
   const int lane = threadIdx.x & 31;
   const uint32_t B = 1u << a.bbits, warps = gridDim.x * (blockDim.x >> 5);
   const int rem = 2 * a.k - a.bbits;
