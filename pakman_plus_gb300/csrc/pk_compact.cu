@@ -630,8 +630,11 @@ struct Replay {
   int np, ns;
 };
 
+// Bound: the wait for its scattered reads (57 of 63 cycles an instruction), so twelve CTAs an
+// SM rather than the registers it would take: contigs of 4.0M nodes 8.05 -> 7.78 ms in all;
+// sixteen spill and give that back.
 template <typename KeyT, int PASS>
-__global__ void __launch_bounds__(128) k_cp_apply(Side<KeyT> a, Side<KeyT> b, uint32_t n, int L,
+__global__ void __launch_bounds__(128, 12) k_cp_apply(Side<KeyT> a, Side<KeyT> b, uint32_t n, int L,
                                                   const uint32_t* __restrict__ old_of,
                                                   Scanned<uint32_t> inoff, uint32_t* __restrict__ inlist,
                                                   const Tr* __restrict__ tr, const uint64_t* __restrict__ ar,
