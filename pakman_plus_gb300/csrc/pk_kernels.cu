@@ -8,11 +8,12 @@
 //   k_coarse_offsets   each chunk's segment of every coarse region
 //   k_scatter_coarse   roll again, keys to their coarse region through shared-memory rings
 //   k_scatter_fine     per slice of a coarse region: keys to their bucket, staged by bucket
-//   k_giant_chunks     chunk items of buckets too large for one CTA
+//   k_giant_chunks     chunk and part items of buckets too large for one CTA
 //   k_bucket_table     per bucket: hash-aggregate in smem, sort the distinct keys, write
 //                      the (k-mer, count) rows and the count histogram
 //   k_cutoff           first minimum of the count histogram over [1, t)
-//   k_filter_kept      kept rows (count >= cutoff), dense, with a decoupled look-back
+//   k_kept_offsets     kept rows (count >= cutoff) per bucket and their prefix over the buckets
+//   k_filter_kept      the kept rows, dense
 //   k_macro_nodes      per (k-1)-mer unit: merge the suffix-side and prefix-side
 //                      streams of kept k-mers into macro-node records
 //   k_wire             initial wiring of every macro-node
@@ -259,30 +260,6 @@ __device__ __forceinline__ uint32_t block_exclusive_sum(uint32_t v, uint32_t* s_
   total = s_warp[32];
   __syncthreads();
   return res;
-}
-
-// Block-wide OR and AND of a key (result in x_or/x_and of every thread).
-template <typename KeyT>
-__device__ void block_or_and(KeyT& x_or, KeyT& x_and, KeyT* s_red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  uint64_t olo = (uint64_t)x_or, ohi = (uint64_t)(x_or >> 32 >> 32);
-  uint64_t alo = (uint64_t)x_and, ahi = (uint64_t)(x_and >> 32 >> 32);
-  for (int o = 16; o > 0; o >>= 1) {
-    olo |= __shfl_xor_sync(FULLMASK, olo, o);
-    ohi |= __shfl_xor_sync(FULLMASK, ohi, o);
-    alo &= __shfl_xor_sync(FULLMASK, alo, o);
-    ahi &= __shfl_xor_sync(FULLMASK, ahi, o);
-  }
-  if (lane == 0) {
-    s_red[warp] = (KeyT)olo | ((KeyT)ohi << 32 << 32);
-    s_red[nw + warp] = (KeyT)alo | ((KeyT)ahi << 32 << 32);
-  }
-  __syncthreads();
-  KeyT ro = 0, ra = ~(KeyT)0;
-  for (int w = 0; w < nw; w++) { ro |= s_red[w]; ra &= s_red[nw + w]; }
-  x_or = ro;
-  x_and = ra;
-  __syncthreads();
 }
 
 // Four input bytes: their 2-bit codes (byte 0 in the top bits of the low byte), a mask of
