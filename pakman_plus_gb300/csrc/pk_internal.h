@@ -67,6 +67,7 @@ struct Scalars {                    // device-side scalars of one job
   uint32_t ticket_fcount;
   uint32_t n_chunk_items;           // chunk items of giant buckets (table kernel)
   uint32_t n_giants;                // giant buckets
+  uint32_t part_beats;              // passes of giant buckets' parts so far
   unsigned long long n_unique;      // U
   unsigned long long n_kept;        // V
   // zeroed together before macro-nodes are built

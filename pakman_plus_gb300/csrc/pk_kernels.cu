@@ -1709,8 +1709,9 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
   // Work tickets: the chunk items of giant buckets first (tickets [0, nci)), then their
   // parts, then the other buckets.  A part waits (bounded) until its bucket's chunks are
   // reduced, and before it writes rows until the parts before it have counted theirs: items
-  // of earlier tickets, held by CTAs that wait on still earlier ones, so the waits end.  Thread 0 takes the next ticket when a bucket starts and its extent
-  // once the bucket's keys are in, so neither is waited for between buckets.
+  // of earlier tickets, held by CTAs that wait on still earlier ones, so the waits end.
+  // Thread 0 takes the next ticket when a bucket starts and its extent once the bucket's keys
+  // are in, so neither is waited for between buckets.
   uint32_t next_t = 0, next_base = 0, next_end = 0;
   bool have_extent = true;
   auto take_ticket = [&]() {
@@ -1816,12 +1817,20 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
       if (tid == 0) {
         unsigned long long w = kLbIncl;
         if (item % kGiantParts) {
+          // the parts before may have hundreds of sub-ranges to count, one part after the
+          // other, so the limit holds for the time in which no part gets through one
           int spins = 0;
           const int max_spins = spin_limit(a.spin_limit);
+          uint32_t beats = 0;  // at the last time that the limit was reached
           while ((w = ld_relaxed(word - 1)) == 0) {
             if (++spins >= max_spins) {
-              atomicOr(&a.sc->err, ERR_LOOKBACK);
-              break;
+              const uint32_t now = *(const volatile uint32_t*)&a.sc->part_beats;
+              if (now == beats) {
+                atomicOr(&a.sc->err, ERR_LOOKBACK);
+                break;
+              }
+              beats = now;
+              spins = 0;
             }
             __nanosleep(spins < 64 ? 32 : 256);
           }
@@ -1860,6 +1869,7 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
       if (GIANT && part)
         giant_pass<KeyT, T>(a, keys_rw, base, n, g0, nch, raws, whole, lo, hi, rmask, skey, scnt, hmask, ulimit, bins,
                             dsh, bmask, &s_ovf, &s_unew);
+      if (GIANT && part && tid == 0) atomicAdd(&a.sc->part_beats, 1u);
       for (uint32_t i0 = 0; i0 < n && !(GIANT && part); i0 += PF * T) {
         if (warp_flag(&s_ovf)) break;
         KeyT rr[PF];
