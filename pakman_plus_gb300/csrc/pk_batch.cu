@@ -96,20 +96,7 @@ pk_status dev_alloc(pk_ctx* ctx, DevBuf& b, size_t bytes, cudaStream_t s) {
     ctx->used -= b.bytes;
     b = DevBuf{};
   }
-  bytes = std::max<size_t>(256, (bytes + 255) & ~(size_t)255);
-  const uint64_t now = ctx->used.fetch_add(bytes) + bytes;
-  if (ctx->budget && now > ctx->budget) {
-    ctx->used -= bytes;
-    return set_error(PK_ERR_NOMEM, "HBM budget exceeded by the batch buffers");
-  }
-  cudaError_t e = cudaMallocFromPoolAsync(&b.p, bytes, ctx->pool, s);
-  if (e != cudaSuccess) {
-    ctx->used -= bytes;
-    b.p = nullptr;
-    return set_error(PK_ERR_NOMEM, std::string("batch buffer: ") + cudaGetErrorString(e));
-  }
-  b.bytes = bytes;
-  return PK_OK;
+  return ctx_alloc(ctx, s, b, bytes);
 }
 
 void dev_free(pk_ctx* ctx, DevBuf& b, cudaStream_t s) {

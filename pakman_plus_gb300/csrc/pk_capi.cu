@@ -41,10 +41,13 @@ pk_status pk::set_device(pk_ctx* c) {
 }
 
 // ------------------------------------------------------------ device blocks -----
+// A cached block of at least `bytes`: up to an eighth (or 64 KB) larger, but with a budget of
+// just that size, as every byte of it counts there.
 static void* cache_take(pk_ctx* c, size_t bytes, size_t* block) {
+  const size_t most = c->budget ? bytes : std::max(bytes + bytes / 8, bytes + 65536);
   std::lock_guard<std::mutex> lk(c->cache_mu);
   auto it = c->cache.lower_bound(bytes);
-  if (it == c->cache.end() || it->first > std::max(bytes + bytes / 8, bytes + 65536)) return nullptr;
+  if (it == c->cache.end() || it->first > most) return nullptr;
   void* p = it->second;
   *block = it->first;
   c->cached -= it->first;
@@ -52,29 +55,37 @@ static void* cache_take(pk_ctx* c, size_t bytes, size_t* block) {
   return p;
 }
 
-// Frees cached blocks, largest first, until at most `keep` bytes are cached.
+// Gives the cached blocks back to the pool when they are more than `keep` bytes: all of them,
+// as the pool joins what is free and a block here and there leaves it pieces that nothing fits.
 static void cache_trim(pk_ctx* c, uint64_t keep) {
   std::lock_guard<std::mutex> lk(c->cache_mu);
-  while (!c->cache.empty() && c->cached > keep) {
-    auto it = std::prev(c->cache.end());
-    cudaFree(it->second);  // idle: nothing to wait for
-    c->cached -= it->first;
-    c->cache.erase(it);
-  }
+  if (c->cached <= keep) return;
+  for (auto& b : c->cache) cudaFree(b.second);  // idle: nothing to wait for
+  c->cache.clear();
+  c->cached = 0;
 }
 
 static void cache_put(pk_ctx* c, DevBuf& b) {
   if (b.p) {
     c->used -= b.bytes;
-    uint64_t keep = c->cache_limit;
-    if (c->budget) keep = std::min<uint64_t>(keep, c->budget - std::min<uint64_t>(c->budget, c->used.load()));
     bool room;
     {
+      // what is in use is read under the lock: an allocation that is not in it yet trims later
       std::lock_guard<std::mutex> lk(c->cache_mu);
-      room = c->cached + b.block <= keep;
+      uint64_t keep = c->cache_limit;
+      if (c->budget) keep = std::min<uint64_t>(keep, c->budget - std::min<uint64_t>(c->budget, c->used.load()));
+      // the largest blocks make room: a job of few bytes is the one that feels an allocation
+      while (c->cached + b.bytes > keep && !c->cache.empty()) {
+        auto it = std::prev(c->cache.end());
+        if (it->first <= b.bytes) break;
+        cudaFree(it->second);  // idle: nothing to wait for
+        c->cached -= it->first;
+        c->cache.erase(it);
+      }
+      room = c->cached + b.bytes <= keep;
       if (room) {
-        c->cache.emplace(b.block, b.p);
-        c->cached += b.block;
+        c->cache.emplace(b.bytes, b.p);
+        c->cached += b.bytes;
       }
     }
     if (!room) cudaFree(b.p);
@@ -82,13 +93,10 @@ static void cache_put(pk_ctx* c, DevBuf& b) {
   b = DevBuf{};
 }
 
-pk_status pk::job_alloc(pk_job* j, DevBuf& b, size_t bytes) {
-  if (b.p && b.bytes >= bytes) return PK_OK;
-  if (j->graph_mode) return fail(PK_ERR_STATE, "batch buffers are smaller than a set needs");
-  job_free(j, b);
-  pk_ctx* c = j->ctx;
-  if (bytes == 0) bytes = 16;
-  bytes = (bytes + 255) & ~(size_t)255;
+// Every device buffer of the context comes from here: charged whole to the budget, which
+// blocks in use and cached blocks share.
+pk_status pk::ctx_alloc(pk_ctx* c, cudaStream_t st, DevBuf& b, size_t bytes) {
+  bytes = std::max<size_t>(256, (bytes + 255) & ~(size_t)255);
   uint64_t now = c->used.fetch_add(bytes) + bytes;
   if (c->budget && now > c->budget) {
     c->used -= bytes;
@@ -100,21 +108,28 @@ pk_status pk::job_alloc(pk_job* j, DevBuf& b, size_t bytes) {
   void* p = cache_take(c, bytes, &block);
   if (!p) {
     if (c->budget) cache_trim(c, c->budget - now);  // what is in use and what is kept stay within it
-    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, c->pool, j->stream);
+    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, c->pool, st);
     if (e != cudaSuccess) {
       cudaGetLastError();
       cache_trim(c, 0);
-      e = cudaMallocFromPoolAsync(&p, bytes, c->pool, j->stream);
+      e = cudaMallocFromPoolAsync(&p, bytes, c->pool, st);
     }
     if (e != cudaSuccess) {
       c->used -= bytes;
       return fail(PK_ERR_NOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
     }
   }
+  c->used += block - bytes;
   b.p = p;
-  b.bytes = bytes;
-  b.block = block;
+  b.bytes = block;
   return PK_OK;
+}
+
+pk_status pk::job_alloc(pk_job* j, DevBuf& b, size_t bytes) {
+  if (b.p && b.bytes >= bytes) return PK_OK;
+  if (j->graph_mode) return fail(PK_ERR_STATE, "batch buffers are smaller than a set needs");
+  job_free(j, b);
+  return ctx_alloc(j->ctx, j->stream, b, bytes);
 }
 
 void pk::job_free(pk_job* j, DevBuf& b) {

@@ -47,8 +47,7 @@ struct pk_ctx {
 
 struct DevBuf {
   void* p = nullptr;
-  size_t bytes = 0;  // usable and charged to the budget
-  size_t block = 0;  // of the device block (at most an eighth or 64 KB more)
+  size_t bytes = 0;  // of the device block: all usable, all charged to the budget
 };
 
 enum Stage {
@@ -134,6 +133,9 @@ struct pk_job {
 
 namespace pk {
 pk_status set_device(pk_ctx* c);
+// a block for an empty buffer: from the context's idle blocks or its pool, which gets the idle
+// blocks back before a budget or the device refuses
+pk_status ctx_alloc(pk_ctx* c, cudaStream_t st, DevBuf& b, size_t bytes);
 pk_status job_alloc(pk_job* j, DevBuf& b, size_t bytes);
 // releases a buffer that the stream may still use (stream-ordered), or one that is idle
 void job_free(pk_job* j, DevBuf& b);
