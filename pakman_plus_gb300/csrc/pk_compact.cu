@@ -987,7 +987,8 @@ __global__ void __launch_bounds__(128) k_walk(Side<KeyT> s, int L, const uint2* 
                                               WContig* __restrict__ contigs, uint32_t ccap, uint32_t pcap,
                                               unsigned long long* recorded, uint32_t* err) {
   // one walk per warp: independent walks diverge completely, so they do not share one.
-  // All lanes step together (same loads); lane 0 stores the frames.
+  // All lanes take the same steps (same loads); lane 0 stores the frames.  Between its stores
+  // and the others' loads, and between those and its next store there, the warp meets.
   const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (b >= nb) return;
@@ -1019,6 +1020,7 @@ __global__ void __launch_bounds__(128) k_walk(Side<KeyT> s, int L, const uint2* 
       rem = (int32_t)y.y;
       d = y.z;
       len = y.w;
+      __syncwarp();  // before lane 0 stores the next frame here
       continue;
     }
     const WStep w = ld_step(step + base + wi);
