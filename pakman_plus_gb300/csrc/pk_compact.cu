@@ -1438,7 +1438,7 @@ pk_status cp_finish(pk_job* j, CpState& c) {
 }
 
 template <typename KeyT>
-pk_status cp_walk(pk_job* j, CpState& c) {
+pk_status cp_walk(pk_job* j, CpState& c, bool record) {
   Side<KeyT> a = side_of<KeyT>(c, c.cur);
   const uint64_t n = c.n;
   cudaStream_t st = j->stream;
@@ -1468,9 +1468,11 @@ pk_status cp_walk(pk_job* j, CpState& c) {
   PK_TRY(cp_alloc(j, c.wk_pos, sizeof(uint4) * (B + 1)));
   // room for the contigs and pieces that the counting walk records: walks of a compacted map
   // visit most wires a few times at most
-  const uint64_t pcap = std::min<uint64_t>(kWalkRecords, 2 * (c.E + n) + 1024), ccap = pcap / 4;
-  PK_TRY(cp_alloc(j, c.wk_pieces, sizeof(WPiece) * pcap));
-  PK_TRY(cp_alloc(j, c.wk_contigs, sizeof(WContig) * ccap));
+  const uint64_t pcap = record ? std::min<uint64_t>(kWalkRecords, 2 * (c.E + n) + 1024) : 0, ccap = pcap / 4;
+  if (record) {
+    PK_TRY(cp_alloc(j, c.wk_pieces, sizeof(WPiece) * pcap));
+    PK_TRY(cp_alloc(j, c.wk_contigs, sizeof(WContig) * ccap));
+  }
   PK_TRY(cp_alloc(j, c.tot, 2 * sizeof(unsigned long long)));
   PK_CUDA(cudaMemsetAsync(c.tot.p, 0, 2 * sizeof(unsigned long long), st));
   if (B)
@@ -1510,6 +1512,15 @@ pk_status cp_walk(pk_job* j, CpState& c) {
   c.wk_depth = (uint32_t)cap;
   c.wk_done = true;
   return PK_OK;
+}
+
+// Frees what the compaction's rounds needed and what a walk has taken, down to the map itself.
+void cp_shrink(pk_job* j, CpState& c) {
+  for (DevBuf& d : c.side[c.cur ^ 1]) job_free(j, d);
+  DevBuf* rest[] = {&c.in_part, &c.is_id,  &c.tkey,  &c.tr,        &c.tgt,     &c.incnt,  &c.inoff,    &c.fill,
+                    &c.inlist,  &c.ecol,   &c.eoff2, &c.old_of,    &c.ubuf,    &c.wk_off, &c.wk_out,   &c.wk_links,
+                    &c.wk_steps, &c.wk_resume, &c.wk_path, &c.wk_pieces, &c.wk_contigs};
+  for (DevBuf* d : rest) job_free(j, *d);
 }
 
 }  // namespace
@@ -1668,7 +1679,11 @@ extern "C" pk_status pk_walk(pk_job* j, pk_walk_info* info) {
   PK_TRY(set_device(j->ctx));
   c.wk_done = false;
   mark_begin(j, ST_WALK);
-  const pk_status s = c.wide ? cp_walk<u128>(j, c) : cp_walk<uint64_t>(j, c);
+  pk_status s = c.wide ? cp_walk<u128>(j, c, true) : cp_walk<uint64_t>(j, c, true);
+  if (s == PK_ERR_NOMEM) {  // with no more than the map beside it, and without records
+    cp_shrink(j, c);
+    s = c.wide ? cp_walk<u128>(j, c, false) : cp_walk<uint64_t>(j, c, false);
+  }
   mark_end(j, ST_WALK);
   PK_TRY(s);
   if (info) {
