@@ -436,6 +436,19 @@ int pk::auto_bucket_bits(uint64_t F, int k, int wide) {
   return partition_bits((wide ? 0.45 : 0.62) * (double)F, k, wide);
 }
 
+// The digits of a table that is there already (loaded, or merged from pieces): up to 1000 rows
+// per bucket, 768 of which a joined macro-node unit takes.  With 4000, units were sorted in
+// segments: 5.0M rows, load to macro-nodes, 0.81 ms at 4000, 0.70 at 2000, 0.68 at 1000, 0.69
+// at 400.
+int pk::row_bits(uint64_t rows, const pk_params* p) {
+  int b = p->bucket_bits;
+  if (!b) {
+    b = 2;
+    while (b < kMaxPartitionBits && (double)rows / (double)(1u << b) > 1000.0) b++;
+  }
+  return std::max(2, std::min(b, std::min(kMaxPartitionBits, 2 * p->k - 2)));
+}
+
 // The digits the counting pass histograms when the partition's own follow from its window
 // count: enough for long reads (0.85 windows per byte) where a digit more is cheap, as many
 // as the histogram holds at most.
@@ -774,15 +787,7 @@ pk_status pk_table_load(pk_job* j, const void* keys, const uint32_t* counts, uin
   j->F = 0;
   j->N = n;
   j->stage = 0;
-  int bb = p->bucket_bits;
-  // up to 1000 rows per bucket, 768 of which a joined macro-node unit takes.  With 4000, units
-  // were sorted in segments: 5.0M rows, load to macro-nodes, 0.81 ms at 4000, 0.70 at 2000,
-  // 0.68 at 1000, 0.69 at 400
-  if (!bb) {
-    bb = 2;
-    while (bb < kMaxPartitionBits && (double)n / (double)(1u << bb) > 1000.0) bb++;
-  }
-  j->bbits = std::max(2, std::min(bb, std::min(kMaxPartitionBits, 2 * k - 2)));
+  j->bbits = row_bits(n, p);
   const int B = 1 << j->bbits;
   if (on_device) {
     std::swap(j->tkeys, nk);

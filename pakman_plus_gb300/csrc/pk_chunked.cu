@@ -305,17 +305,11 @@ pk_status pk::count_pieces(pk_job* j, const char* host, uint64_t n, const pk_par
   std::swap(j->tcounts, j->acc_counts[cur]);
   release_piece_buffers(j);
   j->bsmall_valid = false;  // the merged table has no per-bucket small-count histogram
-  const int k = p->k;
-  int bb = p->bucket_bits;
-  if (!bb) {  // about 4000 rows per bucket, as for a loaded table
-    bb = 2;
-    while (bb < kMaxPartBits && (double)rows / (double)(1u << bb) > 4000.0) bb++;
-  }
-  j->bbits = std::max(2, std::min(bb, std::min(kMaxPartBits, 2 * k - 2)));
+  j->bbits = row_bits(rows, p);
   const int B = 1 << j->bbits;
   PK_TRY(job_alloc(j, j->bstart, sizeof(uint32_t) * (B + 1)));
   PK_TRY(job_alloc(j, j->tu, sizeof(uint32_t) * (size_t)B));
-  PK_CUDA(launch_table_bounds(j->tkeys.p, rows, j->bbits, k, (uint32_t*)j->bstart.p, (uint32_t*)j->tu.p,
+  PK_CUDA(launch_table_bounds(j->tkeys.p, rows, j->bbits, p->k, (uint32_t*)j->bstart.p, (uint32_t*)j->tu.p,
                               j->wide, j->stream));
   Scalars init{};
   memset(&init, 0, sizeof(init));

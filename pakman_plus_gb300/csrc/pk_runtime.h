@@ -144,6 +144,7 @@ void job_free_all(pk_job* j);  // waits for the job's stream
 void cp_free(pk_job* j);  // the compaction state, if any
 pk_status check_params(const pk_params* p);
 int auto_bucket_bits(uint64_t F, int k, int wide);
+int row_bits(uint64_t rows, const pk_params* p);
 // device FASTA -> resident table; in graph mode no host synchronisation happens and
 // the window count is taken as j->ncap
 pk_status count_impl(pk_job* j, const void* d_fasta, uint64_t n, const pk_params* p);
