@@ -23,7 +23,6 @@ enum : uint32_t {
   ERR_LOOKBACK = 2u,      // a bounded look-back wait ran out
   ERR_BUCKET = 4u,        // a bucket could not be split small enough for on-chip counting
   ERR_MN_CAPACITY = 8u,   // a macro-node segment exceeded on-chip capacity
-  ERR_TICKET = 16u,       // work ticket overrun (should not happen)
   ERR_BOUNDS = 32u,       // a computed index fell outside its buffer (write skipped)
 };
 
@@ -73,7 +72,6 @@ struct Scalars {                    // device-side scalars of one job
   // zeroed together before macro-nodes are built
   unsigned long long mn_begin[0];
   unsigned long long n_nodes;       // M
-  unsigned long long n_kept_rows;   // V as counted by the kept offsets
   uint32_t ticket_mn;
   uint32_t ticket_filter;
   uint32_t n_big;                   // macro-node units of more than one segment

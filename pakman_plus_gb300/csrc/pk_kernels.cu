@@ -2288,7 +2288,6 @@ __global__ void __launch_bounds__(kKeptT) k_kept_offsets(FilterArgs a) {
     if (threadIdx.x == 0) {
       if (tile) st_relaxed(&a.flags[tile], kLbIncl | (before + tot));
       s_before = before;
-      if (tile == tiles - 1) a.sc->n_kept_rows = before + tot;
     }
   }
   __syncthreads();
