@@ -890,7 +890,10 @@ __global__ void __launch_bounds__(256) k_coarse_offsets(const uint32_t* __restri
 // or 8 keys: six CTAs an SM instead of two wait at their barriers at other times.  Bacterial
 // reads (2^14 buckets, 2^7 fine): 0.90 -> 0.77 ms; three CTAs of 4096-key slices 0.80 ms, of
 // 8192 1.28 ms (they spill).  With 2^10 fine buckets 4096-key slices lose (25 Mbp long-k path
-// 22.6 -> 26.0 ms).
+// 22.6 -> 26.0 ms).  The line between, quarter against whole slices: 64-bit keys at 2^8 fine
+// buckets 0.85 against 0.93 ms (254M keys) and 1.58 against 1.70 ms (472M), at 2^9 3.16 against
+// 1.41 ms; 128-bit keys at 2^8 1.23 against 1.20, at 2^9 4.94 against 1.79 ms (195M).  So it
+// could lie at 2^8 for 64-bit keys; it is the same for both widths.
 constexpr int kFewFine = 7;
 template <typename KeyT, bool FEW>
 struct FineCfg {
