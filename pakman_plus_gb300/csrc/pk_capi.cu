@@ -1153,6 +1153,8 @@ static pk_status run_all(pk_job* j, const void* fasta, uint64_t n, const pk_para
   j->no_wait = p && n <= kSmallRun && p->chunking != 1 && j->ctx->budget == 0;
   pk_status s = host ? pk_count(j, (const char*)fasta, n, p) : pk_count_device(j, fasta, n, p);
   if (s == PK_OK) s = run_rest(j, p, out);
+  // an allocation that failed on the way: the caller's buffer may still be read
+  if (s != PK_OK && j->no_wait) cudaStreamSynchronize(j->stream);
   j->no_wait = false;
   return s;
 }
