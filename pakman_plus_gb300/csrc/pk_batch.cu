@@ -145,9 +145,9 @@ pk_status presize(pk_job* j, uint64_t fmax, int k, int bbits, int t, int sms) {
   PK_TRY(job_alloc(j, j->flags_m, 8 * (((size_t)B + 255) / 256 + mn_flag_words(bbits)) + 4 * (size_t)B));
   PK_TRY(job_alloc(j, j->gfirst, 4 * (size_t)B));
   PK_TRY(job_alloc(j, j->gcount, 4 * (size_t)B));
-  PK_TRY(job_alloc(j, j->chunk_bucket, 4 * (fmax / kChunkKeys + 1)));
+  PK_TRY(job_alloc(j, j->chunk_bucket, 4 * (fmax / chunk_keys(k > 32) + 1)));
   PK_TRY(job_alloc(j, j->gdone, 4 * (size_t)B));
-  PK_TRY(job_alloc(j, j->chunk_u, 4 * (fmax / kChunkKeys + 1)));
+  PK_TRY(job_alloc(j, j->chunk_u, 4 * (fmax / chunk_keys(k > 32) + 1)));
   PK_TRY(job_alloc(j, j->gpart, giant_part_bytes(fmax)));
   return PK_OK;
 }

@@ -616,8 +616,9 @@ static pk_status table_impl(pk_job* j, uint64_t N, int t) {
     PK_TRY(job_alloc(j, j->gfirst, sizeof(uint32_t) * (size_t)B));
     PK_TRY(job_alloc(j, j->gcount, sizeof(uint32_t) * (size_t)B));
     PK_TRY(job_alloc(j, j->gdone, sizeof(uint32_t) * (size_t)B));
-    PK_TRY(job_alloc(j, j->chunk_bucket, sizeof(uint32_t) * (size_t)(N / kChunkKeys + 1)));
-    PK_TRY(job_alloc(j, j->chunk_u, sizeof(uint32_t) * (size_t)(N / kChunkKeys + 1)));
+    const uint64_t chunks = N / chunk_keys(j->wide) + 1;
+    PK_TRY(job_alloc(j, j->chunk_bucket, sizeof(uint32_t) * chunks));
+    PK_TRY(job_alloc(j, j->chunk_u, sizeof(uint32_t) * chunks));
     PK_TRY(job_alloc(j, j->gpart, giant_part_bytes(N)));
   }
   PK_TRY(job_alloc(j, j->bsmall, sizeof(uint32_t) * kSmallCounts * (size_t)B));
@@ -647,7 +648,7 @@ static pk_status table_impl(pk_job* j, uint64_t N, int t) {
   b.spin_limit = (int)j->wait_limit;
   b.sc = j->d_sc;
   if (giants)
-    PK_CUDA(launch_giant_chunks(b, (uint32_t*)j->gfirst.p, (uint32_t*)j->gcount.p, (uint32_t*)j->chunk_bucket.p,
+    PK_CUDA(launch_giant_chunks(b, j->wide, (uint32_t*)j->gfirst.p, (uint32_t*)j->gcount.p, (uint32_t*)j->chunk_bucket.p,
                                 glist, j->stream));
   PK_CUDA(launch_bucket_table(b, j->wide, j->table_ctas > 0 ? j->table_ctas * thread_sms(j->ctx->sms) : 0, j->stream));
   mark_end(j, ST_TABLE);

@@ -49,8 +49,7 @@ constexpr int kSortBinBits = 10;    // top remainder bits of the per-bucket coun
 constexpr int kBinMax = 128;        // largest bin sorted by ranking (else bitonic sort)
 // Giant buckets (skewed input: a homopolymer or tandem repeat and its error variants)
 // are first reduced chunk by chunk, by many CTAs, to (key, count) pairs.
-constexpr int kChunkKeys = 32768;                   // keys per chunk of a giant bucket
-constexpr uint32_t kGiantKeys = 16u * kChunkKeys;   // a bucket this large is giant
+constexpr uint32_t kGiantKeys = 1u << 19;           // a bucket this large is giant
 constexpr int kGiantParts = 16;                     // work items that count one giant bucket
 constexpr uint32_t kChunkRaw = 0xffffffffu;         // chunk left as keys (too many distinct)
 
@@ -191,12 +190,13 @@ void set_thread_sms(int n);
 int thread_sms(int device_sms);
 
 cudaError_t launch_line_scan(const CountArgs& a, cudaStream_t st);
-// chunk items of the giant buckets (n_b >= kGiantKeys): floor(n_b / kChunkKeys)
+// chunk items of the giant buckets (n_b >= kGiantKeys): floor(n_b / chunk_keys)
 // consecutive items each, from gfirst[b], gcount[b] of them; chunk_bucket maps an item
 // to its bucket; sc->n_chunk_items = all items; sc->n_giants and glist: the buckets; gdone,
 // gpart and the giants' rows of bsmall = 0
-cudaError_t launch_giant_chunks(const BucketArgs& a, uint32_t* gfirst, uint32_t* gcount, uint32_t* chunk_bucket,
-                                uint32_t* glist, cudaStream_t st);
+int chunk_keys(int wide);
+cudaError_t launch_giant_chunks(const BucketArgs& a, int wide, uint32_t* gfirst, uint32_t* gcount,
+                                uint32_t* chunk_bucket, uint32_t* glist, cudaStream_t st);
 size_t giant_part_bytes(unsigned long long keys);  // gpart, then glist
 // the line scan in two halves: per-tile newline counts for tiles [tile0, tile0 + ntiles)
 // (any order, any number of launches), then the prefix over all tiles

@@ -1259,13 +1259,19 @@ struct BucketCfg;
 // 1.76 ms), 1024 with giant buckets (low-complexity reads: whole path 0.91 against
 // 0.99 ms); 128-bit keys 512, whose four keys in
 // flight need the registers (25 Mbp long-k, 2^18 buckets: 10.9 ms; 768 with two keys in
-// flight 13.7 ms).  Keys loaded ahead: four (64-bit keys with two 1.84, with eight 1.88 ms).
+// flight 13.7 ms).  Keys per chunk of a giant bucket: one that has more distinct keys than half a
+// table stays as it is, and every sub-range of the bucket then reads all its keys.  By the
+// substitution rate, windows of 55 low-complexity bases at 1 % have about 3300 distinct ones
+// in 32768 and 1050 in 8192, so 128-bit keys (half a table is 2048) take 8192.  6 Mbp, 60x,
+// k = 55: 14.6 s with 32768, 0.96 s with 16384, 1.21 s with 8192, 1.52 s with 4096; k = 64, 40x:
+// 8.3, 2.4, 1.06 and 1.33 s.  Keys loaded ahead: four (64-bit keys with two 1.84, with eight 1.88 ms).
 template <>
 struct BucketCfg<uint64_t> {
   static constexpr int H = 8192;   // table slots
   static constexpr int T = 768;    // threads
   static constexpr int TG = 1024;  // threads when there are giant buckets
   static constexpr int PF = 4;     // keys loaded per thread before inserting
+  static constexpr int CH = 32768; // keys per chunk of a giant bucket
 };
 template <>
 struct BucketCfg<u128> {
@@ -1273,6 +1279,7 @@ struct BucketCfg<u128> {
   static constexpr int T = 512;
   static constexpr int TG = 512;
   static constexpr int PF = 4;
+  static constexpr int CH = 8192;
 };
 
 // Two CTAs fit an SM: for 64-bit keys 115 KB each (96 KB of slots, the sort's order and
@@ -1341,7 +1348,7 @@ __device__ __forceinline__ void emit_row(const BucketArgs& a, KeyT* __restrict__
 }
 
 // Chunk items of the giant buckets (one thread per bucket): a bucket of at least
-// kGiantKeys keys reserves floor(n / kChunkKeys) consecutive chunk items, gfirst[b] the
+// kGiantKeys keys reserves floor(n / chunk_keys) consecutive chunk items, gfirst[b] the
 // first and gcount[b] how many, and marks them as its own in chunk_bucket; the number
 // of chunk items ends in sc->n_chunk_items (zero beforehand); gdone = 0.  Its kGiantParts
 // part items find it in glist; their look-back words and its small-count histogram, which
@@ -1350,11 +1357,11 @@ __global__ void __launch_bounds__(256) k_giant_chunks(const uint32_t* __restrict
                                                       uint32_t* gfirst, uint32_t* gcount,
                                                       uint32_t* chunk_bucket, uint32_t* gdone,
                                                       unsigned long long* gpart, uint32_t* glist,
-                                                      uint32_t* bsmall, Scalars* sc) {
+                                                      uint32_t* bsmall, uint32_t chunk_keys, Scalars* sc) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   const uint32_t n = bstart[b + 1] - bstart[b];
-  const uint32_t c = n >= kGiantKeys ? n / kChunkKeys : 0u;
+  const uint32_t c = n >= kGiantKeys ? n / chunk_keys : 0u;
   gdone[b] = 0;
   gcount[b] = c;
   uint32_t g0 = 0;
@@ -1385,10 +1392,10 @@ __device__ __forceinline__ void clear_table(KeyT* skey, uint32_t* scnt, uint32_t
   for (int i = threadIdx.x; i < (1 << kSortBinBits); i += T) bins[i] = 0;
 }
 
-// One chunk item: keys [cb, cb + kChunkKeys) of a giant bucket are aggregated on chip.
+// One chunk item: keys [cb, cb + CH) of a giant bucket are aggregated on chip.
 // When their distinct keys fit half the table they are written back over the chunk's
 // own slots as (remainder, count) pairs -- remainders in slots [cb, cb + u), counts as
-// uint32 from slot cb + kChunkKeys / 2 on -- and chunk_u = u; otherwise the chunk keeps
+// uint32 from slot cb + CH / 2 on -- and chunk_u = u; otherwise the chunk keeps
 // its keys and chunk_u = kChunkRaw.  The bucket item reads the pairs in place of the
 // keys, so a heavy k-mer's copies are summed by many CTAs instead of one.  The table is
 // empty before and after.
@@ -1396,17 +1403,17 @@ template <typename KeyT, int T>
 __device__ __forceinline__ void aggregate_chunk(const BucketArgs& a, KeyT* keys_rw, unsigned long long cb,
                                                 uint32_t item, uint32_t beta, KeyT rmask, KeyT* skey,
                                                 uint32_t* scnt, uint32_t* s_flag, uint32_t* s_cnt) {
-  constexpr int H = BucketCfg<KeyT>::H;
+  constexpr int H = BucketCfg<KeyT>::H, CH = BucketCfg<KeyT>::CH;
   constexpr int PF = BucketCfg<KeyT>::PF;
   const KeyT EMPTY = ~(KeyT)0;
   const int tid = threadIdx.x, lane = tid & 31;
-  for (uint32_t i0 = 0; i0 < (uint32_t)kChunkKeys; i0 += PF * T) {
+  for (uint32_t i0 = 0; i0 < (uint32_t)CH; i0 += PF * T) {
     if (warp_flag(s_flag)) break;
     KeyT rr[PF];
 #pragma unroll
     for (int q = 0; q < PF; q++) {
       const uint32_t i = i0 + q * T + tid;
-      rr[q] = i < (uint32_t)kChunkKeys ? keys_rw[cb + i] & rmask : EMPTY;
+      rr[q] = i < (uint32_t)CH ? keys_rw[cb + i] & rmask : EMPTY;
     }
     uint32_t fresh = 0;
 #pragma unroll
@@ -1429,7 +1436,7 @@ __device__ __forceinline__ void aggregate_chunk(const BucketArgs& a, KeyT* keys_
     *s_flag = 0;
   }
   __syncthreads();
-  uint32_t* pc = reinterpret_cast<uint32_t*>(keys_rw + cb + kChunkKeys / 2);
+  uint32_t* pc = reinterpret_cast<uint32_t*>(keys_rw + cb + CH / 2);
   for (uint32_t i0 = 0; i0 < (uint32_t)H; i0 += T) {
     const uint32_t i = i0 + tid;
     const KeyT x = i < (uint32_t)H ? skey[i] : EMPTY;
@@ -1461,7 +1468,7 @@ __device__ __forceinline__ void aggregate_chunk(const BucketArgs& a, KeyT* keys_
 // entries it will read: the chunks' pairs (or keys, where a chunk stayed raw) and the
 // keys after the last chunk; `raws` tells whether any chunk stayed raw.  On expiry it sets
 // ERR_LOOKBACK and *s_fail.
-template <int T>
+template <int CH, int T>
 __device__ __forceinline__ uint32_t giant_entries(const BucketArgs& a, uint32_t beta, uint32_t n, uint32_t g0,
                                                uint32_t nch, uint32_t* s_warp, uint32_t* s_fail, bool& raws) {
   const int tid = threadIdx.x;
@@ -1483,12 +1490,12 @@ __device__ __forceinline__ uint32_t giant_entries(const BucketArgs& a, uint32_t 
   for (uint32_t j = tid; j < nch; j += T) {
     const uint32_t cu = __ldcg(&a.chunk_u[g0 + j]);
     raw |= cu == kChunkRaw;
-    part += cu == kChunkRaw ? (uint32_t)kChunkKeys : cu;
+    part += cu == kChunkRaw ? (uint32_t)CH : cu;
   }
   raws = __syncthreads_or(raw) != 0;
   uint32_t tot;
   block_exclusive_sum(part, s_warp, tot);
-  return tot + (n - nch * (uint32_t)kChunkKeys);
+  return tot + (n - nch * (uint32_t)CH);
 }
 
 // The remainder range [lo, hi) of part `part` of a giant bucket, by thread 0's view in *s_lo
@@ -1504,6 +1511,7 @@ __device__ __forceinline__ void giant_range(const BucketArgs& a, const KeyT* key
                                             KeyT* samp, KeyT* s_lo, KeyT* s_end) {
   static_assert(kSplitSamples % kGiantParts == 0, "quantiles are samples");
   constexpr uint32_t PER = kSplitSamples / kGiantParts;
+  constexpr int CH = BucketCfg<KeyT>::CH;
   const uint32_t tid = threadIdx.x;
   if (n_eff <= (uint32_t)BucketCfg<KeyT>::H / 2) {
     if (tid == 0) {
@@ -1516,9 +1524,9 @@ __device__ __forceinline__ void giant_range(const BucketArgs& a, const KeyT* key
   KeyT mine = 0;
   if (tid < (uint32_t)kSplitSamples) {
     const uint32_t j = (uint32_t)(((unsigned long long)tid * nch) / kSplitSamples);
-    const uint32_t len = min(__ldcg(&a.chunk_u[g0 + j]), (uint32_t)kChunkKeys);  // raw: all of them
+    const uint32_t len = min(__ldcg(&a.chunk_u[g0 + j]), (uint32_t)CH);  // raw: all of them
     const uint32_t e = len ? (tid * 2654435761u >> 8) % len : 0u;
-    mine = ldcg_key(keys_rw + ((unsigned long long)base + (unsigned long long)j * kChunkKeys + e)) & rmask;
+    mine = ldcg_key(keys_rw + ((unsigned long long)base + (unsigned long long)j * CH + e)) & rmask;
     samp[tid] = mine;
   }
   if (tid == 0) {
@@ -1551,10 +1559,11 @@ __device__ __forceinline__ void giant_pass(const BucketArgs& a, const KeyT* keys
                                            uint32_t* bins, int dsh, uint32_t bmask, uint32_t* s_ovf,
                                            uint32_t* s_unew) {
   constexpr int GP = 4;  // loads in flight
+  constexpr int CH = BucketCfg<KeyT>::CH;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // entries [i, len) of the chunk at cb, `step` apart, GP at a time
   auto read = [&](unsigned long long cb, uint32_t i0, uint32_t len, uint32_t step, bool pairs) {
-    const uint32_t* pc = reinterpret_cast<const uint32_t*>(keys_rw + cb + kChunkKeys / 2);
+    const uint32_t* pc = reinterpret_cast<const uint32_t*>(keys_rw + cb + CH / 2);
     KeyT r[GP];
     uint32_t c[GP];
 #pragma unroll
@@ -1587,15 +1596,15 @@ __device__ __forceinline__ void giant_pass(const BucketArgs& a, const KeyT* keys
     if (len == kChunkRaw) continue;
     for (uint32_t i0 = 0; i0 < len; i0 += 32 * GP) {
       if (warp_flag(s_ovf)) break;
-      read((unsigned long long)base + (unsigned long long)j * kChunkKeys, i0 + lane, len, 32, true);
+      read((unsigned long long)base + (unsigned long long)j * CH, i0 + lane, len, 32, true);
     }
   }
   for (uint32_t j = raws ? 0 : nch; j <= nch; j++) {
     if (j < nch && __ldcg(&a.chunk_u[g0 + j]) != kChunkRaw) continue;
-    const uint32_t len = j < nch ? (uint32_t)kChunkKeys : n - nch * (uint32_t)kChunkKeys;
+    const uint32_t len = j < nch ? (uint32_t)CH : n - nch * (uint32_t)CH;
     for (uint32_t i0 = 0; i0 < len; i0 += GP * T) {
       if (warp_flag(s_ovf)) break;
-      read((unsigned long long)base + (unsigned long long)j * kChunkKeys, i0 + tid, len, T, false);
+      read((unsigned long long)base + (unsigned long long)j * CH, i0 + tid, len, T, false);
     }
   }
 }
@@ -1661,6 +1670,7 @@ template <typename KeyT, bool GIANT, int T>
 __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
   using SM = BucketSmem<KeyT>;
   constexpr int H = SM::H;
+  static_assert(H <= BucketCfg<KeyT>::CH, "a chunk's pairs: keys in its first half, counts in its second");
   constexpr int BINS = SM::BINS;
   constexpr int HALF = H / 2;
   constexpr int PF = BucketCfg<KeyT>::PF;
@@ -1768,7 +1778,7 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
       if (tid == 0) {
         const uint32_t gb = a.chunk_bucket[tk];
         s_nb[0] = gb;
-        s_nb[1] = a.bstart[gb] + (tk - a.gfirst[gb]) * (uint32_t)kChunkKeys;
+        s_nb[1] = a.bstart[gb] + (tk - a.gfirst[gb]) * (uint32_t)BucketCfg<KeyT>::CH;
       }
       __syncthreads();
       aggregate_chunk<KeyT, T>(a, keys_rw, s_nb[1], tk, s_nb[0], rmask, skey, scnt, &s_ovf, &s_unew);
@@ -1793,7 +1803,7 @@ __global__ void __launch_bounds__(T, 2) k_bucket_table(BucketArgs a) {
     bool failed = false, raws = false;
     if (GIANT) {
       __syncthreads();
-      if (part) n_eff = giant_entries<T>(a, beta, n, g0, nch, s_warp, &s_fail, raws);
+      if (part) n_eff = giant_entries<BucketCfg<KeyT>::CH, T>(a, beta, n, g0, nch, s_warp, &s_fail, raws);
       failed = s_fail != 0;  // a giant bucket whose chunks did not finish in time
       if (part && !failed) {
         giant_range<KeyT>(a, keys_rw, base, n_eff, g0, nch, item % kGiantParts, rmask, rtop,
@@ -3177,11 +3187,13 @@ cudaError_t launch_bucket_table(const BucketArgs& a, int wide, int grid, cudaStr
   return wide ? launch_bucket_t<u128>(a, grid, st) : launch_bucket_t<uint64_t>(a, grid, st);
 }
 
-cudaError_t launch_giant_chunks(const BucketArgs& a, uint32_t* gfirst, uint32_t* gcount, uint32_t* chunk_bucket,
-                                uint32_t* glist, cudaStream_t st) {
+int chunk_keys(int wide) { return wide ? BucketCfg<u128>::CH : BucketCfg<uint64_t>::CH; }
+
+cudaError_t launch_giant_chunks(const BucketArgs& a, int wide, uint32_t* gfirst, uint32_t* gcount,
+                                uint32_t* chunk_bucket, uint32_t* glist, cudaStream_t st) {
   const int B = 1 << a.bbits;
   pk::note_launch(), k_giant_chunks<<<(B + 255) / 256, 256, 0, st>>>(a.bstart, B, gfirst, gcount, chunk_bucket, a.gdone,
-                                                                    a.gpart, glist, a.bsmall, a.sc);
+                                                                    a.gpart, glist, a.bsmall, (uint32_t)chunk_keys(wide), a.sc);
   return cudaGetLastError();
 }
 
