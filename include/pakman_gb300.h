@@ -290,9 +290,10 @@ pk_status pk_copy_walk_contigs(pk_job* job, uint64_t* offsets, uint8_t* bases);
 pk_status pk_summary_get(pk_job* job, pk_summary* out);
 
 /* ---- bounded device waits -----------------------------------------------------------
- * Kernels that wait on other CTAs (the decoupled look-back of the kept-row filter and of
- * the macro-node kernel, a giant bucket waiting for its chunks) poll a bounded number of
- * times with a short sleep between polls, then set an error bit and return, so the call
+ * Kernels that wait on other CTAs (the decoupled look-back of the kept-row offsets and of
+ * the macro-node kernel, a giant bucket's parts waiting for its chunks and, while any part
+ * moves, for one another) poll a bounded number of times with a short sleep between polls,
+ * then set an error bit and return, so the call
  * fails with PK_ERR_DEVICE and the context stays usable.  spins = polls before a wait
  * gives up (0 = the default, about 1-2 s).  withhold_unit >= 0 makes that macro-node work
  * unit publish nothing, so the waits of the units after it run out: a fault injected on
